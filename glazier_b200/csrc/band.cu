@@ -190,7 +190,7 @@ __device__ __forceinline__ void band_price(const SweepLaunch &a, const BandPass 
     const int vol_old = base_old.x + dv, surf_old = base_old.y + ds;
     unpack_delta(prev_new, dv, ds);
     const int vol_new = base_new.x + dv, surf_new = base_new.y + ds;
-    delta = size_terms<UNIFORM>(a, old, nw, t_old, t_new, vol_old, vol_new, surf_old, surf_new, ds_old, ds_new, delta);
+    delta = size_terms<UNIFORM>(a, a.t, old, nw, t_old, t_new, vol_old, vol_new, surf_old, surf_new, ds_old, ds_new, delta);
     const float u = to_f32(draw(v.key_accept, target));
     if (!(delta <= 0.0f || u < metropolis_exp(__fmul_rn(-delta, a.beta)))) return;
     a.labels[target] = nw;

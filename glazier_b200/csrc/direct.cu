@@ -1,0 +1,348 @@
+// The direct sweep: a colour pass with no staging at all, the labels and
+// tallies read where they lie. It takes the lattices whose passes the window
+// rings of sweep.cu do not pay for: lean planes of at most 1024^2, lean
+// volumes, and models with every term on small lattices.
+//
+// What bounds it is latency. A pass is a chain of dependent reads (labels,
+// then the two cells' tallies and types, then for some copies moments,
+// fields or activity) and a copy's arithmetic, on too few targets to fill the
+// GPU, so the work is laid out to shorten that chain and to keep a warp's
+// lanes on the same part of it:
+//   - Everything a pass can do before the previous pass has finished comes
+//     before its programmatic wait: the tables into shared memory, each
+//     thread's target and its pick's draw (the clock of a replayed step is
+//     written a whole graph earlier).
+//   - A small pass prices each target in its own thread; in a plane the
+//     neighbour labels come with the target's own, so the chain is labels,
+//     tallies, commit. A larger one gathers the unlike targets, about a
+//     fifth, into a queue that whole warps price from its front.
+//   - Pricing has no branch on the common path, so its reads and sums overlap.
+//   - The tally rotation is shared out over the grid and taken by each
+//     block's last threads.
+// Measured per MCS (the step graph, back to back), against the pass that read
+// its launch from shared memory and its tables where they lie, and launched
+// plainly: lean planes of four types 27.2 -> 16.2 us at 256^2 and 30.6 -> 18.9
+// at 512^2; the two-field tissue (length, chemotaxis) 55.5 -> 31.1 us at
+// 256^2, 62.1 -> 35.1 at 512^2 and 114.9 -> 62.7 at 1024^2. A pass of the
+// 256^2 plane is about 4 us, of which 0.8 is the graph's kernel-to-kernel
+// time and the rest the chain.
+
+#include <atomic>
+#include <cstdlib>
+
+#include "direct.cuh"
+
+namespace glz {
+
+// The view of a pass: from the launch, or for a step replayed from a graph
+// from the engine's clock (the pass's number gives the tally slots, the step
+// its draws), as pass_launch (engine.cu) sets them on the host.
+struct DirectView {
+    PassView v;
+    TermView t;
+    int2 *vs_next_base;
+    long long *vs_clear;
+    long long *mom_next_base;
+    long long *mom_clear;
+};
+
+__device__ __forceinline__ DirectView direct_view(const SweepLaunch &a) {
+    DirectView d;
+    if (!a.clock) {
+        d.v = PassView{a.colour, a.key_pick, a.key_accept, a.vs_base, a.vs_prev, a.vs_cur};
+        d.t = TermView{a.mom_base, a.mom_prev, a.mom_cur, a.field_cur};
+        d.vs_next_base = a.vs_next_base;
+        d.vs_clear = a.vs_clear;
+        d.mom_next_base = a.mom_next_base;
+        d.mom_clear = a.mom_clear;
+        return d;
+    }
+    const EngineClock c = *a.clock;
+    const unsigned long long p = (unsigned long long)(c.pass + a.colour);
+    const int32_t step = (int32_t)c.step;
+    const int b = (int)(p % 2), n = 1 - b, cur = (int)(p % 3), next = cur == 2 ? 0 : cur + 1,
+              prev = cur == 0 ? 2 : cur - 1;
+    d.v = PassView{a.colour,
+                   stream_key(a.seed, step, a.colour, 0),
+                   stream_key(a.seed, step, a.colour, 1),
+                   a.tal.vs_base[b],
+                   a.tal.vs_delta[prev],
+                   reinterpret_cast<unsigned long long *>(a.tal.vs_delta[cur])};
+    d.t = TermView{a.tal.mom_base[b], a.tal.mom_delta[prev],
+                   reinterpret_cast<unsigned long long *>(a.tal.mom_delta[cur]), c.field_cur};
+    d.vs_next_base = a.tal.vs_base[n];
+    d.vs_clear = a.tal.vs_delta[next];
+    d.mom_next_base = a.tal.mom_base[n];
+    d.mom_clear = a.tal.mom_delta[next];
+    return d;
+}
+
+// This block's share of the tally rotation (engine.h): an equal run of the
+// labels, and of the moment words, from the block's last thread back.
+template <bool EXTRAS>
+__device__ __forceinline__ void rotate_share(const SweepLaunch &a, const DirectView &d) {
+    const int n = a.n_live ? *a.n_live : a.n_labels;
+    const int from = (int)(blockDim.x - 1u - threadIdx.x);
+    const int share = (n + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int first = (int)blockIdx.x * share, last = min(n, first + share);
+    for (int l = first + from; l < last; l += (int)blockDim.x) {
+        int dv, ds;
+        unpack_delta(d.v.vs_prev[l], dv, ds);
+        const int2 b = d.v.vs_base[l];
+        d.vs_next_base[l] = make_int2(b.x + dv, b.y + ds);
+        d.vs_clear[l] = 0;
+    }
+    if (EXTRAS && a.tracks) {
+        const long long words = (long long)last * a.g.nm;
+        for (long long k = (long long)first * a.g.nm + from; k < words; k += blockDim.x) {
+            d.mom_next_base[k] = d.t.base[k] + d.t.prev[k];
+            d.mom_clear[k] = 0;
+        }
+    }
+}
+
+// How a pass's targets are shared out (the launch's FORM).
+constexpr int kPlain = 0;  // one target per thread, priced where it lies
+constexpr int kWarp = 1;   // each warp queues the unlike of its 32 kWarpK targets
+constexpr int kBlock = 2;  // each block gathers the unlike of its targets into one queue
+
+// From a million targets a pass a warp's own queue needs no block barrier
+// and is the faster (0.37 against 0.51 ms per MCS at 256^3 for one target a
+// thread).
+constexpr int kWarpK = 4;
+// A block's targets per thread at most (per MCS at 1024^2: 37.3 us with two,
+// 52.0 with one).
+constexpr int kBlockK = 2;
+constexpr int kBlockThreads = 256;
+
+// Passes of the lean models are held to 64 registers, four blocks of 256 per
+// SM, so that a 2^18-target pass of two targets a thread is one wave (at
+// 128^3: 0.060 ms per MCS against 0.073 uncapped, 0.065 at 48 registers); the
+// every-term passes to 128, two blocks of 256 (uncapped they take up to 200,
+// one block: 48 against 70 us per MCS for the 512^2 tissue).
+template <bool EXTRAS>
+constexpr int kDirectMinBlocks = EXTRAS ? 2 : 4;
+
+template <int DIM, int NOFF, bool UNIFORM, int FORM, bool EXTRAS>
+__global__ void __launch_bounds__(kBlockThreads, kDirectMinBlocks<EXTRAS>)
+    direct_sweep_kernel(const __grid_constant__ SweepLaunch a) {
+    const int targets = (a.g.w / 2) * (a.g.h / 2) * (DIM == 3 ? a.g.d / 2 : 1);
+    __shared__ TypeSmem<EXTRAS> types;
+    const TypeTables T = UNIFORM && !EXTRAS ? a.t : load_types<EXTRAS>(a, types);
+    const DirectView d = direct_view(a);
+    const PassView &v = d.v;
+    const GlobalPass acc{a, v};
+    const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    if constexpr (FORM == kPlain) {
+        const int j = (int)(blockIdx.x * blockDim.x) + tid;
+        int x = 0, y = 0, z = 0, pick = 0;
+        if (j < targets) {
+            direct_site<DIM>(a, a.colour, j, x, y, z);
+            pick = pick_of<NOFF>(draw(v.key_pick, (uint32_t)((z * a.g.h + y) * a.g.w + x)));
+        }
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        if (!(UNIFORM && !EXTRAS)) __syncthreads();  // the tables are in place
+        if (j < targets) {
+            if constexpr (DIM == 2) {
+                // a plane's neighbour labels come with the target's own: one
+                // round trip, not two
+                NeighbourLabels<DIM, NOFF, GlobalPass> ln(a, acc, x, y, z);
+                ln.load();
+                const uint32_t old = acc.label(x, y, z), nw = ln.picked(pick);
+                if (old != nw)
+                    direct_copy<DIM, NOFF, UNIFORM, GlobalPass, NeighbourLabels<DIM, NOFF, GlobalPass>, EXTRAS>(
+                        a, T, acc, ln, v.key_accept, x, y, z, pick, old, nw, &d.t);
+            } else {
+                const uint32_t old = acc.label(x, y, z), nw = picked_label<DIM, NOFF>(a, acc, x, y, z, pick);
+                const NeighbourReads<DIM, NOFF, GlobalPass> ln(a, acc, x, y, z);
+                if (old != nw)
+                    direct_copy<DIM, NOFF, UNIFORM, GlobalPass, NeighbourReads<DIM, NOFF, GlobalPass>, EXTRAS>(
+                        a, T, acc, ln, v.key_accept, x, y, z, pick, old, nw, &d.t);
+            }
+        }
+        rotate_share<EXTRAS>(a, d);
+    } else if constexpr (FORM == kBlock) {
+        __shared__ int queue[kBlockThreads * kBlockK];
+        __shared__ uint8_t picks[kBlockThreads * kBlockK];
+        __shared__ uint2 pair[kBlockThreads * kBlockK];  // (old, new) labels of each queued copy
+        __shared__ int counts[kBlockThreads / 32];
+        const int nt = (int)blockDim.x;
+        // the block's targets: direct_span of them, at most nt kBlockK
+        const int first = (int)blockIdx.x * a.direct_span;
+        const int last = min(first + a.direct_span, targets);
+        int site[kBlockK], picked[kBlockK];
+        int tx[kBlockK], ty[kBlockK], tz[kBlockK];
+#pragma unroll
+        for (int k = 0; k < kBlockK; ++k) {
+            const int j = first + k * nt + tid;
+            site[k] = j < last ? j : -1;
+            picked[k] = 0;
+            tx[k] = ty[k] = tz[k] = 0;
+            if (j < last) {
+                direct_site<DIM>(a, a.colour, j, tx[k], ty[k], tz[k]);
+                picked[k] = pick_of<NOFF>(draw(v.key_pick, (uint32_t)((tz[k] * a.g.h + ty[k]) * a.g.w + tx[k])));
+            }
+        }
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        unsigned masks[kBlockK];
+        uint2 labels[kBlockK];
+        int mine = 0;
+#pragma unroll
+        for (int k = 0; k < kBlockK; ++k) {
+            labels[k] = make_uint2(0u, 0u);
+            if (site[k] >= 0)
+                labels[k] = make_uint2(acc.label(tx[k], ty[k], tz[k]),
+                                       picked_label<DIM, NOFF>(a, acc, tx[k], ty[k], tz[k], picked[k]));
+        }
+#pragma unroll
+        for (int k = 0; k < kBlockK; ++k) {
+            masks[k] = __ballot_sync(0xffffffffu, labels[k].x != labels[k].y);
+            mine += __popc(masks[k]);
+        }
+        if (lane == 0) counts[warp] = mine;
+        __syncthreads();
+        int at = 0, total = 0;
+        for (int w = 0; w < nt / 32; ++w) {
+            at += w < warp ? counts[w] : 0;
+            total += counts[w];
+        }
+#pragma unroll
+        for (int k = 0; k < kBlockK; ++k) {
+            if (masks[k] & (1u << lane)) {
+                const int e = at + __popc(masks[k] & below);
+                queue[e] = site[k];
+                picks[e] = (uint8_t)picked[k];
+                pair[e] = labels[k];
+            }
+            at += __popc(masks[k]);
+        }
+        __syncthreads();
+        for (int e = tid; e < total; e += nt) {
+            int x, y, z;
+            direct_site<DIM>(a, a.colour, queue[e], x, y, z);
+            const NeighbourReads<DIM, NOFF, GlobalPass> ln(a, acc, x, y, z);
+            direct_copy<DIM, NOFF, UNIFORM, GlobalPass, NeighbourReads<DIM, NOFF, GlobalPass>, EXTRAS>(
+                a, T, acc, ln, v.key_accept, x, y, z, picks[e], pair[e].x, pair[e].y, &d.t);
+        }
+        rotate_share<EXTRAS>(a, d);
+    } else {
+        __shared__ int queue[kBlockThreads / 32][32 * kWarpK];
+        __shared__ uint8_t picks[kBlockThreads / 32][32 * kWarpK];
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        if (!(UNIFORM && !EXTRAS)) __syncthreads();  // the tables are in place
+        const int first = (int)((blockIdx.x * (blockDim.x / 32) + warp) * 32 * kWarpK);
+        int total = 0;
+#pragma unroll
+        for (int k = 0; k < kWarpK; ++k) {
+            const int j = first + k * 32 + lane;
+            bool unlike = false;
+            int pick = 0;
+            if (j < targets) {
+                int x, y, z;
+                direct_site<DIM>(a, a.colour, j, x, y, z);
+                pick = pick_of<NOFF>(draw(v.key_pick, (uint32_t)((z * a.g.h + y) * a.g.w + x)));
+                unlike = acc.label(x, y, z) != picked_label<DIM, NOFF>(a, acc, x, y, z, pick);
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, unlike);
+            if (unlike) {
+                queue[warp][total + __popc(m & below)] = j;
+                picks[warp][total + __popc(m & below)] = (uint8_t)pick;
+            }
+            total += __popc(m);
+        }
+        __syncwarp();
+        for (int e = lane; e < total; e += 32) {
+            int x, y, z;
+            direct_site<DIM>(a, a.colour, queue[warp][e], x, y, z);
+            const int pick = picks[warp][e];
+            const NeighbourReads<DIM, NOFF, GlobalPass> ln(a, acc, x, y, z);
+            direct_copy<DIM, NOFF, UNIFORM, GlobalPass, NeighbourReads<DIM, NOFF, GlobalPass>, EXTRAS>(
+                a, T, acc, ln, v.key_accept, x, y, z, pick, acc.label(x, y, z),
+                picked_label<DIM, NOFF>(a, acc, x, y, z, pick), &d.t);
+        }
+        rotate_share<EXTRAS>(a, d);
+    }
+}
+
+int programmatic_launch() {
+    static const int on = [] {
+        const char *env = std::getenv("GLAZIER_SWEEP_PDL");
+        return env && env[0] == '0' ? 0 : 1;
+    }();
+    return on;
+}
+
+// The device's SM count, or 0 if it cannot be read: a device attribute only,
+// so a launch being captured into a graph may ask.
+static int sm_count() {
+    static std::atomic<int> sms_once{0};  // handles on other host threads may launch too
+    int sms = sms_once.load(std::memory_order_acquire);
+    if (!sms) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) {
+            cudaGetLastError();
+            return 0;
+        }
+        sms_once.store(sms, std::memory_order_release);
+    }
+    return sms;
+}
+
+template <int DIM, int NOFF, bool UNIFORM>
+cudaError_t launch_direct(const SweepLaunch &a, cudaStream_t stream) {
+    const int targets = (a.g.w / 2) * (a.g.h / 2) * (DIM == 3 ? a.g.d / 2 : 1);
+    const bool warp = a.compact == 1, block = a.compact == 2;
+    SweepLaunch b = a;
+    // Every-term blocks are half as wide: their 128 registers a thread leave
+    // room for two blocks of 256 an SM, and four of 128 fill it as well but
+    // wait for one another less (62.7 against 64.9 us per MCS at 1024^2).
+    const int threads = block && !a.lean ? kBlockThreads / 2 : kBlockThreads;
+    int per_block = threads * (warp ? kWarpK : (block ? kBlockK : 1));
+    int grid = (targets + per_block - 1) / per_block;
+    if (block) {
+        const int slots = sm_count() * kDirectMinBlocks<false>;
+        if (a.lean && slots > 0) {
+            // Spread the pass evenly over whole waves of resident blocks, so
+            // that no SM holds more of its targets than another (at 128^3 and
+            // 1024^2: 592 blocks of 443 targets instead of 512 of 512 on 148
+            // SMs).
+            const int spread = (grid + slots - 1) / slots * slots;
+            per_block = (targets + spread - 1) / spread;
+            grid = (targets + per_block - 1) / per_block;
+        }
+        b.direct_span = per_block;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = programmatic_launch();
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (!a.lean)  // every term: length, chemotaxis, connectivity, motility, drift, nematic, moments
+        return warp    ? cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kWarp, true>, b)
+               : block ? cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kBlock, true>, b)
+                       : cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kPlain, true>, b);
+    return warp    ? cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kWarp, false>, b)
+           : block ? cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kBlock, false>, b)
+                   : cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kPlain, false>, b);
+}
+
+template cudaError_t launch_direct<2, 4, true>(const SweepLaunch &, cudaStream_t);
+template cudaError_t launch_direct<2, 4, false>(const SweepLaunch &, cudaStream_t);
+template cudaError_t launch_direct<2, 8, true>(const SweepLaunch &, cudaStream_t);
+template cudaError_t launch_direct<2, 8, false>(const SweepLaunch &, cudaStream_t);
+template cudaError_t launch_direct<3, 6, true>(const SweepLaunch &, cudaStream_t);
+template cudaError_t launch_direct<3, 6, false>(const SweepLaunch &, cudaStream_t);
+template cudaError_t launch_direct<3, 18, true>(const SweepLaunch &, cudaStream_t);
+template cudaError_t launch_direct<3, 18, false>(const SweepLaunch &, cudaStream_t);
+template cudaError_t launch_direct<3, 26, true>(const SweepLaunch &, cudaStream_t);
+template cudaError_t launch_direct<3, 26, false>(const SweepLaunch &, cudaStream_t);
+
+}  // namespace glz

@@ -114,15 +114,14 @@ struct glz_gpu {
     float *nematic = nullptr;  // 2 per site, with the nematic term
     float *activity = nullptr;  // sites, with motility
     uint2 *pending = nullptr;   // a motility pass's accepted copies
-    int *pending_count = nullptr;
+    int *pending_count = nullptr;  // by the pass's parity
     int substeps[glz::kMaxSpecies] = {};
     float fd[glz::kMaxSpecies] = {}, fdecay[glz::kMaxSpecies] = {};
 
     // per-type tables
-    float *contact = nullptr, *tv = nullptr, *lv = nullptr, *ts = nullptr, *ls = nullptr;
-    float *chemo = nullptr, *sec = nullptr, *upt = nullptr, *ext = nullptr, *maxact = nullptr, *lamact = nullptr;
-    double *tl = nullptr, *ll = nullptr, *divv = nullptr, *death = nullptr, *lnem = nullptr;
-    uint8_t *connected = nullptr;
+    unsigned char *types = nullptr;  // the tables a sweep reads, laid out by TypeLayout
+    float *sec = nullptr, *upt = nullptr;
+    double *divv = nullptr, *death = nullptr;
 
     // state
     uint32_t *labels = nullptr;
@@ -192,21 +191,24 @@ struct glz_gpu {
 
     glz::TypeTables tables() const {
         glz::TypeTables tt{};
-        tt.contact = contact;
-        tt.target_volume = tv;
-        tt.lambda_volume = lv;
-        tt.target_surface = ts;
-        tt.lambda_surface = ls;
-        tt.target_length = tl;
-        tt.lambda_length = ll;
+        const glz::TypeLayout L(n_types, n_species);
+        const auto f32 = [&](int at) { return reinterpret_cast<const float *>(types + at); };
+        const auto f64 = [&](int at) { return reinterpret_cast<const double *>(types + at); };
+        tt.contact = f32(L.contact);
+        tt.target_volume = f32(L.target_volume);
+        tt.lambda_volume = f32(L.lambda_volume);
+        tt.target_surface = f32(L.target_surface);
+        tt.lambda_surface = f32(L.lambda_surface);
+        tt.target_length = f64(L.target_length);
+        tt.lambda_length = f64(L.lambda_length);
         tt.division_volume = divv;
         tt.death_rate = death;
-        tt.connected = connected;
-        tt.chemotaxis = chemo;
-        tt.external = ext;
-        tt.max_activity = maxact;
-        tt.lambda_activity = lamact;
-        tt.lambda_nematic = lnem;
+        tt.connected = types + L.connected;
+        tt.chemotaxis = f32(L.chemotaxis);
+        tt.external = f32(L.external);
+        tt.max_activity = f32(L.max_activity);
+        tt.lambda_activity = f32(L.lambda_activity);
+        tt.lambda_nematic = f64(L.lambda_nematic);
         tt.secretion = sec;
         tt.uptake = upt;
         return tt;
@@ -441,8 +443,11 @@ glz::SweepLaunch pass_launch(glz_gpu *h, int colour) {
     a.nematic = h->nematic;
     a.activity = h->activity;
     a.pending = h->pending;
-    a.pending_count = h->pending_count;
-    for (int s = 0; s < h->n_species; ++s) a.fields[s] = h->field_ptr(s, h->field_cur[s]);
+    // two counts, by the pass's parity (the colour's, since a step has an even number of passes)
+    a.pending_count = h->pending_count ? h->pending_count + (colour & 1) : nullptr;
+    a.pending_clear = h->pending_count ? h->pending_count + ((colour & 1) ^ 1) : nullptr;
+    a.field_buf = h->field_buf;
+    for (int s = 0; s < h->n_species; ++s) a.field_cur |= (unsigned)(h->field_cur[s] & 1) << s;
     a.use_tma = h->use_tma;
     a.lean = h->lean;
     a.direct = h->direct;
@@ -656,7 +661,6 @@ int queue_clocked_step(glz_gpu *h) {
         a.clock = h->clock;
         a.seed = h->seed;
         a.tal = h->t;
-        a.field_buf = h->field_buf;
         CU(glz::launch_sweep(a, h->stream));
         if (h->has_motility) CU(glz::launch_apply_copies(a, h->activity, h->stream));
     }
@@ -1041,20 +1045,7 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
         h->fd[s] = (float)(at(m->diffusion, s) / (double)h->substeps[s]);
         h->fdecay[s] = (float)(at(m->decay, s) / (double)h->substeps[s]);
     }
-    if (has_conn) {
-        int all[26][3];
-        int n = offsets_for(3, d, all);  // the full Moore / 26 ring (connectivity.rs:23-29)
-        g.ring_n = n;
-        std::memcpy(g.ring, all, sizeof all);
-        for (int a = 0; a < n; ++a) {
-            uint32_t mask = 0;
-            for (int b = 0; b < n; ++b)
-                if (std::abs(all[a][0] - all[b][0]) <= 1 && std::abs(all[a][1] - all[b][1]) <= 1 &&
-                    std::abs(all[a][2] - all[b][2]) <= 1)
-                    mask |= 1u << b;
-            g.adjacency[a] = mask;
-        }
-    }
+    if (has_conn) g.ring_n = g.dim == 3 ? 26 : 8;  // the full Moore ring (connectivity.rs:23-29)
 
     // GLAZIER_SWEEP_LEAN=0 keeps every model on the general sweep kernel.
     const char *lean_env = std::getenv("GLAZIER_SWEEP_LEAN");
@@ -1078,15 +1069,19 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
     // staging costs more than it saves.
     const long long direct_most_general = g.dim == 2 ? 1024LL * 1024LL : 128LL * 128LL * 128LL;
     h->direct = direct_mode == 1 || (direct_mode == -1 && sites <= (h->lean ? direct_most : direct_most_general));
-    // From 2^18 targets a pass the direct kernel gathers each block's unlike
-    // copies into one queue priced by whole warps, and from a million it
-    // queues each warp's (GLAZIER_SWEEP_COMPACT=0: neither, =1: the warp's,
-    // =2: the block's, at any size).
+    // From 2^18 targets a pass (with other terms, past 2^16) the direct kernel
+    // gathers each block's unlike copies into one queue priced by whole
+    // warps, and from a million it queues each warp's
+    // (GLAZIER_SWEEP_COMPACT=0: neither, =1: the warp's, =2: the block's, at
+    // any size). Per MCS of the two-field tissue, priced in place against
+    // gathered: 31.1 and 31.7 us at 256^2, 35.1 and 35.0 at 512^2, 51.6 and
+    // 36.6 at 640^2, 92.7 and 62.7 at 1024^2.
     const char *compact_env = std::getenv("GLAZIER_SWEEP_COMPACT");
     const int compact_mode = compact_env ? (compact_env[0] == '0' ? 0 : (compact_env[0] == '2' ? 2 : 1)) : -1;
     const long long targets = sites / g.ncol;
+    const long long gather_from = h->lean ? glz::kDirectGatherFrom : glz::kDirectGatherEveryFrom;
     h->compact = compact_mode >= 0 ? compact_mode
-                                   : (targets >= glz::kDirectCompactFrom ? 1 : (targets >= glz::kDirectGatherFrom ? 2 : 0));
+                                   : (targets >= glz::kDirectCompactFrom ? 1 : (targets >= gather_from ? 2 : 0));
     // With no fields, division or death there is nothing between colour
     // passes: a direct plane of at most 512^2 sites runs every MCS of a call
     // in one cooperative launch, which saves more launch time than its grid
@@ -1114,12 +1109,26 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
     h->host_ts = ts;
     h->host_ls = ls;
     int rc;
-    if ((rc = upload(h, &h->contact, contact)) || (rc = upload(h, &h->tv, tv)) || (rc = upload(h, &h->lv, lv)) ||
-        (rc = upload(h, &h->ts, ts)) || (rc = upload(h, &h->ls, ls)) || (rc = upload(h, &h->tl, tl)) ||
-        (rc = upload(h, &h->ll, ll)) || (rc = upload(h, &h->divv, divv)) || (rc = upload(h, &h->death, death)) ||
-        (rc = upload(h, &h->connected, conn)) || (rc = upload(h, &h->chemo, chemo)) || (rc = upload(h, &h->sec, sec)) ||
-        (rc = upload(h, &h->upt, upt)) || (rc = upload(h, &h->ext, ext)) || (rc = upload(h, &h->maxact, maxact)) ||
-        (rc = upload(h, &h->lamact, lamact)) || (rc = upload(h, &h->lnem, lnem)))
+    const glz::TypeLayout L(nt, ns);
+    std::vector<unsigned char> types(L.bytes, 0);
+    const auto place = [&](int at, const auto &table) {
+        if (!table.empty()) std::memcpy(types.data() + at, table.data(), table.size() * sizeof table[0]);
+    };
+    place(L.contact, contact);
+    place(L.target_volume, tv);
+    place(L.lambda_volume, lv);
+    place(L.target_surface, ts);
+    place(L.lambda_surface, ls);
+    place(L.target_length, tl);
+    place(L.lambda_length, ll);
+    place(L.lambda_nematic, lnem);
+    place(L.max_activity, maxact);
+    place(L.lambda_activity, lamact);
+    place(L.external, ext);
+    place(L.chemotaxis, chemo);
+    place(L.connected, conn);
+    if ((rc = upload(h, &h->types, types)) || (rc = upload(h, &h->divv, divv)) || (rc = upload(h, &h->death, death)) ||
+        (rc = upload(h, &h->sec, sec)) || (rc = upload(h, &h->upt, upt)))
         return bail(rc);
 
     if ((rc = dev_alloc(&h->labels, (size_t)sites))) return bail(rc);
@@ -1173,8 +1182,8 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
         if (cudaMemcpy(h->activity, act.data(), sites * sizeof(float), cudaMemcpyHostToDevice))
             return bail(fail(GLZ_DRIVER, "activity upload failed"));
         if ((rc = dev_alloc(&h->pending, (size_t)(sites / g.ncol + 1)))) return bail(rc);
-        if ((rc = dev_alloc(&h->pending_count, 1))) return bail(rc);
-        if (cudaMemset(h->pending_count, 0, sizeof(int))) return bail(fail(GLZ_DRIVER, "memset failed"));
+        if ((rc = dev_alloc(&h->pending_count, 2))) return bail(rc);
+        if (cudaMemset(h->pending_count, 0, 2 * sizeof(int))) return bail(fail(GLZ_DRIVER, "memset failed"));
     }
     if ((rc = dev_alloc(&h->error_flag, 1))) return bail(rc);
     if ((rc = dev_alloc(&h->clock, 1))) return bail(rc);
@@ -1420,10 +1429,8 @@ int glz_gpu_device_field(glz_gpu *h, int index, void **field) {
 void glz_gpu_destroy(glz_gpu *h) {
     if (!h) return;
     if (h->stream) cudaStreamSynchronize(h->stream);
-    cudaFree(h->contact); cudaFree(h->tv); cudaFree(h->lv); cudaFree(h->ts); cudaFree(h->ls);
-    cudaFree(h->chemo); cudaFree(h->sec); cudaFree(h->upt); cudaFree(h->ext); cudaFree(h->maxact); cudaFree(h->lamact);
-    cudaFree(h->activity); cudaFree(h->pending); cudaFree(h->pending_count); cudaFree(h->nematic); cudaFree(h->lnem);
-    cudaFree(h->tl); cudaFree(h->ll); cudaFree(h->divv); cudaFree(h->death); cudaFree(h->connected);
+    cudaFree(h->types); cudaFree(h->sec); cudaFree(h->upt); cudaFree(h->divv); cudaFree(h->death);
+    cudaFree(h->activity); cudaFree(h->pending); cudaFree(h->pending_count); cudaFree(h->nematic);
     cudaFree(h->labels); cudaFree(h->cell_type); cudaFree(h->field_buf); cudaFree(h->dose);
     cudaFree(h->error_flag); cudaFree(h->medium); cudaFree(h->barrier); cudaFree(h->counters);
     free_tallies(h->t);

@@ -20,9 +20,7 @@ struct Geometry {
     int w, h, d, dim, ncol, sites;
     int n_off;          // energy neighbourhood (lattice.rs:69-88)
     int off[26][3];
-    int ring_n;         // connectivity ring (connectivity.rs:23-29), 0 when off
-    int ring[26][3];
-    uint32_t adjacency[26];
+    int ring_n;         // positions of the connectivity veto's ring, 0 when off
     int nm;             // exact moment sums per cell: 5 in a plane, 9 in a volume
     // w, h and their halves (a colour's targets per row and rows per plane)
     // as multiply-shift dividers; set_dividers fills them from w and h
@@ -47,6 +45,25 @@ struct TypeTables {
     const float *max_activity, *lambda_activity;   // the motility (Act) term
     const double *lambda_nematic;
 };
+
+// The tables a sweep prices with sit in one allocation (an engine's, or a
+// replica's of the ensemble up to lambda_surface), in this order, so a block
+// copies them into shared memory as one run of words: byte offsets for
+// n types and ns species. The first `lean` bytes are all that contact, volume
+// and surface terms read.
+struct TypeLayout {
+    int contact, target_volume, lambda_volume, target_surface, lambda_surface, lean;
+    int target_length, lambda_length, lambda_nematic;
+    int max_activity, lambda_activity, external, chemotaxis, connected, bytes;
+    __host__ __device__ constexpr TypeLayout(int n, int ns)
+        : contact(0), target_volume(4 * n * n), lambda_volume(target_volume + 4 * n),
+          target_surface(lambda_volume + 4 * n), lambda_surface(target_surface + 4 * n), lean(lambda_surface + 4 * n),
+          target_length((lean + 7) / 8 * 8), lambda_length(target_length + 8 * n),
+          lambda_nematic(lambda_length + 8 * n), max_activity(lambda_nematic + 8 * n),
+          lambda_activity(max_activity + 4 * n), external(lambda_activity + 4 * n), chemotaxis(external + 12 * n),
+          connected(chemotaxis + 4 * n * ns), bytes((connected + n + 3) / 4 * 4) {}
+};
+constexpr int kSmemTypes = 16;  // tables of up to this many types are held in shared memory
 
 // The per-cell tallies a colour pass reads, in the rotation that gives every
 // pass a snapshot without an extra launch:
@@ -117,13 +134,13 @@ struct SweepLaunch {
     // for launch_apply_copies.
     const float *activity;
     uint2 *pending;
-    int *pending_count;
-    const float *fields[kMaxSpecies];
+    int *pending_count;  // this pass's, and the other pass parity's (cleared for the next pass)
+    int *pending_clear;
     int use_tma;
     int lean;                // take the lean kernel: no length, chemotaxis, connectivity or moment tracking
     int direct;              // a lean model small enough for the direct kernel (one thread per target)
     int compact;             // the direct kernel queues unlike copies before pricing them: 1 per warp, 2 per block
-    int direct_span;         // targets a block of the block-queued direct kernel takes (0: 256 a thread-row)
+    int direct_span;         // targets a block of the block-queued direct kernel takes
     int max_ctas;            // > 0 caps the persistent grid (each CTA then walks more tiles)
     const void *tensor_map;  // CUtensorMap in device-visible memory, or null
     int *error_flag;
@@ -133,7 +150,8 @@ struct SweepLaunch {
     const EngineClock *clock;
     uint64_t seed;
     Tallies tal;
-    float *field_buf;  // two buffers per species, species-major
+    float *field_buf;    // two buffers per species, species-major
+    unsigned field_cur;  // bit s: the buffer holding species s (a clocked launch reads the clock's)
 };
 
 cudaError_t launch_sweep(const SweepLaunch &a, cudaStream_t stream);
@@ -154,8 +172,10 @@ struct ResidentLaunch {
 // cudaErrorCooperativeLaunchTooLarge (and nothing launched) when the blocks
 // cannot all be resident at once.
 // Targets a pass from which the direct kernel queues a block's unlike copies
-// (kDirectGatherFrom) and from which a warp's (kDirectCompactFrom).
+// (kDirectGatherFrom; with terms past contact, volume and surface,
+// kDirectGatherEveryFrom) and from which a warp's (kDirectCompactFrom).
 constexpr int kDirectGatherFrom = 1 << 18;
+constexpr int kDirectGatherEveryFrom = (1 << 16) + 1;
 constexpr int kDirectCompactFrom = 1 << 20;
 
 cudaError_t launch_resident_sweep(const ResidentLaunch &r, cudaStream_t stream);
@@ -173,7 +193,7 @@ cudaError_t launch_band_sweep(const ResidentLaunch &r, cudaStream_t stream);
 bool band_sweep_fits(int w, int h);
 
 // Apply a motility pass's listed copies: the label, and the activity of a
-// type with a maximum (lib.rs:696-698); then clear the list.
+// type with a maximum (lib.rs:696-698); then clear the next pass's count.
 cudaError_t launch_apply_copies(const SweepLaunch &a, float *activity, cudaStream_t stream);
 
 // The activity's memory runs down by one each Monte Carlo step

@@ -8,6 +8,44 @@
 
 namespace glz {
 
+// Shared memory for the tables of up to kSmemTypes types. A launch's tables
+// are few bytes read by every copy, each behind the one before it (a type's
+// weight, then its target): read where they lie they cost a cold kernel a
+// chain of up to eight L2 round trips.
+template <bool EXTRAS>
+struct alignas(8) TypeSmem {
+    unsigned char bytes[EXTRAS ? TypeLayout(kSmemTypes, kMaxSpecies).bytes : TypeLayout(kSmemTypes, 0).lean];
+};
+
+// Copy the launch's tables in (all of the block's threads; the caller's next
+// block barrier publishes them) and give where to read them. Reads nothing a
+// pass writes, so it may come before a programmatic wait.
+template <bool EXTRAS>
+__device__ __forceinline__ TypeTables load_types(const SweepLaunch &a, TypeSmem<EXTRAS> &S) {
+    TypeTables t = a.t;
+    if (a.n_types > kSmemTypes) return t;
+    const TypeLayout L(a.n_types, a.n_species);
+    const uint32_t *src = reinterpret_cast<const uint32_t *>(a.t.contact);
+    uint32_t *dst = reinterpret_cast<uint32_t *>(S.bytes);
+    for (int i = threadIdx.x; i < (EXTRAS ? L.bytes : L.lean) / 4; i += blockDim.x) dst[i] = src[i];
+    t.contact = reinterpret_cast<const float *>(S.bytes + L.contact);
+    t.target_volume = reinterpret_cast<const float *>(S.bytes + L.target_volume);
+    t.lambda_volume = reinterpret_cast<const float *>(S.bytes + L.lambda_volume);
+    t.target_surface = reinterpret_cast<const float *>(S.bytes + L.target_surface);
+    t.lambda_surface = reinterpret_cast<const float *>(S.bytes + L.lambda_surface);
+    if (EXTRAS) {
+        t.target_length = reinterpret_cast<const double *>(S.bytes + L.target_length);
+        t.lambda_length = reinterpret_cast<const double *>(S.bytes + L.lambda_length);
+        t.lambda_nematic = reinterpret_cast<const double *>(S.bytes + L.lambda_nematic);
+        t.max_activity = reinterpret_cast<const float *>(S.bytes + L.max_activity);
+        t.lambda_activity = reinterpret_cast<const float *>(S.bytes + L.lambda_activity);
+        t.external = reinterpret_cast<const float *>(S.bytes + L.external);
+        t.chemotaxis = reinterpret_cast<const float *>(S.bytes + L.chemotaxis);
+        t.connected = S.bytes + L.connected;
+    }
+    return t;
+}
+
 __device__ __forceinline__ uint32_t smem_addr(const void *p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
@@ -19,39 +57,24 @@ __device__ __forceinline__ uint32_t smem_addr(const void *p) {
 //   volume:  lambda ((v -/+ 1 - V_t)^2 - (v - V_t)^2) = lambda (1 -/+ 2 (v - V_t))
 //   surface: lambda ((s + ds - S_t)^2 - (s - S_t)^2) = lambda ds (2 (s - S_t) + ds)
 template <bool UNIFORM>
-__device__ __forceinline__ float size_terms(const SweepLaunch &a, uint32_t old, uint32_t nw, int t_old, int t_new,
+__device__ __forceinline__ float size_terms(const SweepLaunch &a, const TypeTables &t, uint32_t old, uint32_t nw, int t_old, int t_new,
                                             int vol_old, int vol_new, int surf_old, int surf_new, int ds_old,
                                             int ds_new, float delta) {
-    if (old != 0) {
-        const float lam = UNIFORM ? a.u_lambda_volume : a.t.lambda_volume[t_old];
-        if (lam != 0.0f) {
-            const float e = __fsub_rn((float)vol_old, UNIFORM ? a.u_target_volume : a.t.target_volume[t_old]);
-            delta = __fadd_rn(delta, __fmul_rn(lam, __fsub_rn(1.0f, __fmul_rn(2.0f, e))));
-        }
-    }
-    if (nw != 0) {
-        const float lam = UNIFORM ? a.u_lambda_volume : a.t.lambda_volume[t_new];
-        if (lam != 0.0f) {
-            const float e = __fsub_rn((float)vol_new, UNIFORM ? a.u_target_volume : a.t.target_volume[t_new]);
-            delta = __fadd_rn(delta, __fmul_rn(lam, __fadd_rn(__fmul_rn(2.0f, e), 1.0f)));
-        }
-    }
-    if (old != 0) {
-        const float lam = UNIFORM ? a.u_lambda_surface : a.t.lambda_surface[t_old];
-        if (lam != 0.0f) {
-            const float e = __fsub_rn((float)surf_old, UNIFORM ? a.u_target_surface : a.t.target_surface[t_old]);
-            const float d = (float)ds_old;
-            delta = __fadd_rn(delta, __fmul_rn(lam, __fmul_rn(d, __fadd_rn(__fmul_rn(2.0f, e), d))));
-        }
-    }
-    if (nw != 0) {
-        const float lam = UNIFORM ? a.u_lambda_surface : a.t.lambda_surface[t_new];
-        if (lam != 0.0f) {
-            const float e = __fsub_rn((float)surf_new, UNIFORM ? a.u_target_surface : a.t.target_surface[t_new]);
-            const float d = (float)ds_new;
-            delta = __fadd_rn(delta, __fmul_rn(lam, __fmul_rn(d, __fadd_rn(__fmul_rn(2.0f, e), d))));
-        }
-    }
+    // No branch: the medium, and a type whose weight is zero, add a zero,
+    // which leaves the sum's bits alone.
+    const float lv_old = old != 0 ? (UNIFORM ? a.u_lambda_volume : t.lambda_volume[t_old]) : 0.0f;
+    const float lv_new = nw != 0 ? (UNIFORM ? a.u_lambda_volume : t.lambda_volume[t_new]) : 0.0f;
+    const float ls_old = old != 0 ? (UNIFORM ? a.u_lambda_surface : t.lambda_surface[t_old]) : 0.0f;
+    const float ls_new = nw != 0 ? (UNIFORM ? a.u_lambda_surface : t.lambda_surface[t_new]) : 0.0f;
+    const float ev_old = __fsub_rn((float)vol_old, UNIFORM ? a.u_target_volume : t.target_volume[t_old]);
+    const float ev_new = __fsub_rn((float)vol_new, UNIFORM ? a.u_target_volume : t.target_volume[t_new]);
+    const float es_old = __fsub_rn((float)surf_old, UNIFORM ? a.u_target_surface : t.target_surface[t_old]);
+    const float es_new = __fsub_rn((float)surf_new, UNIFORM ? a.u_target_surface : t.target_surface[t_new]);
+    const float d_old = (float)ds_old, d_new = (float)ds_new;
+    delta = __fadd_rn(delta, __fmul_rn(lv_old, __fsub_rn(1.0f, __fmul_rn(2.0f, ev_old))));
+    delta = __fadd_rn(delta, __fmul_rn(lv_new, __fadd_rn(__fmul_rn(2.0f, ev_new), 1.0f)));
+    delta = __fadd_rn(delta, __fmul_rn(ls_old, __fmul_rn(d_old, __fadd_rn(__fmul_rn(2.0f, es_old), d_old))));
+    delta = __fadd_rn(delta, __fmul_rn(ls_new, __fmul_rn(d_new, __fadd_rn(__fmul_rn(2.0f, es_new), d_new))));
     return delta;
 }
 

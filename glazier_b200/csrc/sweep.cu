@@ -31,9 +31,11 @@
 #include <cstdlib>
 
 #include "device.cuh"
+#include "direct.cuh"
 #include "engine.h"
 #include "neighbours.cuh"
 #include "pricing.cuh"
+#include "terms.cuh"
 
 namespace glz {
 
@@ -75,7 +77,6 @@ __host__ __device__ constexpr int window_offset(int k) {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-constexpr int kSmemTypes = 16;  // contact tables up to 16 types live in shared memory
 constexpr long long kWaitLimit = 1LL << 24;
 
 template <int DIM>
@@ -93,127 +94,6 @@ struct SweepSmem {
     int wring[26];
     alignas(8) unsigned long long mbar[2];
 };
-
-// The dominant eigenvalue of a symmetric 3x3 by twenty rounds of power
-// iteration and a Rayleigh quotient, as the serial engine takes it
-// (moments.rs:165-186).
-__device__ double power_lambda(const double c[3][3]) {
-    double v0 = 1.0, v1 = 0.7, v2 = 0.3;
-    for (int round = 0; round < 20; ++round) {
-        double w0 = c[0][0] * v0 + c[0][1] * v1 + c[0][2] * v2;
-        double w1 = c[1][0] * v0 + c[1][1] * v1 + c[1][2] * v2;
-        double w2 = c[2][0] * v0 + c[2][1] * v1 + c[2][2] * v2;
-        double norm = sqrt(w0 * w0 + w1 * w1 + w2 * w2);
-        if (norm < 1e-15) return 0.0;
-        v0 = w0 / norm;
-        v1 = w1 / norm;
-        v2 = w2 / norm;
-    }
-    double w0 = c[0][0] * v0 + c[0][1] * v1 + c[0][2] * v2;
-    double w1 = c[1][0] * v0 + c[1][1] * v1 + c[1][2] * v2;
-    double w2 = c[2][0] * v0 + c[2][1] * v1 + c[2][2] * v2;
-    double lambda = v0 * w0 + v1 * w1 + v2 * w2;
-    return lambda > 0.0 ? lambda : 0.0;
-}
-
-// 4 sqrt(lambda_max) of a cell's covariance from its n sites and exact sums
-// (moments.rs:150-155); a plane takes the 2x2 closed form.
-template <int DIM>
-__device__ double axis_length(long long n, const long long *m) {
-    if (n < 2) return 0.0;
-    double dn = (double)n;
-    if (DIM == 2) {
-        double mx = (double)m[0] / dn, my = (double)m[1] / dn;
-        double cxx = (double)m[2] / dn - mx * mx;
-        double cyy = (double)m[3] / dn - my * my;
-        double cxy = (double)m[4] / dn - mx * my;
-        double half = 0.5 * (cxx + cyy), diff = 0.5 * (cxx - cyy);
-        double lambda = half + sqrt(diff * diff + cxy * cxy);
-        return 4.0 * sqrt(lambda > 0.0 ? lambda : 0.0);
-    } else {
-        double mx = (double)m[0] / dn, my = (double)m[1] / dn, mz = (double)m[2] / dn;
-        double c[3][3];
-        c[0][0] = (double)m[3] / dn - mx * mx;
-        c[1][1] = (double)m[4] / dn - my * my;
-        c[2][2] = (double)m[5] / dn - mz * mz;
-        c[0][1] = c[1][0] = (double)m[6] / dn - mx * my;
-        c[0][2] = c[2][0] = (double)m[7] / dn - mx * mz;
-        c[1][2] = c[2][1] = (double)m[8] / dn - my * mz;
-        return 4.0 * sqrt(power_lambda(c));
-    }
-}
-
-template <int DIM>
-__device__ __forceinline__ void site_terms(int ux, int uy, int uz, long long *t) {
-    if (DIM == 2) {
-        t[0] = ux; t[1] = uy; t[2] = (long long)ux * ux; t[3] = (long long)uy * uy; t[4] = (long long)ux * uy;
-    } else {
-        t[0] = ux; t[1] = uy; t[2] = uz;
-        t[3] = (long long)ux * ux; t[4] = (long long)uy * uy; t[5] = (long long)uz * uz;
-        t[6] = (long long)ux * uy; t[7] = (long long)ux * uz; t[8] = (long long)uy * uz;
-    }
-}
-
-// Change in a cell's length energy (cpu.rs:291-305) when the site with sum
-// terms `terms` leaves (sign -1) or joins (+1) it, from the pass snapshot.
-template <int DIM>
-__device__ __noinline__ double length_delta(const SweepLaunch &a, int type, int label, long long n,
-                                            const long long *terms, int sign) {
-    constexpr int NM = DIM == 2 ? 5 : 9;
-    const size_t at = (size_t)label * a.g.nm;  // the moment words of a cell: NM, then the nematic sums
-    long long m[NM], after[NM];
-#pragma unroll
-    for (int k = 0; k < NM; ++k) {
-        m[k] = a.mom_base[at + k] + a.mom_prev[at + k];
-        after[k] = m[k] + sign * terms[k];
-    }
-    double tl = a.t.target_length[type];
-    double before = axis_length<DIM>(n, m) - tl;
-    double now = axis_length<DIM>(n + sign, after) - tl;
-    return a.t.lambda_length[type] * (now * now - before * before);
-}
-
-// Change in a cell's nematic energy (cpu.rs:315-332, lib.rs:603-637) when the
-// site with sum terms `terms` (its moment terms, then its field components in
-// fixed point) leaves (sign -1) or joins (+1) it: -lambda (f' . a' - f . a),
-// f the cell's field sum and a its anisotropy, from the pass snapshot.
-template <int DIM>
-__device__ __noinline__ double nematic_delta(const SweepLaunch &a, int type, int label, long long n,
-                                             const long long *terms, int sign) {
-    constexpr int NM = DIM == 2 ? 5 : 9;
-    const size_t at = (size_t)label * a.g.nm;
-    long long m[NM + 2], after[NM + 2];
-#pragma unroll
-    for (int k = 0; k < NM + 2; ++k) {
-        m[k] = a.mom_base[at + k] + a.mom_prev[at + k];
-        after[k] = m[k] + sign * terms[k];
-    }
-    double a0, a1, b0, b1;
-    anisotropy<DIM>(n, m, a0, a1);
-    anisotropy<DIM>(n + sign, after, b0, b1);
-    const double scale = 1.0 / 4294967296.0;
-    const double before = (double)m[NM] * scale * a0 + (double)m[NM + 1] * scale * a1;
-    const double now = (double)after[NM] * scale * b0 + (double)after[NM + 1] * scale * b1;
-    return -a.t.lambda_nematic[type] * (now - before);
-}
-
-// lib.rs:371-389: whether the ring positions in `present` are one piece.
-__device__ __forceinline__ bool one_piece(uint32_t present, const uint32_t *adjacency) {
-    if (present == 0u || (present & (present - 1u)) == 0u) return true;
-    uint32_t reached = present & (~present + 1u);
-    for (int round = 0; round < 26; ++round) {
-        uint32_t grown = reached, rest = reached;
-        while (rest) {
-            int k = __ffs(rest) - 1;
-            grown |= adjacency[k];
-            rest &= rest - 1u;
-        }
-        grown &= present;
-        if (grown == reached) break;
-        reached = grown;
-    }
-    return reached == present;
-}
 
 // Position of target j of a tile: local coordinates in the tile.
 template <int DIM>
@@ -240,134 +120,27 @@ __device__ __noinline__ bool keeps_other_colour(const SweepLaunch &a, uint32_t o
 }
 
 // The connectivity veto (lib.rs:511-521): the ring positions of `old` around
-// the target must be one piece.
-__device__ __noinline__ bool ring_one_piece(const SweepLaunch &a, const int *wring, const uint32_t *win, int wc,
-                                            uint32_t old) {
+// the target must be one piece. `wring` holds the ring's window offsets.
+template <int DIM>
+__device__ __noinline__ bool ring_one_piece(const int *wring, const uint32_t *win, int wc, uint32_t old) {
     uint32_t present = 0;
-    for (int k = 0; k < a.g.ring_n; ++k)
-        if (win[wc + wring[k]] == old) present |= 1u << k;
-    return one_piece(present, a.g.adjacency);
-}
-
-// The moment-sum terms of the target site in a cell's own frame.
-template <int DIM>
-__device__ __forceinline__ void terms_of(const SweepLaunch &a, uint32_t label, int x, int y, int z, long long *t) {
-    const int *an = &a.anchor[(size_t)label * 4];
-    site_terms<DIM>(fold_int(x - an[0], a.g.w), fold_int(y - an[1], a.g.h), fold_int(z - an[2], a.g.d), t);
-}
-
-// The geometric mean of the activity over the sites of `label` around `site`
-// (x, y, z), the site itself included; zero as soon as one of them has none
-// left (lib.rs:391-424, motility.rs:58-79). Labels and activity are the
-// pass's starting values: a pass with motility defers its writes.
-template <int DIM>
-__device__ __noinline__ float activity_mean(const SweepLaunch &a, uint32_t site, int x, int y, int z,
-                                            uint32_t label) {
-    const float here = a.activity[site];
-    if (!(here > 0.0f)) return 0.0f;
-    float log_sum = motility_log(here), count = 1.0f;
-    const int W = a.g.w, H = a.g.h, D = a.g.d;
-    for (int k = 0; k < a.g.n_off; ++k) {
-        const uint32_t n = (uint32_t)(((size_t)wrap(z + a.g.off[k][2], D) * H + wrap(y + a.g.off[k][1], H)) * W +
-                                      wrap(x + a.g.off[k][0], W));
-        if (n == site || a.labels[n] != label) continue;
-        const float v = a.activity[n];
-        if (!(v > 0.0f)) return 0.0f;
-        log_sum = __fadd_rn(log_sum, motility_log(v));
-        count = __fadd_rn(count, 1.0f);
-    }
-    return metropolis_exp(__fdiv_rn(log_sum, count));
-}
-
-// The length, chemotaxis, motility and drift terms of a copy (cpu.rs:291-305,
-// 341-395).
-template <int DIM>
-__device__ __noinline__ float extra_terms(const SweepLaunch &a, uint32_t old, uint32_t nw, int t_old, int t_new,
-                                          int vol_old, int vol_new, int x, int y, int z, int pick, uint32_t target,
-                                          float delta) {
-    constexpr int NM = DIM == 2 ? 5 : 9;
-    const int W = a.g.w, H = a.g.h, D = a.g.d;
-    // the length and nematic terms, leaving cell first (lib.rs:578-639)
-    if (a.has_length || a.has_nematic) {
-        long long terms[NM + 2];
-        if (a.has_nematic) {
-            terms[NM] = nematic_fixed(a.nematic[2 * (size_t)target]);
-            terms[NM + 1] = nematic_fixed(a.nematic[2 * (size_t)target + 1]);
-        }
-        const bool len_old = a.has_length && a.t.lambda_length[t_old] != 0.0;
-        const bool nem_old = a.has_nematic && a.t.lambda_nematic[t_old] != 0.0;
-        if (old != 0 && (len_old || nem_old)) {
-            terms_of<DIM>(a, old, x, y, z, terms);
-            if (len_old) delta = __fadd_rn(delta, (float)length_delta<DIM>(a, t_old, old, vol_old, terms, -1));
-            if (nem_old) delta = __fadd_rn(delta, (float)nematic_delta<DIM>(a, t_old, old, vol_old, terms, -1));
-        }
-        const bool len_new = a.has_length && a.t.lambda_length[t_new] != 0.0;
-        const bool nem_new = a.has_nematic && a.t.lambda_nematic[t_new] != 0.0;
-        if (nw != 0 && (len_new || nem_new)) {
-            terms_of<DIM>(a, nw, x, y, z, terms);
-            if (len_new) delta = __fadd_rn(delta, (float)length_delta<DIM>(a, t_new, nw, vol_new, terms, 1));
-            if (nem_new) delta = __fadd_rn(delta, (float)nematic_delta<DIM>(a, t_new, nw, vol_new, terms, 1));
-        }
-    }
-    const int ox = a.g.off[pick][0], oy = a.g.off[pick][1], oz = a.g.off[pick][2];
-    const int sx = wrap(x + ox, W), sy = wrap(y + oy, H), sz = wrap(z + oz, D);
-    if (a.has_chemotaxis && nw != 0) {
-        const uint32_t source = (uint32_t)(((size_t)sz * H + sy) * W + sx);
-        for (int s = 0; s < a.n_species; ++s) {
-            const float lam = a.t.chemotaxis[t_new * a.n_species + s];
-            if (lam == 0.0f) continue;
-            const float *f = a.fields[s];
-            delta = __fsub_rn(delta, __fmul_rn(lam, __fsub_rn(f[target], f[source])));
-        }
-    }
-    // Motility (cpu.rs:346-352, lib.rs:656-663): the cell's memory pulls it
-    // where it has been.
-    if (a.has_motility && nw != 0) {
-        const float lam = a.t.lambda_activity[t_new], top = a.t.max_activity[t_new];
-        if (lam != 0.0f && top > 0.0f) {
-            const uint32_t source = (uint32_t)(((size_t)sz * H + sy) * W + sx);
-            const float into = activity_mean<DIM>(a, source, sx, sy, sz, nw);
-            const float out_of = activity_mean<DIM>(a, target, x, y, z, old);
-            delta = __fsub_rn(delta, __fmul_rn(__fdiv_rn(lam, top), __fsub_rn(into, out_of)));
-        }
-    }
-    // The drift (cpu.rs:360-369, lib.rs:664-673): work e . (target - source),
-    // the step folded onto the lattice.
-    if (a.has_external && nw != 0) {
-        const float ex = a.t.external[3 * t_new], ey = a.t.external[3 * t_new + 1], ez = a.t.external[3 * t_new + 2];
-        if (ex != 0.0f || ey != 0.0f || ez != 0.0f) {
-            const float fx = (float)fold_int(x - sx, W), fy = (float)fold_int(y - sy, H), fz = (float)fold_int(z - sz, D);
-            delta = __fsub_rn(delta, __fadd_rn(__fadd_rn(__fmul_rn(ex, fx), __fmul_rn(ey, fy)), __fmul_rn(ez, fz)));
-        }
-    }
-    return delta;
-}
-
-// The moment sums follow an accepted copy: the site leaves `old` and joins `nw`.
-template <int DIM>
-__device__ __noinline__ void commit_moments(const SweepLaunch &a, uint32_t old, uint32_t nw, int x, int y, int z) {
-    constexpr int NM = DIM == 2 ? 5 : 9;
-    const int nm = a.g.nm;
-    long long terms[NM], q[2] = {0, 0};
-    if (a.has_nematic) {
-        const size_t site = ((size_t)z * a.g.h + y) * a.g.w + x;
-        q[0] = nematic_fixed(a.nematic[2 * site]);
-        q[1] = nematic_fixed(a.nematic[2 * site + 1]);
-    }
-    if (old != 0) {
-        terms_of<DIM>(a, old, x, y, z, terms);
 #pragma unroll
-        for (int k = 0; k < NM; ++k) atomicAdd(&a.mom_cur[(size_t)old * nm + k], (unsigned long long)(-terms[k]));
-        if (a.has_nematic)
-            for (int k = 0; k < 2; ++k) atomicAdd(&a.mom_cur[(size_t)old * nm + NM + k], (unsigned long long)(-q[k]));
-    }
-    if (nw != 0) {
-        terms_of<DIM>(a, nw, x, y, z, terms);
-#pragma unroll
-        for (int k = 0; k < NM; ++k) atomicAdd(&a.mom_cur[(size_t)nw * nm + k], (unsigned long long)terms[k]);
-        if (a.has_nematic)
-            for (int k = 0; k < 2; ++k) atomicAdd(&a.mom_cur[(size_t)nw * nm + NM + k], (unsigned long long)q[k]);
-    }
+    for (int k = 0; k < kRing<DIM>; ++k)
+        if (win[wc + wring[k]] == old) present |= 1u << cube_bit<DIM, kRing<DIM>>(k);
+    return one_piece<DIM>(present);
+}
+
+template <int DIM, int NOFF>
+__device__ __noinline__ float tile_extra_terms(const SweepLaunch &a, uint32_t old, uint32_t nw, int t_old, int t_new,
+                                               int vol_old, int vol_new, int x, int y, int z, int pick,
+                                               uint32_t target, float delta) {
+    const TermView v{a.mom_base, a.mom_prev, a.mom_cur, a.field_cur};
+    return extra_terms<DIM, NOFF>(a, a.t, v, old, nw, t_old, t_new, vol_old, vol_new, x, y, z, pick, target, delta);
+}
+
+template <int DIM>
+__device__ __noinline__ void tile_commit_moments(const SweepLaunch &a, uint32_t old, uint32_t nw, int x, int y, int z) {
+    commit_moments<DIM>(a, a.mom_cur, old, nw, anchor_of(a, old), anchor_of(a, nw), x, y, z);
 }
 
 // Price one copy attempt whose neighbour pick is known to carry another label
@@ -448,7 +221,7 @@ __device__ __forceinline__ void price_and_commit(const SweepLaunch &a, const int
         // A like neighbour is a site of another colour, since every neighbour
         // of a target is; only a target with none needs the per-colour count.
         if (like_old == 0 && !keeps_other_colour(a, old)) return;
-        if (EXTRAS && a.g.ring_n > 0 && a.t.connected[t_old] && !ring_one_piece(a, wring, win, wc, old)) return;
+        if (EXTRAS && a.g.ring_n > 0 && a.t.connected[t_old] && !ring_one_piece<DIM>(wring, win, wc, old)) return;
     }
     const int ds_old = 2 * like_old - NOFF;
     const int ds_new = NOFF - 2 * like_new;
@@ -463,9 +236,9 @@ __device__ __forceinline__ void price_and_commit(const SweepLaunch &a, const int
         vol_new = base_new.x + dv;
         surf_new = base_new.y + ds;
     }
-    delta = size_terms<UNIFORM>(a, old, nw, t_old, t_new, vol_old, vol_new, surf_old, surf_new, ds_old, ds_new, delta);
+    delta = size_terms<UNIFORM>(a, a.t, old, nw, t_old, t_new, vol_old, vol_new, surf_old, surf_new, ds_old, ds_new, delta);
     if (EXTRAS && (a.has_length || a.has_chemotaxis || a.has_external || a.has_motility || a.has_nematic))
-        delta = extra_terms<DIM>(a, old, nw, t_old, t_new, vol_old, vol_new, x, y, z, pick, target, delta);
+        delta = tile_extra_terms<DIM, NOFF>(a, old, nw, t_old, t_new, vol_old, vol_new, x, y, z, pick, target, delta);
 
     // Metropolis: a copy that lowers the energy (or keeps it) is taken, else
     // with probability exp(-delta / T). The draw and the exponential are
@@ -490,7 +263,7 @@ __device__ __forceinline__ void price_and_commit(const SweepLaunch &a, const int
         atomicAdd(&a.vs_cur[nw], pack_delta(1, ds_new));
         atomicAdd(&a.vol_by_colour[(size_t)nw * a.g.ncol + a.colour], 1);
     }
-    if (EXTRAS && a.tracks) commit_moments<DIM>(a, old, nw, x, y, z);
+    if (EXTRAS && a.tracks) tile_commit_moments<DIM>(a, old, nw, x, y, z);
 }
 
 template <int DIM>
@@ -695,7 +468,7 @@ __global__ void __launch_bounds__(kThreads, GLZ_SWEEP_MIN_BLOCKS) sweep_kernel(c
     if (small_types)
         for (int i = tid; i < a.n_types * a.n_types; i += blockDim.x) S.contact[i] = a.t.contact[i];
     if (tid < NOFF) S.woff[tid] = (a.g.off[tid][2] * T::PY + a.g.off[tid][1]) * T::PX + a.g.off[tid][0];
-    if (tid < a.g.ring_n) S.wring[tid] = (a.g.ring[tid][2] * T::PY + a.g.ring[tid][1]) * T::PX + a.g.ring[tid][0];
+    if (tid < kRing<DIM>) S.wring[tid] = window_offset<DIM, kRing<DIM>>(tid);
     if (tid == 0) {
         S.queued = 0;
         S.taken = 0;
@@ -1102,367 +875,6 @@ __global__ void __launch_bounds__(kLeanThreads, GLZ_LEAN_MIN_BLOCKS)
     }
 }
 
-// ---------------------------------------------------------------- the direct sweep
-//
-// Small lattices of the lean models take a kernel with no staging at all:
-// one thread per target, the labels read where they lie (a target's
-// neighbours are other colours, which no copy in the pass changes), priced
-// with price_and_commit's arithmetic operation for operation. The lean
-// kernel's window ring, patches and queues cost more latency than they save
-// when a pass is a few tiles.
-// The per-pass view of the tallies and draws a direct pass reads.
-struct PassView {
-    int colour;
-    uint64_t key_pick, key_accept;
-    const int2 *vs_base;
-    const long long *vs_prev;
-    unsigned long long *vs_cur;
-};
-
-// The per-colour guard of keeps_other_colour, for a direct pass.
-__device__ __noinline__ bool direct_keeps_other_colour(const SweepLaunch &a, int colour, uint32_t old) {
-    int other = 0;
-    for (int c = 0; c < a.g.ncol; ++c)
-        if (c != colour) other += a.vol_by_colour[(size_t)old * a.g.ncol + c];
-    return other != 0;
-}
-
-// Where a direct pass finds and puts labels and tallies: global memory.
-struct GlobalPass {
-    const SweepLaunch &a;
-    const PassView &v;
-    __device__ __forceinline__ uint32_t label(int x, int y, int z) const {
-        return a.labels[(z * a.g.h + y) * a.g.w + x];
-    }
-    __device__ __forceinline__ int2 base(uint32_t l) const { return v.vs_base[l]; }
-    __device__ __forceinline__ long long prev(uint32_t l) const { return v.vs_prev[l]; }
-    __device__ __forceinline__ bool keeps_other_colour(uint32_t old) const {
-        return direct_keeps_other_colour(a, v.colour, old);
-    }
-    __device__ __forceinline__ void put(uint32_t target, int, int, int, uint32_t nw) const { a.labels[target] = nw; }
-    __device__ __forceinline__ void tally(uint32_t l, int dv, int ds) const {
-        atomicAdd(&v.vs_cur[l], pack_delta(dv, ds));
-        atomicAdd(&a.vol_by_colour[(size_t)l * a.g.ncol + v.colour], dv);
-    }
-};
-
-// Site (x, y, z) of target j of colour `colour` in a direct pass.
-template <int DIM>
-__device__ __forceinline__ void direct_site(const SweepLaunch &a, int colour, int j, int &x, int &y, int &z) {
-    const uint32_t row = udiv(a.g.div_hw, (uint32_t)j), plane = udiv(a.g.div_hh, row);
-    x = 2 * (int)((uint32_t)j - row * (uint32_t)(a.g.w / 2)) + (colour & 1);
-    y = 2 * (int)(row - plane * (uint32_t)(a.g.h / 2)) + ((colour >> 1) & 1);
-    z = DIM == 3 ? 2 * (int)plane + ((colour >> 2) & 1) : 0;
-}
-
-// The connectivity veto (lib.rs:511-521) for a direct pass: the ring
-// positions of `old` around target (x, y, z), read where they lie, must be
-// one piece.
-__device__ __noinline__ bool direct_ring_one_piece(const SweepLaunch &a, int x, int y, int z, uint32_t old) {
-    const int W = a.g.w, H = a.g.h, D = a.g.d;
-    uint32_t present = 0;
-    for (int k = 0; k < a.g.ring_n; ++k) {
-        const int nx = wrap(x + a.g.ring[k][0], W), ny = wrap(y + a.g.ring[k][1], H), nz = wrap(z + a.g.ring[k][2], D);
-        if (a.labels[((size_t)nz * H + ny) * W + nx] == old) present |= 1u << k;
-    }
-    return one_piece(present, a.g.adjacency);
-}
-
-// The offset of neighbour `pick`, chosen among compile-time constants (the
-// 26-neighbourhood has a closed form) rather than read from a table.
-template <int DIM, int NOFF>
-__device__ __forceinline__ void pick_offset(int pick, int &dx, int &dy, int &dz) {
-    if constexpr (DIM == 3 && NOFF == 26) {
-        dx = neighbour_offset<3, 26>(pick, 0);
-        dy = neighbour_offset<3, 26>(pick, 1);
-        dz = neighbour_offset<3, 26>(pick, 2);
-    } else {
-        dx = dy = dz = 0;
-#pragma unroll
-        for (int k = 0; k < NOFF; ++k)
-            if (k == pick) {
-                dx = neighbour_offset<DIM, NOFF>(k, 0);
-                dy = neighbour_offset<DIM, NOFF>(k, 1);
-                dz = neighbour_offset<DIM, NOFF>(k, 2);
-            }
-    }
-}
-
-// The copy attempt at target (x, y, z) of a direct pass, its labels and
-// tallies found through `acc`: a target's neighbours are other colours, which
-// no copy in the pass changes. Priced with price_and_commit's arithmetic
-// operation for operation.
-template <int DIM, int NOFF, bool UNIFORM, class Access, bool EXTRAS = false>
-__device__ __forceinline__ void direct_target(const SweepLaunch &a, const Access &acc, uint64_t key_pick,
-                                              uint64_t key_accept, int x, int y, int z, int known_pick = -1,
-                                              bool known_labels = false, uint32_t known_old = 0,
-                                              uint32_t known_new = 0) {
-    const int W = a.g.w, H = a.g.h, D = a.g.d;
-    const int xm = x == 0 ? W - 1 : x - 1, xp = x == W - 1 ? 0 : x + 1;
-    const int ym = y == 0 ? H - 1 : y - 1, yp = y == H - 1 ? 0 : y + 1;
-    const int zm = z == 0 ? D - 1 : z - 1, zp = z == D - 1 ? 0 : z + 1;
-    const auto at = [&](int k) -> uint32_t {
-        const int dx = neighbour_offset<DIM, NOFF>(k, 0), dy = neighbour_offset<DIM, NOFF>(k, 1),
-                  dz = neighbour_offset<DIM, NOFF>(k, 2);
-        const int nx = dx < 0 ? xm : (dx > 0 ? xp : x), ny = dy < 0 ? ym : (dy > 0 ? yp : y),
-                  nz = dz < 0 ? zm : (dz > 0 ? zp : z);
-        return acc.label(nx, ny, nz);
-    };
-    const uint32_t target = (uint32_t)((z * H + y) * W + x);
-    const int pick = known_pick >= 0 ? known_pick : pick_of<NOFF>(draw(key_pick, target));
-    int dx, dy, dz;
-    pick_offset<DIM, NOFF>(pick, dx, dy, dz);
-    // A caller that read the two labels earlier in the pass passes them: the
-    // target's changes only by its own commit and the neighbour is another
-    // colour, so they are still the pass's.
-    const uint32_t nw = known_labels ? known_new
-                                     : acc.label(dx < 0 ? xm : (dx > 0 ? xp : x), dy < 0 ? ym : (dy > 0 ? yp : y),
-                                                 dz < 0 ? zm : (dz > 0 ? zp : z));
-    const uint32_t old = known_labels ? known_old : acc.label(x, y, z);
-    if (old == nw) return;
-    const int2 base_old = acc.base(old), base_new = acc.base(nw);
-    const long long prev_old = acc.prev(old), prev_new = acc.prev(nw);
-    const int t_old = UNIFORM ? a.uniform_type : a.cell_type[old];
-    const int t_new = UNIFORM ? a.uniform_type : a.cell_type[nw];
-    float delta = 0.0f;
-    int like_old = 0, like_new = 0;
-    if (UNIFORM) {
-#pragma unroll
-        for (int k = 0; k < NOFF; ++k) {
-            const uint32_t ln = at(k);
-            like_old += ln == old;
-            like_new += ln == nw;
-        }
-        delta = __fmul_rn(a.uniform_contact, (float)(like_old - like_new));
-    } else {
-#pragma unroll
-        for (int k = 0; k < NOFF; ++k) {
-            const uint32_t ln = at(k);
-            const int tn = ln == old ? t_old : (ln == nw ? t_new : (int)a.cell_type[ln]);
-            if (ln != old)
-                delta = __fsub_rn(delta, a.t.contact[t_old * a.n_types + tn]);
-            else
-                ++like_old;
-            if (ln != nw)
-                delta = __fadd_rn(delta, a.t.contact[t_new * a.n_types + tn]);
-            else
-                ++like_new;
-        }
-    }
-    if (old != 0 && like_old == 0 && !acc.keeps_other_colour(old)) return;
-    if (EXTRAS && old != 0 && a.g.ring_n > 0 && a.t.connected[t_old] && !direct_ring_one_piece(a, x, y, z, old))
-        return;
-    const int ds_old = 2 * like_old - NOFF;
-    const int ds_new = NOFF - 2 * like_new;
-    int dv, ds;
-    unpack_delta(prev_old, dv, ds);
-    const int vol_old = base_old.x + dv, surf_old = base_old.y + ds;
-    unpack_delta(prev_new, dv, ds);
-    const int vol_new = base_new.x + dv, surf_new = base_new.y + ds;
-    delta = size_terms<UNIFORM>(a, old, nw, t_old, t_new, vol_old, vol_new, surf_old, surf_new, ds_old, ds_new, delta);
-    if (EXTRAS && (a.has_length || a.has_chemotaxis || a.has_external || a.has_motility || a.has_nematic))
-        delta = extra_terms<DIM>(a, old, nw, t_old, t_new, vol_old, vol_new, x, y, z, pick, target, delta);
-    const float u = to_f32(draw(key_accept, target));
-    if (!(delta <= 0.0f || u < metropolis_exp(__fmul_rn(-delta, a.beta)))) return;
-    if (EXTRAS && a.has_motility) {
-        const int k = atomicAdd(a.pending_count, 1);
-        a.pending[k] = make_uint2(target, nw);
-    } else {
-        acc.put(target, x, y, z, nw);
-    }
-    if (old != 0) acc.tally(old, -1, ds_old);
-    if (nw != 0) acc.tally(nw, 1, ds_new);
-    if (EXTRAS && a.tracks) commit_moments<DIM>(a, old, nw, x, y, z);
-}
-
-// K 0: one target per thread, priced where it lies. K > 0: each warp takes
-// 32 K consecutive targets; every lane draws its targets' picks and compares
-// the two labels, the targets whose pick carries another label go into the
-// warp's queue, and the warp prices the queue in full rounds, so that a
-// round's lanes all have a copy to price. The queue pays on large passes
-// (0.37 against 0.51 ms per MCS at 256^3 with K 4); below a million targets
-// a pass (kDirectCompactFrom, engine.h) the block-queued form below, with its
-// wider grid, hides more latency.
-constexpr int kDirectCompactK = 4;
-// K < 0: the block's 256 |K| consecutive targets are drawn and compared by
-// all its threads, the unlike ones gathered into one block-wide queue, and
-// the queue priced from its front by as many whole warps as it needs: the
-// plain form's wide grid, with a warp's lanes busy in the pricing rounds.
-// Two targets a thread (per MCS at 1024^2: 37.3 us with two, 52.0 with one;
-// at 128^3, with the register cap below, 0.060 ms with two, 0.062 with one).
-template <int DIM>
-constexpr int kDirectBlockK = -2;
-
-// Direct passes of the lean models are held to 64 registers, four blocks of
-// 256 per SM, so that a 2^18-target pass of two targets a thread is one wave
-// (at 128^3: 0.060 ms per MCS against 0.073 uncapped, 0.065 at 48 registers);
-// the every-term passes keep their registers (capped, they spill and slow).
-template <bool EXTRAS>
-constexpr int kDirectMinBlocks = EXTRAS ? 1 : 4;
-
-template <int DIM, int NOFF, bool UNIFORM, int K, bool EXTRAS>
-__device__ __forceinline__ void direct_sweep_body(const SweepLaunch &a) {
-    const int targets = (a.g.w / 2) * (a.g.h / 2) * (DIM == 3 ? a.g.d / 2 : 1);
-    const PassView v{a.colour, a.key_pick, a.key_accept, a.vs_base, a.vs_prev, a.vs_cur};
-    const GlobalPass acc{a, v};
-    if constexpr (K == 0) {
-        const int j = blockIdx.x * blockDim.x + threadIdx.x;
-        if (j < targets) {
-            int x, y, z;
-            direct_site<DIM>(a, a.colour, j, x, y, z);
-            direct_target<DIM, NOFF, UNIFORM, GlobalPass, EXTRAS>(a, acc, v.key_pick, v.key_accept, x, y, z);
-        }
-    } else if constexpr (K < 0) {
-        constexpr int KB = -K;
-        __shared__ int queue[256 * KB];
-        __shared__ uint8_t picks[256 * KB];
-        __shared__ uint2 pair[256 * KB];  // (old, new) labels of each queued copy, as the light step read them
-        __shared__ int counts[8];
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        const unsigned below = (1u << lane) - 1u;
-        // The block's targets [first, last): direct_span of them (at most 256 KB)
-        // when the launch spreads the pass evenly over the SMs' resident
-        // blocks, else 256 KB.
-        const int span = a.direct_span > 0 ? a.direct_span : 256 * KB;
-        const int first = (int)blockIdx.x * span;
-        const int last = min(first + span, targets);
-        unsigned masks[KB];
-        int picked[KB];
-        uint2 labels[KB];
-        int mine = 0;
-#pragma unroll
-        for (int k = 0; k < KB; ++k) {
-            const int j = first + k * 256 + (int)threadIdx.x;
-            bool unlike = false;
-            int pick = 0;
-            labels[k] = make_uint2(0u, 0u);
-            if (j < last) {
-                int x, y, z;
-                direct_site<DIM>(a, a.colour, j, x, y, z);
-                pick = pick_of<NOFF>(draw(v.key_pick, (uint32_t)((z * a.g.h + y) * a.g.w + x)));
-                int dx, dy, dz;
-                pick_offset<DIM, NOFF>(pick, dx, dy, dz);
-                const int nx = x + dx < 0 ? a.g.w - 1 : (x + dx >= a.g.w ? 0 : x + dx);
-                const int ny = y + dy < 0 ? a.g.h - 1 : (y + dy >= a.g.h ? 0 : y + dy);
-                const int nz = z + dz < 0 ? a.g.d - 1 : (z + dz >= a.g.d ? 0 : z + dz);
-                labels[k] = make_uint2(acc.label(x, y, z), acc.label(nx, ny, nz));
-                unlike = labels[k].x != labels[k].y;
-            }
-            masks[k] = __ballot_sync(0xffffffffu, unlike);
-            picked[k] = pick;
-            mine += __popc(masks[k]);
-        }
-        if (lane == 0) counts[warp] = mine;
-        __syncthreads();
-        int at = 0, total = 0;
-#pragma unroll
-        for (int w = 0; w < 8; ++w) {
-            at += w < warp ? counts[w] : 0;
-            total += counts[w];
-        }
-#pragma unroll
-        for (int k = 0; k < KB; ++k) {
-            if (masks[k] & (1u << lane)) {
-                queue[at + __popc(masks[k] & below)] = first + k * 256 + (int)threadIdx.x;
-                picks[at + __popc(masks[k] & below)] = (uint8_t)picked[k];
-                pair[at + __popc(masks[k] & below)] = labels[k];
-            }
-            at += __popc(masks[k]);
-        }
-        __syncthreads();
-        for (int e = (int)threadIdx.x; e < total; e += 256) {
-            int x, y, z;
-            direct_site<DIM>(a, a.colour, queue[e], x, y, z);
-            const uint2 ln = pair[e];
-            direct_target<DIM, NOFF, UNIFORM, GlobalPass, EXTRAS>(a, acc, v.key_pick, v.key_accept, x, y, z, picks[e],
-                                                                  true, ln.x, ln.y);
-        }
-    } else {
-        __shared__ int queue[8][32 * K];
-        __shared__ uint8_t picks[8][32 * K];
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        const unsigned below = (1u << lane) - 1u;
-        const int first = (blockIdx.x * 8 + warp) * 32 * K;
-        int total = 0;
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const int j = first + k * 32 + lane;
-            bool unlike = false;
-            int pick = 0;
-            if (j < targets) {
-                int x, y, z;
-                direct_site<DIM>(a, a.colour, j, x, y, z);
-                pick = pick_of<NOFF>(draw(v.key_pick, (uint32_t)((z * a.g.h + y) * a.g.w + x)));
-                int dx, dy, dz;
-                pick_offset<DIM, NOFF>(pick, dx, dy, dz);
-                const int nx = x + dx < 0 ? a.g.w - 1 : (x + dx >= a.g.w ? 0 : x + dx);
-                const int ny = y + dy < 0 ? a.g.h - 1 : (y + dy >= a.g.h ? 0 : y + dy);
-                const int nz = z + dz < 0 ? a.g.d - 1 : (z + dz >= a.g.d ? 0 : z + dz);
-                unlike = acc.label(x, y, z) != acc.label(nx, ny, nz);
-            }
-            const unsigned m = __ballot_sync(0xffffffffu, unlike);
-            if (unlike) {
-                queue[warp][total + __popc(m & below)] = j;
-                picks[warp][total + __popc(m & below)] = (uint8_t)pick;
-            }
-            total += __popc(m);
-        }
-        __syncwarp();
-        for (int e = lane; e < total; e += 32) {
-            int x, y, z;
-            direct_site<DIM>(a, a.colour, queue[warp][e], x, y, z);
-            direct_target<DIM, NOFF, UNIFORM, GlobalPass, EXTRAS>(a, acc, v.key_pick, v.key_accept, x, y, z,
-                                                                  picks[warp][e]);
-        }
-    }
-    rotate_tallies<DIM>(a);
-}
-
-template <int DIM, int NOFF, bool UNIFORM, int K, bool EXTRAS>
-__global__ void __launch_bounds__(256, kDirectMinBlocks<EXTRAS>) direct_sweep_kernel(const __grid_constant__ SweepLaunch a) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    direct_sweep_body<DIM, NOFF, UNIFORM, K, EXTRAS>(a);
-}
-
-// A clocked launch's pass fields from the engine clock, as pass_launch
-// (engine.cu) sets them on the host: the step and its draws, the tally slots
-// of the pass's number, each species' current field buffer.
-__device__ __forceinline__ void clock_patch(SweepLaunch &d) {
-    const EngineClock c = *d.clock;
-    const long long p = c.pass + d.colour;
-    d.step = (int32_t)c.step;
-    d.key_pick = stream_key(d.seed, d.step, d.colour, 0);
-    d.key_accept = stream_key(d.seed, d.step, d.colour, 1);
-    d.vs_base = d.tal.vs_base[p % 2];
-    d.vs_prev = d.tal.vs_delta[(p + 2) % 3];
-    d.vs_cur = reinterpret_cast<unsigned long long *>(d.tal.vs_delta[p % 3]);
-    d.vs_next_base = d.tal.vs_base[(p + 1) % 2];
-    d.vs_clear = d.tal.vs_delta[(p + 1) % 3];
-    d.mom_base = d.tal.mom_base[p % 2];
-    d.mom_prev = d.tal.mom_delta[(p + 2) % 3];
-    d.mom_cur = reinterpret_cast<unsigned long long *>(d.tal.mom_delta[p % 3]);
-    d.mom_next_base = d.tal.mom_base[(p + 1) % 2];
-    d.mom_clear = d.tal.mom_delta[(p + 1) % 3];
-    for (int s = 0; s < d.n_species; ++s)
-        d.fields[s] = d.field_buf + ((size_t)2 * s + ((c.field_cur >> s) & 1u)) * (size_t)d.g.sites;
-}
-
-// The direct pass of a step replayed from a graph: the block copies the
-// launch into shared memory, patches it from the clock and prices from there.
-template <int DIM, int NOFF, bool UNIFORM, int K, bool EXTRAS>
-__global__ void __launch_bounds__(256, kDirectMinBlocks<EXTRAS>) direct_sweep_clocked(const __grid_constant__ SweepLaunch a) {
-    __shared__ SweepLaunch d;
-    static_assert(sizeof(SweepLaunch) % sizeof(int) == 0, "the launch copies as words");
-    const int *src = reinterpret_cast<const int *>(&a);
-    int *dst = reinterpret_cast<int *>(&d);
-    for (int i = threadIdx.x; i < (int)(sizeof(SweepLaunch) / sizeof(int)); i += blockDim.x) dst[i] = src[i];
-    __syncthreads();
-    if (threadIdx.x == 0) clock_patch(d);
-    __syncthreads();
-    direct_sweep_body<DIM, NOFF, UNIFORM, K, EXTRAS>(d);
-}
-
 // ---------------------------------------------------------------- the resident sweep
 //
 // A small lean model with nothing between its colour passes but the passes
@@ -1523,7 +935,7 @@ __global__ void __launch_bounds__(256) resident_sweep_kernel(const __grid_consta
             if (j < targets) {
                 int x, y, z;
                 direct_site<DIM>(a, c, j, x, y, z);
-                direct_target<DIM, NOFF, UNIFORM>(a, GlobalPass{a, v}, v.key_pick, v.key_accept, x, y, z);
+                direct_target<DIM, NOFF, UNIFORM>(a, a.t, GlobalPass{a, v}, v.key_pick, v.key_accept, x, y, z);
             }
             // the rotation for the next pass, which no thread of this one reads
             int2 *next_base = r.vs_base[(p + 1) % 2];
@@ -1767,7 +1179,10 @@ __global__ void __launch_bounds__(kClusterThreads, 1) cluster_sweep_kernel(const
             for (int e = tid; e < total; e += nth) {
                 const int t = queue[e];
                 const int y = yf + 2 * (t / hw), x = 2 * (t % hw) + (c & 1);
-                direct_target<2, NOFF, UNIFORM>(a, acc, key_pick, key_accept, x, y, 0, (int)picks[e]);
+                const int pick = picks[e];
+                const NeighbourReads<2, NOFF, ClusterPass> ln(a, acc, x, y, 0);
+                direct_copy<2, NOFF, UNIFORM>(a, a.t, acc, ln, key_accept, x, y, 0, pick, acc.label(x, y, 0),
+                                              picked_label<2, NOFF>(a, acc, x, y, 0, pick));
             }
             // this CTA's labels' rotation for the next pass, which no thread of this one reads
             int2 *next_base = base + ((p + 1) % 2) * L.Lc;
@@ -1857,86 +1272,6 @@ cudaError_t launch_cluster_sweep(const ResidentLaunch &r, cudaStream_t stream) {
 }
 
 template <int DIM, int NOFF, bool UNIFORM>
-static cudaError_t launch_direct(const SweepLaunch &a, cudaStream_t stream);
-
-// Whether sweeps launch programmatically (GLAZIER_SWEEP_PDL=0: plainly).
-static int programmatic_launch() {
-    static const int on = [] {
-        const char *env = std::getenv("GLAZIER_SWEEP_PDL");
-        return env && env[0] == '0' ? 0 : 1;
-    }();
-    return on;
-}
-
-// Blocks of the block-queued direct kernel that the device holds at once by
-// its launch bounds (SMs x kDirectMinBlocks blocks of 256 threads; the lean
-// form's 64-register cap makes that exactly four per SM); 0 if the SM count
-// cannot be read. A device attribute only, so a launch being captured into
-// a graph may ask.
-static int gathered_slots(bool extras) {
-    static std::atomic<int> sms_once{0};  // handles on other host threads may launch too
-    int sms = sms_once.load(std::memory_order_acquire);
-    if (!sms) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) {
-            cudaGetLastError();
-            return 0;
-        }
-        sms_once.store(sms, std::memory_order_release);
-    }
-    return sms * (extras ? kDirectMinBlocks<true> : kDirectMinBlocks<false>);
-}
-
-template <int DIM, int NOFF, bool UNIFORM>
-static cudaError_t launch_direct(const SweepLaunch &a, cudaStream_t stream) {
-    const int targets = (a.g.w / 2) * (a.g.h / 2) * (DIM == 3 ? a.g.d / 2 : 1);
-    const bool compact = a.compact == 1, gathered = a.compact == 2;
-    const int per_block = 256 * (compact ? kDirectCompactK : (gathered ? -kDirectBlockK<DIM> : 1));
-    int grid = (targets + per_block - 1) / per_block;
-    SweepLaunch b = a;
-    b.direct_span = 0;
-    if (gathered) {
-        // Spread the pass evenly over whole waves of resident blocks, so that
-        // no SM holds more of its targets than another (at 128^3 and 1024^2:
-        // 592 blocks of 443 targets instead of 512 of 512 on 148 SMs).
-        const int slots = gathered_slots(!a.lean);
-        if (slots > 0) {
-            const int waves = (grid + slots - 1) / slots;
-            const int spread = waves * slots;
-            b.direct_span = (targets + spread - 1) / spread;
-            grid = (targets + b.direct_span - 1) / b.direct_span;
-        }
-    }
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(256);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    // a motility pass follows its predecessor's copy list and a memset, not a kernel
-    attr[0].val.programmaticStreamSerializationAllowed = programmatic_launch() && !a.has_motility;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (a.clock) {  // a step captured into a graph: plain launches, pass fields from the clock
-        cfg.numAttrs = 0;
-        if (!a.lean)
-            return compact    ? cudaLaunchKernelEx(&cfg, direct_sweep_clocked<DIM, NOFF, UNIFORM, kDirectCompactK, true>, b)
-                   : gathered ? cudaLaunchKernelEx(&cfg, direct_sweep_clocked<DIM, NOFF, UNIFORM, kDirectBlockK<DIM>, true>, b)
-                              : cudaLaunchKernelEx(&cfg, direct_sweep_clocked<DIM, NOFF, UNIFORM, 0, true>, b);
-        return compact    ? cudaLaunchKernelEx(&cfg, direct_sweep_clocked<DIM, NOFF, UNIFORM, kDirectCompactK, false>, b)
-               : gathered ? cudaLaunchKernelEx(&cfg, direct_sweep_clocked<DIM, NOFF, UNIFORM, kDirectBlockK<DIM>, false>, b)
-                          : cudaLaunchKernelEx(&cfg, direct_sweep_clocked<DIM, NOFF, UNIFORM, 0, false>, b);
-    }
-    if (!a.lean)  // every term: length, chemotaxis, connectivity, motility, drift, nematic, moments
-        return compact    ? cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kDirectCompactK, true>, b)
-               : gathered ? cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kDirectBlockK<DIM>, true>, b)
-                          : cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, 0, true>, b);
-    return compact    ? cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kDirectCompactK, false>, b)
-           : gathered ? cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kDirectBlockK<DIM>, false>, b)
-                      : cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, 0, false>, b);
-}
-
-template <int DIM, int NOFF, bool UNIFORM>
 static cudaError_t launch_lean(const SweepLaunch &a, const CUtensorMap &tmap, cudaStream_t stream) {
     using T = Tile<DIM>;
     static std::atomic<int> grid_cap_once{0};  // handles on other host threads may launch too
@@ -2006,8 +1341,7 @@ static cudaError_t launch(const SweepLaunch &a, cudaStream_t stream) {
     const int grid_cap = grid_cap_once.load(std::memory_order_acquire);
     int grid = tiles < grid_cap ? tiles : grid_cap;
     if (a.max_ctas > 0 && grid > a.max_ctas) grid = a.max_ctas;
-    // programmatic launch as the lean kernel's, except for a motility pass,
-    // which follows its predecessor's copy list and a memset, not a kernel
+    // programmatic launch as the lean kernel's
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(kThreads);
@@ -2015,7 +1349,7 @@ static cudaError_t launch(const SweepLaunch &a, cudaStream_t stream) {
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = programmatic_launch() && !a.has_motility;
+    attr[0].val.programmaticStreamSerializationAllowed = programmatic_launch();
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, sweep_kernel<DIM, NOFF, UNIFORM>, a, tmap);
@@ -2034,8 +1368,13 @@ static cudaError_t launch_any(const SweepLaunch &a, cudaStream_t stream) {
     return cudaErrorInvalidValue;
 }
 
+// The pass's listed copies; the other pass parity's count, which the copies
+// before these emptied, is set to zero for the next pass.
 __global__ void apply_copies_kernel(const __grid_constant__ SweepLaunch a, float *activity) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int count = *a.pending_count;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *a.pending_clear = 0;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
         const uint2 p = a.pending[k];
         a.labels[p.x] = p.y;
@@ -2046,15 +1385,33 @@ __global__ void apply_copies_kernel(const __grid_constant__ SweepLaunch a, float
     }
 }
 
+// A kernel launch that may start while the previous kernel on the stream
+// ends; the kernel waits (griddepcontrol.wait) before it reads pass data.
+template <class... Params, class... Args>
+static cudaError_t launch_after(void (*kernel)(Params...), int grid, cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(256);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = programmatic_launch();
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 cudaError_t launch_apply_copies(const SweepLaunch &a, float *activity, cudaStream_t stream) {
-    // at most one copy per target, and a pass has sites / colours targets
+    // at most one copy per target, and a pass has sites / colours targets;
+    // an accepted one is rare enough that a fraction of that grid covers them
     const int most = a.g.sites / a.g.ncol + 1;
-    apply_copies_kernel<<<(most + 255) / 256, 256, 0, stream>>>(a, activity);
-    if (cudaError_t e = cudaGetLastError()) return e;
-    return cudaMemsetAsync(a.pending_count, 0, sizeof(int), stream);
+    const int blocks = (most + 2047) / 2048;
+    return launch_after(apply_copies_kernel, blocks, stream, a, activity);
 }
 
 __global__ void activity_decay_kernel(float *activity, int sites) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= sites) return;
     const float v = activity[i];
@@ -2062,8 +1419,7 @@ __global__ void activity_decay_kernel(float *activity, int sites) {
 }
 
 cudaError_t launch_activity_decay(float *activity, int sites, cudaStream_t stream) {
-    activity_decay_kernel<<<(sites + 255) / 256, 256, 0, stream>>>(activity, sites);
-    return cudaGetLastError();
+    return launch_after(activity_decay_kernel, (sites + 255) / 256, stream, activity, sites);
 }
 
 cudaError_t launch_sweep(const SweepLaunch &a, cudaStream_t stream) {
@@ -2505,7 +1861,7 @@ __device__ __forceinline__ void direct_ensemble_tile(const EnsembleLaunch &e, Sw
     const int jy = (lt / tiles_x) * BY + (int)threadIdx.x / BX;
     if (jx < hw && jy < hh) {
         const PassView v{colour, d.key_pick, d.key_accept, d.vs_base, d.vs_prev, d.vs_cur};
-        direct_target<2, NOFF, UNIFORM, GlobalPass, false>(d, GlobalPass{d, v}, v.key_pick, v.key_accept,
+        direct_target<2, NOFF, UNIFORM, GlobalPass, false>(d, d.t, GlobalPass{d, v}, v.key_pick, v.key_accept,
                                                            2 * jx + (colour & 1), 2 * jy + ((colour >> 1) & 1), 0);
     }
     __syncthreads();  // `d` and `where` serve the block's next tile
