@@ -40,6 +40,7 @@ struct GlobalPass {
     __device__ __forceinline__ uint32_t label(int x, int y, int z) const {
         return a.labels[(z * a.g.h + y) * a.g.w + x];
     }
+    __device__ __forceinline__ int type(uint32_t l) const { return a.cell_type[l]; }
     __device__ __forceinline__ int2 base(uint32_t l) const { return v.vs_base[l]; }
     __device__ __forceinline__ long long prev(uint32_t l) const { return v.vs_prev[l]; }
     __device__ __forceinline__ bool keeps_other_colour(uint32_t old) const {
@@ -146,8 +147,8 @@ __device__ __forceinline__ void direct_copy(const SweepLaunch &a, const TypeTabl
     const uint32_t target = (uint32_t)((z * H + y) * W + x);
     const int2 base_old = acc.base(old), base_new = acc.base(nw);
     const long long prev_old = acc.prev(old), prev_new = acc.prev(nw);
-    const int t_old = UNIFORM ? a.uniform_type : a.cell_type[old];
-    const int t_new = UNIFORM ? a.uniform_type : a.cell_type[nw];
+    const int t_old = UNIFORM ? a.uniform_type : acc.type(old);
+    const int t_new = UNIFORM ? a.uniform_type : acc.type(nw);
     // the moment commit's anchors, read here so the commit does not wait
     int4 an_old = make_int4(0, 0, 0, 0), an_new = an_old;
     if (EXTRAS && a.tracks) {
@@ -175,7 +176,7 @@ __device__ __forceinline__ void direct_copy(const SweepLaunch &a, const TypeTabl
             const uint32_t ln = neighbour(k);
             const bool is_old = ln == old, is_new = ln == nw;
             int tn = is_old ? t_old : t_new;
-            if (!is_old && !is_new) tn = a.cell_type[ln];
+            if (!is_old && !is_new) tn = acc.type(ln);
             const float j_old = T.contact[t_old * a.n_types + tn], j_new = T.contact[t_new * a.n_types + tn];
             delta = __fsub_rn(delta, is_old ? 0.0f : j_old);
             delta = __fadd_rn(delta, is_new ? 0.0f : j_new);

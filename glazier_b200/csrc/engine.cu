@@ -136,10 +136,9 @@ struct glz_gpu {
     bool lean = false;    // the sweep prices contact, volume and surface only
     bool direct = false;  // ... on a lattice small enough for the direct kernel
     int compact = 0;      // ... queueing a warp's unlike copies (1, large passes) or a block's (2)
-    bool resident = false;  // ... with nothing between passes: every MCS in one launch
-    bool cluster = false;   // ... a plane, in one thread-block cluster's shared memory
+    bool cluster = false;   // ... a small plane with nothing between passes, in one cluster's shared memory
     bool band = false;      // ... a large plane, streamed by row bands in one launch per call
-    unsigned *barrier = nullptr;  // the resident sweep's grid barrier
+    unsigned *barrier = nullptr;  // the band sweep's grid barrier
     int max_ctas = 0;
     int uniform = -1;
     bool uniform_exact = false;
@@ -594,16 +593,14 @@ int check_error_flag(glz_gpu *h) {
     if (flag == 1) return fail(GLZ_DRIVER, "a sweep tile's tensor copy did not complete within its wait limit");
     if (flag == 2) return fail(GLZ_INVALID, "a label is not below the cell type count");
     if (flag == 3) return fail(GLZ_DRIVER, "the sweep's shared-memory window was not 128-byte aligned");
-    if (flag == 4) return fail(GLZ_DRIVER, "a resident sweep's grid barrier did not complete within its wait limit");
+    if (flag == 4) return fail(GLZ_DRIVER, "a launch's grid barrier did not complete within its wait limit");
     return GLZ_OK;
 }
 
-// The step schedule, with each phase bracketed by events when `ms` is given.
-// Every MCS of the call in one cooperative launch. GLZ_OK with *done false
-// when the blocks cannot all be resident (nothing launched; the caller runs
+// Up to `steps` MCS of the call in one cluster launch. GLZ_OK with *done false
+// when the plane does not fit a cluster (nothing launched; the caller runs
 // the passes one by one, and later calls do too).
-int run_resident(glz_gpu *h, uint64_t steps, double *ms, bool *done) {
-    *done = false;
+int run_cluster(glz_gpu *h, uint64_t steps, bool *done) {
     glz::ResidentLaunch r{};
     r.a = pass_launch(h, 0);
     r.seed = h->seed;
@@ -612,44 +609,17 @@ int run_resident(glz_gpu *h, uint64_t steps, double *ms, bool *done) {
     r.pass0 = (long long)h->pass_no;
     for (int k = 0; k < 2; ++k) r.vs_base[k] = h->t.vs_base[k];
     for (int k = 0; k < 3; ++k) r.vs_delta[k] = h->t.vs_delta[k];
-    r.barrier = h->barrier;
-    cudaEvent_t ev[2] = {};
-    if (ms) {
-        for (auto &e : ev) CU(cudaEventCreate(&e));
-        ms[0] = ms[1] = ms[2] = 0.0;
-    }
-    CU(cudaMemsetAsync(h->barrier, 0, 2 * sizeof(unsigned), h->stream));
-    if (ms) CU(cudaEventRecord(ev[0], h->stream));
-    cudaError_t e = cudaErrorNotSupported;
-    if (h->cluster) {
-        e = glz::launch_cluster_sweep(r, h->stream);
-        if (e == cudaErrorNotSupported) {
-            cudaGetLastError();
-            h->cluster = false;  // and later calls: the plane does not fit a cluster
-        }
-    }
-    if (!h->cluster) e = glz::launch_resident_sweep(r, h->stream);
-    if (e == cudaErrorCooperativeLaunchTooLarge) {
+    const cudaError_t e = glz::launch_cluster_sweep(r, h->stream);
+    *done = e == cudaSuccess;
+    if (e == cudaErrorNotSupported) {
         cudaGetLastError();
-        h->resident = false;
-        for (auto &x : ev)
-            if (x) cudaEventDestroy(x);
+        h->cluster = false;
         return GLZ_OK;
     }
-    if (e != cudaSuccess) return fail(GLZ_DRIVER, std::string("resident sweep: ") + cudaGetErrorString(e));
-    if (ms) {
-        CU(cudaEventRecord(ev[1], h->stream));
-        CU(cudaEventSynchronize(ev[1]));
-        float t = 0.0f;
-        CU(cudaEventElapsedTime(&t, ev[0], ev[1]));
-        ms[0] = t;
-        for (auto &x : ev) cudaEventDestroy(x);
-    }
+    if (e != cudaSuccess) return fail(GLZ_DRIVER, std::string("cluster sweep: ") + cudaGetErrorString(e));
     h->pass_no += steps * (uint64_t)h->g.ncol;
     h->mcs += steps;
-    *done = true;
-    CU(cudaStreamSynchronize(h->stream));
-    return check_error_flag(h);
+    return GLZ_OK;
 }
 
 // One step with clocked launches, for capture: the direct passes (and the
@@ -758,9 +728,8 @@ int run_graph(glz_gpu *h, uint64_t steps) {
         CU(cudaGraphLaunch(h->step_exec, h->stream));
         advance_host(h);
     }
-    CU(cudaStreamSynchronize(h->stream));
     if (int rc = sync_count(h)) return rc;
-    return check_error_flag(h);
+    return check_error_flag(h);  // waits for the stream
 }
 
 // The band sweep's step schedule: every MCS of the call in one launch when
@@ -833,29 +802,34 @@ int run_band(glz_gpu *h, uint64_t steps, double *ms) {
 
 int run_steps(glz_gpu *h, uint64_t steps, double *ms) {
     if (h->band) return run_band(h, steps, ms);
-    if (!ms && h->graph_on && h->direct && !h->resident && steps > 0) return run_graph(h, steps);
-    // resident launches of at most 65536 MCS, so the barrier's arrival count
-    // (blocks x passes) stays far inside 32 bits
-    double total[3] = {0.0, 0.0, 0.0};
-    while (h->resident && steps > 0) {
-        const uint64_t chunk = steps < 65536 ? steps : 65536;
-        bool done = false;
-        double part[3];
-        if (int rc = run_resident(h, chunk, ms ? part : nullptr, &done)) return rc;
-        if (!done) break;
-        if (ms)
-            for (int k = 0; k < 3; ++k) total[k] += part[k];
-        steps -= chunk;
-    }
-    if (ms && steps == 0) {
-        for (int k = 0; k < 3; ++k) ms[k] = total[k];
-        return GLZ_OK;
-    }
-    if (steps == 0) return GLZ_OK;
+    // A model with nothing between its passes is queued pass by pass: a pass
+    // takes the device longer than its launch takes the host, and passes
+    // launched programmatically on the stream follow one another closer than
+    // a graph's replays do (per MCS at 512^2, three types: 16.0 us queued,
+    // 18.9 replayed; 17.3 and 21.2 at 1024^2, one type).
+    const bool between = h->n_species > 0 || h->has_pop || h->infect_species >= 0;
+    if (!ms && h->graph_on && h->direct && between && steps > 0) return run_graph(h, steps);
     cudaEvent_t ev[6] = {};
     if (ms) {
         for (auto &e : ev) CU(cudaEventCreate(&e));
         ms[0] = ms[1] = ms[2] = 0.0;
+    }
+    if (h->cluster && steps > 0) {
+        if (ms) CU(cudaEventRecord(ev[0], h->stream));
+        // launches of at most 65536 MCS
+        while (h->cluster && steps > 0) {
+            const uint64_t chunk = steps < 65536 ? steps : 65536;
+            bool done = false;
+            if (int rc = run_cluster(h, chunk, &done)) return rc;
+            if (done) steps -= chunk;
+        }
+        if (ms) {
+            CU(cudaEventRecord(ev[1], h->stream));
+            CU(cudaEventSynchronize(ev[1]));
+            float t = 0.0f;
+            CU(cudaEventElapsedTime(&t, ev[0], ev[1]));
+            ms[0] = t;
+        }
     }
     int rc = GLZ_OK;
     for (uint64_t r = 0; r < steps && rc == GLZ_OK; ++r) {
@@ -889,16 +863,15 @@ int run_steps(glz_gpu *h, uint64_t steps, double *ms) {
         for (auto &e : ev)
             if (e) cudaEventDestroy(e);
     if (rc != GLZ_OK) return rc;
-    CU(cudaStreamSynchronize(h->stream));
     if (int rc2 = sync_count(h)) return rc2;
-    return check_error_flag(h);
+    return check_error_flag(h);  // waits for the stream
 }
 
 }  // namespace
 
 namespace glz {
 
-bool engine_replays(const glz_gpu *h) { return h->graph_on && h->direct && !h->resident && !h->band; }
+bool engine_replays(const glz_gpu *h) { return h->graph_on && h->direct && !h->cluster && !h->band; }
 
 int engine_begin_replays(glz_gpu *h) {
     if (int rc = upload_clock(h)) return rc;
@@ -1069,33 +1042,35 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
     // staging costs more than it saves.
     const long long direct_most_general = g.dim == 2 ? 1024LL * 1024LL : 128LL * 128LL * 128LL;
     h->direct = direct_mode == 1 || (direct_mode == -1 && sites <= (h->lean ? direct_most : direct_most_general));
-    // From 2^18 targets a pass (with other terms, past 2^16) the direct kernel
-    // gathers each block's unlike copies into one queue priced by whole
-    // warps, and from a million it queues each warp's
+    // Past a number of targets a pass the direct kernel gathers each block's
+    // unlike copies into one queue priced by whole warps, and from a million
+    // it queues each warp's
     // (GLAZIER_SWEEP_COMPACT=0: neither, =1: the warp's, =2: the block's, at
     // any size). Per MCS of the two-field tissue, priced in place against
     // gathered: 31.1 and 31.7 us at 256^2, 35.1 and 35.0 at 512^2, 51.6 and
-    // 36.6 at 640^2, 92.7 and 62.7 at 1024^2.
+    // 36.6 at 640^2, 92.7 and 62.7 at 1024^2. Of the lean plane: 11.9 and 13.9
+    // at 512^2, 13.9 and 15.7 at 768^2 (a last target a thread of one wave of
+    // blocks), 20.9 and 16.7 at 896^2; of the lean volume (26 neighbours):
+    // 24.2 and 28.4 at 64^3, 28.9 and 30.7 at 80^3, 35.6 and 33.4 at 96^3.
     const char *compact_env = std::getenv("GLAZIER_SWEEP_COMPACT");
     const int compact_mode = compact_env ? (compact_env[0] == '0' ? 0 : (compact_env[0] == '2' ? 2 : 1)) : -1;
     const long long targets = sites / g.ncol;
-    const long long gather_from = h->lean ? glz::kDirectGatherFrom : glz::kDirectGatherEveryFrom;
+    const long long gather_from = !h->lean ? glz::kDirectGatherEveryFrom
+                                  : g.dim == 2 ? glz::kDirectGatherFrom : glz::kDirectGatherVolumeFrom;
     h->compact = compact_mode >= 0 ? compact_mode
                                    : (targets >= glz::kDirectCompactFrom ? 1 : (targets >= gather_from ? 2 : 0));
-    // With no fields, division or death there is nothing between colour
-    // passes: a direct plane of at most 512^2 sites runs every MCS of a call
-    // in one cooperative launch, which saves more launch time than its grid
-    // barrier costs (in a volume the barrier and its L2 reads lose to a
-    // launch per pass). GLAZIER_SWEEP_RESIDENT=0: a launch per pass, =1: one
-    // launch at any size or dimension.
+    // A small lean plane with nothing between its colour passes (no fields,
+    // division or death) runs every MCS of a call in one thread-block
+    // cluster (GLAZIER_SWEEP_RESIDENT=0 or GLAZIER_SWEEP_CLUSTER=0: a launch
+    // per pass; RESIDENT=1: the cluster at any size that fits one). Per MCS,
+    // the cluster against a launch per pass: 6.0 and 9.9 us at 128^2, 7.8 and
+    // 10.1 at 196 x 180, 11.0 and 10.5 at 256^2.
     const char *resident_env = std::getenv("GLAZIER_SWEEP_RESIDENT");
     const int resident_mode = resident_env ? (resident_env[0] == '0' ? 0 : 1) : -1;
-    h->resident = h->lean && h->direct && ns == 0 && !h->has_pop &&
-                  (resident_mode == 1 || (resident_mode == -1 && g.dim == 2 && sites <= 512LL * 512LL));
-    // A resident plane runs in one thread-block cluster when it fits one
-    // (GLAZIER_SWEEP_CLUSTER=0: the cooperative grid instead).
     const char *cluster_env = std::getenv("GLAZIER_SWEEP_CLUSTER");
-    h->cluster = h->resident && g.dim == 2 && !(cluster_env && cluster_env[0] == '0');
+    h->cluster = h->lean && h->direct && ns == 0 && !h->has_pop && g.dim == 2 &&
+                 !(cluster_env && cluster_env[0] == '0') &&
+                 (resident_mode == 1 || (resident_mode == -1 && sites < 256LL * 256LL));
     // The band sweep (every colour pass of a call in one launch, rows
     // streamed by bands) runs a lean plane only when asked
     // (GLAZIER_SWEEP_BAND=1) and its rows are whole 16-byte units: at 2048^2,
@@ -1103,7 +1078,7 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
     // (0.169 against 0.145 ms per MCS at 4096^2, L2 flushed).
     const char *band_env = std::getenv("GLAZIER_SWEEP_BAND");
     h->band = h->lean && g.dim == 2 && band_env && band_env[0] == '1' && glz::band_sweep_fits(w, hh);
-    if (h->band) h->direct = h->resident = h->cluster = false;
+    if (h->band) h->direct = h->cluster = false;
     h->host_tv = tv;
     h->host_lv = lv;
     h->host_ts = ts;
@@ -1406,7 +1381,6 @@ const char *glz_gpu_sweep_kernel(const glz_gpu *h) {
     if (!h) return "";
     if (h->band) return "band";
     if (h->cluster) return "cluster";
-    if (h->resident) return "resident";
     if (h->direct) return h->compact == 1 ? "compact" : (h->compact == 2 ? "gathered" : "direct");
     return h->lean ? "lean" : "general";
 }

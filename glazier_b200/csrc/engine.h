@@ -156,8 +156,8 @@ struct SweepLaunch {
 
 cudaError_t launch_sweep(const SweepLaunch &a, cudaStream_t stream);
 
-// Every requested MCS of a small lean model with nothing between its passes
-// in one cooperative launch (sweep.cu, the resident sweep).
+// Every requested MCS of a lean model with nothing between its passes in one
+// launch (the cluster sweep, the band sweep).
 struct ResidentLaunch {
     SweepLaunch a;           // static fields; the pass fields are set per pass
     uint64_t seed;
@@ -169,18 +169,17 @@ struct ResidentLaunch {
     unsigned *barrier;       // [0] arrivals, [1] barriers completed; zero at launch
 };
 
-// cudaErrorCooperativeLaunchTooLarge (and nothing launched) when the blocks
-// cannot all be resident at once.
 // Targets a pass from which the direct kernel queues a block's unlike copies
-// (kDirectGatherFrom; with terms past contact, volume and surface,
-// kDirectGatherEveryFrom) and from which a warp's (kDirectCompactFrom).
-constexpr int kDirectGatherFrom = 1 << 18;
+// (of a lean plane: more than 148 SMs' four blocks of 256 take at once; of a
+// lean volume; with terms past contact, volume and surface) and from which a
+// warp's.
+constexpr int kDirectGatherFrom = 148 * 4 * 256 + 1;
+constexpr int kDirectGatherVolumeFrom = 5 << 14;
 constexpr int kDirectGatherEveryFrom = (1 << 16) + 1;
 constexpr int kDirectCompactFrom = 1 << 20;
 
-cudaError_t launch_resident_sweep(const ResidentLaunch &r, cudaStream_t stream);
-// The same MCS in one thread-block cluster holding a small plane in shared
-// memory; cudaErrorNotSupported (nothing launched) when it does not fit one.
+// Every requested MCS of a small lean plane in one thread-block cluster holding
+// it in shared memory; cudaErrorNotSupported (nothing launched) when it does not fit one.
 cudaError_t launch_cluster_sweep(const ResidentLaunch &r, cudaStream_t stream);
 
 // Every MCS of a call (or one MCS, when fields run between steps) of a large

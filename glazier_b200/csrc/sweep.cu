@@ -24,7 +24,6 @@
 // atomics whose order does not matter; a pass is therefore deterministic and
 // a host replay of the same schedule reproduces it bit for bit.
 
-#include <cooperative_groups.h>
 #include <atomic>
 #include <cuda.h>
 
@@ -875,25 +874,12 @@ __global__ void __launch_bounds__(kLeanThreads, GLZ_LEAN_MIN_BLOCKS)
     }
 }
 
-// ---------------------------------------------------------------- the resident sweep
-//
-// A small lean model with nothing between its colour passes but the passes
-// (no fields, division, death or infection) runs every requested MCS in one
-// cooperative launch: the direct pass's work per target, the tally rotation,
-// then a grid barrier, pass after pass. Each pass's draws and tally slots
-// follow from its number as the host would set them. Reads of what other
-// blocks wrote in earlier passes are plain loads: the barrier's gpu-scope
-// release (each block's fence and arrival) and acquire (the waiting thread's
-// acquire load and fence, then the block barrier) order them after those
-// writes, whatever an SM's L1 held before. The barrier's wait is bounded: a
-// block that gives up sets error flag 4 and returns, and the others then
-// give up at their next barrier.
-
+// A grid barrier for the ensemble's cooperative launches.
 // polls of the barrier word (each an L2 round trip, so the limit is seconds)
 constexpr long long kBarrierLimit = 1LL << 22;
 
 // Barrier number k of the launch (k = 0, 1, ...): false if it timed out.
-__device__ __forceinline__ bool resident_barrier(unsigned *bar, unsigned k) {
+__device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned k) {
     __shared__ int ok;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -919,202 +905,172 @@ __device__ __forceinline__ bool resident_barrier(unsigned *bar, unsigned k) {
     return ok != 0;
 }
 
-template <int DIM, int NOFF, bool UNIFORM>
-__global__ void __launch_bounds__(256) resident_sweep_kernel(const __grid_constant__ ResidentLaunch r) {
-    const SweepLaunch &a = r.a;
-    const int targets = (a.g.w / 2) * (a.g.h / 2) * (DIM == 3 ? a.g.d / 2 : 1);
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    unsigned k = 0;
-    for (int m = 0; m < r.mcs; ++m) {
-        const int32_t step = (int32_t)((uint32_t)r.step0 + (uint32_t)m);
-        for (int c = 0; c < a.g.ncol; ++c) {
-            const long long p = r.pass0 + (long long)m * a.g.ncol + c;
-            const PassView v{c, stream_key(r.seed, step, c, 0), stream_key(r.seed, step, c, 1), r.vs_base[p % 2],
-                             r.vs_delta[(p + 2) % 3], reinterpret_cast<unsigned long long *>(r.vs_delta[p % 3])};
-            if (j < targets) {
-                int x, y, z;
-                direct_site<DIM>(a, c, j, x, y, z);
-                direct_target<DIM, NOFF, UNIFORM>(a, a.t, GlobalPass{a, v}, v.key_pick, v.key_accept, x, y, z);
-            }
-            // the rotation for the next pass, which no thread of this one reads
-            int2 *next_base = r.vs_base[(p + 1) % 2];
-            long long *clear = r.vs_delta[(p + 1) % 3];
-            for (size_t l = j; l < (size_t)a.n_labels; l += stride) {
-                int dv, ds;
-                unpack_delta(v.vs_prev[l], dv, ds);
-                const int2 b = v.vs_base[l];
-                next_base[l] = make_int2(b.x + dv, b.y + ds);
-                clear[l] = 0;
-            }
-            if (!resident_barrier(r.barrier, k++)) {
-                if (threadIdx.x == 0) atomicExch(a.error_flag, 4);
-                return;
-            }
-        }
-    }
-}
-
-// Run `mcs` MCS of a small lean model in one cooperative launch, or return
-// cudaErrorCooperativeLaunchTooLarge (nothing launched) when its blocks
-// cannot all be resident.
-template <int DIM, int NOFF, bool UNIFORM>
-static cudaError_t launch_resident(const ResidentLaunch &r, cudaStream_t stream) {
-    const int targets = (r.a.g.w / 2) * (r.a.g.h / 2) * (DIM == 3 ? r.a.g.d / 2 : 1);
-    const int blocks = (targets + 255) / 256;
-    static std::atomic<int> most_once{0};  // handles on other host threads may launch too
-    if (!most_once.load(std::memory_order_acquire)) {
-        int dev = 0, sms = 0, per_sm = 0;
-        if (cudaError_t e = cudaGetDevice(&dev)) return e;
-        if (cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) return e;
-        if (cudaError_t e =
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, resident_sweep_kernel<DIM, NOFF, UNIFORM>, 256, 0))
-            return e;
-        most_once.store(sms * per_sm, std::memory_order_release);
-    }
-    const int most = most_once.load(std::memory_order_acquire);
-    if (blocks > most) return cudaErrorCooperativeLaunchTooLarge;
-    void *args[] = {const_cast<ResidentLaunch *>(&r)};
-    return cudaLaunchCooperativeKernel((const void *)resident_sweep_kernel<DIM, NOFF, UNIFORM>, dim3(blocks), dim3(256),
-                                       args, 0, stream);
-}
-
-template <bool UNIFORM>
-static cudaError_t resident_any(const ResidentLaunch &r, cudaStream_t stream) {
-    if (r.a.g.dim == 2) {
-        if (r.a.g.n_off == 4) return launch_resident<2, 4, UNIFORM>(r, stream);
-        if (r.a.g.n_off == 8) return launch_resident<2, 8, UNIFORM>(r, stream);
-    } else {
-        if (r.a.g.n_off == 6) return launch_resident<3, 6, UNIFORM>(r, stream);
-        if (r.a.g.n_off == 18) return launch_resident<3, 18, UNIFORM>(r, stream);
-        if (r.a.g.n_off == 26) return launch_resident<3, 26, UNIFORM>(r, stream);
-    }
-    return cudaErrorInvalidValue;
-}
-
-cudaError_t launch_resident_sweep(const ResidentLaunch &r, cudaStream_t stream) {
-    for (int k = 0; k < r.a.g.n_off; ++k)
-        for (int axis = 0; axis < 3; ++axis) {
-            const int want = r.a.g.dim == 2 ? (r.a.g.n_off == 4 ? neighbour_offset<2, 4>(k, axis)
-                                                                 : neighbour_offset<2, 8>(k, axis))
-                                            : (r.a.g.n_off == 6    ? neighbour_offset<3, 6>(k, axis)
-                                               : r.a.g.n_off == 18 ? neighbour_offset<3, 18>(k, axis)
-                                                                   : neighbour_offset<3, 26>(k, axis));
-            if (r.a.g.off[k][axis] != want) return cudaErrorInvalidValue;
-        }
-    return r.a.uniform_type >= 0 && r.a.uniform_contact_exact ? resident_any<true>(r, stream)
-                                                              : resident_any<false>(r, stream);
-}
-
 // ---------------------------------------------------------------- the cluster sweep
 //
-// A small plane of a model the resident sweep takes runs every MCS of a call
-// in ONE thread-block cluster: the lattice split by rows over the cluster's
-// CTAs and held in their shared memory, the tallies dealt by label (label l
-// in CTA l mod C), every read or atomic on another CTA's part through
-// distributed shared memory, and the cluster's hardware barrier between
-// passes. The copies, draws and tally rotation are the resident sweep's;
-// the lattice and tallies go back to global memory at the end.
+// A small plane of a lean model with nothing between its colour passes (no
+// fields, division, death or infection) runs every MCS of a call in ONE
+// thread-block cluster, its lattice and tallies in the CTAs' shared memory:
+//   - The lattice is split by rows over the CTAs, an even number of rows
+//     each, with a copy of the row either side. A copy committed to a CTA's
+//     first or last row is also written to the neighbour's copy of it, so
+//     every label a pass reads is in the CTA's own shared memory.
+//   - The tallies are dealt by label (label l in CTA l mod C), read and
+//     changed through distributed shared memory. Cell types are held whole by
+//     every CTA.
+//   - Each thread's targets are the same sites of every pass but for the
+//     colour's offset, and the next pass's picks are drawn between the
+//     cluster barrier's arrive and its wait, so a pass starts at its label
+//     reads. The unlike targets go into the CTA's queue with their labels,
+//     and whole warps price it.
+// The copies, draws and tally rotation are the direct sweep's; the lattice
+// and tallies go back to global memory at the end. What bounds a pass is its
+// chain: labels, queue, the two cells' tallies across the cluster, pricing,
+// the commits' atomics, the barrier (1.5 us a pass at 128^2; 2.4 when every
+// label was read through a table of row pointers into the CTAs, the picks
+// were drawn at the pass's start and a target's coordinates divided out).
 
-constexpr int kClusterThreads = 1024;
-#ifndef GLZ_CLUSTER_MAX
-#define GLZ_CLUSTER_MAX 16
-#endif
-constexpr int kClusterMax = GLZ_CLUSTER_MAX;  // CTAs of a cluster at most (16 is the non-portable limit)
-// A plane takes a cluster of at least kClusterMin CTAs (fewer only when it
-// has fewer rows), more while a CTA would hold more targets than threads:
-// a pass's work per CTA is what bounds it, so spreading a 128^2 plane over
-// 8 SMs rather than 4 cuts its 100 MCS from 1.17 to 0.99 ms.
-#ifndef GLZ_CLUSTER_MIN
-#define GLZ_CLUSTER_MIN 8
-#endif
-constexpr int kClusterMin = GLZ_CLUSTER_MIN;  // a power of two
+constexpr int kClusterThreads = 1024;  // a CTA's threads at most
+constexpr int kClusterMost = 16;       // CTAs of a cluster at most (16 is the non-portable limit)
 constexpr int kClusterSmem = 200 * 1024;
-#ifndef GLZ_CLUSTER_PER_THREAD
-#define GLZ_CLUSTER_PER_THREAD 1
-#endif
-constexpr int kClusterPerThread = GLZ_CLUSTER_PER_THREAD;  // a pass's targets a thread draws at most
+constexpr int kClusterPerThread = 4;  // a thread's targets a pass at most
 
 // Shared-memory layout of one CTA of a C-CTA cluster sweep (bytes from the
-// start): delta[3][Lc] (i64), base[2][Lc] (int2), the pointer tables
-// (delta 3C, base 2C, volc C), rows[H], slab[R W] (u32), volc[Lc][4] (i32),
-// the pass's queue of unlike copies (target index, pick) with room for every
-// target of the CTA's rows, and the queue's two fill counters.
+// start): delta[3][Lc] (i64), base[2][Lc] (int2), the queue (uint4 each),
+// slab[R + 2][W] (u32), volc[Lc][4] (i32), the types, the queue's two fill
+// counters.
 struct ClusterLayout {
     int C, R, Lc, qcap;
-    size_t delta, base, dptr, bptr, vptr, rows, slab, volc, queue, picks, qn, bytes;
+    size_t delta, base, queue, slab, volc, types, qn, bytes;
     __host__ __device__ ClusterLayout(int w, int h, int n_labels, int c) : C(c) {
-        R = (h + c - 1) / c;
+        R = 2 * ((h / 2 + c - 1) / c);
         Lc = (n_labels + c - 1) / c;
-        qcap = (R + 1) / 2 * (w / 2);
+        qcap = R / 2 * (w / 2);
         delta = 0;
         base = delta + 3 * (size_t)Lc * 8;
-        dptr = base + 2 * (size_t)Lc * 8;
-        bptr = dptr + 3 * (size_t)c * 8;
-        vptr = bptr + 2 * (size_t)c * 8;
-        rows = vptr + (size_t)c * 8;
-        slab = rows + (size_t)h * 8;
-        volc = slab + ((size_t)R * w * 4 + 15) / 16 * 16;
-        queue = volc + (size_t)Lc * 16;
-        picks = queue + (size_t)qcap * 4;
-        qn = picks + ((size_t)qcap + 15) / 16 * 16;
+        queue = (base + 2 * (size_t)Lc * 8 + 15) / 16 * 16;
+        slab = queue + (size_t)qcap * 16;
+        volc = slab + ((size_t)(R + 2) * w * 4 + 15) / 16 * 16;
+        types = volc + (size_t)Lc * 16;
+        qn = types + ((size_t)n_labels + 15) / 16 * 16;
         bytes = qn + 16;
     }
 };
 
-// Labels and tallies of a cluster pass: `rows[y]` is row y in whichever CTA
-// holds it; a label's tallies sit in CTA l & mask at index l >> shift.
+// The address of a CTA's own shared memory as it appears in CTA `rank` of the
+// cluster, and the reads and changes that take such an address.
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t own, int rank) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(own), "r"(rank));
+    return a;
+}
+
+__device__ __forceinline__ int2 cluster_ld_int2(uint32_t a) {
+    int2 v;
+    asm volatile("ld.shared::cluster.v2.s32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
+    return v;
+}
+
+__device__ __forceinline__ long long cluster_ld_i64(uint32_t a) {
+    long long v;
+    asm volatile("ld.shared::cluster.s64 %0, [%1];" : "=l"(v) : "r"(a));
+    return v;
+}
+
+__device__ __forceinline__ int cluster_ld_int(uint32_t a) {
+    int v;
+    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+
+__device__ __forceinline__ void cluster_st(uint32_t a, uint32_t v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+
+__device__ __forceinline__ void cluster_add(uint32_t a, unsigned long long v) {
+    asm volatile("red.relaxed.cluster.shared::cluster.add.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+}
+
+__device__ __forceinline__ void cluster_add(uint32_t a, int v) {
+    asm volatile("red.relaxed.cluster.shared::cluster.add.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
+// Labels and tallies of a cluster pass. `row` is the target's row of the
+// slab, set per copy.
 struct ClusterPass {
-    uint32_t *const *rows;
-    int2 *const *bptr;         // [slot * C + rank]
-    long long *const *dptr;    // [slot * C + rank]
-    int *const *vptr;          // [rank]
-    int C, shift, mask, colour, bslot, pslot, cslot;
-    __device__ __forceinline__ uint32_t label(int x, int y, int) const { return rows[y][x]; }
-    __device__ __forceinline__ int2 base(uint32_t l) const { return bptr[bslot * C + (l & mask)][l >> shift]; }
-    __device__ __forceinline__ long long prev(uint32_t l) const { return dptr[pslot * C + (l & mask)][l >> shift]; }
+    uint32_t base_at, prev_at, cur_at, volc_at;  // this pass's slots in the CTA's own shared memory
+    const uint8_t *types;
+    int shift, mask, colour;
+    uint32_t *slab_row;         // the target's row in the slab
+    uint32_t halo_up, halo_dn;  // the neighbours' copies of the CTA's first and last row
+    bool first, last;           // the target's row is the CTA's first, last
+    __device__ __forceinline__ int type(uint32_t l) const { return types[l]; }
+    __device__ __forceinline__ int2 base(uint32_t l) const {
+        return cluster_ld_int2(cluster_addr(base_at + (l >> shift) * 8, (int)(l & mask)));
+    }
+    __device__ __forceinline__ long long prev(uint32_t l) const {
+        return cluster_ld_i64(cluster_addr(prev_at + (l >> shift) * 8, (int)(l & mask)));
+    }
     __device__ __forceinline__ bool keeps_other_colour(uint32_t old) const {
-        const int *v = vptr[old & mask] + (size_t)(old >> shift) * 4;
+        const uint32_t v = cluster_addr(volc_at + (old >> shift) * 16, (int)(old & mask));
         int other = 0;
         for (int c = 0; c < 4; ++c)
-            if (c != colour) other += v[c];
+            if (c != colour) other += cluster_ld_int(v + 4 * c);
         return other != 0;
     }
-    __device__ __forceinline__ void put(uint32_t, int x, int y, int, uint32_t nw) const { rows[y][x] = nw; }
+    __device__ __forceinline__ void put(uint32_t, int x, int, int, uint32_t nw) const {
+        slab_row[x] = nw;
+        if (first) cluster_st(halo_up + 4 * x, nw);
+        if (last) cluster_st(halo_dn + 4 * x, nw);
+    }
     __device__ __forceinline__ void tally(uint32_t l, int dv, int ds) const {
-        atomicAdd(reinterpret_cast<unsigned long long *>(&dptr[cslot * C + (l & mask)][l >> shift]),
-                  pack_delta(dv, ds));
-        atomicAdd(&vptr[l & mask][(size_t)(l >> shift) * 4 + colour], dv);
+        cluster_add(cluster_addr(cur_at + (l >> shift) * 8, (int)(l & mask)), pack_delta(dv, ds));
+        cluster_add(cluster_addr(volc_at + (l >> shift) * 16 + 4 * colour, (int)(l & mask)), dv);
     }
 };
 
-template <int NOFF, bool UNIFORM>
+// A target's energy neighbours in the slab: its row and the rows either side.
+template <int NOFF>
+struct SlabLabels {
+    const uint32_t *row;
+    int W, x, xm, xp;
+    __device__ __forceinline__ uint32_t operator()(int k) const {
+        const int dx = neighbour_offset<2, NOFF>(k, 0), dy = neighbour_offset<2, NOFF>(k, 1);
+        return row[dy * W + (dx < 0 ? xm : (dx > 0 ? xp : x))];
+    }
+    __device__ __forceinline__ uint32_t ring(int) const { return 0; }
+};
+
+template <int NOFF, bool UNIFORM, int TPT>
 __global__ void __launch_bounds__(kClusterThreads, 1) cluster_sweep_kernel(const __grid_constant__ ResidentLaunch r) {
-    namespace cg = cooperative_groups;
-    cg::cluster_group cluster = cg::this_cluster();
     const SweepLaunch &a = r.a;
-    const int C = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
-    const int W = a.g.w, H = a.g.h, n_labels = a.n_labels;
+    int C, rank;
+    asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(C));
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const int W = a.g.w, H = a.g.h, n_labels = a.n_labels, hw = W / 2;
     const ClusterLayout L(W, H, n_labels, C);
-    const int tid = threadIdx.x, nth = blockDim.x;
+    const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31;
+    __shared__ TypeSmem<false> tables;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     long long *delta = reinterpret_cast<long long *>(smem_raw + L.delta);
     int2 *base = reinterpret_cast<int2 *>(smem_raw + L.base);
-    long long **dptr = reinterpret_cast<long long **>(smem_raw + L.dptr);
-    int2 **bptr = reinterpret_cast<int2 **>(smem_raw + L.bptr);
-    int **vptr = reinterpret_cast<int **>(smem_raw + L.vptr);
-    uint32_t **rows = reinterpret_cast<uint32_t **>(smem_raw + L.rows);
-    uint32_t *slab = reinterpret_cast<uint32_t *>(smem_raw + L.slab);
+    uint4 *queue = reinterpret_cast<uint4 *>(smem_raw + L.queue);
+    uint32_t *slab = reinterpret_cast<uint32_t *>(smem_raw + L.slab);  // row y0 - 1 first
     int *volc = reinterpret_cast<int *>(smem_raw + L.volc);
-    int *queue = reinterpret_cast<int *>(smem_raw + L.queue);
-    uint8_t *picks = reinterpret_cast<uint8_t *>(smem_raw + L.picks);
+    uint8_t *types = smem_raw + L.types;
     int *qn = reinterpret_cast<int *>(smem_raw + L.qn);
-    const int y0 = rank * L.R, y1 = min(H, y0 + L.R);
-    const int lane = tid & 31;
+    const TypeTables T = UNIFORM ? a.t : load_types<false>(a, tables);
+    const int y0 = min(H, rank * L.R), y1 = min(H, y0 + L.R), rows = y1 - y0;
     if (tid < 2) qn[tid] = 0;
 
-    // this CTA's rows and labels, and where every CTA's parts lie
-    for (int i = tid; i < (y1 - y0) * W; i += nth) slab[i] = a.labels[(size_t)y0 * W + i];
+    // this CTA's rows and the two about them, its labels' tallies, the types
+    if (rows > 0)
+        for (int i = tid; i < (rows + 2) * W; i += nth) {
+            const int k = i / W, y = y0 - 1 + k;
+            slab[i] = a.labels[(size_t)(y < 0 ? H - 1 : (y >= H ? y - H : y)) * W + (i - k * W)];
+        }
     for (int i = tid; i < L.Lc; i += nth) {
         const int l = i * C + rank;
         const bool in = l < n_labels;
@@ -1122,84 +1078,123 @@ __global__ void __launch_bounds__(kClusterThreads, 1) cluster_sweep_kernel(const
         for (int k = 0; k < 3; ++k) delta[k * L.Lc + i] = in ? r.vs_delta[k][l] : 0;
         for (int c = 0; c < 4; ++c) volc[i * 4 + c] = in ? a.vol_by_colour[(size_t)l * 4 + c] : 0;
     }
-    for (int y = tid; y < H; y += nth) {
-        const int o = y / L.R;
-        rows[y] = cluster.map_shared_rank(slab, o) + (size_t)(y - o * L.R) * W;
-    }
-    for (int i = tid; i < C; i += nth) {
-        for (int k = 0; k < 3; ++k) dptr[k * C + i] = cluster.map_shared_rank(delta + k * L.Lc, i);
-        for (int k = 0; k < 2; ++k) bptr[k * C + i] = cluster.map_shared_rank(base + k * L.Lc, i);
-        vptr[i] = cluster.map_shared_rank(volc, i);
-    }
-    cluster.sync();  // every CTA's part in place before any is read
+    if (!UNIFORM)
+        for (int i = tid; i < n_labels; i += nth) types[i] = a.cell_type[i];
+    // The CTA's first row is the row after the CTA before's last, its last
+    // row the one before the next's first.
+    const int filled = (H - 1) / L.R;  // the last CTA with rows
+    const int up = rank == 0 ? filled : rank - 1, dn = rank >= filled ? 0 : rank + 1;
+    const int up_rows = min(H, (up + 1) * L.R) - up * L.R;
+    ClusterPass acc;
+    acc.types = types;
+    acc.shift = __ffs(C) - 1;
+    acc.mask = C - 1;
+    acc.volc_at = smem_addr(volc);
+    acc.halo_up = cluster_addr(smem_addr(slab) + (uint32_t)((up_rows + 1) * W) * 4u, up);
+    acc.halo_dn = cluster_addr(smem_addr(slab), dn);
+    const uint32_t base_at = smem_addr(base), delta_at = smem_addr(delta);
 
-    const int hw = W / 2;
+    // this thread's targets, the same in every pass but for the colour's offset
+    const int count = rows / 2 * hw;
+    int tx[TPT], ty[TPT], pick[TPT];
+#pragma unroll
+    for (int k = 0; k < TPT; ++k) {
+        const int t = k * nth + tid, j = t / hw;
+        tx[k] = t < count ? 2 * (t - j * hw) : -1;
+        ty[k] = 2 * j;
+    }
+    const auto draw_picks = [&](uint64_t key, int c) {
+#pragma unroll
+        for (int k = 0; k < TPT; ++k)
+            if (tx[k] >= 0)
+                pick[k] = pick_of<NOFF>(
+                    draw(key, (uint32_t)((y0 + ty[k] + ((c >> 1) & 1)) * W + tx[k] + (c & 1))));
+    };
+    uint32_t step = (uint32_t)r.step0;
+    draw_picks(stream_key(r.seed, (int32_t)step, 0, 0), 0);
+    cluster_arrive();  // every CTA's part in place before any is read
+    cluster_wait();
+
+    int b = (int)(r.pass0 % 2), cur = (int)(r.pass0 % 3), parity = 0;
     for (int m = 0; m < r.mcs; ++m) {
-        const int32_t step = (int32_t)((uint32_t)r.step0 + (uint32_t)m);
         for (int c = 0; c < 4; ++c) {
-            const long long p = r.pass0 + (long long)m * 4 + c;
-            const ClusterPass acc{rows, bptr, dptr, vptr, C, __ffs(C) - 1, C - 1, c,
-                                  (int)(p % 2), (int)((p + 2) % 3), (int)(p % 3)};
-            const uint64_t key_pick = stream_key(r.seed, step, c, 0), key_accept = stream_key(r.seed, step, c, 1);
-            // this CTA's targets of colour c: rows of its slab of the colour's
-            // parity. Every thread draws its targets' picks and compares the
-            // two labels; the unlike ones go into the CTA's queue (a warp's
-            // slots reserved at once), which whole warps then price from its
-            // front. A pass's copies read only its snapshot and other
-            // colours' labels and commit by atomics, so the queue's order
-            // changes nothing.
-            const int yf = y0 + ((y0 & 1) != ((c >> 1) & 1));
-            const int count = yf < y1 ? (y1 - yf + 1) / 2 * hw : 0;
-            int *fill = qn + (p & 1);
-            for (int t0 = 0; t0 < count; t0 += nth) {
-                const int t = t0 + tid;
-                bool unlike = false;
-                int pick = 0;
-                if (t < count) {
-                    const int y = yf + 2 * (t / hw), x = 2 * (t % hw) + (c & 1);
-                    pick = pick_of<NOFF>(draw(key_pick, (uint32_t)(y * W + x)));
+            const int next = cur == 2 ? 0 : cur + 1, prev = cur == 0 ? 2 : cur - 1;
+            const int cx = c & 1, cy = (c >> 1) & 1;
+            acc.colour = c;
+            acc.base_at = base_at + (uint32_t)(b * L.Lc) * 8u;
+            acc.prev_at = delta_at + (uint32_t)(prev * L.Lc) * 8u;
+            acc.cur_at = delta_at + (uint32_t)(cur * L.Lc) * 8u;
+            const uint64_t key_accept = stream_key(r.seed, (int32_t)step, c, 1);
+            // Light step: the two labels of every target; the unlike go into
+            // the queue (a warp's slots reserved at once). A pass's copies
+            // read only its snapshot and other colours' labels and commit by
+            // atomics, so the queue's order changes nothing.
+            int *fill = qn + parity;
+            uint2 ln[TPT];
+            unsigned masks[TPT];
+            int mine = 0;
+#pragma unroll
+            for (int k = 0; k < TPT; ++k) {
+                ln[k] = make_uint2(0u, 0u);
+                if (tx[k] >= 0) {
                     int dx, dy, dz;
-                    pick_offset<2, NOFF>(pick, dx, dy, dz);
-                    const int nx = x + dx < 0 ? W - 1 : (x + dx >= W ? 0 : x + dx);
-                    const int ny = y + dy < 0 ? H - 1 : (y + dy >= H ? 0 : y + dy);
-                    unlike = acc.label(x, y, 0) != acc.label(nx, ny, 0);
+                    pick_offset<2, NOFF>(pick[k], dx, dy, dz);
+                    const int x = tx[k] + cx, sx = x + dx;
+                    const uint32_t *row = slab + (ty[k] + cy + 1) * W;
+                    ln[k] = make_uint2(row[x], row[dy * W + (sx < 0 ? W - 1 : (sx >= W ? 0 : sx))]);
                 }
-                const unsigned m = __ballot_sync(0xffffffffu, unlike);
-                int slot = 0;
-                if (lane == 0 && m) slot = atomicAdd(fill, __popc(m));
-                slot = __shfl_sync(0xffffffffu, slot, 0) + __popc(m & ((1u << lane) - 1u));
-                if (unlike) {
-                    queue[slot] = t;
-                    picks[slot] = (uint8_t)pick;
-                }
+            }
+#pragma unroll
+            for (int k = 0; k < TPT; ++k) {
+                masks[k] = __ballot_sync(0xffffffffu, ln[k].x != ln[k].y);
+                mine += __popc(masks[k]);
+            }
+            int slot = 0;
+            if (lane == 0 && mine) slot = atomicAdd(fill, mine);
+            slot = __shfl_sync(0xffffffffu, slot, 0);
+#pragma unroll
+            for (int k = 0; k < TPT; ++k) {
+                if (masks[k] & (1u << lane))
+                    queue[slot + __popc(masks[k] & ((1u << lane) - 1u))] =
+                        make_uint4((uint32_t)(tx[k] + cx), (uint32_t)(ty[k] + cy) | ((uint32_t)pick[k] << 28), ln[k].x,
+                                   ln[k].y);
+                slot += __popc(masks[k]);
             }
             __syncthreads();
             const int total = *fill;
-            if (tid == 0) qn[(p + 1) & 1] = 0;  // the next pass's counter; no thread reads it before the cluster barrier
-            for (int e = tid; e < total; e += nth) {
-                const int t = queue[e];
-                const int y = yf + 2 * (t / hw), x = 2 * (t % hw) + (c & 1);
-                const int pick = picks[e];
-                const NeighbourReads<2, NOFF, ClusterPass> ln(a, acc, x, y, 0);
-                direct_copy<2, NOFF, UNIFORM>(a, a.t, acc, ln, key_accept, x, y, 0, pick, acc.label(x, y, 0),
-                                              picked_label<2, NOFF>(a, acc, x, y, 0, pick));
-            }
-            // this CTA's labels' rotation for the next pass, which no thread of this one reads
-            int2 *next_base = base + ((p + 1) % 2) * L.Lc;
-            long long *clear = delta + ((p + 1) % 3) * L.Lc;
-            for (int i = tid; i < L.Lc; i += nth) {
+            if (tid == 0) qn[parity ^ 1] = 0;  // the next pass's counter; no thread reads it before the cluster barrier
+            // this CTA's labels' rotation for the next pass, which no thread
+            // of this one reads, from the last thread back
+            for (int i = nth - 1 - tid; i < L.Lc; i += nth) {
                 int dv, ds;
-                unpack_delta(delta[acc.pslot * L.Lc + i], dv, ds);
-                const int2 b = base[acc.bslot * L.Lc + i];
-                next_base[i] = make_int2(b.x + dv, b.y + ds);
-                clear[i] = 0;
+                unpack_delta(delta[prev * L.Lc + i], dv, ds);
+                const int2 v = base[b * L.Lc + i];
+                base[(b ^ 1) * L.Lc + i] = make_int2(v.x + dv, v.y + ds);
+                delta[next * L.Lc + i] = 0;
             }
-            cluster.sync();
+            for (int e = tid; e < total; e += nth) {
+                const uint4 q = queue[e];
+                const int x = (int)q.x, row = (int)(q.y & 0xfffffffu);
+                acc.slab_row = slab + (row + 1) * W;
+                acc.first = row == 0;
+                acc.last = row == rows - 1;
+                const SlabLabels<NOFF> labels{acc.slab_row, W, x, x == 0 ? W - 1 : x - 1, x == W - 1 ? 0 : x + 1};
+                direct_copy<2, NOFF, UNIFORM>(a, T, acc, labels, key_accept, x, y0 + row, 0, (int)(q.y >> 28), q.z, q.w);
+            }
+            cluster_arrive();
+            // the next pass's picks while the others arrive
+            if (c == 3) ++step;
+            const int nc = (c + 1) & 3;
+            draw_picks(stream_key(r.seed, (int32_t)step, nc, 0), nc);
+            cluster_wait();
+            b ^= 1;
+            cur = next;
+            parity ^= 1;
         }
     }
 
     // back to global memory: this CTA's rows and labels
-    for (int i = tid; i < (y1 - y0) * W; i += nth) a.labels[(size_t)y0 * W + i] = slab[i];
+    for (int i = tid; i < rows * W; i += nth) a.labels[(size_t)y0 * W + i] = slab[W + i];
     for (int i = tid; i < L.Lc; i += nth) {
         const int l = i * C + rank;
         if (l >= n_labels) continue;
@@ -1209,52 +1204,69 @@ __global__ void __launch_bounds__(kClusterThreads, 1) cluster_sweep_kernel(const
     }
 }
 
-// Run `mcs` MCS of a small 2D lean model in one cluster; cudaErrorNotSupported
-// (nothing launched) when the plane or its labels do not fit one.
-template <int NOFF, bool UNIFORM>
-static cudaError_t launch_cluster(const ResidentLaunch &r, cudaStream_t stream) {
-    const SweepLaunch &a = r.a;
-    const long long targets = (long long)a.g.w * a.g.h / 4;
-    int want = kClusterMin;
-    while (want < kClusterMax && (long long)want * kClusterThreads < targets) want *= 2;
-    // past kClusterPerThread targets a thread the cooperative grid's wider
-    // spread is faster
-    if ((long long)want * kClusterThreads * kClusterPerThread < targets) return cudaErrorNotSupported;
-    auto kernel = cluster_sweep_kernel<NOFF, UNIFORM>;
-    static std::atomic<bool> ready{false};  // handles on other host threads may launch too
-    if (!ready.load(std::memory_order_acquire)) {
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterSmem) ||
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) {
-            cudaGetLastError();
-            return cudaErrorNotSupported;
-        }
-        ready.store(true, std::memory_order_release);
+// The widest cluster of `kernel` the device schedules with the most shared
+// memory and threads, or 0.
+template <class Kernel>
+static int widest_cluster(Kernel kernel) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterSmem) ||
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) {
+        cudaGetLastError();
+        return 0;
     }
-    // the widest cluster up to `want` CTAs that the device schedules and whose parts fit
-    for (int C = want; C >= 1; C /= 2) {
-        if (C > a.g.h) continue;
-        const ClusterLayout L(a.g.w, a.g.h, a.n_labels, C);
-        if (L.bytes > (size_t)kClusterSmem) break;
+    for (int c = kClusterMost; c >= 1; c /= 2) {
         cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(C);
+        cfg.gridDim = dim3(c);
         cfg.blockDim = dim3(kClusterThreads);
-        cfg.dynamicSmemBytes = L.bytes;
-        cfg.stream = stream;
+        cfg.dynamicSmemBytes = kClusterSmem;
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = C;
+        at[0].val.clusterDim.x = c;
         at[0].val.clusterDim.y = 1;
         at[0].val.clusterDim.z = 1;
         cfg.attrs = at;
         cfg.numAttrs = 1;
         int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters < 1) {
-            cudaGetLastError();
-            continue;
-        }
-        return cudaLaunchKernelEx(&cfg, kernel, r);
+        if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters >= 1) return c;
+        cudaGetLastError();
     }
-    return cudaErrorNotSupported;
+    return 0;
+}
+
+// Run `mcs` MCS of a small 2D lean model in one cluster; cudaErrorNotSupported
+// (nothing launched) when the plane or its labels do not fit one. A plane
+// takes the widest cluster (100 MCS at 128^2: 0.60 ms on 16 CTAs, 0.63 on 8,
+// 0.82 on 4), a thread one target while a CTA's targets are no more than its
+// threads can be.
+template <int NOFF, bool UNIFORM, int TPT>
+static cudaError_t launch_cluster(const ResidentLaunch &r, cudaStream_t stream) {
+    const SweepLaunch &a = r.a;
+    auto kernel = cluster_sweep_kernel<NOFF, UNIFORM, TPT>;
+    static std::atomic<int> widest{-1};  // handles on other host threads may launch too
+    int C = widest.load(std::memory_order_acquire);
+    if (C < 0) {
+        C = widest_cluster(kernel);
+        widest.store(C, std::memory_order_release);
+    }
+    while (C > 1 && C > a.g.h / 2) C /= 2;  // a CTA holds two rows at least
+    if (C < 1) return cudaErrorNotSupported;
+    const ClusterLayout L(a.g.w, a.g.h, a.n_labels, C);
+    if (L.bytes > (size_t)kClusterSmem) return cudaErrorNotSupported;
+    if (L.qcap > TPT * kClusterThreads)
+        return TPT < kClusterPerThread ? launch_cluster<NOFF, UNIFORM, kClusterPerThread>(r, stream)
+                                       : cudaErrorNotSupported;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(C);
+    cfg.blockDim = dim3(((L.qcap + TPT - 1) / TPT + 31) / 32 * 32);
+    cfg.dynamicSmemBytes = L.bytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = C;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, r);
 }
 
 cudaError_t launch_cluster_sweep(const ResidentLaunch &r, cudaStream_t stream) {
@@ -1266,8 +1278,8 @@ cudaError_t launch_cluster_sweep(const ResidentLaunch &r, cudaStream_t stream) {
             if (a.g.off[k][axis] != want) return cudaErrorInvalidValue;
         }
     const bool uniform = a.uniform_type >= 0 && a.uniform_contact_exact;
-    if (a.g.n_off == 4) return uniform ? launch_cluster<4, true>(r, stream) : launch_cluster<4, false>(r, stream);
-    if (a.g.n_off == 8) return uniform ? launch_cluster<8, true>(r, stream) : launch_cluster<8, false>(r, stream);
+    if (a.g.n_off == 4) return uniform ? launch_cluster<4, true, 1>(r, stream) : launch_cluster<4, false, 1>(r, stream);
+    if (a.g.n_off == 8) return uniform ? launch_cluster<8, true, 1>(r, stream) : launch_cluster<8, false, 1>(r, stream);
     return cudaErrorNotSupported;
 }
 
@@ -1911,7 +1923,7 @@ __global__ void __launch_bounds__(BX *BY) direct_ensemble_step_kernel(const __gr
         for (int t = (int)blockIdx.x; t < e.total_tiles; t += (int)gridDim.x)
             direct_ensemble_tile<NOFF, UNIFORM, BX, BY>(e, d, where, t, c, step, pass);
         ensemble_rotate(e, pass);
-        if (c + 1 < e.ncol && !resident_barrier(e.barrier, (unsigned)c)) {
+        if (c + 1 < e.ncol && !grid_barrier(e.barrier, (unsigned)c)) {
             if (threadIdx.x == 0) atomicExch(e.error_flag, 4);
             return;
         }

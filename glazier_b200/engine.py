@@ -158,7 +158,7 @@ class GpuSimulation:
     @property
     def sweep_kernel(self) -> str:
         """The sweep kernel the next step takes ("band", "lean", "direct",
-        "compact", "resident", "cluster" or "general")."""
+        "gathered", "compact", "cluster" or "general")."""
         return _lib.lib().glz_gpu_sweep_kernel(self._h).decode()
 
     def labels(self) -> np.ndarray:

@@ -6,6 +6,11 @@
 - Models of 16 and of 17 types, the most whose tables are held in shared
   memory and the least whose are read where they lie, with and without the
   terms past contact, volume and surface.
+- The lean models' default choice either side of each of its sizes: the
+  cluster up to (not with) 256^2 sites, in place up to one wave of blocks,
+  then gathered; planes of few rows, whose cluster has CTAs without rows or a
+  CTA that is its own neighbour; and a plane whose cluster threads take four
+  targets each.
 
 Every lattice, volume, surface, type and f32 field is the replay's, bit for
 bit.
@@ -86,3 +91,43 @@ def test_tables_in_shared_memory_and_past_it(device, kinds, every, monkeypatch):
     replay.step(12)
     _same(gpu, replay, 1 if every else 0)
     gpu.close()
+
+
+@pytest.mark.parametrize("w, h, d, kernel", [
+    (30, 2, 1, "cluster"), (18, 4, 1, "cluster"), (66, 34, 1, "cluster"), (130, 50, 1, "cluster"),
+    (254, 256, 1, "cluster"), (256, 256, 1, "direct"), (778, 778, 1, "direct"), (780, 780, 1, "gathered"),
+    (80, 80, 80, "direct"), (88, 88, 88, "gathered"),
+])
+@pytest.mark.parametrize("types", [1, 2])
+def test_the_lean_choice_either_side_of_each_size(device, w, h, d, kernel, types):
+    side = 8 if min(w, h) >= 16 else 2
+    gpu, replay = _lean(device, w, h, d, types, side)
+    assert gpu.sweep_kernel == kernel
+    _same(gpu, replay, 0)
+    gpu.close()
+
+
+@pytest.mark.parametrize("types", [1, 2])
+def test_a_cluster_of_four_targets_a_thread(device, types, monkeypatch):
+    monkeypatch.setenv("GLAZIER_SWEEP_RESIDENT", "1")
+    gpu, replay = _lean(device, 512, 260, 1, types, 8)
+    assert gpu.sweep_kernel == "cluster"
+    _same(gpu, replay, 0)
+    gpu.close()
+
+
+def _lean(device, w, h, d, types, side):
+    """The lean model of one or two types after 1 and then 4 MCS on both sides."""
+    vt = float(side**2 if d == 1 else side**3)
+    cell = dict(target_volume=vt, lambda_volume=1.0, target_surface=90.0, lambda_surface=0.05)
+    model = Model(width=w, height=h, depth=d, contact=[0.0, 16.0, 16.0, 16.0, 6.0, 10.25, 16.0, 10.25, 9.125],
+                  types=[CellType(), CellType(**cell), CellType(**cell)], temperature=10.0, neighbour_order=2, seed=5)
+    start = Start.tiled(model, side)
+    if types == 2:
+        start.set_cell_types(1 + np.arange(start.n_cells) % 2)
+    gpu = device.GpuSimulation.from_start(start)
+    replay = ReplayOracle.from_start(start)
+    for chunk in (1, 4):
+        gpu.step(chunk)
+        replay.step(chunk)
+    return gpu, replay
