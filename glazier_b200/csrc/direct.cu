@@ -22,7 +22,7 @@
 // Measured per MCS (the step graph, back to back), against the pass that read
 // its launch from shared memory and its tables where they lie, and launched
 // plainly: lean planes of four types 27.2 -> 16.2 us at 256^2 and 30.6 -> 18.9
-// at 512^2; the two-field tissue (length, chemotaxis) 55.5 -> 31.1 us at
+// at 512^2; the two-field tissue (length, chemotaxis; replayed) 55.5 -> 31.1 us at
 // 256^2, 62.1 -> 35.1 at 512^2 and 114.9 -> 62.7 at 1024^2. A pass of the
 // 256^2 plane is about 4 us, of which 0.8 is the graph's kernel-to-kernel
 // time and the rest the chain.
@@ -141,8 +141,7 @@ __global__ void __launch_bounds__(kBlockThreads, kDirectMinBlocks<EXTRAS>)
             direct_site<DIM>(a, a.colour, j, x, y, z);
             pick = pick_of<NOFF>(draw(v.key_pick, (uint32_t)((z * a.g.h + y) * a.g.w + x)));
         }
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        grid_wait();
         if (!(UNIFORM && !EXTRAS)) __syncthreads();  // the tables are in place
         if (j < targets) {
             if constexpr (DIM == 2) {
@@ -185,8 +184,7 @@ __global__ void __launch_bounds__(kBlockThreads, kDirectMinBlocks<EXTRAS>)
                 picked[k] = pick_of<NOFF>(draw(v.key_pick, (uint32_t)((tz[k] * a.g.h + ty[k]) * a.g.w + tx[k])));
             }
         }
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        grid_wait();
         unsigned masks[kBlockK];
         uint2 labels[kBlockK];
         int mine = 0;
@@ -231,8 +229,7 @@ __global__ void __launch_bounds__(kBlockThreads, kDirectMinBlocks<EXTRAS>)
     } else {
         __shared__ int queue[kBlockThreads / 32][32 * kWarpK];
         __shared__ uint8_t picks[kBlockThreads / 32][32 * kWarpK];
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        grid_wait();
         if (!(UNIFORM && !EXTRAS)) __syncthreads();  // the tables are in place
         const int first = (int)((blockIdx.x * (blockDim.x / 32) + warp) * 32 * kWarpK);
         int total = 0;

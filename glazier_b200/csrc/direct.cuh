@@ -10,6 +10,7 @@
 #include "device.cuh"
 #include "engine.h"
 #include "neighbours.cuh"
+#include "pdl.cuh"
 #include "pricing.cuh"
 #include "terms.cuh"
 
@@ -235,9 +236,6 @@ __device__ __forceinline__ void direct_target(const SweepLaunch &a, const TypeTa
         direct_copy<DIM, NOFF, UNIFORM, Access, NeighbourReads<DIM, NOFF, Access>, EXTRAS>(a, T, acc, ln, key_accept, x, y,
                                                                                            z, pick, old, nw, terms);
 }
-
-// Whether sweeps launch programmatically (GLAZIER_SWEEP_PDL=0: plainly).
-int programmatic_launch();
 
 // A direct pass (direct.cu) of the launch's neighbourhood and pricing form.
 template <int DIM, int NOFF, bool UNIFORM>

@@ -154,29 +154,20 @@ struct glz_gpu {
 
     // Population models keep the live label count on the device (divisions
     // add to it there). The host holds an upper bound of it for the work it
-    // has queued, and after each population step the count is copied into a
-    // pinned slot and marked by an event, so the bound tightens without
-    // waiting for the stream whenever a copy has landed.
-    static constexpr int kCountSlots = 4;
+    // has queued; every eighth step the device also writes the count into
+    // mapped host memory, so the bound tightens without a wait for the stream.
     int *n_live = nullptr;
-    int *n_seen = nullptr;  // pinned, kCountSlots entries
-    cudaEvent_t n_event[kCountSlots] = {};
-    uint64_t n_step[kCountSlots] = {};  // the population step each slot's copy follows
-    uint64_t pop_steps = 0;             // population steps queued
+    unsigned long long *seen = nullptr;  // (step << 32) | the count before that step's divisions
     size_t n_bound = 0;
     // The most cells one step can add: cells at or past their division
     // volume hold disjoint sites, so at most sites / (the least division
     // volume, and at least 4 sites, cpu.rs:681) of them divide.
     size_t born_most = 0;
 
-    // Steps of a direct-kernel engine replay from one captured graph: its
-    // kernels read the step, pass and field buffers from `clock`, so the
-    // same graph serves every step. GLAZIER_ENGINE_GRAPH=0 queues every
-    // launch from the host instead.
+    // The clock of a step captured into a graph (the batched ensemble's): its
+    // kernels read the step, pass and field buffers there, so the same graph
+    // serves every step.
     glz::EngineClock *clock = nullptr;
-    cudaGraphExec_t step_exec = nullptr;
-    bool graph_on = true;
-    uint64_t records_from = 0;  // count records older than this step predate graph replays
     uint64_t arrays_version = 0;  // bumped when the per-label arrays move (a captured step then is stale)
 
     // population scratch, `cap` entries each
@@ -184,7 +175,8 @@ struct glz_gpu {
     double *plan = nullptr;
     int *moved = nullptr;
     uint32_t *daughter = nullptr;
-    int *counters = nullptr;
+    int *first = nullptr;   // every model: a recount's first sites
+    int *flags = nullptr;   // two steps' event flags, then the count's ticket
 
     float *field_ptr(int s, int which) { return field_buf + ((size_t)2 * s + which) * (size_t)g.sites; }
 
@@ -251,11 +243,6 @@ void free_population(glz_gpu *h) {
     h->daughter = nullptr;
 }
 
-void drop_step_graph(glz_gpu *h) {
-    if (h->step_exec) cudaGraphExecDestroy(h->step_exec);
-    h->step_exec = nullptr;
-}
-
 // Per-label arrays sized for `cap` labels. The settled tallies, anchors,
 // per-colour volumes and cell types of the first n_labels entries carry over
 // exactly, so growing never changes a run; every delta word starts at zero.
@@ -315,22 +302,26 @@ int alloc_labels(glz_gpu *h, size_t cap) {
     h->cell_type = types;
     cudaFree(h->dose);
     h->dose = dose;
+    cudaFree(h->first);
+    h->first = nullptr;
+    if (int rc = dev_alloc(&h->first, cap)) return rc;
     h->cap = cap;
-    drop_step_graph(h);  // its kernels hold the old arrays
-    h->arrays_version += 1;
+    h->arrays_version += 1;  // a captured step holds the old arrays
     return GLZ_OK;
 }
 
-// Recount every tally from the lattice; with `when` (a device flag) only if
-// it is nonzero when the recount runs.
-int recount(glz_gpu *h, const int *when = nullptr) {
+// Recount every tally from the lattice. `ending`: as the end of a population
+// step, only if the step had an event; `clocked` for a captured step.
+int recount(glz_gpu *h, bool ending = false, bool clocked = false) {
     const uint64_t p = h->pass_no;
     glz::RecountLaunch r{};
     r.g = h->g;
     r.labels = h->labels;
     r.n_labels = (int)(h->n_live ? h->cap : h->n_labels);
     r.n_live = h->n_live;
-    r.when = when;
+    r.flags = ending ? h->flags : nullptr;
+    r.clock = clocked ? h->clock : nullptr;
+    r.step = (long long)h->mcs;
     r.vs_base = h->t.vs_base[p % 2];
     r.mom_base = h->t.mom_base[p % 2];
     for (int k = 0; k < 3; ++k) {
@@ -339,6 +330,7 @@ int recount(glz_gpu *h, const int *when = nullptr) {
     }
     r.vol_by_colour = h->t.vol_by_colour;
     r.anchor = h->t.anchor;
+    r.first = h->first;
     r.tracks = h->tracks;
     r.nematic = h->has_nematic ? h->nematic : nullptr;
     r.error_flag = h->error_flag;
@@ -465,33 +457,38 @@ int sweep_pass(glz_gpu *h, int colour) {
     return GLZ_OK;
 }
 
-int field_step(glz_gpu *h) {
+// The field rounds of a step; `clocked` for a captured step (the buffers from
+// the clock, the host's left as they are).
+int field_step(glz_gpu *h, bool clocked) {
     int rounds = 0;
     for (int s = 0; s < h->n_species; ++s) rounds = h->substeps[s] > rounds ? h->substeps[s] : rounds;
+    glz::FieldLaunch f{};
+    f.g = h->g;
+    f.n_types = h->n_types;
+    f.n_species = h->n_species;
+    f.labels = h->labels;
+    f.cell_type = h->cell_type;
+    f.secretion = h->sec;
+    f.uptake = h->upt;
+    f.infect_species = h->infect_species;
+    f.infect_from = h->infect_from;
+    f.dose = h->dose;
+    f.field_buf = h->field_buf;
+    for (int s = 0; s < h->n_species; ++s) f.field_cur |= (unsigned)(h->field_cur[s] & 1) << s;
+    f.clock = clocked ? h->clock : nullptr;
     for (int r = 0; r < rounds; ++r) {
-        glz::FieldLaunch f{};
-        f.g = h->g;
-        f.n_species = h->n_species;
         f.round = r;
-        f.labels = h->labels;
-        f.cell_type = h->cell_type;
-        f.secretion = h->sec;
-        f.uptake = h->upt;
-        f.infect_species = h->infect_species;
-        f.infect_from = h->infect_from;
-        f.dose = h->dose;
         for (int s = 0; s < h->n_species; ++s) {
             f.active[s] = r < h->substeps[s];
             f.last[s] = r == h->substeps[s] - 1;
             f.d[s] = h->fd[s];
             f.decay[s] = h->fdecay[s];
-            f.in[s] = h->field_ptr(s, h->field_cur[s]);
-            f.out[s] = h->field_ptr(s, 1 - h->field_cur[s]);
         }
         CU(glz::launch_field_round(f, h->stream));
-        for (int s = 0; s < h->n_species; ++s)
-            if (f.active[s]) h->field_cur[s] = 1 - h->field_cur[s];
     }
+    if (!clocked)
+        for (int s = 0; s < h->n_species; ++s)
+            if (h->substeps[s] & 1) h->field_cur[s] = 1 - h->field_cur[s];
     return GLZ_OK;
 }
 
@@ -511,25 +508,15 @@ size_t capacity_for(const glz_gpu *h, size_t n) {
 }
 
 // Keep room for the next step's divisions. The host's bound of the count
-// comes from the newest count copy that has landed (each step queued after
-// it adds at most its most divisions); only when that is not enough does the
-// host wait for the exact count, and grow when that is not.
+// follows the count the device last wrote (each step after it adds at most
+// its most divisions); only when that is not enough does the host wait for
+// the exact count, and grow when that is not.
 int ensure_capacity(glz_gpu *h) {
     if (after_step(h, h->n_bound) <= h->cap) return GLZ_OK;
-    for (int back = 0; back < glz_gpu::kCountSlots && (uint64_t)back < h->pop_steps; ++back) {
-        const int slot = (int)((h->pop_steps - 1 - (uint64_t)back) % glz_gpu::kCountSlots);
-        if (h->n_step[slot] < h->records_from) break;
-        const cudaError_t q = cudaEventQuery(h->n_event[slot]);
-        if (q == cudaErrorNotReady) {
-            cudaGetLastError();
-            continue;
-        }
-        CU(q);
-        size_t bound = (size_t)h->n_seen[slot];
-        for (uint64_t k = h->n_step[slot] + 1; k < h->pop_steps && bound <= h->cap; ++k) bound = after_step(h, bound);
-        if (bound < h->n_bound) h->n_bound = bound;
-        break;
-    }
+    const unsigned long long seen = *static_cast<volatile unsigned long long *>(h->seen);
+    size_t bound = (size_t)(uint32_t)seen;
+    for (uint32_t k = (uint32_t)h->mcs - (uint32_t)(seen >> 32); k > 0 && bound <= h->cap; --k) bound = after_step(h, bound);
+    if (bound < h->n_bound) h->n_bound = bound;
     if (after_step(h, h->n_bound) <= h->cap) return GLZ_OK;
     if (int rc = sync_count(h)) return rc;
     if (after_step(h, h->n_labels) <= h->cap) return GLZ_OK;
@@ -537,53 +524,47 @@ int ensure_capacity(glz_gpu *h) {
     return alloc_labels(h, capacity_for(h, h->n_labels));
 }
 
-// The population step's launches; `clocked` for a captured step (the settle
-// slots and the death draws' step from the clock).
-int population_launches(glz_gpu *h, bool clocked) {
-    if (clocked)
-        CU(glz::launch_settle_clocked(h->t, h->g.nm, (int)h->cap, h->tracks, h->n_live, h->clock, h->g.ncol,
-                                      h->stream));
-    else if (int rc = settle(h))
-        return rc;
-    // The pass count at the step's end has the parity of its start (ncol is
-    // even), so the base slot below is the same for every step of a graph.
-    const uint64_t p = h->pass_no;
+// The step's per-label end: the infection rule, division and death, and a
+// population model's recount; `clocked` for a captured step (the slots and
+// the death draws' step from the clock). At the end of the step's passes, the
+// step's number not yet counted.
+int step_labels(glz_gpu *h, bool clocked) {
+    if (!h->has_pop && h->infect_species < 0) return GLZ_OK;
+    const uint64_t p = h->pass_no;  // even before and after a step, so the base slot is the same
     glz::PopulationLaunch a{};
     a.g = h->g;
     a.t = h->tables();
     a.labels = h->labels;
-    a.cell_type_in = h->cell_type;
-    a.cell_type_out = h->cell_type;
+    a.cell_type = h->cell_type;
     a.n_labels = (int)h->n_labels;
     a.cap = (int)h->cap;
+    a.has_pop = h->has_pop;
+    a.tracks = h->tracks;
     a.n_live = h->n_live;
-    a.vs_base = h->t.vs_base[p % 2];
-    a.mom_base = h->t.mom_base[p % 2];
+    a.tal = h->t;
+    a.base_slot = (int)(p % 2);
+    a.vol_by_colour = h->t.vol_by_colour;
     a.anchor = h->t.anchor;
+    a.step = (long long)h->mcs;
+    a.pass = (long long)p;
     a.key_death = glz::stream_key(h->seed, (int32_t)h->mcs, glz::kPopulationStream, 0);
+    a.clock = clocked ? h->clock : nullptr;
+    a.seed = h->seed;
+    a.infect_from = h->infect_species >= 0 ? h->infect_from : -1;
+    a.infect_to = h->infect_to;
+    a.infect_threshold = h->infect_threshold;
+    a.dose = h->dose;
     a.mode = h->mode;
     a.plan = h->plan;
     a.moved = h->moved;
     a.daughter = h->daughter;
-    a.counters = h->counters;
-    a.clock = clocked ? h->clock : nullptr;
-    a.seed = h->seed;
-    // plan, count, decide (the count grows on the device), apply; a step
-    // without an event changes nothing and its recount returns at once
-    CU(glz::launch_population_plan(a, h->stream));
-    CU(glz::launch_population_apply(a, h->stream));
-    return recount(h, h->counters + 1);
-}
-
-int population(glz_gpu *h) {
-    if (int rc = ensure_capacity(h)) return rc;
-    if (int rc = population_launches(h, false)) return rc;
-    const int slot = (int)(h->pop_steps % glz_gpu::kCountSlots);
-    CU(cudaMemcpyAsync(&h->n_seen[slot], h->n_live, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    CU(cudaEventRecord(h->n_event[slot], h->stream));
-    h->n_step[slot] = h->pop_steps++;
-    h->n_bound = after_step(h, h->n_bound);
-    return GLZ_OK;
+    a.first = h->first;
+    a.flags = h->flags;
+    a.ticket = h->flags ? h->flags + 2 : nullptr;
+    a.seen = h->seen;
+    a.seen_step = !clocked && h->mcs % 8 == 0 ? (long long)(h->mcs & 0xffffffffu) : -1;
+    CU(glz::launch_step_labels(a, h->stream));
+    return h->has_pop ? recount(h, true, clocked) : GLZ_OK;
 }
 
 int check_error_flag(glz_gpu *h) {
@@ -623,8 +604,8 @@ int run_cluster(glz_gpu *h, uint64_t steps, bool *done) {
 }
 
 // One step with clocked launches, for capture: the direct passes (and the
-// motility copies), the activity decay, the field rounds, the infection rule,
-// the population step, then the clock's advance. Host state is left as it is.
+// motility copies), the activity decay, the field rounds, the per-label end,
+// then the clock's advance. Host state is left as it is.
 int queue_clocked_step(glz_gpu *h) {
     for (int c = 0; c < h->g.ncol; ++c) {
         glz::SweepLaunch a = pass_launch(h, c);
@@ -635,35 +616,8 @@ int queue_clocked_step(glz_gpu *h) {
         if (h->has_motility) CU(glz::launch_apply_copies(a, h->activity, h->stream));
     }
     if (h->has_motility) CU(glz::launch_activity_decay(h->activity, h->g.sites, h->stream));
-    int rounds = 0;
-    for (int s = 0; s < h->n_species; ++s) rounds = h->substeps[s] > rounds ? h->substeps[s] : rounds;
-    for (int r = 0; r < rounds; ++r) {
-        glz::FieldLaunch f{};
-        f.g = h->g;
-        f.n_species = h->n_species;
-        f.round = r;
-        f.labels = h->labels;
-        f.cell_type = h->cell_type;
-        f.secretion = h->sec;
-        f.uptake = h->upt;
-        f.infect_species = h->infect_species;
-        f.infect_from = h->infect_from;
-        f.dose = h->dose;
-        f.clock = h->clock;
-        f.field_buf = h->field_buf;
-        for (int s = 0; s < h->n_species; ++s) {
-            f.active[s] = r < h->substeps[s];
-            f.last[s] = r == h->substeps[s] - 1;
-            f.d[s] = h->fd[s];
-            f.decay[s] = h->fdecay[s];
-        }
-        CU(glz::launch_field_round(f, h->stream));
-    }
-    if (h->infect_species >= 0)
-        CU(glz::launch_infection(h->cell_type, h->dose, (int)(h->n_live ? h->cap : h->n_labels), h->infect_from,
-                                 h->infect_to, h->infect_threshold, h->n_live, h->stream));
-    if (h->has_pop)
-        if (int rc = population_launches(h, true)) return rc;
+    if (int rc = field_step(h, true)) return rc;
+    if (int rc = step_labels(h, true)) return rc;
     CU(glz::launch_engine_clock_advance(h->clock, h->g.ncol, h->stream));
     return GLZ_OK;
 }
@@ -681,15 +635,6 @@ int capture_step_graph(glz_gpu *h, cudaGraph_t *out) {
     }
     if (e != cudaSuccess) return fail(GLZ_DRIVER, std::string("step capture: ") + cudaGetErrorString(e));
     *out = graph;
-    return GLZ_OK;
-}
-
-int capture_step(glz_gpu *h) {
-    cudaGraph_t graph = nullptr;
-    if (int rc = capture_step_graph(h, &graph)) return rc;
-    const cudaError_t ei = cudaGraphInstantiate(&h->step_exec, graph, 0);
-    cudaGraphDestroy(graph);
-    if (ei != cudaSuccess) return fail(GLZ_DRIVER, std::string("step graph: ") + cudaGetErrorString(ei));
     return GLZ_OK;
 }
 
@@ -711,25 +656,6 @@ void advance_host(glz_gpu *h) {
     for (int s = 0; s < h->n_species; ++s)
         if (h->substeps[s] & 1) h->field_cur[s] = 1 - h->field_cur[s];
     if (h->has_pop) h->n_bound = after_step(h, h->n_bound);
-}
-
-// Steps of a direct-kernel engine, one graph replay each. The clock starts
-// from the host's counters; the host keeps them in step with every replay,
-// and checks label room before each (a growth drops the graph, whose kernels
-// hold the old arrays, and the next replay captures it anew).
-int run_graph(glz_gpu *h, uint64_t steps) {
-    if (int rc = upload_clock(h)) return rc;
-    h->records_from = h->pop_steps;  // count records from before the replays say nothing of them
-    for (uint64_t r = 0; r < steps; ++r) {
-        if (h->has_pop)
-            if (int rc = ensure_capacity(h)) return rc;
-        if (!h->step_exec)
-            if (int rc = capture_step(h)) return rc;
-        CU(cudaGraphLaunch(h->step_exec, h->stream));
-        advance_host(h);
-    }
-    if (int rc = sync_count(h)) return rc;
-    return check_error_flag(h);  // waits for the stream
 }
 
 // The band sweep's step schedule: every MCS of the call in one launch when
@@ -778,12 +704,8 @@ int run_band(glz_gpu *h, uint64_t steps, double *ms) {
         h->mcs += chunk;
         if (ms && cudaEventRecord(ev[1], h->stream) != cudaSuccess) return done(fail(GLZ_DRIVER, "event record failed"));
         if (h->n_species > 0)
-            if (int rc = field_step(h)) return done(rc);
-        if (h->infect_species >= 0) {
-            const cudaError_t ei = glz::launch_infection(h->cell_type, h->dose, (int)(h->n_live ? h->cap : h->n_labels), h->infect_from,
-                                                         h->infect_to, h->infect_threshold, h->n_live, h->stream);
-            if (ei != cudaSuccess) return done(fail(GLZ_DRIVER, std::string("infection: ") + cudaGetErrorString(ei)));
-        }
+            if (int rc = field_step(h, false)) return done(rc);
+        if (int rc = step_labels(h, false)) return done(rc);
         if (ms) {
             if (cudaEventRecord(ev[2], h->stream) != cudaSuccess || cudaEventSynchronize(ev[2]) != cudaSuccess)
                 return done(fail(GLZ_DRIVER, "event record failed"));
@@ -802,13 +724,11 @@ int run_band(glz_gpu *h, uint64_t steps, double *ms) {
 
 int run_steps(glz_gpu *h, uint64_t steps, double *ms) {
     if (h->band) return run_band(h, steps, ms);
-    // A model with nothing between its passes is queued pass by pass: a pass
-    // takes the device longer than its launch takes the host, and passes
-    // launched programmatically on the stream follow one another closer than
-    // a graph's replays do (per MCS at 512^2, three types: 16.0 us queued,
-    // 18.9 replayed; 17.3 and 21.2 at 1024^2, one type).
-    const bool between = h->n_species > 0 || h->has_pop || h->infect_species >= 0;
-    if (!ms && h->graph_on && h->direct && between && steps > 0) return run_graph(h, steps);
+    // Steps are queued kernel by kernel: a pass takes the device longer than
+    // its launch takes the host, and kernels launched programmatically on the
+    // stream follow one another closer than a step graph's replays do (per
+    // MCS: lean planes of three types 16.0 us queued and 18.9 replayed at
+    // 512^2; of one type 17.3 and 21.2 at 1024^2).
     cudaEvent_t ev[6] = {};
     if (ms) {
         for (auto &e : ev) CU(cudaEventCreate(&e));
@@ -840,14 +760,11 @@ int run_steps(glz_gpu *h, uint64_t steps, double *ms) {
             if (e != cudaSuccess) rc = fail(GLZ_DRIVER, std::string("activity decay: ") + cudaGetErrorString(e));
         }
         if (ms) CU(cudaEventRecord(ev[1], h->stream));
-        if (rc == GLZ_OK && h->n_species > 0) rc = field_step(h);
-        if (rc == GLZ_OK && h->infect_species >= 0) {
-            const cudaError_t e = glz::launch_infection(h->cell_type, h->dose, (int)(h->n_live ? h->cap : h->n_labels), h->infect_from,
-                                                        h->infect_to, h->infect_threshold, h->n_live, h->stream);
-            if (e != cudaSuccess) rc = fail(GLZ_DRIVER, std::string("infection: ") + cudaGetErrorString(e));
-        }
+        if (rc == GLZ_OK && h->n_species > 0) rc = field_step(h, false);
         if (ms) CU(cudaEventRecord(ev[2], h->stream));
-        if (rc == GLZ_OK && h->has_pop) rc = population(h);
+        if (rc == GLZ_OK && h->has_pop) rc = ensure_capacity(h);
+        if (rc == GLZ_OK) rc = step_labels(h, false);
+        if (h->has_pop) h->n_bound = after_step(h, h->n_bound);
         if (ms) CU(cudaEventRecord(ev[3], h->stream));
         h->mcs += 1;
         if (ms && rc == GLZ_OK) {
@@ -871,11 +788,10 @@ int run_steps(glz_gpu *h, uint64_t steps, double *ms) {
 
 namespace glz {
 
-bool engine_replays(const glz_gpu *h) { return h->graph_on && h->direct && !h->cluster && !h->band; }
+bool engine_replays(const glz_gpu *h) { return h->direct && !h->cluster && !h->band; }
 
 int engine_begin_replays(glz_gpu *h) {
     if (int rc = upload_clock(h)) return rc;
-    h->records_from = h->pop_steps;
     CU(cudaStreamSynchronize(h->stream));
     return GLZ_OK;
 }
@@ -1125,12 +1041,10 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
     if (h->has_pop) {
         const int n = (int)n_labels;
         if ((rc = dev_alloc(&h->n_live, 1))) return bail(rc);
-        if (cudaMemcpy(h->n_live, &n, sizeof n, cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaHostAlloc((void **)&h->n_seen, glz_gpu::kCountSlots * sizeof(int), cudaHostAllocDefault) != cudaSuccess)
+        if (cudaMemcpyAsync(h->n_live, &n, sizeof n, cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+            cudaHostAlloc((void **)&h->seen, sizeof *h->seen, cudaHostAllocMapped) != cudaSuccess)
             return bail(fail(GLZ_DRIVER, "label count set-up failed"));
-        for (auto &e : h->n_event)
-            if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
-                return bail(fail(GLZ_DRIVER, "cannot create an event"));
+        *h->seen = n_labels;
         h->n_bound = n_labels;
     }
 
@@ -1162,10 +1076,10 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
     }
     if ((rc = dev_alloc(&h->error_flag, 1))) return bail(rc);
     if ((rc = dev_alloc(&h->clock, 1))) return bail(rc);
-    if (const char *graph_env = std::getenv("GLAZIER_ENGINE_GRAPH")) h->graph_on = graph_env[0] != '0';
     if ((rc = dev_alloc(&h->barrier, 2))) return bail(rc);
     if ((rc = dev_alloc(&h->medium, 2))) return bail(rc);
-    if ((rc = dev_alloc(&h->counters, 2))) return bail(rc);
+    if ((rc = dev_alloc(&h->flags, 3))) return bail(rc);
+    if (cudaMemsetAsync(h->flags, 0, 3 * sizeof(int), h->stream)) return bail(fail(GLZ_DRIVER, "memset failed"));
     if (cudaMemsetAsync(h->error_flag, 0, sizeof(int), h->stream)) return bail(fail(GLZ_DRIVER, "memset failed"));
 
     // The tensor copy needs rows that are a whole number of 16-byte units.
@@ -1330,13 +1244,12 @@ int glz_gpu_set_infection(glz_gpu *h, int species, int from_type, int to_type, d
     h->infect_threshold = std::llround(threshold * (double)glz::kDoseScale);
     // types now change during a run: the sweep reads them per copy
     h->uniform = -1;
-    drop_step_graph(h);  // its launches carry the rule and the uniform-type pricing
+    h->arrays_version += 1;  // a captured step carries the old rule and the uniform-type pricing
     return GLZ_OK;
 }
 
 int glz_gpu_set_nematic_field(glz_gpu *h, const double *field, size_t len) {
     if (!h) return fail(GLZ_INVALID, "null handle");
-    drop_step_graph(h);
     if (len != 2 * (size_t)h->g.sites) {
         char msg[128];
         std::snprintf(msg, sizeof msg, "nematic field has %zu sites, the lattice %d", len / 2, h->g.sites);
@@ -1357,7 +1270,6 @@ int glz_gpu_set_nematic_field(glz_gpu *h, const double *field, size_t len) {
 
 int glz_gpu_set_nematic_field_device(glz_gpu *h, const float *field, size_t len) {
     if (!h) return fail(GLZ_INVALID, "null handle");
-    drop_step_graph(h);
     if (len != 2 * (size_t)h->g.sites) {
         char msg[128];
         std::snprintf(msg, sizeof msg, "nematic field has %zu sites, the lattice %d", len / 2, h->g.sites);
@@ -1406,15 +1318,12 @@ void glz_gpu_destroy(glz_gpu *h) {
     cudaFree(h->types); cudaFree(h->sec); cudaFree(h->upt); cudaFree(h->divv); cudaFree(h->death);
     cudaFree(h->activity); cudaFree(h->pending); cudaFree(h->pending_count); cudaFree(h->nematic);
     cudaFree(h->labels); cudaFree(h->cell_type); cudaFree(h->field_buf); cudaFree(h->dose);
-    cudaFree(h->error_flag); cudaFree(h->medium); cudaFree(h->barrier); cudaFree(h->counters);
+    cudaFree(h->error_flag); cudaFree(h->medium); cudaFree(h->barrier); cudaFree(h->flags); cudaFree(h->first);
     free_tallies(h->t);
     free_population(h);
-    drop_step_graph(h);
     cudaFree(h->clock);
     cudaFree(h->n_live);
-    if (h->n_seen) cudaFreeHost(h->n_seen);
-    for (auto &e : h->n_event)
-        if (e) cudaEventDestroy(e);
+    if (h->seen) cudaFreeHost(h->seen);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
 }

@@ -254,10 +254,8 @@ int ensemble_grid_cap(int dim, int n_off, bool uniform);
 
 struct FieldLaunch {
     Geometry g;
-    int n_species;
+    int n_types, n_species;
     int round;
-    const float *in[kMaxSpecies];
-    float *out[kMaxSpecies];
     float d[kMaxSpecies], decay[kMaxSpecies];
     int active[kMaxSpecies], last[kMaxSpecies];
     const uint32_t *labels;
@@ -268,20 +266,15 @@ struct FieldLaunch {
     int infect_species = -1;  // -1: no rule
     int infect_from;
     unsigned long long *dose;
-    // Clocked: each species' buffers from the clock's current bit and the
-    // round (`in`, `out` unused), two per species in field_buf.
-    const EngineClock *clock = nullptr;
+    // Two buffers per species, species-major: a round reads the one that
+    // field_cur (or, clocked, the clock) and the round give, and writes the
+    // other. field_cur is as at the step's start in every round.
     float *field_buf = nullptr;
+    unsigned field_cur = 0;
+    const EngineClock *clock = nullptr;
 };
 
 cudaError_t launch_field_round(const FieldLaunch &a, cudaStream_t stream);
-
-// A cell of type `from` whose dose has reached `threshold` (units of 2^-24)
-// turns to type `to`.
-// With `n_live` (device memory) the count is read there and n_labels is the
-// capacity.
-cudaError_t launch_infection(uint8_t *cell_type, const unsigned long long *dose, int n_labels, int from, int to,
-                             long long threshold, const int *n_live, cudaStream_t stream);
 
 // Fixed-point scale of the infection dose: an uptake amount u adds
 // rint(u * 2^24), so the sum is exact and its order does not matter.
@@ -300,14 +293,20 @@ struct RecountLaunch {
     long long *mom_delta[3];
     int *vol_by_colour;
     int *anchor;
+    int *first;  // scratch per label: its first site in scan order
     int tracks;
     const float *nematic;  // with the nematic term: its sums follow the moments
     int *error_flag;  // set to 2 when a label is not below n_labels
     // Population models: the live count in device memory (n_labels is then
-    // the capacity), and a device flag the recount runs only when nonzero
-    // (the population step's event flag). Null: n_labels, and always.
+    // the capacity).
     const int *n_live;
-    const int *when;
+    // The recount at a population step's end: the two steps' event flags (it
+    // runs only when this step's, by the step's or the clock's parity, are
+    // nonzero; the step's own kernels have then cleared the tallies and found
+    // the first sites).
+    const int *flags;
+    const EngineClock *clock;
+    long long step;
 };
 
 cudaError_t launch_recount(const RecountLaunch &a, cudaStream_t stream);
@@ -317,10 +316,6 @@ cudaError_t launch_recount(const RecountLaunch &a, cudaStream_t stream);
 // capacity.
 cudaError_t launch_settle(int2 *vs_base, long long *vs_delta, long long *mom_base, long long *mom_delta, int nm,
                           int n_labels, int tracks, const int *n_live, cudaStream_t stream);
-// The same settle at the end of a clocked step: the slots follow from the
-// clock's pass count after the step's `ncol` passes.
-cudaError_t launch_settle_clocked(const Tallies &t, int nm, int n_labels, int tracks, const int *n_live,
-                                  const EngineClock *clock, int ncol, cudaStream_t stream);
 // Advance an engine's clock by one step of `ncol` passes.
 cudaError_t launch_engine_clock_advance(EngineClock *clock, int ncol, cudaStream_t stream);
 
@@ -333,24 +328,40 @@ struct PopulationLaunch {
     Geometry g;
     TypeTables t;
     uint32_t *labels;
-    const uint8_t *cell_type_in;
-    uint8_t *cell_type_out;  // may alias cell_type_in
-    int n_labels;            // unused: the count lives in n_live
+    uint8_t *cell_type;
+    int n_labels;            // without n_live
     int cap;
-    int *n_live;             // the live label count; decide adds the daughters to it
-    const int2 *vs_base;     // settled tallies
-    const long long *mom_base;
+    int has_pop, tracks;     // has_pop 0: the infection rule alone
+    int *n_live;             // the live label count; the decision adds the daughters to it
+    Tallies tal;
+    int base_slot;           // of the settled tallies (a step has an even number of passes: its start's)
+    int *vol_by_colour;
     const int *anchor;
     uint64_t key_death;      // stream_key(seed, step, kPopulationStream, 0)
-    const EngineClock *clock;  // clocked: the step (for the death draws) from here, with `seed`
+    long long step, pass;    // the step's number; the pass count at its end
+    const EngineClock *clock;  // clocked: step and pass from here, with `seed`
     uint64_t seed;
-    // scratch, n_labels entries each
+    // the infection rule (infect_from -1: none)
+    int infect_from, infect_to;
+    long long infect_threshold;
+    const unsigned long long *dose;
+    // scratch, cap entries each
     unsigned char *mode;
     double *plan;            // 6 per cell: centroid, axis
     int *moved;
     uint32_t *daughter;
-    int *counters;           // [0] daughters issued, [1] events (the recount's `when`)
+    int *first;
+    int *flags;              // two steps' event flags, by the step's parity
+    int *ticket;             // blocks done counting
+    // Where the host sees the count (mapped memory): (step << 32) | the count
+    // before that step's divisions, written when seen_step >= 0.
+    unsigned long long *seen;
+    long long seen_step;
 };
+
+__device__ __forceinline__ int population_parity(const PopulationLaunch &a) {
+    return (int)((a.clock ? a.clock->step : a.step) & 1);
+}
 
 // Record the message glz_last_error() returns on this thread.
 void set_last_error(const std::string &msg);
@@ -375,7 +386,8 @@ int engine_before_replay(glz_gpu *h, cudaStream_t replays, uint64_t *version);
 void engine_after_replay(glz_gpu *h);
 int engine_end_replays(glz_gpu *h);
 
-cudaError_t launch_population_plan(const PopulationLaunch &a, cudaStream_t stream);
-cudaError_t launch_population_apply(const PopulationLaunch &a, cudaStream_t stream);
+// A step's per-label end: the infection rule, division and death; a
+// population model's recount (launch_recount with `flags`) follows it.
+cudaError_t launch_step_labels(const PopulationLaunch &a, cudaStream_t stream);
 
 }  // namespace glz

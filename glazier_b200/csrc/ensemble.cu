@@ -128,6 +128,7 @@ struct glz_ens {
     long long *vs_delta[3] = {};
     int *volc = nullptr;
     int *anchor = nullptr;
+    int *first = nullptr;  // a recount's scratch
     float *tables = nullptr;  // per replica: contact, tv, lv, ts, ls
     uint8_t *connected = nullptr;
     glz::EnsembleReplica *d_reps = nullptr;
@@ -392,7 +393,7 @@ static int create_batched(int n, const glz_model *models, const uint32_t *const 
         (rc = dev_alloc(&h->vs_base[0], cells)) || (rc = dev_alloc(&h->vs_base[1], cells)) ||
         (rc = dev_alloc(&h->vs_delta[0], cells)) || (rc = dev_alloc(&h->vs_delta[1], cells)) ||
         (rc = dev_alloc(&h->vs_delta[2], cells)) || (rc = dev_alloc(&h->volc, cells * h->ncol)) ||
-        (rc = dev_alloc(&h->anchor, cells * 4)) || (rc = dev_alloc(&h->d_reps, (size_t)n)) ||
+        (rc = dev_alloc(&h->anchor, cells * 4)) || (rc = dev_alloc(&h->first, cells)) || (rc = dev_alloc(&h->d_reps, (size_t)n)) ||
         (rc = dev_alloc(&h->d_maps, (size_t)n)) || (rc = dev_alloc(&h->d_prefix, (size_t)n + 1)) ||
         (rc = dev_alloc(&h->d_order, (size_t)n)) || (rc = dev_alloc(&h->d_clock, 1)) ||
         (rc = dev_alloc(&h->d_barrier, 2)) ||
@@ -508,6 +509,7 @@ static int create_batched(int n, const glz_model *models, const uint32_t *const 
         for (int k = 0; k < 3; ++k) rl.vs_delta[k] = h->vs_delta[k] + rep.cell_off;
         rl.vol_by_colour = h->volc + rep.cell_off * h->ncol;
         rl.anchor = h->anchor + rep.cell_off * 4;
+        rl.first = h->first + rep.cell_off;
         rl.tracks = 0;
         rl.error_flag = h->error_flag;
         if (glz::launch_recount(rl, h->stream) != cudaSuccess) return bail(fail(GLZ_DRIVER, "recount failed"));
@@ -882,7 +884,7 @@ void glz_ens_destroy(glz_ens *h) {
     cudaFree(h->labels); cudaFree(h->cell_type);
     for (auto *p : h->vs_base) cudaFree(p);
     for (auto *p : h->vs_delta) cudaFree(p);
-    cudaFree(h->volc); cudaFree(h->anchor); cudaFree(h->tables); cudaFree(h->connected);
+    cudaFree(h->volc); cudaFree(h->first); cudaFree(h->anchor); cudaFree(h->tables); cudaFree(h->connected);
     cudaFree(h->d_reps); cudaFree(h->d_maps); cudaFree(h->d_prefix); cudaFree(h->d_order);
     cudaFree(h->d_clock); cudaFree(h->d_barrier); cudaFree(h->error_flag); cudaFree(h->medium);
     if (h->stream) cudaStreamDestroy(h->stream);

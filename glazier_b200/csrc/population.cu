@@ -1,54 +1,60 @@
-// Division and death, planned per cell on the device.
+// The per-label end of a Monte Carlo step: the infection rule's switches, and
+// division and death, planned per cell on the device.
 //
 // Replaces `run_population` (glazier-cuda/src/lib.rs:1362-1461) and its
 // kernels `cell_circular_sums`, `cell_moments` and `apply_population`
 // (lib.rs:66-142), which took five host round trips every Monte Carlo step.
-// Here every decision is made on the device from the exact moment sums:
-//   plan    per cell: a live cell at or past its division volume (and of at
-//           least four sites, cpu.rs:681) plans a cut through its centroid
-//           perpendicular to its major axis (power iteration on the
-//           covariance, moments.rs:165-186); any other live cell of a type
-//           with a death rate dies when its counter-hash draw falls under the
-//           rate (the reference's `else if`, lib.rs:1406-1423).
-//   count   per site: how many sites each planned cut would move.
-//   decide  one CTA, in label order: a cut that moves nothing or everything
-//           is no division (cpu.rs:697-703); the rest take daughter labels
-//           n_labels, n_labels + 1, ... in their mothers' order, a prefix sum
-//           over the compacted list of dividing cells. The live label count
-//           stays in device memory: decide reads it and adds the daughters,
-//           so no host read stands between steps.
-//   apply   per site: death to medium, the far side of a cut to the daughter.
-// The engine then recounts every tally from the lattice (cpu.rs:649-653),
-// a recount whose kernels return at once when decide found no event.
+// Here every decision is made on the device from the exact moment sums, in
+// four kernels, the last three of which return at once in a step that plans
+// no event:
+//   labels  per cell: the infection rule; the step's pending deltas folded
+//           into the tallies; then a live cell at or past its division volume
+//           (and of at least four sites, cpu.rs:681) plans a cut through its
+//           centroid perpendicular to its major axis (power iteration on the
+//           covariance, moments.rs:165-186), and any other live cell of a
+//           type with a death rate dies when its counter-hash draw falls
+//           under the rate (the reference's `else if`, lib.rs:1406-1423).
+//   count   per site: how many sites each planned cut would move. The last
+//           block to finish decides, in label order: a cut that moves nothing
+//           or everything is no division (cpu.rs:697-703); the rest take
+//           daughter labels n, n + 1, ... in their mothers' order. The live
+//           label count stays in device memory, so no host read stands
+//           between steps.
+//   apply   per site: death to medium, the far side of a cut to the daughter;
+//           every tally zeroed and each label's first site found.
+//   recount (tally.cu) the tallies from the lattice (cpu.rs:649-653).
+// On a small lattice these are chains of a few reads each, so their number is
+// what they cost: a whole run of the 256^2 infection model (200 MCS) takes
+// 11.3 ms with these and the four-site field kernel, 15 with eleven kernels.
 
 #include "device.cuh"
 #include "engine.h"
+#include "pdl.cuh"
+#include "tally.cuh"
+#include "terms.cuh"
 
 namespace glz {
 
+constexpr int kDeath = 1, kDivision = 2;  // a step's event flags
+
 __device__ __forceinline__ double along_cut(const Geometry &g, const int *anchor, const double *plan, uint32_t l,
-                                            size_t i) {
-    const int x = (int)(i % g.w), y = (int)((i / g.w) % g.h), z = (int)(i / ((size_t)g.w * g.h));
-    const int *an = &anchor[4 * (size_t)l];
-    const double ux = (double)fold_int(x - an[0], g.w);
-    const double uy = (double)fold_int(y - an[1], g.h);
-    const double uz = (double)fold_int(z - an[2], g.d);
+                                            uint32_t i) {
+    const uint32_t row = udiv(g.div_w, i), z = udiv(g.div_h, row), x = i - row * (uint32_t)g.w,
+                   y = row - z * (uint32_t)g.h;
+    const int4 an = *reinterpret_cast<const int4 *>(&anchor[4 * (size_t)l]);
+    const double ux = (double)fold_int((int)x - an.x, g.w);
+    const double uy = (double)fold_int((int)y - an.y, g.h);
+    const double uz = (double)fold_int((int)z - an.z, g.d);
     const double *p = &plan[6 * (size_t)l];
     return (ux - p[0]) * p[3] + (uy - p[1]) * p[4] + (uz - p[2]) * p[5];
 }
 
-__global__ void plan_kernel(const __grid_constant__ PopulationLaunch a) {
-    const int l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l >= *a.n_live) return;
-    a.moved[l] = 0;
-    a.mode[l] = 0;
-    if (l == 0) return;
-    const int v = a.vs_base[l].x;
-    if (v <= 0) return;
-    const int t = a.cell_type_in[l];
+// What cell l (of a population model) plans: 0 nothing, kDivision (its cut
+// into the plan table) or kDeath.
+__device__ __forceinline__ int plan_of(const PopulationLaunch &a, int l, int t, int v, const long long *m) {
     const double div_vol = a.t.division_volume[t];
+    if (v <= 0) return 0;
     if (div_vol > 0.0 && (double)v >= div_vol && v >= 4) {
-        const long long *m = &a.mom_base[(size_t)l * a.g.nm];
         const double dn = (double)v;
         double c[3][3], mean[3];
         if (a.g.dim == 2) {
@@ -97,102 +103,185 @@ __global__ void plan_kernel(const __grid_constant__ PopulationLaunch a) {
         p[3] = v0;
         p[4] = v1;
         p[5] = v2;
-        a.mode[l] = 1;
-    } else if (a.t.death_rate[t] > 0.0) {
+        return kDivision;
+    }
+    if (a.t.death_rate[t] > 0.0) {
         const uint64_t key =
             a.clock ? stream_key(a.seed, (int32_t)a.clock->step, kPopulationStream, 0) : a.key_death;
-        if (to_f64(draw(key, (uint32_t)l)) < a.t.death_rate[t]) a.mode[l] = 2;
+        if (to_f64(draw(key, (uint32_t)l)) < a.t.death_rate[t]) return kDeath;
+    }
+    return 0;
+}
+
+__global__ void __launch_bounds__(128) labels_kernel(const __grid_constant__ PopulationLaunch a) {
+    grid_wait();
+    const int l = blockIdx.x * blockDim.x + threadIdx.x;
+    const int n = a.n_live ? *a.n_live : a.n_labels;
+    if (a.has_pop && l == 0 && a.seen_step >= 0) *a.seen = ((unsigned long long)a.seen_step << 32) | (unsigned)n;
+    int event = 0;
+    if (l < n) {
+        int t = a.cell_type[l];
+        if (a.infect_from >= 0 && l > 0 && t == a.infect_from && (long long)a.dose[l] >= a.infect_threshold) {
+            t = a.infect_to;
+            a.cell_type[l] = (uint8_t)t;
+        }
+        if (a.has_pop) {
+            // the slots at the end of the step's passes
+            const long long p = a.clock ? a.clock->pass + a.g.ncol : a.pass;
+            int2 *const base = a.tal.vs_base[p % 2];
+            long long *const delta = a.tal.vs_delta[(p + 2) % 3];
+            int dv, ds;
+            unpack_delta(delta[l], dv, ds);
+            const int2 b = base[l];
+            base[l] = make_int2(b.x + dv, b.y + ds);
+            delta[l] = 0;
+            long long m[11];
+            if (a.tracks) {
+                long long *const mom = a.tal.mom_base[p % 2] + (size_t)l * a.g.nm;
+                long long *const mom_delta = a.tal.mom_delta[(p + 2) % 3] + (size_t)l * a.g.nm;
+#pragma unroll
+                for (int k = 0; k < 11; ++k)
+                    if (k < a.g.nm) m[k] = mom[k] + mom_delta[k];
+#pragma unroll
+                for (int k = 0; k < 11; ++k)
+                    if (k < a.g.nm) {
+                        mom[k] = m[k];
+                        mom_delta[k] = 0;
+                    }
+            }
+            if (l > 0) event = plan_of(a, l, t, b.x + dv, m);
+            a.mode[l] = (unsigned char)event;
+            a.moved[l] = 0;
+        }
+    }
+    if (a.has_pop) {
+        const int any = __reduce_or_sync(0xffffffffu, (unsigned)event);
+        if (any && (threadIdx.x & 31) == 0) atomicOr(&a.flags[population_parity(a)], any);
     }
 }
 
-__global__ void count_cut_kernel(const __grid_constant__ PopulationLaunch a) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)a.g.sites) return;
-    const uint32_t l = a.labels[i];
-    if (l == 0 || a.mode[l] != 1) return;
-    if (along_cut(a.g, a.anchor, a.plan, l, i) > 0.0) atomicAdd(&a.moved[l], 1);
-}
-
-// One CTA walks the labels in order and hands each kept division the next
-// daughter label: a block-wide prefix sum over the flags of each chunk.
-__global__ void __launch_bounds__(1024) decide_kernel(const __grid_constant__ PopulationLaunch a) {
+// Give each kept division the next daughter label, in label order, and add
+// the daughters to the live count; one block.
+__device__ void decide(const PopulationLaunch &a, int *flag) {
+    constexpr int kEach = 8;  // consecutive labels a thread takes
     __shared__ int warp_total[32];
-    __shared__ int running;
-    __shared__ int any_event;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int n_labels = *a.n_live;
-    if (tid == 0) {
-        running = 0;
-        any_event = 0;
-    }
-    __syncthreads();
-    for (int base = 0; base < n_labels; base += blockDim.x) {
-        const int l = base + tid;
-        int keep = 0;
-        if (l < n_labels && l > 0) {
-            const unsigned char m = a.mode[l];
-            if (m == 1) {
-                const int moved = a.moved[l];
-                if (moved > 0 && moved < a.vs_base[l].x)
-                    keep = 1;
-                else
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, warps = blockDim.x >> 5;
+    const int n = *a.n_live;
+    int running = 0, events = 0;
+    for (int base = 0; base < n; base += (int)blockDim.x * kEach) {
+        int keep = 0, mine = 0;
+#pragma unroll
+        for (int k = 0; k < kEach; ++k) {
+            const int l = base + tid * kEach + k;
+            const int m = l < n ? __ldcg(&a.mode[l]) : 0;
+            if (m == kDeath) events |= kDeath;
+            if (m == kDivision) {
+                const int moved = __ldcg(&a.moved[l]);
+                const int volume = a.tal.vs_base[a.base_slot][l].x;
+                if (moved > 0 && moved < volume) {
+                    keep |= 1 << k;
+                    ++mine;
+                } else {
                     a.mode[l] = 0;
+                }
             }
-            if (keep || m == 2) any_event = 1;
         }
-        const unsigned ballot = __ballot_sync(0xffffffffu, keep);
-        const int before_in_warp = __popc(ballot & ((1u << lane) - 1u));
-        if (lane == 0) warp_total[wid] = __popc(ballot);
+        int scan = mine;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, scan, o);
+            if (lane >= o) scan += up;
+        }
+        __syncthreads();  // the totals of the chunk before have been read
+        if (lane == 31) warp_total[wid] = scan;
         __syncthreads();
-        if (wid == 0) {
-            int v = lane < (int)(blockDim.x >> 5) ? warp_total[lane] : 0;
-            for (int o = 1; o < 32; o <<= 1) {
-                const int up = __shfl_up_sync(0xffffffffu, v, o);
-                if (lane >= o) v += up;
+        int before = running + scan - mine;
+        for (int w = 0; w < warps; ++w) {
+            before += w < wid ? warp_total[w] : 0;
+            running += warp_total[w];
+        }
+#pragma unroll
+        for (int k = 0; k < kEach; ++k)
+            if (keep >> k & 1) {
+                const int l = base + tid * kEach + k;
+                const uint32_t d = (uint32_t)(n + before++);
+                a.daughter[l] = d;
+                a.cell_type[d] = a.cell_type[l];
             }
-            warp_total[lane] = v;  // inclusive prefix over warps
-        }
-        __syncthreads();
-        const int warp_before = wid == 0 ? 0 : warp_total[wid - 1];
-        if (keep) {
-            const uint32_t d = (uint32_t)(n_labels + running + warp_before + before_in_warp);
-            a.daughter[l] = d;
-            a.cell_type_out[d] = a.cell_type_in[l];
-        }
-        __syncthreads();
-        if (tid == 0) running += warp_total[(blockDim.x >> 5) - 1];
-        __syncthreads();
     }
+    const int death = __syncthreads_or(events);
     if (tid == 0) {
-        a.counters[0] = running;
-        a.counters[1] = any_event;
-        *a.n_live = n_labels + running;  // every thread read the count before the first barrier
+        *flag = (death ? kDeath : 0) | (running ? kDivision : 0);
+        *a.n_live = n + running;
     }
 }
 
-__global__ void apply_kernel(const __grid_constant__ PopulationLaunch a) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)a.g.sites) return;
-    const uint32_t l = a.labels[i];
-    if (l == 0) return;
-    const unsigned char m = a.mode[l];
-    if (m == 2) {
-        a.labels[i] = 0;
-    } else if (m == 1) {
-        if (along_cut(a.g, a.anchor, a.plan, l, i) > 0.0) a.labels[i] = a.daughter[l];
+__global__ void __launch_bounds__(256) count_kernel(const __grid_constant__ PopulationLaunch a) {
+    __shared__ bool last;
+    grid_wait();
+    const int par = population_parity(a);
+    int *const flag = &a.flags[par];
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.flags[par ^ 1] = 0;  // the next step's, read by no kernel of this one
+    const int events = *flag;
+    if (!events) return;
+    const size_t stride = (size_t)gridDim.x * blockDim.x, first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    // each label's first site starts past them all (apply finds it)
+    for (size_t l = first; l < (size_t)a.cap; l += stride) a.first[l] = INT_MAX;
+    if (!(events & kDivision)) return;
+    for (size_t i = first; i < (size_t)a.g.sites; i += stride) {
+        const uint32_t l = a.labels[i];
+        if (l != 0 && a.mode[l] == kDivision && along_cut(a.g, a.anchor, a.plan, l, (uint32_t)i) > 0.0)
+            atomicAdd(&a.moved[l], 1);
     }
+    // the last block to arrive sees every other block's counts
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(a.ticket, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    decide(a, flag);
+    if (threadIdx.x == 0) *a.ticket = 0;
 }
 
-cudaError_t launch_population_plan(const PopulationLaunch &a, cudaStream_t stream) {
-    plan_kernel<<<(a.cap + 255) / 256, 256, 0, stream>>>(a);
-    count_cut_kernel<<<(a.g.sites + 255) / 256, 256, 0, stream>>>(a);
-    decide_kernel<<<1, 1024, 0, stream>>>(a);
-    return cudaGetLastError();
+__global__ void __launch_bounds__(256) apply_kernel(const __grid_constant__ PopulationLaunch a) {
+    grid_wait();
+    if (!a.flags[population_parity(a)]) return;
+    const size_t stride = (size_t)gridDim.x * blockDim.x, begin = (size_t)blockIdx.x * blockDim.x;
+    for (size_t base = begin; base < (size_t)a.g.sites; base += stride) {
+        const size_t i = base + threadIdx.x;
+        uint32_t l = i < (size_t)a.g.sites ? a.labels[i] : 0u;
+        if (l != 0) {
+            const unsigned char m = a.mode[l];
+            if (m == kDeath) {
+                a.labels[i] = l = 0;
+            } else if (m == kDivision && along_cut(a.g, a.anchor, a.plan, l, (uint32_t)i) > 0.0) {
+                a.labels[i] = l = a.daughter[l];
+            }
+        }
+        first_site(a.first, l, (int)i);
+    }
+    RecountLaunch r{};
+    r.g = a.g;
+    r.vs_base = a.tal.vs_base[a.base_slot];
+    r.mom_base = a.tal.mom_base[a.base_slot];
+    for (int k = 0; k < 3; ++k) {
+        r.vs_delta[k] = a.tal.vs_delta[k];
+        r.mom_delta[k] = a.tal.mom_delta[k];
+    }
+    r.vol_by_colour = a.vol_by_colour;
+    r.tracks = a.tracks;
+    for (size_t l = begin + threadIdx.x; l < (size_t)*a.n_live; l += stride) clear_tallies(r, (int)l);
 }
 
-cudaError_t launch_population_apply(const PopulationLaunch &a, cudaStream_t stream) {
-    apply_kernel<<<(a.g.sites + 255) / 256, 256, 0, stream>>>(a);
-    return cudaGetLastError();
+cudaError_t launch_step_labels(const PopulationLaunch &a, cudaStream_t stream) {
+    const int n = a.n_live ? a.cap : a.n_labels;
+    if (cudaError_t e = launch_after(labels_kernel, dim3((unsigned)((n + 127) / 128)), 128, stream, a)) return e;
+    if (!a.has_pop) return cudaSuccess;
+    // at most eight blocks an SM, so a step without an event starts few
+    const long long sites = ((long long)a.g.sites + 255) / 256;
+    const dim3 grid((unsigned)(sites < 1184 ? sites : 1184));
+    if (cudaError_t e = launch_after(count_kernel, grid, 256, stream, a)) return e;
+    return launch_after(apply_kernel, grid, 256, stream, a);
 }
 
 }  // namespace glz

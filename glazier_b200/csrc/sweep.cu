@@ -33,6 +33,7 @@
 #include "direct.cuh"
 #include "engine.h"
 #include "neighbours.cuh"
+#include "pdl.cuh"
 #include "pricing.cuh"
 #include "terms.cuh"
 
@@ -1383,8 +1384,7 @@ static cudaError_t launch_any(const SweepLaunch &a, cudaStream_t stream) {
 // The pass's listed copies; the other pass parity's count, which the copies
 // before these emptied, is set to zero for the next pass.
 __global__ void apply_copies_kernel(const __grid_constant__ SweepLaunch a, float *activity) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    grid_wait();
     const int count = *a.pending_count;
     if (blockIdx.x == 0 && threadIdx.x == 0) *a.pending_clear = 0;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
@@ -1397,33 +1397,16 @@ __global__ void apply_copies_kernel(const __grid_constant__ SweepLaunch a, float
     }
 }
 
-// A kernel launch that may start while the previous kernel on the stream
-// ends; the kernel waits (griddepcontrol.wait) before it reads pass data.
-template <class... Params, class... Args>
-static cudaError_t launch_after(void (*kernel)(Params...), int grid, cudaStream_t stream, Args... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(256);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = programmatic_launch();
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 cudaError_t launch_apply_copies(const SweepLaunch &a, float *activity, cudaStream_t stream) {
     // at most one copy per target, and a pass has sites / colours targets;
     // an accepted one is rare enough that a fraction of that grid covers them
     const int most = a.g.sites / a.g.ncol + 1;
     const int blocks = (most + 2047) / 2048;
-    return launch_after(apply_copies_kernel, blocks, stream, a, activity);
+    return launch_after(apply_copies_kernel, dim3((unsigned)blocks), 256, stream, a, activity);
 }
 
 __global__ void activity_decay_kernel(float *activity, int sites) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    grid_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= sites) return;
     const float v = activity[i];
@@ -1431,7 +1414,7 @@ __global__ void activity_decay_kernel(float *activity, int sites) {
 }
 
 cudaError_t launch_activity_decay(float *activity, int sites, cudaStream_t stream) {
-    return launch_after(activity_decay_kernel, (sites + 255) / 256, stream, activity, sites);
+    return launch_after(activity_decay_kernel, dim3((unsigned)((sites + 255) / 256)), 256, stream, activity, sites);
 }
 
 cudaError_t launch_sweep(const SweepLaunch &a, cudaStream_t stream) {

@@ -13,6 +13,8 @@
 #include "device.cuh"
 #include "engine.h"
 #include "neighbours.cuh"
+#include "pdl.cuh"
+#include "tally.cuh"
 
 namespace glz {
 
@@ -30,34 +32,54 @@ __device__ __forceinline__ void coords_of(const Geometry &g, size_t i, int &x, i
 // population model, else the launch's.
 __device__ __forceinline__ int recount_labels(const RecountLaunch &a) { return a.n_live ? *a.n_live : a.n_labels; }
 
-// Whether a conditional recount runs (the population step's event flag).
-__device__ __forceinline__ bool recount_runs(const RecountLaunch &a) { return !a.when || *a.when != 0; }
-
-// The tallies a recount rebuilds, zeroed for the live labels (a conditional
-// recount's stand-in for its memsets).
-__global__ void clear_tallies_kernel(const __grid_constant__ RecountLaunch a) {
-    if (!recount_runs(a)) return;
+__global__ void __launch_bounds__(256) clear_tallies_kernel(const __grid_constant__ RecountLaunch a) {
     const int l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l >= recount_labels(a)) return;
-    a.vs_base[l] = make_int2(0, 0);
-    for (int c = 0; c < a.g.ncol; ++c) a.vol_by_colour[(size_t)l * a.g.ncol + c] = 0;
-    for (int k = 0; k < 3; ++k) a.vs_delta[k][l] = 0;
-    if (a.tracks)
-        for (int j = 0; j < a.g.nm; ++j) {
-            a.mom_base[(size_t)l * a.g.nm + j] = 0;
-            for (int k = 0; k < 3; ++k) a.mom_delta[k][(size_t)l * a.g.nm + j] = 0;
-        }
+    clear_tallies(a, l);
+    a.first[l] = INT_MAX;
 }
 
-__global__ void fill_anchor_kernel(const __grid_constant__ RecountLaunch a) {
-    if (!recount_runs(a)) return;
-    int *anchor = a.anchor;
-    const int l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l >= recount_labels(a)) return;
-    anchor[4 * l + 0] = 0;
-    anchor[4 * l + 1] = 0;
-    anchor[4 * l + 2] = 0;
-    anchor[4 * l + 3] = INT_MAX;
+__global__ void __launch_bounds__(256) first_sites_kernel(const __grid_constant__ RecountLaunch a) {
+    grid_wait();
+    const uint32_t n_labels = (uint32_t)recount_labels(a);
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t l = i < (size_t)a.g.sites ? a.labels[i] : 0u;
+    if (l >= n_labels) l = 0u;  // recount_counts_kernel reports it
+    first_site(a.first, l, (int)i);
+}
+
+// Sum of (u0 + k)^2 for k = 0 .. n - 1.
+__device__ __forceinline__ long long squares_from(long long u0, long long n) {
+    return n * u0 * u0 + u0 * n * (n - 1) + (n - 1) * n * (2 * n - 1) / 6;
+}
+
+// A run of `len` sites of label l along x from (x, y, z), into its moment
+// words about its first site: the offsets along a run are consecutive unless
+// the run crosses the fold half a span away, so its sums are closed forms
+// and the run is one atomic a word, not one a site.
+template <int DIM>
+__device__ __forceinline__ void run_moments(const RecountLaunch &a, uint32_t l, int x, int y, int z, int len) {
+    const uint32_t f = (uint32_t)a.first[l];
+    const uint32_t row = udiv(a.g.div_w, f), pl = udiv(a.g.div_h, row);
+    const int ax = (int)(f - row * (uint32_t)a.g.w), ay = (int)(row - pl * (uint32_t)a.g.h), az = (int)pl;
+    const long long u0 = fold_int(x - ax, a.g.w), u1 = fold_int(x + len - 1 - ax, a.g.w);
+    const long long uy = fold_int(y - ay, a.g.h), uz = fold_int(z - az, a.g.d);
+    long long s1 = 0, s2 = 0;
+    if (u1 - u0 == len - 1) {
+        s1 = len * (u0 + u1) / 2;
+        s2 = squares_from(u0, len);
+    } else {
+        for (int k = 0; k < len; ++k) {
+            const long long u = fold_int(x + k - ax, a.g.w);
+            s1 += u;
+            s2 += u * u;
+        }
+    }
+    const long long words[9] = {s1,      len * uy, DIM == 2 ? s2 : len * uz, DIM == 2 ? len * uy * uy : s2,
+                                DIM == 2 ? s1 * uy : len * uy * uy, len * uz * uz, s1 * uy, s1 * uz, len * uy * uz};
+    unsigned long long *m = reinterpret_cast<unsigned long long *>(&a.mom_base[(size_t)l * a.g.nm]);
+#pragma unroll
+    for (int k = 0; k < (DIM == 2 ? 5 : 9); ++k) atomicAdd(&m[k], (unsigned long long)words[k]);
 }
 
 // Unlike-label neighbours of site i (label l) at (x, y, z), in 32-bit index
@@ -82,11 +104,12 @@ __device__ __forceinline__ int unlike_neighbours(const Geometry &g, const uint32
     return bonds;
 }
 
-// Volume, unlike-bond surface, per-colour volume and first site of every
-// label. Blocks run along lattice rows (x across threads, one row per block
+// Volume, unlike-bond surface, per-colour volume and moment sums of every
+// label, and its anchor (its first site). The medium has no tally (its counts
+// are medium_count_kernel's). Blocks run along lattice rows (x across threads, one row per block
 // row), so a warp holds 32 consecutive sites of one row and a cell usually
-// covers a run of lanes: each run adds its counts through its first lane
-// (whose site is also the run's first), one atomic per run, not per site.
+// covers a run of lanes: each run adds its counts through its first lane,
+// one atomic per run, not per site.
 // Along a row only x changes, so a run's sites alternate between two
 // colours, starting with its first lane's. A label that comes back later in
 // the warp starts another run. Neighbour addresses are the compile-time
@@ -94,7 +117,8 @@ __device__ __forceinline__ int unlike_neighbours(const Geometry &g, const uint32
 template <int DIM, int NOFF>
 __global__ void recount_counts_kernel(const __grid_constant__ RecountLaunch a) {
     constexpr uint32_t kNone = 0xffffffffu;
-    if (!recount_runs(a)) return;
+    grid_wait();
+    if (a.flags && !a.flags[(a.clock ? a.clock->step : a.step) & 1]) return;
     const uint32_t n_labels = (uint32_t)recount_labels(a);
     const int W = a.g.w, H = a.g.h, D = a.g.d;
     const int lane = threadIdx.x & 31;
@@ -109,6 +133,7 @@ __global__ void recount_counts_kernel(const __grid_constant__ RecountLaunch a) {
             l = kNone;
         }
         int bonds = 0;
+        if (l == 0) l = kNone;
         if (l != kNone) {
             const int ym = y == 0 ? H - 1 : y - 1, yp = y == H - 1 ? 0 : y + 1;
             const int zm = z == 0 ? D - 1 : z - 1, zp = z == D - 1 ? 0 : z + 1;
@@ -144,10 +169,18 @@ __global__ void recount_counts_kernel(const __grid_constant__ RecountLaunch a) {
             const int run_bonds = scan_last - scan + bonds;
             atomicAdd(&a.vs_base[l].x, len);
             if (run_bonds) atomicAdd(&a.vs_base[l].y, run_bonds);
-            atomicMin(&a.anchor[4 * (size_t)l + 3], (int)i);
+            if (a.first[l] == (int)i)
+                *reinterpret_cast<int4 *>(&a.anchor[4 * (size_t)l]) = make_int4(x, y, z, (int)i);
+            if (a.tracks) run_moments<DIM>(a, l, x, y, z, len);
             int *by_colour = &a.vol_by_colour[(size_t)l * a.g.ncol];
             atomicAdd(&by_colour[colour], (len + 1) / 2);
             if (len > 1) atomicAdd(&by_colour[colour ^ 1], len / 2);
+        }
+        if (a.nematic && l != kNone) {
+            constexpr int NM = DIM == 2 ? 5 : 9;
+            unsigned long long *m = reinterpret_cast<unsigned long long *>(&a.mom_base[(size_t)l * a.g.nm]);
+            atomicAdd(&m[NM], (unsigned long long)nematic_fixed(a.nematic[2 * (size_t)i]));
+            atomicAdd(&m[NM + 1], (unsigned long long)nematic_fixed(a.nematic[2 * (size_t)i + 1]));
         }
     }
 }
@@ -160,8 +193,7 @@ static cudaError_t launch_counts(const RecountLaunch &a, cudaStream_t stream) {
     const int bx = a.g.w >= 256 ? 256 : (a.g.w + 31) / 32 * 32;
     const int rows = a.g.h * a.g.d;
     const dim3 grid((unsigned)((a.g.w + bx - 1) / bx), (unsigned)(rows < 65535 ? rows : 65535));
-    recount_counts_kernel<DIM, NOFF><<<grid, bx, 0, stream>>>(a);
-    return cudaGetLastError();
+    return launch_after(recount_counts_kernel<DIM, NOFF>, grid, bx, stream, a);
 }
 
 static cudaError_t launch_counts_any(const RecountLaunch &a, cudaStream_t stream) {
@@ -176,79 +208,17 @@ static cudaError_t launch_counts_any(const RecountLaunch &a, cudaStream_t stream
     return cudaErrorInvalidValue;
 }
 
-__global__ void recount_anchor_kernel(const __grid_constant__ RecountLaunch a) {
-    if (!recount_runs(a)) return;
-    const int l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l >= recount_labels(a)) return;
-    const int first = a.anchor[4 * l + 3];
-    if (first == INT_MAX) return;
-    int x, y, z;
-    coords_of(a.g, (size_t)first, x, y, z);
-    a.anchor[4 * l + 0] = x;
-    a.anchor[4 * l + 1] = y;
-    a.anchor[4 * l + 2] = z;
-}
-
-__global__ void recount_moments_kernel(const __grid_constant__ RecountLaunch a) {
-    if (!recount_runs(a)) return;
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)a.g.sites) return;
-    const uint32_t l = a.labels[i];
-    if (l == 0 || l >= (uint32_t)recount_labels(a)) return;
-    int x, y, z;
-    coords_of(a.g, i, x, y, z);
-    const int *an = &a.anchor[4 * (size_t)l];
-    const long long ux = fold_int(x - an[0], a.g.w);
-    const long long uy = fold_int(y - an[1], a.g.h);
-    const long long uz = fold_int(z - an[2], a.g.d);
-    unsigned long long *m = reinterpret_cast<unsigned long long *>(&a.mom_base[(size_t)l * a.g.nm]);
-    if (a.g.dim == 2) {
-        atomicAdd(&m[0], (unsigned long long)ux);
-        atomicAdd(&m[1], (unsigned long long)uy);
-        atomicAdd(&m[2], (unsigned long long)(ux * ux));
-        atomicAdd(&m[3], (unsigned long long)(uy * uy));
-        atomicAdd(&m[4], (unsigned long long)(ux * uy));
-    } else {
-        atomicAdd(&m[0], (unsigned long long)ux);
-        atomicAdd(&m[1], (unsigned long long)uy);
-        atomicAdd(&m[2], (unsigned long long)uz);
-        atomicAdd(&m[3], (unsigned long long)(ux * ux));
-        atomicAdd(&m[4], (unsigned long long)(uy * uy));
-        atomicAdd(&m[5], (unsigned long long)(uz * uz));
-        atomicAdd(&m[6], (unsigned long long)(ux * uy));
-        atomicAdd(&m[7], (unsigned long long)(ux * uz));
-        atomicAdd(&m[8], (unsigned long long)(uy * uz));
-    }
-    if (a.nematic) {
-        const int g = a.g.dim == 2 ? 5 : 9;
-        atomicAdd(&m[g], (unsigned long long)nematic_fixed(a.nematic[2 * i]));
-        atomicAdd(&m[g + 1], (unsigned long long)nematic_fixed(a.nematic[2 * i + 1]));
-    }
-}
-
 cudaError_t launch_recount(const RecountLaunch &a, cudaStream_t stream) {
-    const size_t n = (size_t)a.n_labels;  // the count, or the capacity with n_live
-    const int lb = (int)((n + 255) / 256);
-    const int sb = (a.g.sites + 255) / 256;
-    if (a.n_live || a.when) {
-        clear_tallies_kernel<<<lb, 256, 0, stream>>>(a);
-    } else {
-        cudaError_t e;
-        if ((e = cudaMemsetAsync(a.vs_base, 0, n * sizeof(int2), stream))) return e;
-        if ((e = cudaMemsetAsync(a.vol_by_colour, 0, n * a.g.ncol * sizeof(int), stream))) return e;
-        for (int k = 0; k < 3; ++k)
-            if ((e = cudaMemsetAsync(a.vs_delta[k], 0, n * sizeof(long long), stream))) return e;
-        if (a.tracks) {
-            if ((e = cudaMemsetAsync(a.mom_base, 0, n * a.g.nm * sizeof(long long), stream))) return e;
-            for (int k = 0; k < 3; ++k)
-                if ((e = cudaMemsetAsync(a.mom_delta[k], 0, n * a.g.nm * sizeof(long long), stream))) return e;
-        }
+    if (!a.first || !a.anchor) return cudaErrorInvalidValue;
+    if (!a.flags) {
+        const size_t n = (size_t)a.n_labels;  // the count, or the capacity with n_live
+        clear_tallies_kernel<<<(int)((n + 255) / 256), 256, 0, stream>>>(a);
+        if (cudaError_t e = cudaGetLastError()) return e;
+        if (cudaError_t e =
+                launch_after(first_sites_kernel, dim3((unsigned)((a.g.sites + 255) / 256)), 256, stream, a))
+            return e;
     }
-    fill_anchor_kernel<<<lb, 256, 0, stream>>>(a);
-    if (cudaError_t e = launch_counts_any(a, stream)) return e;
-    recount_anchor_kernel<<<lb, 256, 0, stream>>>(a);
-    if (a.tracks) recount_moments_kernel<<<sb, 256, 0, stream>>>(a);
-    return cudaGetLastError();
+    return launch_counts_any(a, stream);
 }
 
 __device__ __forceinline__ void settle_one(int l, int2 *vs_base, long long *vs_delta, long long *mom_base,
@@ -261,31 +231,15 @@ __global__ void settle_kernel(int2 *vs_base, long long *vs_delta, long long *mom
     settle_one(l, vs_base, vs_delta, mom_base, mom_delta, nm, tracks);
 }
 
-// The slots at the end of a clocked step: pass number clock->pass + ncol.
-__global__ void settle_clocked_kernel(const Tallies t, int nm, int n, int tracks, const int *n_live,
-                                      const EngineClock *clock, int ncol) {
-    const int l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l >= (n_live ? *n_live : n)) return;
-    const long long p = clock->pass + ncol;
-    settle_one(l, t.vs_base[p % 2], t.vs_delta[(p + 2) % 3], t.mom_base[p % 2], t.mom_delta[(p + 2) % 3], nm, tracks);
-}
-
 __global__ void engine_clock_kernel(EngineClock *clock, int ncol) {
+    grid_wait();
     clock->step += 1;
     clock->pass += ncol;
     clock->field_cur ^= clock->field_flip;
 }
 
-cudaError_t launch_settle_clocked(const Tallies &t, int nm, int n_labels, int tracks, const int *n_live,
-                                  const EngineClock *clock, int ncol, cudaStream_t stream) {
-    if (n_labels <= 0) return cudaSuccess;
-    settle_clocked_kernel<<<(n_labels + 255) / 256, 256, 0, stream>>>(t, nm, n_labels, tracks, n_live, clock, ncol);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_engine_clock_advance(EngineClock *clock, int ncol, cudaStream_t stream) {
-    engine_clock_kernel<<<1, 1, 0, stream>>>(clock, ncol);
-    return cudaGetLastError();
+    return launch_after(engine_clock_kernel, dim3(1), 1, stream, clock, ncol);
 }
 
 __device__ __forceinline__ void settle_one(int l, int2 *vs_base, long long *vs_delta, long long *mom_base,

@@ -63,9 +63,10 @@ def test_the_infection_model_either_side_of_the_gathering_size(device, size, ker
 
 
 @pytest.mark.parametrize("every", [False, True])
-@pytest.mark.parametrize("kinds", [16, 17])
-def test_tables_in_shared_memory_and_past_it(device, kinds, every, monkeypatch):
-    """`kinds` types in all; without the other terms the passes are launched
+@pytest.mark.parametrize("kinds, width", [(16, 70), (17, 70), (16, 72), (17, 72)])
+def test_tables_in_shared_memory_and_past_it(device, kinds, width, every, monkeypatch):
+    """`kinds` types in all, on rows that are and are not whole multiples of
+    four sites (the field step's two kernels); without the other terms the passes are launched
     one by one, so the same kernel runs with and without them."""
     monkeypatch.setenv("GLAZIER_SWEEP_RESIDENT", "0")
     n = kinds
@@ -76,7 +77,7 @@ def test_tables_in_shared_memory_and_past_it(device, kinds, every, monkeypatch):
                     external=(0.1 * t, -0.2, 0.0)) if every else {}
         types.append(CellType(target_volume=60.0 + t, lambda_volume=1.0 + 0.1 * t, target_surface=90.0 + t,
                               lambda_surface=0.02 * (t % 4), **more))
-    model = Model(width=70, height=62, contact=contact, types=types, temperature=11.0, neighbour_order=2, seed=9)
+    model = Model(width=width, height=62, contact=contact, types=types, temperature=11.0, neighbour_order=2, seed=9)
     if every:
         model.species = [Species("signal", 0.2, 0.01, 1.0)]
         model.secretion = [[0.02 * t] for t in range(n)]
@@ -131,3 +132,29 @@ def _lean(device, w, h, d, types, side):
         gpu.step(chunk)
         replay.step(chunk)
     return gpu, replay
+
+
+@pytest.mark.parametrize("depth", [1, 16])
+def test_many_divisions_and_deaths_in_a_step(device, depth):
+    """Thousands of cells, most of which divide within a few steps, so a
+    step's daughters are numbered over several chunks of labels, the label
+    capacity grows during a call, and cells straddle the periodic edge."""
+    w, h = (512, 500) if depth == 1 else (128, 100)
+    side = 8 if depth == 1 else 4
+    v = float(side**2 if depth == 1 else side**3)
+    model = Model(width=w, height=h, depth=depth, contact=[0.0, 12.0, 12.0, 12.0, 8.0, 10.0, 12.0, 10.0, 8.0],
+                  types=[CellType(), CellType(target_volume=2 * v, lambda_volume=2.0, division_volume=1.05 * v),
+                         CellType(target_volume=v, lambda_volume=2.0, death_rate=0.02)],
+                  temperature=12.0, neighbour_order=2, seed=13)
+    start = Start.tiled(model, side)
+    start.set_cell_types(1 + (np.arange(start.n_cells) % 7 == 3))
+    gpu = device.GpuSimulation.from_start(start)
+    replay = ReplayOracle.from_start(start)
+    for chunk in (3, 17):
+        gpu.step(chunk)
+        replay.step(chunk)
+        assert gpu.n_labels == replay.n_labels
+        _same(gpu, replay, 0)
+    # more labels than one chunk of the decision holds, and divisions among them
+    assert start.n_cells > 2048 and gpu.n_labels > start.n_cells + 1
+    gpu.close()
