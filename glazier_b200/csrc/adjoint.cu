@@ -98,10 +98,10 @@ __device__ __forceinline__ void grid_wait() {
 }
 
 template <class Kernel, class... Args>
-cudaError_t launch_after(Kernel kernel, int grid, size_t smem, cudaStream_t stream, Args... args) {
+cudaError_t launch_blocks(Kernel kernel, dim3 grid, int threads, size_t smem, cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kThreads);
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -110,6 +110,11 @@ cudaError_t launch_after(Kernel kernel, int grid, size_t smem, cudaStream_t stre
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+template <class Kernel, class... Args>
+cudaError_t launch_after(Kernel kernel, int grid, size_t smem, cudaStream_t stream, Args... args) {
+    return launch_blocks(kernel, dim3((unsigned)grid), kThreads, smem, stream, args...);
 }
 
 struct Species {
@@ -662,6 +667,300 @@ __global__ void __launch_bounds__(kThreads) backward_quads(const __grid_constant
     for (int k = threadIdx.x; k < a.n_grads; k += blockDim.x) global_row[k] = row[k];
 }
 
+// Planes of rows of whole multiples of four sites take several rounds a
+// launch: a block holds a tile of kTileX by kTileY sites of one species with
+// kHalo sites about it in shared memory and runs up to kHalo rounds there,
+// each valid one site less far out than the round before, so a round costs a
+// block barrier and not a launch, and neighbouring tiles repeat the rounds of
+// their common margin (1.4 times the sites at 64 x 32 with a halo of 4).
+// Species do not meet in a field step, so each has blocks of its own. A round
+// of a 512^2 field was a launch of a few dependent reads on L2-resident data:
+// 3.8 us forward and 9.4 backward, whatever the arithmetic. At 512^2 with two
+// species, 50 steps and a checkpoint every 10 (host clock of the calls) the
+// forward takes 135 us (189 one round a launch) and the backward 415 (686); at
+// 1024^2, 286 (377) and 1410 (2025). Issue slots and shared-memory latency
+// bound a round now. Tiles of 16, 24 or 40 rows, blocks of 256, 320 or 512
+// threads, and two quads a thread one under the other were all slower at
+// 512^2, and so was copying each round's inputs in a round ahead.
+// Each site's arithmetic is the one-round kernels', operation for operation.
+constexpr int kHalo = 4;  // rounds a launch at most; a whole quad, so tiles stay aligned
+constexpr int kTileX = 64, kTileY = 32;
+constexpr int kRegionX = kTileX + 2 * kHalo, kRegionY = kTileY + 2 * kHalo;
+constexpr int kRegionQuads = kRegionX / 4;
+constexpr int kTileThreads = 384;
+constexpr int kQuadsEach = (kRegionY * kRegionQuads + kTileThreads - 1) / kTileThreads;
+constexpr int kTileTypes = 16;  // owner types whose rates and sums a tile kernel holds at most
+
+struct TileForward {
+    Grid g;
+    int n_species, n_types, steps;
+    const uint8_t *owner;  // the first step's owner types
+    const float *sec, *upt, *de;
+    int k[glz::kMaxSpecies];             // sub-steps a step
+    const float *in[glz::kMaxSpecies];   // the first step's input
+    float *keep[glz::kMaxSpecies][kHalo];  // by round: where to keep the exchange input (null: nowhere)
+    float *post[glz::kMaxSpecies][kHalo];  // by round: where to store its output (null: nowhere)
+};
+
+struct TileBackward {
+    Grid g;
+    int n_species, n_types, steps;
+    const uint8_t *owner;  // the first step's owner types (the last the launch takes back)
+    const float *sec, *upt, *de;
+    int k[glz::kMaxSpecies];
+    const float *lam[glz::kMaxSpecies];
+    float *lam_in[glz::kMaxSpecies];
+    const float *u[glz::kMaxSpecies][kHalo];     // by round, last first: its sub-step's input
+    const float *exch[glz::kMaxSpecies][kHalo];  // by round, a step's last: the exchange input
+    double *sums;  // each thread's running gradient sums: [block][value][thread]
+    int fresh;     // the sums start at zero
+};
+
+// A thread's quads of a tile's region: region row and first column, the
+// lattice site they wrap to, and whether they are the tile's own.
+struct TileQuads {
+    int cell[kQuadsEach];  // offset in the region, -1 past its end
+    int row[kQuadsEach], col[kQuadsEach];
+    uint32_t site[kQuadsEach];
+    bool mine[kQuadsEach];
+    __device__ __forceinline__ TileQuads(const Grid &g, int x0, int y0) {
+#pragma unroll
+        for (int n = 0; n < kQuadsEach; ++n) {
+            const int q = (int)threadIdx.x + n * kTileThreads;
+            row[n] = q / kRegionQuads;
+            col[n] = q - row[n] * kRegionQuads;
+            cell[n] = row[n] < kRegionY ? 4 * q : -1;
+            const int y = y0 - kHalo + row[n], x = x0 - kHalo + 4 * col[n];
+            site[n] = (uint32_t)glz::wrap(y, g.h) * (uint32_t)g.w + (uint32_t)glz::wrap(x, g.w);
+            mine[n] = row[n] >= kHalo && row[n] < kHalo + kTileY && col[n] >= 1 && col[n] < kRegionQuads - 1 &&
+                      y < g.h && x < g.w;
+        }
+    }
+    // whether quad n has a site within `margin` of the tile
+    __device__ __forceinline__ bool within(int n, int margin) const {
+        return cell[n] >= 0 && row[n] >= kHalo - margin && row[n] < kHalo + kTileY + margin &&
+               (margin > 0 || (col[n] >= 1 && col[n] < kRegionQuads - 1));
+    }
+};
+
+// The diffusion and decay of a quad of region cells, from `b`.
+__device__ __forceinline__ void quad_step(const float *b, int cell, float d, float e, float h[4], float v[4]) {
+    float up[4], dn[4], none[4] = {}, sum[4];
+    ld4(b + cell, h);
+    ld4(b + cell - kRegionX, up);
+    ld4(b + cell + kRegionX, dn);
+    quad_sums(false, h, b[cell - 1], b[cell + 4], up, dn, none, none, sum);
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+        v[c] = __fsub_rn(__fadd_rn(h[c], __fmul_rn(d, __fsub_rn(sum[c], __fmul_rn(4.0f, h[c])))), __fmul_rn(e, h[c]));
+}
+
+// The species' rates by owner type, (sec, upt), in shared memory, and the slot
+// of owner `o`: the medium's has none of either.
+__device__ __forceinline__ void tile_rates(const float *sec, const float *upt, int s, int n_species, int n_types,
+                                           float2 *rates) {
+    const int t = (int)threadIdx.x;
+    if (t <= n_types)
+        rates[t] = t < n_types ? make_float2(sec[t * n_species + s], upt[t * n_species + s]) : make_float2(0.0f, 0.0f);
+}
+
+__global__ void __launch_bounds__(kTileThreads) tile_forward(const __grid_constant__ TileForward a) {
+    __shared__ alignas(16) float region[2][kRegionX * kRegionY];
+    __shared__ float2 rates[kTileTypes + 1];
+    const int s = (int)blockIdx.z, k = a.k[s], rounds = a.steps * k;
+    const TileQuads Q(a.g, (int)blockIdx.x * kTileX, (int)blockIdx.y * kTileY);
+    grid_wait();
+    tile_rates(a.sec, a.upt, s, a.n_species, a.n_types, rates);
+    const float d = a.de[s], e = a.de[a.n_species + s];
+#pragma unroll
+    for (int n = 0; n < kQuadsEach; ++n)
+        if (Q.cell[n] >= 0) {
+            float v[4];
+            ld4(a.in[s] + Q.site[n], v);
+            st4(region[0] + Q.cell[n], v);
+        }
+    int at = 0;
+    for (int t = 0, r = 0; t < a.steps; ++t) {
+        int own[kQuadsEach][4];
+#pragma unroll
+        for (int n = 0; n < kQuadsEach; ++n)
+            if (Q.cell[n] >= 0) ld4(a.owner + (size_t)t * a.g.sites + Q.site[n], own[n]);
+        for (int j = 0; j < k; ++j, ++r) {
+            __syncthreads();  // the round before is in place (and the rates)
+            const float *b = region[at];
+            float *next = region[at ^ 1];
+            float *const keep = a.keep[s][r], *const post = a.post[s][r];
+            const bool last = j == k - 1;
+#pragma unroll
+            for (int n = 0; n < kQuadsEach; ++n) {
+                if (!Q.within(n, rounds - 1 - r)) continue;
+                float h[4], v[4];
+                quad_step(b, Q.cell[n], d, e, h, v);
+                if (last) {
+                    if (keep && Q.mine[n]) st4(keep + Q.site[n], v);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const bool cell = own[n][c] != kMedium;
+                        const float2 rate = rates[cell ? own[n][c] : a.n_types];
+                        float w = __fadd_rn(v[c], rate.x);
+                        w = __fsub_rn(w, __fmul_rn(rate.y, w));
+                        w = w < 0.0f ? 0.0f : w;
+                        v[c] = cell ? w : v[c];
+                    }
+                }
+                st4(next + Q.cell[n], v);
+                if (post && Q.mine[n]) st4(post + Q.site[n], v);
+            }
+            at ^= 1;
+        }
+    }
+}
+
+// The rounds of `steps` steps backward. Each thread adds its quads' gradient
+// terms, round by round and in x order, to running sums that it takes up from
+// the launch before and leaves for the next: whatever the checkpoint interval
+// cuts launches into, a thread adds the same terms in the same order. The
+// sums by owner type sit in shared memory, a column a thread (a select among
+// registers cost more than the rest of the exchange).
+__host__ __device__ constexpr size_t tile_backward_smem(int n_types) {
+    return sizeof(double) * 2 * kTileThreads * (n_types + 1) + sizeof(float) * 2 * kRegionX * kRegionY;
+}
+
+__global__ void __launch_bounds__(kTileThreads, 2) tile_backward(const __grid_constant__ TileBackward a) {
+    extern __shared__ __align__(16) unsigned char dynamic[];
+    __shared__ float2 rates[kTileTypes + 1];
+    const int T = a.n_types, tid = (int)threadIdx.x;
+    float *const region = reinterpret_cast<float *>(dynamic);  // two of kRegionX * kRegionY
+    // [type][sec, upt][thread], the medium's slot last (its sums go nowhere)
+    double *const by_type = reinterpret_cast<double *>(region + 2 * kRegionX * kRegionY) + tid;
+    const int s = (int)blockIdx.z, k = a.k[s], rounds = a.steps * k;
+    const int block = ((int)blockIdx.z * (int)gridDim.y + (int)blockIdx.y) * (int)gridDim.x + (int)blockIdx.x;
+    const TileQuads Q(a.g, (int)blockIdx.x * kTileX, (int)blockIdx.y * kTileY);
+    grid_wait();
+    tile_rates(a.sec, a.upt, s, a.n_species, T, rates);
+    const float d = a.de[s], e = a.de[a.n_species + s];
+    double *const sums = a.sums + (size_t)block * (2 + 2 * T) * kTileThreads + tid;
+    double gd = 0.0, ge = 0.0;
+    if (!a.fresh) {
+        gd = sums[0];
+        ge = sums[kTileThreads];
+    }
+    for (int v = 0; v < 2 * T; ++v) by_type[v * kTileThreads] = a.fresh ? 0.0 : sums[(2 + v) * kTileThreads];
+    by_type[2 * T * kTileThreads] = by_type[(2 * T + 1) * kTileThreads] = 0.0;
+#pragma unroll
+    for (int n = 0; n < kQuadsEach; ++n)
+        if (Q.cell[n] >= 0) {
+            float v[4];
+            ld4(a.lam[s] + Q.site[n], v);
+            st4(region + Q.cell[n], v);
+        }
+    __syncthreads();
+    int at = 0;
+    for (int t = a.steps - 1, r = 0; t >= 0; --t) {
+        for (int j = k - 1; j >= 0; --j, ++r) {
+            const int margin = rounds - 1 - r;
+            float *const b = region + at * kRegionX * kRegionY, *const next = region + (at ^ 1) * kRegionX * kRegionY;
+            const float *const u = a.u[s][r];
+            if (j == k - 1) {
+                // through the exchange, at the site
+                const float *const exch = a.exch[s][r];
+                float x[kQuadsEach][4];
+                int own[kQuadsEach][4];
+#pragma unroll
+                for (int n = 0; n < kQuadsEach; ++n)
+                    if (Q.within(n, margin + 1)) {
+                        ld4(exch + Q.site[n], x[n]);
+                        ld4(a.owner + (size_t)t * a.g.sites + Q.site[n], own[n]);
+                    }
+#pragma unroll
+                for (int n = 0; n < kQuadsEach; ++n) {
+                    if (!Q.within(n, margin + 1)) continue;
+                    float l[4];
+                    ld4(b + Q.cell[n], l);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const bool cell = own[n][c] != kMedium;
+                        const int o = cell ? own[n][c] : T;
+                        const float2 rate = rates[o];
+                        const float v1 = __fadd_rn(x[n][c], rate.x);
+                        const float v2 = __fsub_rn(v1, __fmul_rn(rate.y, v1));
+                        const float lv = v2 < 0.0f ? 0.0f : l[c];
+                        const float l1 = __fmul_rn(lv, __fsub_rn(1.0f, rate.y));
+                        l[c] = cell ? l1 : l[c];
+                        if (Q.mine[n]) {
+                            double *const sum = by_type + 2 * o * kTileThreads;
+                            sum[0] += (double)l1;
+                            sum[kTileThreads] -= (double)__fmul_rn(lv, v1);
+                        }
+                    }
+                    st4(b + Q.cell[n], l);
+                }
+                __syncthreads();
+            }
+#pragma unroll
+            for (int n = 0; n < kQuadsEach; ++n) {
+                if (!Q.within(n, margin)) continue;
+                float l[4], li[4];
+                quad_step(b, Q.cell[n], d, e, l, li);
+                st4(next + Q.cell[n], li);
+                if (Q.mine[n]) {
+                    const uint32_t W = (uint32_t)a.g.w, all = (uint32_t)a.g.sites, site = Q.site[n];
+                    const uint32_t x = site - glz::udiv(a.g.div_w, site) * W;
+                    float h[4], hu[4], hd[4], none[4] = {}, us[4];
+                    ld4(u + site, h);
+                    ld4(u + (site < W ? site + all - W : site - W), hu);
+                    ld4(u + (site + W >= all ? site + W - all : site + W), hd);
+                    quad_sums(false, h, u[x == 0 ? site + W - 1 : site - 1], u[x + 4 == W ? site + 4 - W : site + 4], hu,
+                              hd, none, none, us);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        gd += (double)__fmul_rn(l[c], __fsub_rn(us[c], __fmul_rn(4.0f, h[c])));
+                        ge -= (double)__fmul_rn(l[c], h[c]);
+                    }
+                }
+            }
+            __syncthreads();
+            at ^= 1;
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < kQuadsEach; ++n)
+        if (Q.mine[n]) {
+            float v[4];
+            ld4(region + at * kRegionX * kRegionY + Q.cell[n], v);
+            st4(a.lam_in[s] + Q.site[n], v);
+        }
+    sums[0] = gd;
+    sums[kTileThreads] = ge;
+    for (int v = 0; v < 2 * T; ++v) sums[(2 + v) * kTileThreads] = by_type[v * kTileThreads];
+}
+
+// Gradient blockIdx.x from every thread's sums: thread i adds thread i's (and
+// i + kThreads's) of each of its species' tiles in order, then the block's
+// threads are summed.
+__global__ void __launch_bounds__(kThreads) tile_gradients(const double *__restrict__ sums, int tiles, int n_species,
+                                                           int n_types, double *__restrict__ grads) {
+    __shared__ double scratch[kWarps];
+    grid_wait();
+    // gradient layout: d, e per species, then sec, upt per (type, species);
+    // a species' values: d, e, then (sec, upt) by type
+    const int S = n_species, g = (int)blockIdx.x, values = 2 + 2 * n_types;
+    int s = g % S, v = g / S;
+    if (g >= 2 * S) {
+        const int i = g - 2 * S, table = i / (n_types * S), t = (i - table * n_types * S) / S;
+        v = 2 + 2 * t + table;
+    }
+    const double *p = sums + ((size_t)s * tiles * values + v) * kTileThreads;
+    const size_t stride = (size_t)values * kTileThreads;
+    double total = 0.0;
+    for (int i = (int)threadIdx.x; i < kTileThreads; i += kThreads) {
+#pragma unroll 8
+        for (int b = 0; b < tiles; ++b) total += p[(size_t)b * stride + i];
+    }
+    total = block_sum(total, scratch);
+    if (threadIdx.x == 0) grads[g] = total;
+}
+
 // grads[k] = the sum over blocks of partial[b][k], one warp per k: lane l
 // adds rows l, l + 32, ... in order, then the warp's lanes are summed by the
 // fixed shuffle tree, so the order depends on the block count alone.
@@ -701,7 +1000,7 @@ struct glz_adj {
     float *staging = nullptr;                  // pinned: the rate tables on their way in
     float *d_de = nullptr;      // per-sub-step d then e per species
     float *final_out = nullptr; // n_species * sites: the forward's last step, copied to the caller
-    double *partial = nullptr;  // kBlocks rows of n_grads
+    double *partial = nullptr;  // kBlocks rows of n_grads, or the tile kernels' running sums
     double *d_grads = nullptr;  // n_grads: d, e per species, then sec, upt per (type, species)
     std::vector<double> params;
     std::vector<int> k;
@@ -724,6 +1023,27 @@ bool quads(const glz_adj *h) { return h->g.w % 4 == 0; }
 int blocks_for(const glz_adj *h) {
     const long long items = quads(h) ? h->g.sites / 4 : h->g.sites;
     return (int)((items + kThreads - 1) / kThreads);
+}
+
+// Planes that take the tile kernels: rows of whole quads, few enough owner
+// types, and few enough sites that the threads' running sums stay small
+// beside the fields (15 bytes a site of a species at four types).
+bool tile_plane(const glz_adj *h) {
+    return h->g.dim == 2 && quads(h) && h->n_types <= kTileTypes && h->g.sites <= (1 << 20);
+}
+// ... when every species' sub-steps fit a launch's rounds.
+bool tiled(const glz_adj *h) { return tile_plane(h) && h->kmax <= kHalo; }
+int steps_each(const glz_adj *h) { return kHalo / h->kmax; }
+dim3 tile_grid(const glz_adj *h) {
+    return dim3((unsigned)((h->g.w + kTileX - 1) / kTileX), (unsigned)((h->g.h + kTileY - 1) / kTileY),
+                (unsigned)h->n_species);
+}
+size_t partial_doubles(const glz_adj *h) {
+    const size_t rows = (size_t)kBlocks * n_grads(h);
+    if (!tile_plane(h)) return rows;
+    const dim3 grid = tile_grid(h);
+    const size_t sums = (size_t)grid.x * grid.y * grid.z * (2 + 2 * h->n_types) * kTileThreads;
+    return sums > rows ? sums : rows;
 }
 
 int launch_forward(glz_adj *h, const ForwardRound &a) {
@@ -838,11 +1158,85 @@ int keep_step(glz_adj *h, int sg, int local, int len, float *last_out) {
     return GLZ_OK;
 }
 
-// Recompute segment `sg`, keeping every sub-step state; its last step's
-// output is not needed.
-int recompute(glz_adj *h, int sg, int len) {
+// Steps `local` .. `local + n - 1` of segment `sg` in one tile launch, keeping
+// every sub-step state as keep_step does; `out` may name where a step's output
+// goes besides (the last of the segment, or none).
+int tile_keep(glz_adj *h, int sg, int local, int n, int len, float *last_out) {
+    TileForward a{};
+    a.g = h->g;
+    a.n_species = h->n_species;
+    a.n_types = h->n_types;
+    a.steps = n;
+    a.owner = h->owner + (size_t)(sg * h->every + local) * h->g.sites;
+    a.sec = h->d_sec;
+    a.upt = h->d_upt;
+    a.de = h->d_de;
+    for (int s = 0; s < h->n_species; ++s) {
+        a.k[s] = h->k[s];
+        a.in[s] = seg_state(h, sg, local, 0, s);
+        for (int i = 0, r = 0; i < n; ++i)
+            for (int j = 0; j < h->k[s]; ++j, ++r) {
+                const int step = local + i;
+                if (j < h->k[s] - 1) {
+                    a.post[s][r] = seg_state(h, sg, step, j + 1, s);
+                    continue;
+                }
+                a.keep[s][r] = seg_state(h, sg, step, h->k[s], s);
+                a.post[s][r] = step + 1 < len ? seg_state(h, sg, step + 1, 0, s)
+                                              : (last_out ? last_out + (size_t)s * h->g.sites : nullptr);
+            }
+    }
+    CU(launch_blocks(tile_forward, tile_grid(h), kTileThreads, 0, h->stream, a));
+    return GLZ_OK;
+}
+
+// keep_step for a whole segment.
+int keep_segment(glz_adj *h, int sg, int len, float *last_out) {
+    if (tiled(h)) {
+        for (int local = 0; local < len; local += steps_each(h)) {
+            const int n = len - local < steps_each(h) ? len - local : steps_each(h);
+            if (int rc = tile_keep(h, sg, local, n, len, last_out)) return rc;
+        }
+        return GLZ_OK;
+    }
     for (int local = 0; local < len; ++local)
-        if (int rc = keep_step(h, sg, local, len, nullptr)) return rc;
+        if (int rc = keep_step(h, sg, local, len, last_out)) return rc;
+    return GLZ_OK;
+}
+
+// Every step forward up to the last segment's first, tile launches of several
+// steps each: the checkpoints on the way, and each launch's last output to a
+// work buffer when it is no checkpoint.
+int tile_forward_to(glz_adj *h, int t_last) {
+    const size_t n_all = field_floats(h), sites = h->g.sites;
+    const float *cur = h->ckpt;
+    for (int t = 0; t < t_last; t += steps_each(h)) {
+        const int n = t_last - t < steps_each(h) ? t_last - t : steps_each(h);
+        TileForward a{};
+        a.g = h->g;
+        a.n_species = h->n_species;
+        a.n_types = h->n_types;
+        a.steps = n;
+        a.owner = h->owner + (size_t)t * sites;
+        a.sec = h->d_sec;
+        a.upt = h->d_upt;
+        a.de = h->d_de;
+        float *dst = nullptr;
+        for (int i = 1; i <= n; ++i) {
+            float *to = (t + i) % h->every == 0 ? h->ckpt + (size_t)((t + i) / h->every) * n_all : nullptr;
+            if (i == n) {
+                if (!to) to = cur == h->work[0] ? h->work[1] : h->work[0];
+                dst = to;
+            }
+            for (int s = 0; to && s < h->n_species; ++s) a.post[s][i * h->k[s] - 1] = to + (size_t)s * sites;
+        }
+        for (int s = 0; s < h->n_species; ++s) {
+            a.k[s] = h->k[s];
+            a.in[s] = cur + (size_t)s * sites;
+        }
+        CU(launch_blocks(tile_forward, tile_grid(h), kTileThreads, 0, h->stream, a));
+        cur = dst;
+    }
     return GLZ_OK;
 }
 
@@ -879,7 +1273,9 @@ int forward_sequence(glz_adj *h) {
     const size_t n = field_floats(h);
     const int last = (h->steps - 1) / h->every, t_last = last * h->every;
     const float *cur = h->ckpt;
-    for (int t = 0; t < t_last; ++t) {
+    if (tiled(h))
+        if (int rc = tile_forward_to(h, t_last)) return rc;
+    for (int t = tiled(h) ? t_last : 0; t < t_last; ++t) {
         float *dst;
         if ((t + 1) % h->every == 0)
             dst = h->ckpt + (size_t)((t + 1) / h->every) * n;
@@ -888,8 +1284,53 @@ int forward_sequence(glz_adj *h) {
         if (int rc = step_forward(h, t, cur, dst)) return rc;
         cur = dst;
     }
-    for (int t = t_last; t < h->steps; ++t)
-        if (int rc = keep_step(h, last, t - t_last, h->steps - t_last, h->final_out)) return rc;
+    return keep_segment(h, last, h->steps - t_last, h->final_out);
+}
+
+// backward_sequence by tile launches of several steps each.
+int tile_backward_sequence(glz_adj *h) {
+    const int S = h->n_species;
+    int cur = 0;
+    TileBackward a{};
+    a.g = h->g;
+    a.n_species = S;
+    a.n_types = h->n_types;
+    a.sec = h->d_sec;
+    a.upt = h->d_upt;
+    a.de = h->d_de;
+    a.sums = h->partial;
+    a.fresh = 1;
+    const dim3 grid = tile_grid(h);
+    const size_t smem = tile_backward_smem(h->n_types);
+    CU(cudaFuncSetAttribute(tile_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int nseg = (h->steps + h->every - 1) / h->every;
+    for (int sg = nseg - 1; sg >= 0; --sg) {
+        const int t0 = sg * h->every, len = (t0 + h->every < h->steps ? t0 + h->every : h->steps) - t0;
+        // the forward left the last segment's states in place
+        if (sg < nseg - 1)
+            if (int rc = keep_segment(h, sg, len, nullptr)) return rc;
+        for (int end = len; end > 0; end -= steps_each(h)) {
+            const int n = end < steps_each(h) ? end : steps_each(h), local = end - n;
+            a.steps = n;
+            a.owner = h->owner + (size_t)(t0 + local) * h->g.sites;
+            for (int s = 0; s < S; ++s) {
+                a.k[s] = h->k[s];
+                a.lam[s] = h->lam[cur] + (size_t)s * h->g.sites;
+                a.lam_in[s] = h->lam[1 - cur] + (size_t)s * h->g.sites;
+                for (int step = end - 1, r = 0; step >= local; --step)
+                    for (int j = h->k[s] - 1; j >= 0; --j, ++r) {
+                        a.u[s][r] = seg_state(h, sg, step, j, s);
+                        a.exch[s][r] = seg_state(h, sg, step, h->k[s], s);
+                    }
+            }
+            CU(launch_blocks(tile_backward, grid, kTileThreads, smem, h->stream, a));
+            a.fresh = 0;
+            cur = 1 - cur;
+        }
+    }
+    CU(launch_after(tile_gradients, n_grads(h), 0, h->stream, (const double *)h->partial, (int)(grid.x * grid.y), S,
+                    h->n_types, h->d_grads));
+    for (int s = 0; s < S; ++s) h->bwd_cur[s] = cur;
     return GLZ_OK;
 }
 
@@ -897,6 +1338,7 @@ int forward_sequence(glz_adj *h) {
 // by segment from the last: recompute the segment's sub-step states, then
 // its rounds backward; the per-block gradient rows summed at the end.
 int backward_sequence(glz_adj *h) {
+    if (tiled(h)) return tile_backward_sequence(h);
     const int S = h->n_species, T = h->n_types, G = n_grads(h);
     const size_t sites = h->g.sites;
     const int grid = blocks_for(h) < kBlocks ? blocks_for(h) : kBlocks;
@@ -923,7 +1365,7 @@ int backward_sequence(glz_adj *h) {
         const int t0 = sg * h->every, len = (t0 + h->every < h->steps ? t0 + h->every : h->steps) - t0;
         // the forward left the last segment's states in place
         if (sg < nseg - 1)
-            if (int rc = recompute(h, sg, len)) return rc;
+            if (int rc = keep_segment(h, sg, len, nullptr)) return rc;
         for (int local = len - 1; local >= 0; --local) {
             a.owner = h->owner + (size_t)(t0 + local) * sites;
             for (int r = h->kmax - 1; r >= 0; --r) {
@@ -988,7 +1430,7 @@ int glz_adj_create(int width, int height, int depth, int n_species, int n_types,
         cudaMalloc(&h->d_sec, table_floats(h) * 4) != cudaSuccess ||
         cudaMallocHost(&h->staging, table_floats(h) * 4) != cudaSuccess ||
         cudaMalloc(&h->final_out, n * sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&h->partial, (size_t)kBlocks * n_grads(h) * 8) != cudaSuccess ||
+        cudaMalloc(&h->partial, partial_doubles(h) * 8) != cudaSuccess ||
         cudaMalloc(&h->d_grads, (size_t)n_grads(h) * 8) != cudaSuccess)
         return bail(fail(GLZ_DRIVER, "adjoint allocation failed"));
     h->d_upt = h->d_sec + (size_t)n_types * n_species;
