@@ -1,7 +1,7 @@
 // The direct sweep: a colour pass with no staging at all, the labels and
 // tallies read where they lie. It takes the lattices whose passes the window
 // rings of sweep.cu do not pay for: lean planes of at most 1024^2, lean
-// volumes, and models with every term on small lattices.
+// volumes, and models with every term.
 //
 // What bounds it is latency. A pass is a chain of dependent reads (labels,
 // then the two cells' tallies and types, then for some copies moments,
@@ -115,16 +115,24 @@ constexpr int kWarpK = 4;
 constexpr int kBlockK = 2;
 constexpr int kBlockThreads = 256;
 
-// Passes of the lean models are held to 64 registers, four blocks of 256 per
-// SM, so that a 2^18-target pass of two targets a thread is one wave (at
-// 128^3: 0.060 ms per MCS against 0.073 uncapped, 0.065 at 48 registers); the
-// every-term passes to 128, two blocks of 256 (uncapped they take up to 200,
-// one block: 48 against 70 us per MCS for the 512^2 tissue).
-template <bool EXTRAS>
-constexpr int kDirectMinBlocks = EXTRAS ? 2 : 4;
+// Every-term passes of more targets than the device's blocks hold at once
+// gather in blocks of kBlockThreads at 64 registers, some spilled: what the
+// spills cost is less than what the warps give (per MCS of the two-field
+// tissue, 128 registers and 64: 53.7 and 46.7 us at 1024^2, 162.6 and 130.2
+// at 2048^2; 31.9 and 37.0 at 640^2, where a pass is a single wave).
+constexpr int kBlockWide = 3;
+
+// Blocks of kBlockThreads an SM holds, which caps a thread's registers. The
+// lean models' 64 registers make a 2^18-target pass of two targets a thread
+// one wave (at 128^3: 0.060 ms per MCS against 0.073 uncapped, 0.065 at 48);
+// small every-term passes keep 128 (uncapped they take up to 200, one block:
+// 48 against 70 us per MCS for the 512^2 tissue), large ones 64.
+constexpr int direct_blocks(int form, bool extras) {
+    return extras && (form == kPlain || form == kBlock) ? 2 : 4;
+}
 
 template <int DIM, int NOFF, bool UNIFORM, int FORM, bool EXTRAS>
-__global__ void __launch_bounds__(kBlockThreads, kDirectMinBlocks<EXTRAS>)
+__global__ void __launch_bounds__(kBlockThreads, direct_blocks(FORM, EXTRAS))
     direct_sweep_kernel(const __grid_constant__ SweepLaunch a) {
     const int targets = (a.g.w / 2) * (a.g.h / 2) * (DIM == 3 ? a.g.d / 2 : 1);
     __shared__ TypeSmem<EXTRAS> types;
@@ -162,7 +170,7 @@ __global__ void __launch_bounds__(kBlockThreads, kDirectMinBlocks<EXTRAS>)
             }
         }
         rotate_share<EXTRAS>(a, d);
-    } else if constexpr (FORM == kBlock) {
+    } else if constexpr (FORM == kBlock || FORM == kBlockWide) {
         __shared__ int queue[kBlockThreads * kBlockK];
         __shared__ uint8_t picks[kBlockThreads * kBlockK];
         __shared__ uint2 pair[kBlockThreads * kBlockK];  // (old, new) labels of each queued copy
@@ -293,15 +301,16 @@ template <int DIM, int NOFF, bool UNIFORM>
 cudaError_t launch_direct(const SweepLaunch &a, cudaStream_t stream) {
     const int targets = (a.g.w / 2) * (a.g.h / 2) * (DIM == 3 ? a.g.d / 2 : 1);
     const bool warp = a.compact == 1, block = a.compact == 2;
+    const bool wide = block && !a.lean && targets >= kDirectGatherFrom;
     SweepLaunch b = a;
-    // Every-term blocks are half as wide: their 128 registers a thread leave
-    // room for two blocks of 256 an SM, and four of 128 fill it as well but
-    // wait for one another less (62.7 against 64.9 us per MCS at 1024^2).
-    const int threads = block && !a.lean ? kBlockThreads / 2 : kBlockThreads;
+    // Every-term blocks of 128 registers a thread are half as wide: four of
+    // 128 threads fill an SM as two of 256 do but wait for one another less
+    // (62.7 against 64.9 us per MCS at 1024^2).
+    const int threads = block && !a.lean && !wide ? kBlockThreads / 2 : kBlockThreads;
     int per_block = threads * (warp ? kWarpK : (block ? kBlockK : 1));
     int grid = (targets + per_block - 1) / per_block;
     if (block) {
-        const int slots = sm_count() * kDirectMinBlocks<false>;
+        const int slots = sm_count() * direct_blocks(kBlock, false);
         if (a.lean && slots > 0) {
             // Spread the pass evenly over whole waves of resident blocks, so
             // that no SM holds more of its targets than another (at 128^3 and
@@ -324,6 +333,7 @@ cudaError_t launch_direct(const SweepLaunch &a, cudaStream_t stream) {
     cfg.numAttrs = 1;
     if (!a.lean)  // every term: length, chemotaxis, connectivity, motility, drift, nematic, moments
         return warp    ? cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kWarp, true>, b)
+               : wide  ? cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kBlockWide, true>, b)
                : block ? cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kBlock, true>, b)
                        : cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kPlain, true>, b);
     return warp    ? cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kWarp, false>, b)

@@ -953,26 +953,31 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
     const int direct_mode = direct_env ? (direct_env[0] == '0' ? 0 : 1) : -1;
     const long long direct_most = g.dim == 2 ? 1024LL * 1024LL : sites;
     // Models with other terms (length, chemotaxis, connectivity, motility,
-    // drift, nematic, division and death) take the direct kernel on planes up
-    // to 1024^2 and volumes up to 128^3, where the tiled kernel's window
-    // staging costs more than it saves.
-    const long long direct_most_general = g.dim == 2 ? 1024LL * 1024LL : 128LL * 128LL * 128LL;
-    h->direct = direct_mode == 1 || (direct_mode == -1 && sites <= (h->lean ? direct_most : direct_most_general));
+    // drift, nematic, division and death) take the direct kernel at any size:
+    // the tiled kernel's window staging costs more than it saves (per MCS of
+    // the two-field tissue, direct against tiled: 72 and 115 us at 1400^2, 130
+    // and 168 at 2048^2, 450 and 525 at 4096^2; of the infected slab's model
+    // 296 and 574 at 128^3, 461 and 750 at 160^3).
+    h->direct = direct_mode == 1 || (direct_mode == -1 && (!h->lean || sites <= direct_most));
     // Past a number of targets a pass the direct kernel gathers each block's
     // unlike copies into one queue priced by whole warps, and from a million
     // it queues each warp's
     // (GLAZIER_SWEEP_COMPACT=0: neither, =1: the warp's, =2: the block's, at
     // any size). Per MCS of the two-field tissue, priced in place against
     // gathered: 31.1 and 31.7 us at 256^2, 35.1 and 35.0 at 512^2, 51.6 and
-    // 36.6 at 640^2, 92.7 and 62.7 at 1024^2. Of the lean plane: 11.9 and 13.9
+    // 36.6 at 640^2, 92.7 and 62.7 at 1024^2 (of the slab's model 147 and 162
+    // at 64 x 64 x 32, 179 and 191 at 96 x 96 x 64, 386 and 300 at 128^3), by
+    // warps against by blocks 130 and 130 at 2048^2, 450 and 479 at 4096^2. Of
+    // the lean plane: 11.9 and 13.9
     // at 512^2, 13.9 and 15.7 at 768^2 (a last target a thread of one wave of
     // blocks), 20.9 and 16.7 at 896^2; of the lean volume (26 neighbours):
     // 24.2 and 28.4 at 64^3, 28.9 and 30.7 at 80^3, 35.6 and 33.4 at 96^3.
     const char *compact_env = std::getenv("GLAZIER_SWEEP_COMPACT");
     const int compact_mode = compact_env ? (compact_env[0] == '0' ? 0 : (compact_env[0] == '2' ? 2 : 1)) : -1;
     const long long targets = sites / g.ncol;
-    const long long gather_from = !h->lean ? glz::kDirectGatherEveryFrom
-                                  : g.dim == 2 ? glz::kDirectGatherFrom : glz::kDirectGatherVolumeFrom;
+    const long long gather_from = g.dim == 3 ? glz::kDirectGatherVolumeFrom
+                                  : h->lean  ? glz::kDirectGatherFrom
+                                             : glz::kDirectGatherEveryFrom;
     h->compact = compact_mode >= 0 ? compact_mode
                                    : (targets >= glz::kDirectCompactFrom ? 1 : (targets >= gather_from ? 2 : 0));
     // A small lean plane with nothing between its colour passes (no fields,

@@ -171,8 +171,8 @@ struct ResidentLaunch {
 
 // Targets a pass from which the direct kernel queues a block's unlike copies
 // (of a lean plane: more than 148 SMs' four blocks of 256 take at once; of a
-// lean volume; with terms past contact, volume and surface) and from which a
-// warp's.
+// volume; of a plane with terms past contact, volume and surface) and from
+// which a warp's.
 constexpr int kDirectGatherFrom = 148 * 4 * 256 + 1;
 constexpr int kDirectGatherVolumeFrom = 5 << 14;
 constexpr int kDirectGatherEveryFrom = (1 << 16) + 1;

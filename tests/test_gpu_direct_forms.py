@@ -1,8 +1,9 @@
 """The direct sweep's forms at the edges of their ranges, against the replay.
 
-- The two-field infection model (every term but motility) on the largest
-  plane priced in place (512^2, 2^16 targets a pass) and just past it, where a
-  block's unlike copies are gathered: the default choice on both sides.
+- The two-field infection model (every term but motility) either side of each
+  size from which its passes take another form, and a volume of every term
+  past the size from which the gathering blocks are the wide ones: the default
+  choices.
 - Models of 16 and of 17 types, the most whose tables are held in shared
   memory and the least whose are read where they lie, with and without the
   terms past contact, volume and surface.
@@ -47,9 +48,12 @@ def _same(gpu, replay, species: int) -> None:
         assert np.array_equal(gpu.field(k).astype(np.float32), replay.field(k))
 
 
-@pytest.mark.parametrize("size, kernel", [(512, "direct"), (514, "gathered")])
-def test_the_infection_model_either_side_of_the_gathering_size(device, size, kernel):
-    start = infection_start(seed=3, size=size, grid=32, immune=64)
+@pytest.mark.parametrize("size, kernel", [(512, "direct"), (514, "gathered"), (778, "gathered"), (780, "gathered"),
+                                          (2046, "gathered"), (2048, "compact")])
+def test_the_infection_model_either_side_of_each_size(device, size, kernel):
+    """At 780^2 a pass has more targets than one wave of blocks, and the
+    gathering blocks are the wide ones; from 2048^2 warps queue their own."""
+    start = infection_start(seed=3, size=size, grid=size // 16, immune=64)
     gpu = device.GpuSimulation.from_start(start)
     assert gpu.sweep_kernel == kernel
     replay = ReplayOracle.from_start(start)
@@ -157,4 +161,24 @@ def test_many_divisions_and_deaths_in_a_step(device, depth):
         _same(gpu, replay, 0)
     # more labels than one chunk of the decision holds, and divisions among them
     assert start.n_cells > 2048 and gpu.n_labels > start.n_cells + 1
+    gpu.close()
+
+
+def test_a_volume_of_every_term_in_wide_blocks(device):
+    """More than 148 x 4 x 256 targets a pass, with the veto, motility, drift,
+    chemotaxis, length, death and a field of two sub-steps."""
+    cell = dict(target_volume=216.0, lambda_volume=2.0, connected=True, max_activity=20.0, lambda_activity=60.0,
+                external=(0.0, 0.0, 1.0), death_rate=0.002, target_surface=300.0, lambda_surface=0.05)
+    model = Model(width=108, height=110, depth=104, contact=[0.0, 16.0, 16.0, 16.0, 8.0, 9.0, 16.0, 9.0, 8.0],
+                  types=[CellType(), CellType(**cell), CellType(target_length=8.0, lambda_length=0.5, **cell)],
+                  temperature=10.0, neighbour_order=2, seed=29, species=[Species("signal", 0.3, 0.01, 0.0)],
+                  secretion=[[0.0], [0.2], [0.1]], uptake=[[0.0], [0.0], [0.05]], chemotaxis=[[0.0], [10.0], [5.0]])
+    start = Start.tiled(model, 6)
+    start.set_cell_types(1 + np.arange(start.n_cells) % 2)
+    gpu = device.GpuSimulation.from_start(start)
+    assert gpu.sweep_kernel == "gathered" and model.sites // 8 > 148 * 4 * 256
+    replay = ReplayOracle.from_start(start)
+    gpu.step(3)
+    replay.step(3)
+    _same(gpu, replay, 1)
     gpu.close()
