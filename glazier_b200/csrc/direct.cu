@@ -1,7 +1,7 @@
 // The direct sweep: a colour pass with no staging at all, the labels and
 // tallies read where they lie. It takes the lattices whose passes the window
-// rings of sweep.cu do not pay for: lean planes of at most 1024^2, lean
-// volumes, and models with every term.
+// rings of sweep.cu do not pay for: lean planes under 2048^2, lean volumes,
+// and models with every term.
 //
 // What bounds it is latency. A pass is a chain of dependent reads (labels,
 // then the two cells' tallies and types, then for some copies moments,

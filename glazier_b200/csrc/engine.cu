@@ -940,18 +940,16 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
     const char *lean_env = std::getenv("GLAZIER_SWEEP_LEAN");
     h->lean = !h->has_length && !h->tracks && !h->has_chemotaxis && !h->has_external && !h->has_motility && !has_conn &&
               !(lean_env && lean_env[0] == '0');
-    // A lean plane of at most 1024^2 sites, or a lean volume of any size,
-    // takes the direct kernel: one thread per target reading the lattice
-    // through the caches beats the lean kernel's window ring there (per MCS,
-    // L2 flushed: 0.035 against 0.040 ms at 1024^2; 0.37 against 0.91 ms at
-    // 256^3 and 0.64 against 1.07 ms at 320^3, a lattice past L2; at 2048^2
-    // and 4096^2 the lean kernel leads: 100 MCS back to back at 2048^2 take
-    // 5.8 ms on it against 7.8 ms on the warp-queued direct kernel, though a
-    // single MCS after an L2 flush is 6 % faster on the latter).
-    // GLAZIER_SWEEP_DIRECT=0: never, =1: at any size.
+    // A lean plane under 2048^2 sites, or a lean volume of any size, takes the
+    // direct kernel, which reads the lattice through the caches: the lean
+    // kernel's window ring pays on large planes only (per MCS, direct against
+    // lean: 17.7 and 32.0 us at 1100^2, 29.0 and 49.5 at 1448^2, 158 and 129 at
+    // 4096^2; 0.37 against 0.91 ms at 256^3 and 0.64 against 1.07 ms at 320^3,
+    // a lattice past L2, L2 flushed). GLAZIER_SWEEP_DIRECT=0: never, =1: at any
+    // size.
     const char *direct_env = std::getenv("GLAZIER_SWEEP_DIRECT");
     const int direct_mode = direct_env ? (direct_env[0] == '0' ? 0 : 1) : -1;
-    const long long direct_most = g.dim == 2 ? 1024LL * 1024LL : sites;
+    const long long direct_most = g.dim == 2 ? 2048LL * 2048LL - 1 : sites;
     // Models with other terms (length, chemotaxis, connectivity, motility,
     // drift, nematic, division and death) take the direct kernel at any size:
     // the tiled kernel's window staging costs more than it saves (per MCS of
@@ -960,7 +958,7 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
     // 296 and 574 at 128^3, 461 and 750 at 160^3).
     h->direct = direct_mode == 1 || (direct_mode == -1 && (!h->lean || sites <= direct_most));
     // Past a number of targets a pass the direct kernel gathers each block's
-    // unlike copies into one queue priced by whole warps, and from a million
+    // unlike copies into one queue priced by whole warps, and past a larger one
     // it queues each warp's
     // (GLAZIER_SWEEP_COMPACT=0: neither, =1: the warp's, =2: the block's, at
     // any size). Per MCS of the two-field tissue, priced in place against
@@ -970,7 +968,9 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
     // warps against by blocks 130 and 130 at 2048^2, 450 and 479 at 4096^2. Of
     // the lean plane: 11.9 and 13.9
     // at 512^2, 13.9 and 15.7 at 768^2 (a last target a thread of one wave of
-    // blocks), 20.9 and 16.7 at 896^2; of the lean volume (26 neighbours):
+    // blocks), 20.9 and 16.7 at 896^2, by blocks against by warps 17.7 and 21.7
+    // at 1100^2, 29.1 and 28.7 at 1300^2, 30.3 and 29.0 at 1448^2; of the lean
+    // volume (26 neighbours):
     // 24.2 and 28.4 at 64^3, 28.9 and 30.7 at 80^3, 35.6 and 33.4 at 96^3.
     const char *compact_env = std::getenv("GLAZIER_SWEEP_COMPACT");
     const int compact_mode = compact_env ? (compact_env[0] == '0' ? 0 : (compact_env[0] == '2' ? 2 : 1)) : -1;
@@ -978,8 +978,8 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
     const long long gather_from = g.dim == 3 ? glz::kDirectGatherVolumeFrom
                                   : h->lean  ? glz::kDirectGatherFrom
                                              : glz::kDirectGatherEveryFrom;
-    h->compact = compact_mode >= 0 ? compact_mode
-                                   : (targets >= glz::kDirectCompactFrom ? 1 : (targets >= gather_from ? 2 : 0));
+    const long long compact_from = h->lean && g.dim == 2 ? glz::kDirectCompactPlaneFrom : glz::kDirectCompactFrom;
+    h->compact = compact_mode >= 0 ? compact_mode : (targets >= compact_from ? 1 : (targets >= gather_from ? 2 : 0));
     // A small lean plane with nothing between its colour passes (no fields,
     // division or death) runs every MCS of a call in one thread-block
     // cluster (GLAZIER_SWEEP_RESIDENT=0 or GLAZIER_SWEEP_CLUSTER=0: a launch

@@ -172,10 +172,11 @@ struct ResidentLaunch {
 // Targets a pass from which the direct kernel queues a block's unlike copies
 // (of a lean plane: more than 148 SMs' four blocks of 256 take at once; of a
 // volume; of a plane with terms past contact, volume and surface) and from
-// which a warp's.
+// which a warp's (of a lean plane; of the others).
 constexpr int kDirectGatherFrom = 148 * 4 * 256 + 1;
 constexpr int kDirectGatherVolumeFrom = 5 << 14;
 constexpr int kDirectGatherEveryFrom = (1 << 16) + 1;
+constexpr int kDirectCompactPlaneFrom = 3 << 17;
 constexpr int kDirectCompactFrom = 1 << 20;
 
 // Every requested MCS of a small lean plane in one thread-block cluster holding

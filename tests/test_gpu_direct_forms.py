@@ -101,6 +101,7 @@ def test_tables_in_shared_memory_and_past_it(device, kinds, width, every, monkey
 @pytest.mark.parametrize("w, h, d, kernel", [
     (30, 2, 1, "cluster"), (18, 4, 1, "cluster"), (66, 34, 1, "cluster"), (130, 50, 1, "cluster"),
     (254, 256, 1, "cluster"), (256, 256, 1, "direct"), (778, 778, 1, "direct"), (780, 780, 1, "gathered"),
+    (1254, 1252, 1, "gathered"), (1256, 1254, 1, "compact"), (2048, 2046, 1, "compact"), (2050, 2048, 1, "lean"),
     (80, 80, 80, "direct"), (88, 88, 88, "gathered"),
 ])
 @pytest.mark.parametrize("types", [1, 2])
