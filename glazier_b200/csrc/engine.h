@@ -234,14 +234,20 @@ struct EnsembleLaunch {
     int *error_flag;
     // 0: the windowed persistent kernel (128 x 32 tiles); 1, 2, 3: one block
     // per tile of 32 x 8, 16 x 16 or 64 x 4 targets of a plane, priced where
-    // they lie (tile_prefix and total_tiles then count those tiles)
+    // they lie (tile_prefix and total_tiles then count those tiles);
+    // kEnsembleRuns: a block per run of kEnsembleRun consecutive targets of a
+    // replica (total_tiles counts the runs)
     int tile_shape;
+    const int2 *runs;  // per run: its replica, its first target
     // The colour schedule of the direct shapes: 0 a launch per colour pass;
     // 1 every pass of the step in one cooperative launch, blocks striding
     // over the tiles, a grid barrier (bounded, error flag 4) between passes.
     int one_launch;
     unsigned *barrier;  // [0] arrivals, [1] barriers completed; zero at launch
 };
+
+constexpr int kEnsembleRuns = 4;    // the tile shape of runs
+constexpr int kEnsembleRun = 1024;  // targets a run
 
 // Targets per tile along x and y of ensemble tile shape `shape` (1, 2, 3).
 inline void ensemble_tile(int shape, int &bx, int &by) {

@@ -134,6 +134,7 @@ struct glz_ens {
     glz::EnsembleReplica *d_reps = nullptr;
     CUtensorMap *d_maps = nullptr;
     int *d_prefix = nullptr, *d_order = nullptr;
+    int2 *d_runs = nullptr;  // every replica's runs
     glz::EnsembleClock *d_clock = nullptr;
     int *error_flag = nullptr;
     unsigned long long *medium = nullptr;
@@ -181,16 +182,23 @@ void drop_graph(glz_ens *h) {
 // direct blocks' over its targets.
 int tiles_of(const glz_ens *h, const Replica &rep, int shape) {
     if (shape == 0) return rep.tiles;
+    if (shape == glz::kEnsembleRuns)
+        return (rep.g.sites / h->ncol + glz::kEnsembleRun - 1) / glz::kEnsembleRun;
     int bx, by;
     glz::ensemble_tile(shape, bx, by);
     return ((rep.g.w / 2 + bx - 1) / bx) * ((rep.g.h / 2 + by - 1) / by);
 }
 
+// The runs' schedule, of replicas in their own order: what an ensemble starts
+// on and a candidate of the autotuner's, not one that callers name.
+constexpr int kRunsSchedule = 16;
+
 // Lay the replicas' tiles out in schedule order (`schedule` bit 0: largest
-// first; bits 1-2: the tile shape) and upload the order.
+// first; bits 1-2: the tile shape; or kRunsSchedule) and upload the order.
 int set_schedule(glz_ens *h, int schedule, int max_ctas) {
-    const int shape = (schedule >> 1) & 3, one = (schedule >> 3) & 1;
-    if (shape > 0 && h->dim != 2) return fail(GLZ_INVALID, "the direct tile shapes are for planes");
+    const bool runs = (schedule & kRunsSchedule) != 0;
+    const int shape = runs ? glz::kEnsembleRuns : (schedule >> 1) & 3, one = (schedule >> 3) & 1;
+    if (shape > 0 && !runs && h->dim != 2) return fail(GLZ_INVALID, "the direct tile shapes are for planes");
     if (one && shape == 0) return fail(GLZ_INVALID, "one launch per step is a schedule of the direct tile shapes");
     std::vector<int> order(h->n);
     std::iota(order.begin(), order.end(), 0);
@@ -204,6 +212,13 @@ int set_schedule(glz_ens *h, int schedule, int max_ctas) {
     h->one_launch = one;
     CU(cudaMemcpyAsync(h->d_order, order.data(), h->n * sizeof(int), cudaMemcpyHostToDevice, h->stream));
     CU(cudaMemcpyAsync(h->d_prefix, prefix.data(), (h->n + 1) * sizeof(int), cudaMemcpyHostToDevice, h->stream));
+    std::vector<int2> list;
+    if (runs) {
+        list.reserve(h->total_tiles);
+        for (int i = 0; i < h->n; ++i)
+            for (int k = 0; k < prefix[i + 1] - prefix[i]; ++k) list.push_back(make_int2(order[i], k * glz::kEnsembleRun));
+        CU(cudaMemcpyAsync(h->d_runs, list.data(), list.size() * sizeof(int2), cudaMemcpyHostToDevice, h->stream));
+    }
     CU(cudaStreamSynchronize(h->stream));
     h->schedule = schedule;
     h->max_ctas = max_ctas;
@@ -224,6 +239,7 @@ glz::EnsembleLaunch launch_of(glz_ens *h, int colour) {
     e.maps = h->use_tma ? h->d_maps : nullptr;
     e.tile_prefix = h->d_prefix;
     e.order = h->d_order;
+    e.runs = h->d_runs;
     e.clock = h->d_clock;
     for (int k = 0; k < 2; ++k) e.vs_base[k] = h->vs_base[k];
     for (int k = 0; k < 3; ++k) e.vs_delta[k] = h->vs_delta[k];
@@ -389,13 +405,15 @@ static int create_batched(int n, const glz_model *models, const uint32_t *const 
 
     int rc;
     const size_t cells = (size_t)h->total_cells;
+    long long total_runs = 0;
+    for (const Replica &rep : h->reps) total_runs += tiles_of(h, rep, glz::kEnsembleRuns);
     if ((rc = dev_alloc(&h->labels, (size_t)h->total_sites)) || (rc = dev_alloc(&h->cell_type, cells)) ||
         (rc = dev_alloc(&h->vs_base[0], cells)) || (rc = dev_alloc(&h->vs_base[1], cells)) ||
         (rc = dev_alloc(&h->vs_delta[0], cells)) || (rc = dev_alloc(&h->vs_delta[1], cells)) ||
         (rc = dev_alloc(&h->vs_delta[2], cells)) || (rc = dev_alloc(&h->volc, cells * h->ncol)) ||
         (rc = dev_alloc(&h->anchor, cells * 4)) || (rc = dev_alloc(&h->first, cells)) || (rc = dev_alloc(&h->d_reps, (size_t)n)) ||
         (rc = dev_alloc(&h->d_maps, (size_t)n)) || (rc = dev_alloc(&h->d_prefix, (size_t)n + 1)) ||
-        (rc = dev_alloc(&h->d_order, (size_t)n)) || (rc = dev_alloc(&h->d_clock, 1)) ||
+        (rc = dev_alloc(&h->d_order, (size_t)n)) || (rc = dev_alloc(&h->d_runs, (size_t)total_runs)) || (rc = dev_alloc(&h->d_clock, 1)) ||
         (rc = dev_alloc(&h->d_barrier, 2)) ||
         (rc = dev_alloc(&h->error_flag, 1)) || (rc = dev_alloc(&h->medium, 2)))
         return bail(rc);
@@ -515,7 +533,7 @@ static int create_batched(int n, const glz_model *models, const uint32_t *const 
         if (glz::launch_recount(rl, h->stream) != cudaSuccess) return bail(fail(GLZ_DRIVER, "recount failed"));
     }
     if (!glz::ensemble_grid_cap(h->dim, h->n_off, h->uniform)) return bail(fail(GLZ_DRIVER, "kernel setup failed"));
-    if ((rc = set_schedule(h, 0, 0))) return bail(rc);
+    if ((rc = set_schedule(h, kRunsSchedule, 0))) return bail(rc);
     if (cudaStreamSynchronize(h->stream) != cudaSuccess)
         return bail(fail(GLZ_DRIVER, std::string("ensemble setup: ") + cudaGetErrorString(cudaGetLastError())));
     *out = h;
@@ -771,7 +789,8 @@ int glz_ens_autotune(glz_ens *h, uint64_t trial_steps, int *choice) {
     double best = 1e30;
     int best_i = 0, i = 0, rc = GLZ_OK;
     // (schedule, grid cap): replica order x tile shape, the windowed kernel
-    // at three grid sizes, the direct shapes at one block per tile
+    // at three grid sizes, the direct shapes at one block per tile; then the
+    // runs
     std::vector<std::pair<int, int>> cands;
     for (int shape = 0; shape < (h->dim == 2 ? 4 : 1); ++shape)
         for (int order = 0; order < 2; ++order) {
@@ -782,6 +801,7 @@ int glz_ens_autotune(glz_ens *h, uint64_t trial_steps, int *choice) {
                 cands.push_back({order + 2 * shape + 8, 0});  // the step's passes in one launch
             }
         }
+    cands.push_back({kRunsSchedule, 0});
     for (auto [sch, g] : cands) {
         if ((rc = set_schedule(h, sch, g))) break;
         double ms = 0.0;
@@ -884,7 +904,7 @@ void glz_ens_destroy(glz_ens *h) {
     cudaFree(h->labels); cudaFree(h->cell_type);
     for (auto *p : h->vs_base) cudaFree(p);
     for (auto *p : h->vs_delta) cudaFree(p);
-    cudaFree(h->volc); cudaFree(h->first); cudaFree(h->anchor); cudaFree(h->tables); cudaFree(h->connected);
+    cudaFree(h->volc); cudaFree(h->first); cudaFree(h->d_runs); cudaFree(h->anchor); cudaFree(h->tables); cudaFree(h->connected);
     cudaFree(h->d_reps); cudaFree(h->d_maps); cudaFree(h->d_prefix); cudaFree(h->d_order);
     cudaFree(h->d_clock); cudaFree(h->d_barrier); cudaFree(h->error_flag); cudaFree(h->medium);
     if (h->stream) cudaStreamDestroy(h->stream);

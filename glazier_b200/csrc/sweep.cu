@@ -1938,6 +1938,113 @@ static cudaError_t direct_ensemble_shape(const EnsembleLaunch &e, cudaStream_t s
                                        dim3(BX * BY), args, 0, stream);
 }
 
+// ---------------------------------------------------------------- runs of the ensemble
+//
+// One block per run of kEnsembleRun consecutive targets of a replica: the
+// direct sweep's warp-queued pass over every replica's runs at once. The
+// block copies its replica's launch into shared memory and draws its picks
+// before the programmatic wait (nothing of the step writes a launch or the
+// clock); every warp draws and compares its 128 targets, queues the unlike
+// ones with their labels and prices the queue. A replica's last run is all it
+// can waste, where the windowed kernel's tiles lose a quarter of their sites
+// on replicas of uneven sides, and each of its tiles waits for its launch to
+// be found and copied (64 monolayers of 128 to 1024 a side, 12.7 M sites: 254
+// us per MCS windowed, 278 in blocks of 32 x 8 targets priced where they lie).
+constexpr int kRunEach = kEnsembleRun / 256;  // targets a lane
+
+template <int DIM, int NOFF, bool UNIFORM>
+__global__ void __launch_bounds__(256, 4) run_ensemble_kernel(const __grid_constant__ EnsembleLaunch e) {
+    __shared__ SweepLaunch d;
+    __shared__ TypeSmem<false> types;
+    __shared__ uint2 pair[8][32 * kRunEach];  // (old, new) labels of each queued copy
+    __shared__ int queue[8][32 * kRunEach];
+    __shared__ uint8_t picks[8][32 * kRunEach];
+    const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    const int2 run = e.runs[blockIdx.x];
+    const EnsembleReplica &rep = e.replicas[run.x];
+    const EnsembleClock clock = *e.clock;
+    {
+        const int *src = reinterpret_cast<const int *>(&rep.a);
+        int *dst = reinterpret_cast<int *>(&d);
+        for (int i = tid; i < (int)(sizeof(SweepLaunch) / sizeof(int)); i += 256) dst[i] = src[i];
+    }
+    const unsigned long long pass = (unsigned long long)(clock.pass + e.colour);
+    const int32_t step = (int32_t)clock.step;
+    const int b = (int)(pass % 2), cur = (int)(pass % 3), next = cur == 2 ? 0 : cur + 1, prev = cur == 0 ? 2 : cur - 1;
+    const PassView v{e.colour,
+                     stream_key(rep.seed, step, e.colour, 0),
+                     stream_key(rep.seed, step, e.colour, 1),
+                     e.vs_base[b] + rep.cell_off,
+                     e.vs_delta[prev] + rep.cell_off,
+                     reinterpret_cast<unsigned long long *>(e.vs_delta[cur] + rep.cell_off)};
+    __syncthreads();
+    const TypeTables T = UNIFORM ? d.t : load_types<false>(d, types);
+    const GlobalPass acc{d, v};
+    const int targets = (d.g.w / 2) * (d.g.h / 2) * (DIM == 3 ? d.g.d / 2 : 1);
+    const int first = run.y + warp * 32 * kRunEach;
+    int pick[kRunEach];
+#pragma unroll
+    for (int k = 0; k < kRunEach; ++k) {
+        const int j = first + k * 32 + lane;
+        pick[k] = 0;
+        if (j < targets) {
+            int x, y, z;
+            direct_site<DIM>(d, e.colour, j, x, y, z);
+            pick[k] = pick_of<NOFF>(draw(v.key_pick, (uint32_t)((z * d.g.h + y) * d.g.w + x)));
+        }
+    }
+    grid_wait();
+    if (!UNIFORM) __syncthreads();  // the tables are in place
+    uint2 labels[kRunEach];
+#pragma unroll
+    for (int k = 0; k < kRunEach; ++k) {
+        const int j = first + k * 32 + lane;
+        labels[k] = make_uint2(0u, 0u);
+        if (j < targets) {
+            int x, y, z;
+            direct_site<DIM>(d, e.colour, j, x, y, z);
+            labels[k] = make_uint2(acc.label(x, y, z), picked_label<DIM, NOFF>(d, acc, x, y, z, pick[k]));
+        }
+    }
+    int total = 0;
+#pragma unroll
+    for (int k = 0; k < kRunEach; ++k) {
+        const bool unlike = labels[k].x != labels[k].y;
+        const unsigned m = __ballot_sync(0xffffffffu, unlike);
+        if (unlike) {
+            const int at = total + __popc(m & below);
+            queue[warp][at] = first + k * 32 + lane;
+            picks[warp][at] = (uint8_t)pick[k];
+            pair[warp][at] = labels[k];
+        }
+        total += __popc(m);
+    }
+    __syncwarp();
+    for (int q = lane; q < total; q += 32) {
+        int x, y, z;
+        direct_site<DIM>(d, e.colour, queue[warp][q], x, y, z);
+        const NeighbourReads<DIM, NOFF, GlobalPass> ln(d, acc, x, y, z);
+        direct_copy<DIM, NOFF, UNIFORM>(d, T, acc, ln, v.key_accept, x, y, z, picks[warp][q], pair[warp][q].x,
+                                        pair[warp][q].y);
+    }
+    // this block's share of the tally rotation over every replica's cells,
+    // which no thread of this pass reads
+    const int2 *base = e.vs_base[b];
+    int2 *next_base = e.vs_base[b ^ 1];
+    const long long *last_delta = e.vs_delta[prev];
+    long long *clear = e.vs_delta[next];
+    const long long share = (e.total_cells + gridDim.x - 1) / gridDim.x;
+    const long long from = share * blockIdx.x, to = from + share < e.total_cells ? from + share : e.total_cells;
+    for (long long l = from + tid; l < to; l += 256) {
+        int dv, ds;
+        unpack_delta(last_delta[l], dv, ds);
+        const int2 t = base[l];
+        next_base[l] = make_int2(t.x + dv, t.y + ds);
+        clear[l] = 0;
+    }
+}
+
 template <int NOFF, bool UNIFORM>
 static cudaError_t direct_ensemble_launch(const EnsembleLaunch &e, cudaStream_t stream) {
     if (e.total_tiles <= 0) return cudaSuccess;
@@ -1999,6 +2106,8 @@ static int lean_ensemble_cap() {
 
 template <int DIM, int NOFF, bool UNIFORM>
 static cudaError_t ensemble_launch(const EnsembleLaunch &e, cudaStream_t stream) {
+    if (e.tile_shape == kEnsembleRuns)
+        return launch_after(run_ensemble_kernel<DIM, NOFF, UNIFORM>, dim3((unsigned)e.total_tiles), 256, stream, e);
     if (lean_ensemble()) {
         const int cap = lean_ensemble_cap<DIM, NOFF, UNIFORM>();
         if (!cap) return cudaErrorInvalidConfiguration;
@@ -2019,7 +2128,7 @@ static cudaError_t ensemble_launch(const EnsembleLaunch &e, cudaStream_t stream)
 
 template <bool UNIFORM>
 static cudaError_t ensemble_any(const EnsembleLaunch &e, int dim, int n_off, cudaStream_t stream) {
-    if (e.tile_shape > 0) {
+    if (e.tile_shape > 0 && e.tile_shape != kEnsembleRuns) {
         if (dim != 2 || e.tile_shape > 3) return cudaErrorInvalidValue;
         return n_off == 4 ? direct_ensemble_launch<4, UNIFORM>(e, stream) : direct_ensemble_launch<8, UNIFORM>(e, stream);
     }

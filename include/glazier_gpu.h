@@ -223,7 +223,8 @@ int glz_ens_set_infection(glz_ens *h, int replica, int species, int from_type, i
  * windowed persistent kernel's 128 x 32 tiles at three grid sizes, and for
  * planes blocks of 32 x 8, 16 x 16 or 64 x 4 targets priced where they lie)
  * x colour schedule for those blocks (a launch per colour pass, or a step's
- * passes in one cooperative launch with a grid barrier between them).
+ * passes in one cooperative launch with a grid barrier between them); and the
+ * schedule an ensemble starts on, blocks of 1024 consecutive targets.
  * `choice` gets the index of the candidate kept. */
 int glz_ens_autotune(glz_ens *h, uint64_t trial_steps, int *choice);
 /* Choose a schedule directly: bit 0 the replica order (0 as given, 1 largest
