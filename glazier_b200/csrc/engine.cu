@@ -9,6 +9,8 @@
 
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <cmath>
 #include <cstdio>
@@ -29,8 +31,22 @@ namespace {
 thread_local std::string g_error = "no error";
 }
 
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
+
 namespace glz {
 void set_last_error(const std::string &msg) { g_error = msg; }
+
+void prefault(void *p, size_t bytes) {
+    constexpr size_t kLeast = 64 * 1024;
+    if (bytes < kLeast) return;
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    const size_t from = ((size_t)p + page - 1) / page * page, to = ((size_t)p + bytes) / page * page;
+    // a hint: where the kernel or the mapping does not take it, the copy
+    // faults the pages in as it did
+    if (to > from) madvise((void *)from, to - from, MADV_POPULATE_WRITE);
+}
 }
 
 namespace {
@@ -1166,6 +1182,7 @@ int glz_gpu_set_labels_device(glz_gpu *h, const uint32_t *labels, size_t sites) 
 int glz_gpu_labels(glz_gpu *h, uint32_t *out, size_t sites) {
     if (!h || !out) return fail(GLZ_INVALID, "null handle or buffer");
     if (sites != (size_t)h->g.sites) return fail(GLZ_INVALID, "the buffer is not one label per site");
+    glz::prefault(out, sites * sizeof(uint32_t));
     CU(cudaMemcpyAsync(out, h->labels, sites * sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
     CU(cudaStreamSynchronize(h->stream));
     return GLZ_OK;
@@ -1175,6 +1192,7 @@ int glz_gpu_field(glz_gpu *h, int index, double *out, size_t sites) {
     if (!h || !out) return fail(GLZ_INVALID, "null handle or buffer");
     if (index < 0 || index >= h->n_species) return fail(GLZ_INVALID, "no such species");
     if (sites != (size_t)h->g.sites) return fail(GLZ_INVALID, "the buffer is not one value per site");
+    glz::prefault(out, sites * sizeof(double));
     std::vector<float> f(sites);
     CU(cudaMemcpyAsync(f.data(), h->field_ptr(index, h->field_cur[index]), sites * sizeof(float),
                        cudaMemcpyDeviceToHost, h->stream));

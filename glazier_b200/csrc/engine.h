@@ -370,6 +370,13 @@ __device__ __forceinline__ int population_parity(const PopulationLaunch &a) {
     return (int)((a.clock ? a.clock->step : a.step) & 1);
 }
 
+// Have the pages of a host buffer that a copy is about to fill mapped in one
+// call: a fresh buffer's pages otherwise fault one by one inside the driver's
+// copy, which takes five times as long as the copy itself (51 MB in 64
+// lattices: 22 ms, 15 with this, 4.3 into pages already mapped). Changes no
+// content; memory that is mapped costs a page walk.
+void prefault(void *p, size_t bytes);
+
 // Record the message glz_last_error() returns on this thread.
 void set_last_error(const std::string &msg);
 

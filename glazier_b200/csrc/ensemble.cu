@@ -836,6 +836,7 @@ int glz_ens_labels(glz_ens *h, int replica, uint32_t *out, size_t sites) {
     if (g) return glz_gpu_labels(g, out, sites);
     const Replica &rep = h->reps[replica];
     if (sites != (size_t)rep.g.sites) return fail(GLZ_INVALID, "the buffer is not one label per site");
+    glz::prefault(out, sites * 4);
     CU(cudaMemcpyAsync(out, h->labels + rep.label_off, sites * 4, cudaMemcpyDeviceToHost, h->stream));
     CU(cudaStreamSynchronize(h->stream));
     return GLZ_OK;
