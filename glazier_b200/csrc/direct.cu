@@ -29,6 +29,7 @@
 
 #include <atomic>
 #include <cstdlib>
+#include <type_traits>
 
 #include "direct.cuh"
 
@@ -50,7 +51,7 @@ __device__ __forceinline__ DirectView direct_view(const SweepLaunch &a) {
     DirectView d;
     if (!a.clock) {
         d.v = PassView{a.colour, a.key_pick, a.key_accept, a.vs_base, a.vs_prev, a.vs_cur};
-        d.t = TermView{a.mom_base, a.mom_prev, a.mom_cur, a.field_cur};
+        d.t = TermView{a.mom_base, a.mom_prev, a.mom_cur, a.field_cur, nullptr};
         d.vs_next_base = a.vs_next_base;
         d.vs_clear = a.vs_clear;
         d.mom_next_base = a.mom_next_base;
@@ -69,7 +70,7 @@ __device__ __forceinline__ DirectView direct_view(const SweepLaunch &a) {
                    a.tal.vs_delta[prev],
                    reinterpret_cast<unsigned long long *>(a.tal.vs_delta[cur])};
     d.t = TermView{a.tal.mom_base[b], a.tal.mom_delta[prev],
-                   reinterpret_cast<unsigned long long *>(a.tal.mom_delta[cur]), c.field_cur};
+                   reinterpret_cast<unsigned long long *>(a.tal.mom_delta[cur]), c.field_cur, nullptr};
     d.vs_next_base = a.tal.vs_base[n];
     d.vs_clear = a.tal.vs_delta[next];
     d.mom_next_base = a.tal.mom_base[n];
@@ -131,13 +132,19 @@ constexpr int direct_blocks(int form, bool extras) {
     return extras && (form == kPlain || form == kBlock) ? 2 : 4;
 }
 
-template <int DIM, int NOFF, bool UNIFORM, int FORM, bool EXTRAS>
-__global__ void __launch_bounds__(kBlockThreads, direct_blocks(FORM, EXTRAS))
+template <int DIM, int NOFF, bool UNIFORM, int FORM, int TERMS>
+__global__ void __launch_bounds__(kBlockThreads, direct_blocks(FORM, TERMS > 0))
     direct_sweep_kernel(const __grid_constant__ SweepLaunch a) {
+    constexpr bool EXTRAS = TERMS > 0;
     const int targets = (a.g.w / 2) * (a.g.h / 2) * (DIM == 3 ? a.g.d / 2 : 1);
     __shared__ TypeSmem<EXTRAS> types;
     const TypeTables T = UNIFORM && !EXTRAS ? a.t : load_types<EXTRAS>(a, types);
-    const DirectView d = direct_view(a);
+    DirectView d = direct_view(a);
+    __shared__ float logs[TERMS == 2 ? kLogs : 1];
+    if (TERMS == 2) {
+        for (int k = (int)threadIdx.x; k < kLogs; k += (int)blockDim.x) logs[k] = k ? motility_log((float)k) : 0.0f;
+        d.t.logs = logs;
+    }
     const PassView &v = d.v;
     const GlobalPass acc{a, v};
     const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -159,13 +166,13 @@ __global__ void __launch_bounds__(kBlockThreads, direct_blocks(FORM, EXTRAS))
                 ln.load();
                 const uint32_t old = acc.label(x, y, z), nw = ln.picked(pick);
                 if (old != nw)
-                    direct_copy<DIM, NOFF, UNIFORM, GlobalPass, NeighbourLabels<DIM, NOFF, GlobalPass>, EXTRAS>(
+                    direct_copy<DIM, NOFF, UNIFORM, GlobalPass, NeighbourLabels<DIM, NOFF, GlobalPass>, TERMS>(
                         a, T, acc, ln, v.key_accept, x, y, z, pick, old, nw, &d.t);
             } else {
                 const uint32_t old = acc.label(x, y, z), nw = picked_label<DIM, NOFF>(a, acc, x, y, z, pick);
                 const NeighbourReads<DIM, NOFF, GlobalPass> ln(a, acc, x, y, z);
                 if (old != nw)
-                    direct_copy<DIM, NOFF, UNIFORM, GlobalPass, NeighbourReads<DIM, NOFF, GlobalPass>, EXTRAS>(
+                    direct_copy<DIM, NOFF, UNIFORM, GlobalPass, NeighbourReads<DIM, NOFF, GlobalPass>, TERMS>(
                         a, T, acc, ln, v.key_accept, x, y, z, pick, old, nw, &d.t);
             }
         }
@@ -230,7 +237,7 @@ __global__ void __launch_bounds__(kBlockThreads, direct_blocks(FORM, EXTRAS))
             int x, y, z;
             direct_site<DIM>(a, a.colour, queue[e], x, y, z);
             const NeighbourReads<DIM, NOFF, GlobalPass> ln(a, acc, x, y, z);
-            direct_copy<DIM, NOFF, UNIFORM, GlobalPass, NeighbourReads<DIM, NOFF, GlobalPass>, EXTRAS>(
+            direct_copy<DIM, NOFF, UNIFORM, GlobalPass, NeighbourReads<DIM, NOFF, GlobalPass>, TERMS>(
                 a, T, acc, ln, v.key_accept, x, y, z, picks[e], pair[e].x, pair[e].y, &d.t);
         }
         rotate_share<EXTRAS>(a, d);
@@ -265,7 +272,7 @@ __global__ void __launch_bounds__(kBlockThreads, direct_blocks(FORM, EXTRAS))
             direct_site<DIM>(a, a.colour, queue[warp][e], x, y, z);
             const int pick = picks[warp][e];
             const NeighbourReads<DIM, NOFF, GlobalPass> ln(a, acc, x, y, z);
-            direct_copy<DIM, NOFF, UNIFORM, GlobalPass, NeighbourReads<DIM, NOFF, GlobalPass>, EXTRAS>(
+            direct_copy<DIM, NOFF, UNIFORM, GlobalPass, NeighbourReads<DIM, NOFF, GlobalPass>, TERMS>(
                 a, T, acc, ln, v.key_accept, x, y, z, pick, acc.label(x, y, z),
                 picked_label<DIM, NOFF>(a, acc, x, y, z, pick), &d.t);
         }
@@ -331,14 +338,16 @@ cudaError_t launch_direct(const SweepLaunch &a, cudaStream_t stream) {
     attr[0].val.programmaticStreamSerializationAllowed = programmatic_launch();
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (!a.lean)  // every term: length, chemotaxis, connectivity, motility, drift, nematic, moments
-        return warp    ? cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kWarp, true>, b)
-               : wide  ? cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kBlockWide, true>, b)
-               : block ? cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kBlock, true>, b)
-                       : cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kPlain, true>, b);
-    return warp    ? cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kWarp, false>, b)
-           : block ? cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kBlock, false>, b)
-                   : cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kPlain, false>, b);
+    const auto launch = [&](auto terms) {  // the form's kernel with these terms
+        constexpr int TERMS = decltype(terms)::value;
+        if (warp) return cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kWarp, TERMS>, b);
+        if constexpr (TERMS > 0)
+            if (wide) return cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kBlockWide, TERMS>, b);
+        if (block) return cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kBlock, TERMS>, b);
+        return cudaLaunchKernelEx(&cfg, direct_sweep_kernel<DIM, NOFF, UNIFORM, kPlain, TERMS>, b);
+    };
+    if (a.lean) return launch(std::integral_constant<int, 0>{});
+    return a.has_motility ? launch(std::integral_constant<int, 2>{}) : launch(std::integral_constant<int, 1>{});
 }
 
 template cudaError_t launch_direct<2, 4, true>(const SweepLaunch &, cudaStream_t);

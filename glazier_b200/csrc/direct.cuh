@@ -139,8 +139,9 @@ struct NeighbourLabels : NeighbourReads<DIM, NOFF, Access> {
 // has read earlier in the pass (the target's label changes only by its own
 // commit and the neighbour is another colour, so they are still the pass's):
 // priced with price_and_commit's arithmetic operation for operation. `terms`
-// is used with EXTRAS only.
-template <int DIM, int NOFF, bool UNIFORM, class Access, class Labels, bool EXTRAS = false>
+// is used with TERMS only: 0 none past contact, volume and surface, 1 all but
+// motility, 2 all.
+template <int DIM, int NOFF, bool UNIFORM, class Access, class Labels, int TERMS = 0>
 __device__ __forceinline__ void direct_copy(const SweepLaunch &a, const TypeTables &T, const Access &acc,
                                             const Labels &neighbour, uint64_t key_accept, int x, int y, int z, int pick,
                                             uint32_t old, uint32_t nw, const TermView *terms = nullptr) {
@@ -152,20 +153,20 @@ __device__ __forceinline__ void direct_copy(const SweepLaunch &a, const TypeTabl
     const int t_new = UNIFORM ? a.uniform_type : acc.type(nw);
     // the moment commit's anchors, read here so the commit does not wait
     int4 an_old = make_int4(0, 0, 0, 0), an_new = an_old;
-    if (EXTRAS && a.tracks) {
+    if (TERMS && a.tracks) {
         an_old = anchor_of(a, old);
         an_new = anchor_of(a, nw);
     }
     float delta = 0.0f;
     int like_old = 0, like_new = 0;
-    uint32_t present = 0;  // EXTRAS: ring positions of `old` among the energy neighbours, as bits of the veto's cube
+    uint32_t present = 0;  // TERMS: ring positions of `old` among the energy neighbours, as bits of the veto's cube
     if (UNIFORM) {
 #pragma unroll
         for (int k = 0; k < NOFF; ++k) {
             const uint32_t ln = neighbour(k);
             like_old += ln == old;
             like_new += ln == nw;
-            if (EXTRAS && ln == old) present |= 1u << cube_bit<DIM, NOFF>(k);
+            if (TERMS && ln == old) present |= 1u << cube_bit<DIM, NOFF>(k);
         }
         delta = __fmul_rn(a.uniform_contact, (float)(like_old - like_new));
     } else {
@@ -183,11 +184,11 @@ __device__ __forceinline__ void direct_copy(const SweepLaunch &a, const TypeTabl
             delta = __fadd_rn(delta, is_new ? 0.0f : j_new);
             like_old += is_old;
             like_new += is_new;
-            if (EXTRAS && is_old) present |= 1u << cube_bit<DIM, NOFF>(k);
+            if (TERMS && is_old) present |= 1u << cube_bit<DIM, NOFF>(k);
         }
     }
     if (old != 0 && like_old == 0 && !acc.keeps_other_colour(old)) return;
-    if (EXTRAS && old != 0 && a.g.ring_n > 0 && T.connected[t_old]) {
+    if (TERMS && old != 0 && a.g.ring_n > 0 && T.connected[t_old]) {
         // the connectivity veto (lib.rs:511-521); the ring positions the
         // energy neighbourhood leaves out are read here
 #pragma unroll
@@ -208,24 +209,24 @@ __device__ __forceinline__ void direct_copy(const SweepLaunch &a, const TypeTabl
     unpack_delta(prev_new, dv, ds);
     const int vol_new = base_new.x + dv, surf_new = base_new.y + ds;
     delta = size_terms<UNIFORM>(a, T, old, nw, t_old, t_new, vol_old, vol_new, surf_old, surf_new, ds_old, ds_new, delta);
-    if (EXTRAS && (a.has_length || a.has_chemotaxis || a.has_external || a.has_motility || a.has_nematic))
-        delta = extra_terms<DIM, NOFF>(a, T, *terms, old, nw, t_old, t_new, vol_old, vol_new, x, y, z, pick, target, delta);
+    if (TERMS && (a.has_length || a.has_chemotaxis || a.has_external || TERMS == 2 || a.has_nematic))
+        delta = extra_terms<DIM, NOFF, TERMS == 2>(a, T, *terms, old, nw, t_old, t_new, vol_old, vol_new, x, y, z, pick, target, delta);
     const float u = to_f32(draw(key_accept, target));
     if (!(delta <= 0.0f || u < metropolis_exp(__fmul_rn(-delta, a.beta)))) return;
-    if (EXTRAS && a.has_motility) {
+    if (TERMS == 2) {
         const int k = atomicAdd(a.pending_count, 1);
-        a.pending[k] = make_uint2(target, nw);
+        a.pending[k] = make_uint4(target, nw, __float_as_uint(nw != 0 ? T.max_activity[t_new] : 0.0f), 0u);
     } else {
         acc.put(target, x, y, z, nw);
     }
     if (old != 0) acc.tally(old, -1, ds_old);
     if (nw != 0) acc.tally(nw, 1, ds_new);
-    if (EXTRAS && a.tracks) commit_moments<DIM>(a, terms->cur, old, nw, an_old, an_new, x, y, z);
+    if (TERMS && a.tracks) commit_moments<DIM>(a, terms->cur, old, nw, an_old, an_new, x, y, z);
 }
 
 // The whole attempt at target (x, y, z): its pick, its two labels, and the
 // copy when they differ.
-template <int DIM, int NOFF, bool UNIFORM, class Access, bool EXTRAS = false>
+template <int DIM, int NOFF, bool UNIFORM, class Access, int TERMS = 0>
 __device__ __forceinline__ void direct_target(const SweepLaunch &a, const TypeTables &T, const Access &acc, uint64_t key_pick,
                                               uint64_t key_accept, int x, int y, int z,
                                               const TermView *terms = nullptr) {
@@ -233,7 +234,7 @@ __device__ __forceinline__ void direct_target(const SweepLaunch &a, const TypeTa
     const uint32_t old = acc.label(x, y, z), nw = picked_label<DIM, NOFF>(a, acc, x, y, z, pick);
     const NeighbourReads<DIM, NOFF, Access> ln(a, acc, x, y, z);
     if (old != nw)
-        direct_copy<DIM, NOFF, UNIFORM, Access, NeighbourReads<DIM, NOFF, Access>, EXTRAS>(a, T, acc, ln, key_accept, x, y,
+        direct_copy<DIM, NOFF, UNIFORM, Access, NeighbourReads<DIM, NOFF, Access>, TERMS>(a, T, acc, ln, key_accept, x, y,
                                                                                            z, pick, old, nw, terms);
 }
 

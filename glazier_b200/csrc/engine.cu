@@ -129,7 +129,7 @@ struct glz_gpu {
     bool has_motility = false, has_nematic = false;
     float *nematic = nullptr;  // 2 per site, with the nematic term
     float *activity = nullptr;  // sites, with motility
-    uint2 *pending = nullptr;   // a motility pass's accepted copies
+    uint4 *pending = nullptr;   // a motility pass's accepted copies
     int *pending_count = nullptr;  // by the pass's parity
     int substeps[glz::kMaxSpecies] = {};
     float fd[glz::kMaxSpecies] = {}, fdecay[glz::kMaxSpecies] = {};
@@ -552,6 +552,7 @@ int step_labels(glz_gpu *h, bool clocked) {
     a.t = h->tables();
     a.labels = h->labels;
     a.cell_type = h->cell_type;
+    a.n_types = h->n_types;
     a.n_labels = (int)h->n_labels;
     a.cap = (int)h->cap;
     a.has_pop = h->has_pop;
@@ -910,7 +911,7 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
     std::vector<float> contact(nt * nt), tv(nt), lv(nt), ts(nt), ls(nt);
     std::vector<double> tl(nt), ll(nt), divv(nt), death(nt);
     std::vector<uint8_t> conn(nt);
-    bool has_conn = false;
+    bool has_conn = false, has_division = false;
     for (int a = 0; a < nt * nt; ++a) contact[a] = (float)m->contact[a];
     for (int k = 0; k < nt; ++k) {
         tv[k] = (float)at(m->target_volume, k);
@@ -924,9 +925,11 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
         conn[k] = m->connected ? (m->connected[k] != 0) : 0;
         has_conn |= conn[k] != 0;
         h->has_length |= ll[k] != 0.0;
+        has_division |= divv[k] > 0.0;
         h->has_pop |= divv[k] > 0.0 || death[k] > 0.0;
     }
-    h->tracks = h->has_length || h->has_pop || h->has_nematic;
+    // moment sums serve the length and nematic terms and a division's cut
+    h->tracks = h->has_length || has_division || h->has_nematic;
     std::vector<double> lnem(nt);
     for (int k = 0; k < nt; ++k) lnem[k] = at(m->lambda_nematic, k);
     std::vector<float> maxact(nt), lamact(nt);
@@ -1014,7 +1017,7 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
     // 4096^2 and 8192^2 it measured slower than the windowed lean kernel
     // (0.169 against 0.145 ms per MCS at 4096^2, L2 flushed).
     const char *band_env = std::getenv("GLAZIER_SWEEP_BAND");
-    h->band = h->lean && g.dim == 2 && band_env && band_env[0] == '1' && glz::band_sweep_fits(w, hh);
+    h->band = h->lean && !h->has_pop && g.dim == 2 && band_env && band_env[0] == '1' && glz::band_sweep_fits(w, hh);
     if (h->band) h->direct = h->cluster = false;
     h->host_tv = tv;
     h->host_lv = lv;

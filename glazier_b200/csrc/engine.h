@@ -130,10 +130,9 @@ struct SweepLaunch {
     const float *nematic;
     // Motility reads labels and activity two sites from the target, where
     // same-colour targets change during the pass, so a pass with it leaves
-    // both as they were and lists its accepted copies (target, new label)
-    // for launch_apply_copies.
+    // both as they were and lists its accepted copies for launch_apply_copies.
     const float *activity;
-    uint2 *pending;
+    uint4 *pending;  // target, new label, its type's maximum activity (f32 bits)
     int *pending_count;  // this pass's, and the other pass parity's (cleared for the next pass)
     int *pending_clear;
     int use_tma;
@@ -336,6 +335,7 @@ struct PopulationLaunch {
     TypeTables t;
     uint32_t *labels;
     uint8_t *cell_type;
+    int n_types;
     int n_labels;            // without n_live
     int cap;
     int has_pop, tracks;     // has_pop 0: the infection rule alone

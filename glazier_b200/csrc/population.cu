@@ -51,8 +51,8 @@ __device__ __forceinline__ double along_cut(const Geometry &g, const int *anchor
 
 // What cell l (of a population model) plans: 0 nothing, kDivision (its cut
 // into the plan table) or kDeath.
-__device__ __forceinline__ int plan_of(const PopulationLaunch &a, int l, int t, int v, const long long *m) {
-    const double div_vol = a.t.division_volume[t];
+__device__ __forceinline__ int plan_of(const PopulationLaunch &a, int l, double div_vol, double death_rate, int v,
+                                       const long long *m) {
     if (v <= 0) return 0;
     if (div_vol > 0.0 && (double)v >= div_vol && v >= 4) {
         const double dn = (double)v;
@@ -105,35 +105,52 @@ __device__ __forceinline__ int plan_of(const PopulationLaunch &a, int l, int t, 
         p[5] = v2;
         return kDivision;
     }
-    if (a.t.death_rate[t] > 0.0) {
+    if (death_rate > 0.0) {
         const uint64_t key =
             a.clock ? stream_key(a.seed, (int32_t)a.clock->step, kPopulationStream, 0) : a.key_death;
-        if (to_f64(draw(key, (uint32_t)l)) < a.t.death_rate[t]) return kDeath;
+        if (to_f64(draw(key, (uint32_t)l)) < death_rate) return kDeath;
     }
     return 0;
 }
 
+// Every read of a label is requested at once, the label live or not (the
+// arrays hold the capacity), and the types' rates come from shared memory:
+// the count, then the tallies, types, dose and rates each behind the one
+// before were six round trips.
 __global__ void __launch_bounds__(128) labels_kernel(const __grid_constant__ PopulationLaunch a) {
-    grid_wait();
+    __shared__ double rates[2][kSmemTypes];  // division volume, death rate
+    const bool held = a.has_pop && a.n_types <= kSmemTypes;
+    if (held && (int)threadIdx.x < a.n_types) {
+        rates[0][threadIdx.x] = a.t.division_volume[threadIdx.x];
+        rates[1][threadIdx.x] = a.t.death_rate[threadIdx.x];
+    }
+    const double *const division = held ? rates[0] : a.t.division_volume;
+    const double *const death = held ? rates[1] : a.t.death_rate;
+    // the slots at the end of the step's passes (the clock advances after it)
+    const long long p = a.clock ? a.clock->pass + a.g.ncol : a.pass;
+    int2 *const base = a.tal.vs_base[p % 2];
+    long long *const delta = a.tal.vs_delta[(p + 2) % 3];
     const int l = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool room = l < (a.n_live ? a.cap : a.n_labels);
+    __syncthreads();
+    grid_wait();
+    int t = room ? a.cell_type[l] : 0;
+    const long long dose = room && a.infect_from >= 0 ? (long long)a.dose[l] : 0;
+    const long long change = room && a.has_pop ? delta[l] : 0;
+    int2 b = room && a.has_pop ? base[l] : make_int2(0, 0);
     const int n = a.n_live ? *a.n_live : a.n_labels;
     if (a.has_pop && l == 0 && a.seen_step >= 0) *a.seen = ((unsigned long long)a.seen_step << 32) | (unsigned)n;
     int event = 0;
     if (l < n) {
-        int t = a.cell_type[l];
-        if (a.infect_from >= 0 && l > 0 && t == a.infect_from && (long long)a.dose[l] >= a.infect_threshold) {
+        if (a.infect_from >= 0 && l > 0 && t == a.infect_from && dose >= a.infect_threshold) {
             t = a.infect_to;
             a.cell_type[l] = (uint8_t)t;
         }
         if (a.has_pop) {
-            // the slots at the end of the step's passes
-            const long long p = a.clock ? a.clock->pass + a.g.ncol : a.pass;
-            int2 *const base = a.tal.vs_base[p % 2];
-            long long *const delta = a.tal.vs_delta[(p + 2) % 3];
             int dv, ds;
-            unpack_delta(delta[l], dv, ds);
-            const int2 b = base[l];
-            base[l] = make_int2(b.x + dv, b.y + ds);
+            unpack_delta(change, dv, ds);
+            b = make_int2(b.x + dv, b.y + ds);
+            base[l] = b;
             delta[l] = 0;
             long long m[11];
             if (a.tracks) {
@@ -149,7 +166,7 @@ __global__ void __launch_bounds__(128) labels_kernel(const __grid_constant__ Pop
                         mom_delta[k] = 0;
                     }
             }
-            if (l > 0) event = plan_of(a, l, t, b.x + dv, m);
+            if (l > 0) event = plan_of(a, l, division[t], death[t], b.x, m);
             a.mode[l] = (unsigned char)event;
             a.moved[l] = 0;
         }
@@ -277,9 +294,10 @@ cudaError_t launch_step_labels(const PopulationLaunch &a, cudaStream_t stream) {
     const int n = a.n_live ? a.cap : a.n_labels;
     if (cudaError_t e = launch_after(labels_kernel, dim3((unsigned)((n + 127) / 128)), 128, stream, a)) return e;
     if (!a.has_pop) return cudaSuccess;
-    // at most eight blocks an SM, so a step without an event starts few
-    const long long sites = ((long long)a.g.sites + 255) / 256;
-    const dim3 grid((unsigned)(sites < 1184 ? sites : 1184));
+    // at most two blocks an SM up to 2^20 sites, so a step without an event
+    // starts few, and eight past it
+    const long long sites = ((long long)a.g.sites + 255) / 256, most = a.g.sites <= (1 << 20) ? 296 : 1184;
+    const dim3 grid((unsigned)(sites < most ? sites : most));
     if (cudaError_t e = launch_after(count_kernel, grid, 256, stream, a)) return e;
     return launch_after(apply_kernel, grid, 256, stream, a);
 }

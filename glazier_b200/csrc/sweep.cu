@@ -134,8 +134,11 @@ template <int DIM, int NOFF>
 __device__ __noinline__ float tile_extra_terms(const SweepLaunch &a, uint32_t old, uint32_t nw, int t_old, int t_new,
                                                int vol_old, int vol_new, int x, int y, int z, int pick,
                                                uint32_t target, float delta) {
-    const TermView v{a.mom_base, a.mom_prev, a.mom_cur, a.field_cur};
-    return extra_terms<DIM, NOFF>(a, a.t, v, old, nw, t_old, t_new, vol_old, vol_new, x, y, z, pick, target, delta);
+    const TermView v{a.mom_base, a.mom_prev, a.mom_cur, a.field_cur, nullptr};
+    if (!a.has_motility)
+        return extra_terms<DIM, NOFF, false>(a, a.t, v, old, nw, t_old, t_new, vol_old, vol_new, x, y, z, pick, target,
+                                             delta);
+    return extra_terms<DIM, NOFF, true>(a, a.t, v, old, nw, t_old, t_new, vol_old, vol_new, x, y, z, pick, target, delta);
 }
 
 template <int DIM>
@@ -251,7 +254,7 @@ __device__ __forceinline__ void price_and_commit(const SweepLaunch &a, const int
 
     if (EXTRAS && a.has_motility) {
         const int k = atomicAdd(a.pending_count, 1);
-        a.pending[k] = make_uint2(target, nw);
+        a.pending[k] = make_uint4(target, nw, __float_as_uint(nw != 0 ? a.t.max_activity[t_new] : 0.0f), 0u);
     } else {
         a.labels[target] = nw;
     }
@@ -1381,28 +1384,30 @@ static cudaError_t launch_any(const SweepLaunch &a, cudaStream_t stream) {
     return cudaErrorInvalidValue;
 }
 
-// The pass's listed copies; the other pass parity's count, which the copies
-// before these emptied, is set to zero for the next pass.
-__global__ void apply_copies_kernel(const __grid_constant__ SweepLaunch a, float *activity) {
+// The pass's listed copies (target, new label, its type's maximum); the other
+// pass parity's count, which the copies before these emptied, is set to zero
+// for the next pass. An entry is requested beside the count, so a copy is one
+// round trip and its writes.
+__global__ void __launch_bounds__(256) apply_copies_kernel(const __grid_constant__ SweepLaunch a, float *activity, int most) {
     grid_wait();
+    int k = blockIdx.x * blockDim.x + threadIdx.x;
+    uint4 p = k < most ? a.pending[k] : make_uint4(0u, 0u, 0u, 0u);
     const int count = *a.pending_count;
-    if (blockIdx.x == 0 && threadIdx.x == 0) *a.pending_clear = 0;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
-        const uint2 p = a.pending[k];
+    if (k == 0) *a.pending_clear = 0;
+    while (k < count) {
         a.labels[p.x] = p.y;
-        if (p.y != 0) {
-            const float top = a.t.max_activity[a.cell_type[p.y]];
-            if (top > 0.0f) activity[p.x] = top;
-        }
+        const float top = __uint_as_float(p.z);
+        if (top > 0.0f) activity[p.x] = top;
+        k += gridDim.x * blockDim.x;
+        if (k < count) p = a.pending[k];
     }
 }
 
 cudaError_t launch_apply_copies(const SweepLaunch &a, float *activity, cudaStream_t stream) {
-    // at most one copy per target, and a pass has sites / colours targets;
-    // an accepted one is rare enough that a fraction of that grid covers them
+    // at most one copy per target, and a pass has sites / colours targets; an
+    // accepted one is rare enough that a fraction of that grid covers them
     const int most = a.g.sites / a.g.ncol + 1;
-    const int blocks = (most + 2047) / 2048;
-    return launch_after(apply_copies_kernel, dim3((unsigned)blocks), 256, stream, a, activity);
+    return launch_after(apply_copies_kernel, dim3((unsigned)((most + 2047) / 2048)), 256, stream, a, activity, most);
 }
 
 __global__ void activity_decay_kernel(float *activity, int sites) {

@@ -191,8 +191,10 @@ static cudaError_t launch_counts(const RecountLaunch &a, cudaStream_t stream) {
         for (int axis = 0; axis < 3; ++axis)
             if (a.g.off[k][axis] != neighbour_offset<DIM, NOFF>(k, axis)) return cudaErrorInvalidValue;
     const int bx = a.g.w >= 256 ? 256 : (a.g.w + 31) / 32 * 32;
-    const int rows = a.g.h * a.g.d;
-    const dim3 grid((unsigned)((a.g.w + bx - 1) / bx), (unsigned)(rows < 65535 ? rows : 65535));
+    // at a step's end few blocks, which mostly find no event
+    const int rows = a.g.h * a.g.d, across = (a.g.w + bx - 1) / bx;
+    const int most = a.flags && a.g.sites <= (1 << 20) ? (296 * (256 / bx) + across - 1) / across : 65535;
+    const dim3 grid((unsigned)across, (unsigned)(rows < most ? rows : most));
     return launch_after(recount_counts_kernel<DIM, NOFF>, grid, bx, stream, a);
 }
 

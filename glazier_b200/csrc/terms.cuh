@@ -18,6 +18,7 @@ struct TermView {
     const long long *base, *prev;
     unsigned long long *cur;
     unsigned field_cur;
+    const float *logs;  // 0, then motility_log of 1 .. kLogs - 1, in shared memory; or null
 };
 
 __device__ __forceinline__ const float *field_of(const SweepLaunch &a, unsigned field_cur, int s) {
@@ -224,46 +225,68 @@ __device__ __forceinline__ double nematic_delta(const TypeTables &T, int type, l
     return -T.lambda_nematic[type] * (now - before);
 }
 
+// Logs of the whole activities an Act memory runs through (it starts at its
+// maximum and runs down by one a step): motility_log's own values, taken once
+// a block, so a neighbour's log is a table read; the entry of 0 is zero, what
+// a neighbour that does not count adds.
+constexpr int kLogs = 256;
+
+__device__ __forceinline__ int whole_activity(float v) {
+    const int k = (int)v;
+    return k < kLogs && (float)k == v ? k : -1;
+}
+
 // The geometric mean of the activity over the sites of `label` around `site`
 // (x, y, z), the site itself included; zero as soon as one of them has none
 // left (lib.rs:391-424, motility.rs:58-79). Labels and activity are the
-// pass's starting values: a pass with motility defers its writes. The
-// neighbours' labels and activities are requested together and the logs
-// taken without a branch (one that does not count adds a zero, which leaves
-// the sum's bits alone), so the mean is two memory round trips and one
-// chain of additions in the neighbourhood's order, not a round trip a
-// neighbour.
+// pass's starting values: a pass with motility defers its writes.
 template <int DIM, int NOFF>
-__device__ __forceinline__ float activity_mean(const SweepLaunch &a, uint32_t site, int x, int y, int z,
-                                               uint32_t label) {
+__device__ __noinline__ float activity_mean(const SweepLaunch &a, uint32_t site, int x, int y, int z, uint32_t label) {
     const float here = a.activity[site];
     if (!(here > 0.0f)) return 0.0f;
     const Around r = around<DIM>(a.g, x, y, z);
-    float v[NOFF];
-    bool like[NOFF];
-#pragma unroll
+    float log_sum = motility_log(here), count = 1.0f;
     for (int k = 0; k < NOFF; ++k) {
         const uint32_t n = neighbour_site<DIM, NOFF>(a.g, r, x, y, z, k);
-        v[k] = a.activity[n];
-        like[k] = n != site && a.labels[n] == label;
+        if (n == site || a.labels[n] != label) continue;
+        const float v = a.activity[n];
+        if (!(v > 0.0f)) return 0.0f;
+        log_sum = __fadd_rn(log_sum, motility_log(v));
+        count = __fadd_rn(count, 1.0f);
     }
+    return metropolis_exp(__fdiv_rn(log_sum, count));
+}
+
+// The same mean from values already read: `here` the site's activity, v its
+// neighbours', bit k of `like` whether neighbour k carries the label. `known`
+// is false when an activity that counts is not whole (the mean is then not
+// taken here).
+template <int NOFF>
+__device__ __forceinline__ float table_mean(const float *logs, float here, const float *v, uint32_t like, bool &known) {
+    known = true;
+    if (!(here > 0.0f)) return 0.0f;
+    int at[NOFF], least = whole_activity(here);
     bool spent = false;
-    int count = 1;
+    const int own = least;
 #pragma unroll
     for (int k = 0; k < NOFF; ++k) {
-        spent |= like[k] && !(v[k] > 0.0f);
-        count += like[k];
+        const bool counts = like >> k & 1u;
+        at[k] = counts ? whole_activity(v[k]) : 0;
+        least = min(least, at[k]);
+        spent |= counts && !(v[k] > 0.0f);
     }
     if (spent) return 0.0f;
-    float log_sum = motility_log(here);
+    known = least >= 0;
+    if (!known) return 0.0f;
+    float log_sum = logs[own];
 #pragma unroll
-    for (int k = 0; k < NOFF; ++k) log_sum = __fadd_rn(log_sum, like[k] ? motility_log(v[k]) : 0.0f);
-    return metropolis_exp(__fdiv_rn(log_sum, (float)count));
+    for (int k = 0; k < NOFF; ++k) log_sum = __fadd_rn(log_sum, logs[at[k]]);
+    return metropolis_exp(__fdiv_rn(log_sum, (float)(1 + __popc(like))));
 }
 
 // The length, nematic, chemotaxis, motility and drift terms of a copy
-// (cpu.rs:291-332, 341-395).
-template <int DIM, int NOFF>
+// (cpu.rs:291-332, 341-395); the motility term with MOTILE.
+template <int DIM, int NOFF, bool MOTILE>
 __device__ __forceinline__ float extra_terms(const SweepLaunch &a, const TypeTables &T, const TermView &v, uint32_t old, uint32_t nw,
                                              int t_old, int t_new, int vol_old, int vol_new, int x, int y, int z,
                                              int pick, uint32_t target, float delta) {
@@ -322,11 +345,30 @@ __device__ __forceinline__ float extra_terms(const SweepLaunch &a, const TypeTab
     }
     // Motility (cpu.rs:346-352, lib.rs:656-663): the cell's memory pulls it
     // where it has been.
-    if (a.has_motility && nw != 0) {
+    if (MOTILE && nw != 0) {
         const float lam = T.lambda_activity[t_new], top = T.max_activity[t_new];
         if (lam != 0.0f && top > 0.0f) {
-            const float into = activity_mean<DIM, NOFF>(a, source, sx, sy, sz, nw);
-            const float out_of = activity_mean<DIM, NOFF>(a, target, x, y, z, old);
+            float into = 0.0f, out_of = 0.0f;
+            bool known_into = false, known_out = false;
+            if (v.logs) {
+                // every value of both means is requested before any is used
+                const Around rs = around<DIM>(a.g, sx, sy, sz);
+                float at_source[NOFF], at_target[NOFF];
+                uint32_t like_new = 0, like_old = 0;
+#pragma unroll
+                for (int k = 0; k < NOFF; ++k) {
+                    const uint32_t n = neighbour_site<DIM, NOFF>(a.g, rs, sx, sy, sz, k);
+                    const uint32_t m = neighbour_site<DIM, NOFF>(a.g, r, x, y, z, k);
+                    at_source[k] = a.activity[n];
+                    at_target[k] = a.activity[m];
+                    like_new |= (uint32_t)(n != source && a.labels[n] == nw) << k;
+                    like_old |= (uint32_t)(m != target && a.labels[m] == old) << k;
+                }
+                into = table_mean<NOFF>(v.logs, a.activity[source], at_source, like_new, known_into);
+                out_of = table_mean<NOFF>(v.logs, a.activity[target], at_target, like_old, known_out);
+            }
+            if (!known_into) into = activity_mean<DIM, NOFF>(a, source, sx, sy, sz, nw);
+            if (!known_out) out_of = activity_mean<DIM, NOFF>(a, target, x, y, z, old);
             delta = __fsub_rn(delta, __fmul_rn(__fdiv_rn(lam, top), __fsub_rn(into, out_of)));
         }
     }

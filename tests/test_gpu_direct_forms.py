@@ -183,3 +183,39 @@ def test_a_volume_of_every_term_in_wide_blocks(device):
     replay.step(3)
     _same(gpu, replay, 1)
     gpu.close()
+
+
+@pytest.mark.parametrize("depth", [1, 12])
+@pytest.mark.parametrize("top", [20.0, 20.5, 255.0, 256.0, 300.0])
+def test_activities_in_the_log_table_and_past_it(device, depth, top):
+    """Act memories that run through whole activities below 256 (read from a
+    block's table of logs), through halves, and past the table."""
+    cell = dict(target_volume=64.0, lambda_volume=2.0, max_activity=top, lambda_activity=80.0)
+    model = Model(width=48, height=44, depth=depth, contact=[0.0, 16.0, 16.0, 16.0, 8.0, 9.0, 16.0, 9.0, 8.0],
+                  types=[CellType(), CellType(**cell), CellType(target_volume=64.0, lambda_volume=2.0)],
+                  temperature=12.0, neighbour_order=2, seed=31)
+    start = Start.tiled(model, 8 if depth == 1 else 4)
+    start.set_cell_types(1 + np.arange(start.n_cells) % 2)
+    gpu = device.GpuSimulation.from_start(start)
+    replay = ReplayOracle.from_start(start)
+    gpu.step(15)
+    replay.step(15)
+    _same(gpu, replay, 0)
+    gpu.close()
+
+
+def test_deaths_without_divisions_keep_no_moments(device):
+    """Death alone needs no moment sums: every form of the pass still follows
+    the replay through the deaths."""
+    model = Model(width=96, height=80, contact=[0.0, 16.0, 16.0, 8.0],
+                  types=[CellType(), CellType(target_volume=64.0, lambda_volume=2.0, death_rate=0.05)],
+                  temperature=10.0, neighbour_order=2, seed=37)
+    start = Start.tiled(model, 8)
+    gpu = device.GpuSimulation.from_start(start)
+    replay = ReplayOracle.from_start(start)
+    for chunk in (1, 9, 20):
+        gpu.step(chunk)
+        replay.step(chunk)
+        _same(gpu, replay, 0)
+    assert int((gpu.volumes()[1:] == 0).sum()) > 0
+    gpu.close()
