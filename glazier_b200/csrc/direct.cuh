@@ -57,14 +57,29 @@ struct GlobalPass {
 // Site (x, y, z) of target j of colour `colour` in a direct pass.
 template <int DIM>
 __device__ __forceinline__ void direct_site(const SweepLaunch &a, int colour, int j, int &x, int &y, int &z) {
-    const uint32_t row = udiv(a.g.div_hw, (uint32_t)j), plane = udiv(a.g.div_hh, row);
+    const uint32_t row = udiv(a.g.div_hw, (uint32_t)j);
     x = 2 * (int)((uint32_t)j - row * (uint32_t)(a.g.w / 2)) + (colour & 1);
-    y = 2 * (int)(row - plane * (uint32_t)(a.g.h / 2)) + ((colour >> 1) & 1);
-    z = DIM == 3 ? 2 * (int)plane + ((colour >> 2) & 1) : 0;
+    if constexpr (DIM == 2) {
+        y = 2 * (int)row + ((colour >> 1) & 1);
+        z = 0;
+    } else {
+        const uint32_t plane = udiv(a.g.div_hh, row);
+        y = 2 * (int)(row - plane * (uint32_t)(a.g.h / 2)) + ((colour >> 1) & 1);
+        z = 2 * (int)plane + ((colour >> 2) & 1);
+    }
 }
 
-// The offset of neighbour `pick`, chosen among compile-time constants (the
-// 26-neighbourhood has a closed form) rather than read from a table.
+// The offsets of a neighbourhood along an axis, one more than each in two
+// bits, neighbour k's at bit 2 k.
+template <int DIM, int NOFF>
+__host__ __device__ constexpr uint64_t packed_offsets(int axis) {
+    uint64_t bits = 0;
+    for (int k = 0; k < NOFF; ++k) bits |= (uint64_t)(neighbour_offset<DIM, NOFF>(k, axis) + 1) << (2 * k);
+    return bits;
+}
+
+// The offset of neighbour `pick`: a shift of a constant an axis (the
+// 26-neighbourhood has a closed form), not a chain of selects or a table.
 template <int DIM, int NOFF>
 __device__ __forceinline__ void pick_offset(int pick, int &dx, int &dy, int &dz) {
     if constexpr (DIM == 3 && NOFF == 26) {
@@ -72,14 +87,17 @@ __device__ __forceinline__ void pick_offset(int pick, int &dx, int &dy, int &dz)
         dy = neighbour_offset<3, 26>(pick, 1);
         dz = neighbour_offset<3, 26>(pick, 2);
     } else {
-        dx = dy = dz = 0;
-#pragma unroll
-        for (int k = 0; k < NOFF; ++k)
-            if (k == pick) {
-                dx = neighbour_offset<DIM, NOFF>(k, 0);
-                dy = neighbour_offset<DIM, NOFF>(k, 1);
-                dz = neighbour_offset<DIM, NOFF>(k, 2);
-            }
+        constexpr uint64_t X = packed_offsets<DIM, NOFF>(0), Y = packed_offsets<DIM, NOFF>(1),
+                           Z = packed_offsets<DIM, NOFF>(2);
+        if constexpr (2 * NOFF <= 32) {
+            dx = (int)((uint32_t)X >> (2 * pick) & 3u) - 1;
+            dy = (int)((uint32_t)Y >> (2 * pick) & 3u) - 1;
+            dz = DIM == 3 ? (int)((uint32_t)Z >> (2 * pick) & 3u) - 1 : 0;
+        } else {
+            dx = (int)(X >> (2 * pick) & 3u) - 1;
+            dy = (int)(Y >> (2 * pick) & 3u) - 1;
+            dz = (int)(Z >> (2 * pick) & 3u) - 1;
+        }
     }
 }
 
@@ -90,7 +108,7 @@ __device__ __forceinline__ uint32_t picked_label(const SweepLaunch &a, const Acc
     pick_offset<DIM, NOFF>(pick, dx, dy, dz);
     const int nx = x + dx < 0 ? a.g.w - 1 : (x + dx >= a.g.w ? 0 : x + dx);
     const int ny = y + dy < 0 ? a.g.h - 1 : (y + dy >= a.g.h ? 0 : y + dy);
-    const int nz = z + dz < 0 ? a.g.d - 1 : (z + dz >= a.g.d ? 0 : z + dz);
+    const int nz = DIM == 2 ? 0 : (z + dz < 0 ? a.g.d - 1 : (z + dz >= a.g.d ? 0 : z + dz));
     return acc.label(nx, ny, nz);
 }
 

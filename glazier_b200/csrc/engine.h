@@ -140,6 +140,7 @@ struct SweepLaunch {
     int direct;              // a lean model small enough for the direct kernel (one thread per target)
     int compact;             // the direct kernel queues unlike copies before pricing them: 1 per warp, 2 per block
     int direct_span;         // targets a block of the block-queued direct kernel takes
+    int rotate_share;        // labels whose tallies a direct block rotates (without n_live)
     int max_ctas;            // > 0 caps the persistent grid (each CTA then walks more tiles)
     const void *tensor_map;  // CUtensorMap in device-visible memory, or null
     int *error_flag;
