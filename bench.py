@@ -148,7 +148,7 @@ def measured_peak() -> tuple:
 # 4096^2 workload, from an ncu capture of that kernel with cold caches
 # (profiles/lean_sweep_2d_4096.md), with the kernel it was measured on; a
 # figure measured on another kernel is not reported.
-TRAFFIC = {"kernel": "lean", "bytes_per_launch": 79988480.0}
+TRAFFIC = {"kernel": "lean", "bytes_per_launch": 80548862.0}
 
 
 def ensemble_compare(mcs: int, device: int) -> dict:
@@ -685,7 +685,7 @@ def run_ours(args) -> None:
     bytes_per_launch = sites * BYTES_PER_SITE_UPDATE / launches_per_step  # one MCS spread over its launches
     achieved = bytes_per_launch / launch_s / 1e9
     kernel_name = {"band": "band_sweep_kernel<8,1> (one MCS: four colour passes)",
-                   "lean": "lean_sweep_kernel<2,8,1> (one colour pass)"}.get(kernel, kernel)
+                   "lean": "direct_sweep_kernel<2,8,1,1,0> (one colour pass)"}.get(kernel, kernel)
     traffic = TRAFFIC["bytes_per_launch"] if TRAFFIC["kernel"] == kernel else None
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": traffic, "peak_source": peak_kind, "kernel": kernel_name,

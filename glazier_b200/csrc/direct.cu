@@ -1,7 +1,7 @@
 // The direct sweep: a colour pass with no staging at all, the labels and
-// tallies read where they lie. It takes the lattices whose passes the window
-// rings of sweep.cu do not pay for: lean planes under 2048^2, lean volumes,
-// and models with every term.
+// tallies read where they lie. It takes every lean model (contact, volume and
+// surface terms) but the planes small enough for the cluster, and every model
+// with more terms.
 //
 // What bounds it is latency. A pass is a chain of dependent reads (labels,
 // then the two cells' tallies and types, then for some copies moments,
@@ -15,7 +15,8 @@
 //   - A small pass prices each target in its own thread; in a plane the
 //     neighbour labels come with the target's own, so the chain is labels,
 //     tallies, commit. A larger one gathers the unlike targets, about a
-//     fifth, into a queue that whole warps price from its front.
+//     fifth, into a queue that whole warps price from its front; the largest
+//     give each warp a run of targets and a queue of its own.
 //   - Pricing has no branch on the common path, so its reads and sums overlap.
 //   - The tally rotation is shared out over the grid and taken by each
 //     block's last threads.
@@ -107,13 +108,30 @@ __device__ __forceinline__ void rotate_share(const SweepLaunch &a, const DirectV
 
 // How a pass's targets are shared out (the launch's FORM).
 constexpr int kPlain = 0;  // one target per thread, priced where it lies
-constexpr int kWarp = 1;   // each warp queues the unlike of its 32 kWarpK targets
+constexpr int kWarp = 1;   // each warp queues the unlike of a run of targets, and prices it a whole round at a time
 constexpr int kBlock = 2;  // each block gathers the unlike of its targets into one queue
 
-// From a million targets a pass a warp's own queue needs no block barrier
-// and is the faster (0.37 against 0.51 ms per MCS at 256^3 for one target a
-// thread).
+// Past what one wave of gathering blocks holds, each warp takes a run of
+// consecutive targets by itself, 32 kWarpK a step, with no block barrier: what
+// a step leaves in its queue short of a whole round of 32 waits for the next
+// step, so but for the run's last every round is full. Per MCS, priced a step
+// at a time from labels read twice, and so: 41.3 and 37.5 us at 2048^2, 75.6
+// and 64.5 at 3000^2, 139.8 and 107.6 at 4096^2, 0.37 and 0.23 ms at 256^3;
+// the two-field tissue at 2048^2 122 and 107 (a step of 64 targets 121 at
+// 4096^2, of 192 112, of 256 115; the next step's labels read ahead of the
+// pricing 114, and 124 for the tissue, which spills). The large planes'
+// tiled kernel, windows by tensor copies through a ring in shared memory, took
+// 51.3, 103.7 and 131.3 us at these sizes (8192^2: 490 against 399; four
+// neighbours at 4096^2: 326 against 151; two types: 189 against 146). A pass
+// of 4096^2 is bound by issue, 61 % of cycles: 18.9 M warp instructions, and
+// its reads are 1.5 lattices through L2 (2.3 TB/s).
 constexpr int kWarpK = 4;
+// A run's targets at most: longer ones leave the warps further apart in the
+// lattice, shorter ones end in short rounds more often (per MCS with 512, 1024
+// and 2048: 121, 108 and 108 us at 4096^2, 402, 399 and 419 at 8192^2; of the
+// volume with 256 and 1024: 0.234 and 0.248 ms at 256^3).
+constexpr int kRunMost = 1024;
+constexpr int kRunMostVolume = 256;
 // A block's targets per thread at most (per MCS at 1024^2: 37.3 us with two,
 // 52.0 with one).
 constexpr int kBlockK = 2;
@@ -252,40 +270,62 @@ __global__ void __launch_bounds__(kBlockThreads, direct_blocks(FORM, TERMS > 0))
         }
         rotate_share<EXTRAS>(a, d);
     } else {
-        __shared__ int queue[kBlockThreads / 32][32 * kWarpK];
-        __shared__ uint8_t picks[kBlockThreads / 32][32 * kWarpK];
-        grid_wait();
-        if (!(UNIFORM && !EXTRAS)) __syncthreads();  // the tables are in place
-        const int first = (int)((blockIdx.x * (blockDim.x / 32) + warp) * 32 * kWarpK);
+        constexpr int kQueue = 32 * (kWarpK + 1);  // a step's targets after fewer than 32 left of the last
+        __shared__ int queue[kBlockThreads / 32][kQueue];
+        __shared__ uint8_t picks[kBlockThreads / 32][kQueue];
+        __shared__ uint2 pair[kBlockThreads / 32][kQueue];  // (old, new) labels of each queued copy
+        // the warp's run of consecutive targets: direct_span of them
+        const int first = ((int)blockIdx.x * (kBlockThreads / 32) + warp) * a.direct_span;
+        const int last = min(first + a.direct_span, targets);
         int total = 0;
+        if (!(UNIFORM && !EXTRAS)) __syncthreads();  // the tables are in place
+        for (int t = first; t < last; t += 32 * kWarpK) {
+            int tx[kWarpK], ty[kWarpK], tz[kWarpK], pick[kWarpK];
 #pragma unroll
-        for (int k = 0; k < kWarpK; ++k) {
-            const int j = first + k * 32 + lane;
-            bool unlike = false;
-            int pick = 0;
-            if (j < targets) {
-                int x, y, z;
-                direct_site<DIM>(a, a.colour, j, x, y, z);
-                pick = pick_of<NOFF>(draw(v.key_pick, (uint32_t)((z * a.g.h + y) * a.g.w + x)));
-                unlike = acc.label(x, y, z) != picked_label<DIM, NOFF>(a, acc, x, y, z, pick);
+            for (int k = 0; k < kWarpK; ++k) {
+                // past the run's end a lane reads its first target again: no
+                // branch, so the step's reads leave together
+                const int j = t + k * 32 + lane;
+                direct_site<DIM>(a, a.colour, j < last ? j : first, tx[k], ty[k], tz[k]);
+                pick[k] = pick_of<NOFF>(draw(v.key_pick, (uint32_t)((tz[k] * a.g.h + ty[k]) * a.g.w + tx[k])));
             }
-            const unsigned m = __ballot_sync(0xffffffffu, unlike);
-            if (unlike) {
-                queue[warp][total + __popc(m & below)] = j;
-                picks[warp][total + __popc(m & below)] = (uint8_t)pick;
+            if (t == first) grid_wait();  // the first step's draws come before it
+            uint2 labels[kWarpK];
+#pragma unroll
+            for (int k = 0; k < kWarpK; ++k)
+                labels[k] = make_uint2(acc.label(tx[k], ty[k], tz[k]),
+                                       picked_label<DIM, NOFF>(a, acc, tx[k], ty[k], tz[k], pick[k]));
+#pragma unroll
+            for (int k = 0; k < kWarpK; ++k) {
+                const int j = t + k * 32 + lane;
+                const bool unlike = j < last && labels[k].x != labels[k].y;
+                const unsigned m = __ballot_sync(0xffffffffu, unlike);
+                if (unlike) {
+                    const int e = total + __popc(m & below);
+                    queue[warp][e] = j;
+                    picks[warp][e] = (uint8_t)pick[k];
+                    pair[warp][e] = labels[k];
+                }
+                total += __popc(m);
             }
-            total += __popc(m);
+            __syncwarp();
+            // whole rounds of 32 off the queue's end; fewer stay for the next
+            // step, and the last step's are priced as they are
+            const bool more = t + 32 * kWarpK < last;
+            while (total >= 32 || (!more && total > 0)) {
+                const int e = total - 32 + lane;
+                if (e >= 0) {
+                    int x, y, z;
+                    direct_site<DIM>(a, a.colour, queue[warp][e], x, y, z);
+                    const NeighbourReads<DIM, NOFF, GlobalPass> ln(a, acc, x, y, z);
+                    direct_copy<DIM, NOFF, UNIFORM, GlobalPass, NeighbourReads<DIM, NOFF, GlobalPass>, TERMS>(
+                        a, T, acc, ln, v.key_accept, x, y, z, picks[warp][e], pair[warp][e].x, pair[warp][e].y, &d.t);
+                }
+                total = total > 32 ? total - 32 : 0;
+                __syncwarp();
+            }
         }
-        __syncwarp();
-        for (int e = lane; e < total; e += 32) {
-            int x, y, z;
-            direct_site<DIM>(a, a.colour, queue[warp][e], x, y, z);
-            const int pick = picks[warp][e];
-            const NeighbourReads<DIM, NOFF, GlobalPass> ln(a, acc, x, y, z);
-            direct_copy<DIM, NOFF, UNIFORM, GlobalPass, NeighbourReads<DIM, NOFF, GlobalPass>, TERMS>(
-                a, T, acc, ln, v.key_accept, x, y, z, pick, acc.label(x, y, z),
-                picked_label<DIM, NOFF>(a, acc, x, y, z, pick), &d.t);
-        }
+        if (first >= last) grid_wait();
         rotate_share<EXTRAS>(a, d);
     }
 }
@@ -338,6 +378,18 @@ cudaError_t launch_direct(const SweepLaunch &a, cudaStream_t stream) {
             grid = (targets + per_block - 1) / per_block;
         }
         b.direct_span = per_block;
+    }
+    if (warp) {
+        // Equal runs of whole lanes over whole waves of resident warps (or of
+        // the capped grid's), none longer than kRunMost targets unless capped.
+        const int most = DIM == 3 ? kRunMostVolume : kRunMost;
+        long long slots = (long long)sm_count() * direct_blocks(kWarp, false) * (kBlockThreads / 32);
+        if (slots > 0 && a.max_ctas <= 0) slots *= (targets + slots * most - 1) / (slots * most);
+        if (a.max_ctas > 0) slots = (long long)a.max_ctas * (kBlockThreads / 32);
+        const long long even = slots > 0 ? (targets + slots - 1) / slots : 32 * kWarpK;
+        b.direct_span = (int)((even + 31) / 32 * 32);
+        per_block = b.direct_span * (kBlockThreads / 32);
+        grid = (targets + per_block - 1) / per_block;
     }
     b.rotate_share = (a.n_labels + grid - 1) / grid;
     cudaLaunchConfig_t cfg{};

@@ -457,8 +457,8 @@ glz::SweepLaunch pass_launch(glz_gpu *h, int colour) {
     for (int s = 0; s < h->n_species; ++s) a.field_cur |= (unsigned)(h->field_cur[s] & 1) << s;
     a.use_tma = h->use_tma;
     a.lean = h->lean;
-    a.direct = h->direct;
-    a.compact = h->compact;
+    a.direct = h->direct || h->lean;
+    a.compact = h->direct ? h->compact : 1;  // the lean models' large planes: streaming warps
     a.max_ctas = h->max_ctas;
     a.tensor_map = h->use_tma ? &h->tmap : nullptr;
     a.error_flag = h->error_flag;
@@ -959,13 +959,12 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
     const char *lean_env = std::getenv("GLAZIER_SWEEP_LEAN");
     h->lean = !h->has_length && !h->tracks && !h->has_chemotaxis && !h->has_external && !h->has_motility && !has_conn &&
               !(lean_env && lean_env[0] == '0');
-    // A lean plane under 2048^2 sites, or a lean volume of any size, takes the
-    // direct kernel, which reads the lattice through the caches: the lean
-    // kernel's window ring pays on large planes only (per MCS, direct against
-    // lean: 17.7 and 32.0 us at 1100^2, 29.0 and 49.5 at 1448^2, 158 and 129 at
-    // 4096^2; 0.37 against 0.91 ms at 256^3 and 0.64 against 1.07 ms at 320^3,
-    // a lattice past L2, L2 flushed). GLAZIER_SWEEP_DIRECT=0: never, =1: at any
-    // size.
+    // Every lean pass takes the direct kernel (direct.cu), which reads the
+    // lattice through the caches. A plane from 2048^2 sites keeps the name
+    // "lean" and always streams by warps, whose runs GLAZIER_SWEEP_CTAS caps;
+    // under it, and for volumes, the form goes by size.
+    // GLAZIER_SWEEP_DIRECT=0: lean models stream at any size and others take
+    // the tiled kernel, =1: the form goes by size at any size.
     const char *direct_env = std::getenv("GLAZIER_SWEEP_DIRECT");
     const int direct_mode = direct_env ? (direct_env[0] == '0' ? 0 : 1) : -1;
     const long long direct_most = g.dim == 2 ? 2048LL * 2048LL - 1 : sites;
@@ -978,19 +977,21 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
     h->direct = direct_mode == 1 || (direct_mode == -1 && (!h->lean || sites <= direct_most));
     // Past a number of targets a pass the direct kernel gathers each block's
     // unlike copies into one queue priced by whole warps, and past a larger one
-    // it queues each warp's
+    // each warp streams over a run
     // (GLAZIER_SWEEP_COMPACT=0: neither, =1: the warp's, =2: the block's, at
     // any size). Per MCS of the two-field tissue, priced in place against
     // gathered: 31.1 and 31.7 us at 256^2, 35.1 and 35.0 at 512^2, 51.6 and
     // 36.6 at 640^2, 92.7 and 62.7 at 1024^2 (of the slab's model 147 and 162
     // at 64 x 64 x 32, 179 and 191 at 96 x 96 x 64, 386 and 300 at 128^3), by
-    // warps against by blocks 130 and 130 at 2048^2, 450 and 479 at 4096^2. Of
-    // the lean plane: 11.9 and 13.9
+    // warps against by blocks 95.0 and 91.9 at 1800^2, 107 and 119 at 2048^2,
+    // 353 and 435 at 4096^2. Of the lean plane: 11.9 and 13.9
     // at 512^2, 13.9 and 15.7 at 768^2 (a last target a thread of one wave of
-    // blocks), 20.9 and 16.7 at 896^2, by blocks against by warps 17.7 and 21.7
-    // at 1100^2, 29.1 and 28.7 at 1300^2, 30.3 and 29.0 at 1448^2; of the lean
-    // volume (26 neighbours):
-    // 24.2 and 28.4 at 64^3, 28.9 and 30.7 at 80^3, 35.6 and 33.4 at 96^3.
+    // blocks), 20.9 and 16.7 at 896^2, by blocks against by warps 15.8 and 19.2
+    // at 1024^2 (the last wave of gathering blocks holds 1101^2), 24.2 and 21.9
+    // at 1150^2, 26.4 and 23.0 at 1448^2, 47 and 37.5 at 2048^2; of the lean
+    // volume (26 neighbours): 24.2 and 28.4 at 64^3, 28.9 and 30.7 at 80^3,
+    // 35.6 and 33.4 at 96^3, by blocks against by warps 42 and 59 at 128^3,
+    // 73 and 91 at 160^3, 140 and 133 at 204^3, 231 and 233 at 256^3.
     const char *compact_env = std::getenv("GLAZIER_SWEEP_COMPACT");
     const int compact_mode = compact_env ? (compact_env[0] == '0' ? 0 : (compact_env[0] == '2' ? 2 : 1)) : -1;
     const long long targets = sites / g.ncol;
@@ -1014,8 +1015,8 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
     // The band sweep (every colour pass of a call in one launch, rows
     // streamed by bands) runs a lean plane only when asked
     // (GLAZIER_SWEEP_BAND=1) and its rows are whole 16-byte units: at 2048^2,
-    // 4096^2 and 8192^2 it measured slower than the windowed lean kernel
-    // (0.169 against 0.145 ms per MCS at 4096^2, L2 flushed).
+    // 4096^2 and 8192^2 it measured slower than a launch per pass
+    // (0.169 against 0.108 ms per MCS at 4096^2).
     const char *band_env = std::getenv("GLAZIER_SWEEP_BAND");
     h->band = h->lean && !h->has_pop && g.dim == 2 && band_env && band_env[0] == '1' && glz::band_sweep_fits(w, hh);
     if (h->band) h->direct = h->cluster = false;

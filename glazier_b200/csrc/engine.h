@@ -136,10 +136,10 @@ struct SweepLaunch {
     int *pending_count;  // this pass's, and the other pass parity's (cleared for the next pass)
     int *pending_clear;
     int use_tma;
-    int lean;                // take the lean kernel: no length, chemotaxis, connectivity or moment tracking
-    int direct;              // a lean model small enough for the direct kernel (one thread per target)
+    int lean;                // price contact, volume and surface only: no length, chemotaxis, connectivity or moment tracking
+    int direct;              // take the direct kernel
     int compact;             // the direct kernel queues unlike copies before pricing them: 1 per warp, 2 per block
-    int direct_span;         // targets a block of the block-queued direct kernel takes
+    int direct_span;         // targets a block (a streaming warp) of the queueing direct kernel takes
     int rotate_share;        // labels whose tallies a direct block rotates (without n_live)
     int max_ctas;            // > 0 caps the persistent grid (each CTA then walks more tiles)
     const void *tensor_map;  // CUtensorMap in device-visible memory, or null
@@ -172,11 +172,12 @@ struct ResidentLaunch {
 // Targets a pass from which the direct kernel queues a block's unlike copies
 // (of a lean plane: more than 148 SMs' four blocks of 256 take at once; of a
 // volume; of a plane with terms past contact, volume and surface) and from
-// which a warp's (of a lean plane; of the others).
+// which each warp streams over a run of its own (of a lean plane: more than
+// one wave of gathering blocks holds; of the others).
 constexpr int kDirectGatherFrom = 148 * 4 * 256 + 1;
 constexpr int kDirectGatherVolumeFrom = 5 << 14;
 constexpr int kDirectGatherEveryFrom = (1 << 16) + 1;
-constexpr int kDirectCompactPlaneFrom = 3 << 17;
+constexpr int kDirectCompactPlaneFrom = 148 * 4 * 512 + 1;
 constexpr int kDirectCompactFrom = 1 << 20;
 
 // Every requested MCS of a small lean plane in one thread-block cluster holding

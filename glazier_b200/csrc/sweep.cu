@@ -480,7 +480,7 @@ __global__ void __launch_bounds__(kThreads, GLZ_SWEEP_MIN_BLOCKS) sweep_kernel(c
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     // Nothing above reads what the previous pass writes; a programmatic launch
-    // may have started this grid before it ended (see launch_lean).
+    // may have started this grid before it ended (see launch).
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     rotate_tallies<DIM>(a);
@@ -532,12 +532,12 @@ __global__ void __launch_bounds__(kThreads, GLZ_SWEEP_MIN_BLOCKS) sweep_kernel(c
     }
 }
 
-// ---------------------------------------------------------------- the lean sweep
+// ---------------------------------------------------------------- the lean windows
 //
-// Models whose copies price only contact, volume and surface terms (no
-// length, chemotaxis, connectivity veto or moment tracking) take this kernel:
-// the same draws, copies and commits as sweep_kernel, with the work laid out
-// so that no CTA-wide barrier stands between tiles.
+// Replicas whose copies price only contact, volume and surface terms can be
+// swept by the lean ensemble kernel (below): the draws, copies and commits of
+// sweep_kernel, with the work laid out so that no CTA-wide barrier stands
+// between tiles.
 //   - Each warp owns a fixed share of every tile's targets (two rows of them
 //     in a plane) and prices it alone: light pass, its own queue, heavy pass.
 //     Warps drift apart by up to the depth of the window ring.
@@ -550,6 +550,8 @@ __global__ void __launch_bounds__(kThreads, GLZ_SWEEP_MIN_BLOCKS) sweep_kernel(c
 //     (a bounded wait) before pricing. Without tensor copies (rows that are
 //     not whole 16-byte units, or a lattice smaller than a window) every cell
 //     of every window is loaded that way.
+// One lattice's lean passes take the streaming form of direct.cu instead,
+// which measured faster at every size.
 #ifndef GLZ_LEAN_STAGES
 #define GLZ_LEAN_STAGES 3
 #endif
@@ -571,7 +573,6 @@ struct LeanSmem {
     static constexpr int TPW = Tile<DIM>::NT / kLeanWarps;  // targets per warp per tile
     alignas(128) uint32_t win[kLeanStages][WIN_STRIDE];
     uint32_t queue[kLeanWarps][TPW + 32];  // a tile's entries after fewer than 32 held from the tile before
-    float contact[kSmemTypes * kSmemTypes];
     int woff[26];
     int done[kLeanStages];    // warps finished with the buffer's current tile
     int issued[kLeanStages];  // copies issued into the buffer
@@ -589,22 +590,6 @@ template <int DIM>
 __device__ __forceinline__ bool lean_copies(const SweepLaunch &a) {
     using T = Tile<DIM>;
     return a.use_tma && a.g.w >= T::PX && a.g.h >= T::PY && (DIM == 2 || a.g.d >= T::PZ);
-}
-
-// Start tile i of this CTA's list into its buffer: a tensor copy, or a bare
-// arrival when copies are off, so the buffer's phase completes either way.
-template <int DIM>
-__device__ __forceinline__ void lean_issue(const SweepLaunch &a, const CUtensorMap &tmap, LeanSmem<DIM> &S, int i,
-                                           bool copies) {
-    const int slot = i % kLeanStages;
-    S.issued[slot] += 1;
-    if (copies) {
-        int x0, y0, z0;
-        tile_origin<DIM>((int)blockIdx.x + i * (int)gridDim.x, a.g.w, a.g.h, x0, y0, z0);
-        issue_window<DIM>(tmap, S.win[slot], &S.full[slot], x0, y0, z0);
-    } else {
-        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&S.full[slot])) : "memory");
-    }
 }
 
 // The warp's rows of an edge tile's window (rows warp, warp + kLeanWarps, ...):
@@ -637,244 +622,6 @@ __device__ __forceinline__ void lean_patch(const SweepLaunch &a, uint32_t *win, 
             const int px = inside && c >= lo ? hi + (c - lo) : c;
             dst[px] = row[wr(x0 - T::HX + px, W)];
         }
-    }
-}
-
-// The warp is done with tile i's buffer (lane 0 acts); the last warp out
-// refills it with tile i + kLeanStages.
-template <int DIM>
-__device__ __forceinline__ void lean_release(const SweepLaunch &a, const CUtensorMap &tmap, LeanSmem<DIM> &S, int i,
-                                             int mine, bool copies) {
-    if ((threadIdx.x & 31) != 0) return;
-    const int slot = i % kLeanStages;
-    __threadfence_block();
-    if (atomicAdd(&S.done[slot], 1) == kLeanWarps - 1) {
-        S.done[slot] = 0;
-        if (i + kLeanStages < mine) {
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            lean_issue<DIM>(a, tmap, S, i + kLeanStages, copies);
-        }
-    }
-}
-
-template <int DIM, int NOFF, bool UNIFORM>
-__global__ void __launch_bounds__(kLeanThreads, GLZ_LEAN_MIN_BLOCKS)
-    lean_sweep_kernel(const __grid_constant__ SweepLaunch a, const __grid_constant__ CUtensorMap tmap) {
-    using T = Tile<DIM>;
-    using Smem = LeanSmem<DIM>;
-    constexpr int PER_LANE = Smem::TPW / 32;
-    static_assert(Smem::TPW % 32 == 0, "a warp's targets fill whole lanes");
-    static_assert(Smem::WIN_STRIDE * sizeof(uint32_t) % 128 == 0, "window buffers must stay 128-byte aligned");
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    const uint32_t raw = smem_addr(smem_raw);
-    Smem &S = *reinterpret_cast<Smem *>(smem_raw + ((128u - (raw & 127u)) & 127u));
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (smem_addr(S.win[0]) & 127u) {  // never true by construction; refuse rather than copy misaligned
-        if (tid == 0) atomicExch(a.error_flag, 3);
-        return;
-    }
-    const int W = a.g.w, H = a.g.h, D = a.g.d;
-    const int tiles = ((W + T::TX - 1) / T::TX) * ((H + T::TY - 1) / T::TY) * (DIM == 3 ? (D + T::TZ - 1) / T::TZ : 1);
-    const int mine = (int)blockIdx.x < tiles ? (tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-    const bool copies = lean_copies<DIM>(a);
-
-    if (tid == 0) {
-        for (int k = 0; k < kLeanStages; ++k) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&S.full[k])));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&S.patched[k])), "r"(kLeanWarps));
-            S.done[k] = 0;
-            S.issued[k] = 0;
-        }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    const bool small_types = a.n_types <= kSmemTypes;
-    if (!UNIFORM && small_types)
-        for (int k = tid; k < a.n_types * a.n_types; k += blockDim.x) S.contact[k] = a.t.contact[k];
-#pragma unroll
-    for (int k = 0; k < NOFF; ++k)
-        if (tid == k) S.woff[k] = window_offset<DIM, NOFF>(k);
-    // Everything above reads nothing the previous pass writes. Launched
-    // programmatically, this grid may have started before that pass ended:
-    // wait here for it to finish (its labels and tallies visible), then let
-    // the next pass's grid start its own prologue.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    if (tid == 0)
-        for (int i = 0; i < kLeanStages && i < mine; ++i) lean_issue<DIM>(a, tmap, S, i, copies);
-    // Tally rotation (no thread of this pass reads what it writes): the reads
-    // of each thread's first kRotate labels are copied into shared memory now
-    // and finished after the tiles, so their latency hides behind pricing.
-    const size_t rot_stride = (size_t)gridDim.x * blockDim.x;
-    const size_t rot_first = (size_t)blockIdx.x * blockDim.x + tid;
-#pragma unroll
-    for (int k = 0; k < kRotate; ++k) {
-        const size_t l = rot_first + k * rot_stride;
-        if (l < (size_t)a.n_labels) {
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(&S.rot_base[k * kLeanThreads + tid])),
-                         "l"(a.vs_base + l)
-                         : "memory");
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(&S.rot_prev[k * kLeanThreads + tid])),
-                         "l"(a.vs_prev + l)
-                         : "memory");
-        }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    __syncthreads();
-
-    // this lane's targets: offset from the tile's first site, window cell
-    int rel[PER_LANE], cell[PER_LANE];
-#pragma unroll
-    for (int k = 0; k < PER_LANE; ++k) {
-        int lx, ly, lz;
-        target_of<DIM>(warp * Smem::TPW + k * 32 + lane, a.colour, lx, ly, lz);
-        rel[k] = (lz * H + ly) * W + lx;
-        cell[k] = ((lz + T::HZ) * T::PY + (ly + 1)) * T::PX + (lx + T::HX);
-    }
-    uint32_t *queue = S.queue[warp];
-    const unsigned below = (1u << lane) - 1u;
-    uint32_t patch_parity = 0;  // bit k: parity of the next phase of patched[k]
-    // entries held over from the previous tile: queue[0, held), its buffer and origin
-    int held = 0, held_slot = -1, hx0 = 0, hy0 = 0, hz0 = 0;
-    // The CTA's tiles are blockIdx.x + i gridDim.x; their tile coordinates
-    // advance by the grid's own decomposition, so the loop divides nothing.
-    const int tiles_x = (W + T::TX - 1) / T::TX, tiles_y = (H + T::TY - 1) / T::TY;
-    const int step_x = (int)gridDim.x % tiles_x, step_y = ((int)gridDim.x / tiles_x) % tiles_y;
-    const int step_z = (int)gridDim.x / (tiles_x * tiles_y);
-    int tx = (int)blockIdx.x % tiles_x, ty = ((int)blockIdx.x / tiles_x) % tiles_y;
-    int tz = (int)blockIdx.x / (tiles_x * tiles_y);
-
-    for (int i = 0; i < mine; ++i) {
-        const int slot = i % kLeanStages;
-        if (i > 0) {
-            tx += step_x;
-            const int cx = tx >= tiles_x;
-            tx -= cx ? tiles_x : 0;
-            ty += step_y + cx;
-            const int cy = ty >= tiles_y;
-            ty -= cy ? tiles_y : 0;
-            tz += step_z + cy;
-        }
-        const int x0 = tx * T::TX, y0 = ty * T::TY, z0 = DIM == 3 ? tz * T::TZ : 0;
-        uint32_t *win = S.win[slot];
-        bool ok = wait_parity(&S.full[slot], (uint32_t)(i / kLeanStages) & 1u) != 0;
-        const bool edge = !copies || !(x0 >= T::HX && x0 + T::TX + T::HX <= W && y0 >= 1 && y0 + T::TY + 1 <= H &&
-                                       (DIM == 2 || (z0 >= 1 && z0 + T::TZ + 1 <= D)));
-        if (edge && __all_sync(0xffffffffu, ok)) {
-            lean_patch<DIM>(a, win, x0, y0, z0, copies);
-            // generic writes to a buffer a later tensor copy will overwrite
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0)
-                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&S.patched[slot])) : "memory");
-            ok = wait_parity(&S.patched[slot], (patch_parity >> slot) & 1u) != 0;
-            patch_parity ^= 1u << slot;
-        }
-        if (!__all_sync(0xffffffffu, ok)) {
-            // A copy or a warp that never came: flag it, give each buffer's
-            // latest copy its own bounded wait so none lands after exit, stop.
-            if (lane == 0) {
-                atomicExch(a.error_flag, 1);
-                for (int k = 0; k < kLeanStages; ++k)
-                    if (S.issued[k] > 0) wait_parity(&S.full[k], (uint32_t)(S.issued[k] - 1) & 1u);
-            }
-            asm volatile("cp.async.wait_all;" ::: "memory");
-            return;
-        }
-
-        // Light pass: this warp's targets; those whose neighbour pick carries
-        // another label go into the warp's queue, behind the entries held
-        // from the previous tile.
-        const bool full = x0 + T::TX <= W && y0 + T::TY <= H && (DIM == 2 || z0 + T::TZ <= D);
-        const uint32_t tile_base = (uint32_t)((z0 * H + y0) * W + x0);
-        uint32_t entries[PER_LANE];
-        unsigned masks[PER_LANE];
-#pragma unroll
-        for (int k = 0; k < PER_LANE; ++k) {
-            const int j = warp * Smem::TPW + k * 32 + lane;
-            bool in = full;
-            if (!full) {
-                int lx, ly, lz;
-                target_of<DIM>(j, a.colour, lx, ly, lz);
-                in = x0 + lx < W && y0 + ly < H && (DIM == 2 || z0 + lz < D);
-            }
-            bool active = false;
-            int pick = 0;
-            if (in) {
-                pick = pick_of<NOFF>(draw(a.key_pick, tile_base + (uint32_t)rel[k]));
-                active = win[cell[k]] != win[cell[k] + S.woff[pick]];
-            }
-            entries[k] = (uint32_t)j | ((uint32_t)pick << 16);
-            masks[k] = __ballot_sync(0xffffffffu, active);
-        }
-        int total = held;
-#pragma unroll
-        for (int k = 0; k < PER_LANE; ++k) {
-            if (masks[k] & (1u << lane)) queue[total + __popc(masks[k] & below)] = entries[k];
-            total += __popc(masks[k]);
-        }
-        __syncwarp();
-        // Heavy pass: whole rounds of 32 copies, oldest first; entry e is the
-        // previous tile's when e < held. Whatever of the previous tile is still
-        // queued after them goes in one last short round, so that tile's
-        // buffer can be let go; fewer than 32 of this tile's stay held.
-        int taken = 0;
-        for (;;) {
-            const int n = total - taken;
-            if (n < 32 && taken >= held) break;
-            const int e = taken + lane;
-            if (e < total) {
-                const bool before = e < held;
-                price_and_commit<DIM, NOFF, UNIFORM, false>(a, S.woff, S.contact, nullptr,
-                                                            before ? S.win[held_slot] : win, queue[e],
-                                                            before ? hx0 : x0, before ? hy0 : y0,
-                                                            before ? hz0 : z0, small_types);
-            }
-            taken += n < 32 ? n : 32;
-        }
-        __syncwarp();
-        if (held_slot >= 0) lean_release<DIM>(a, tmap, S, i - 1, mine, copies);
-        // move what this tile keeps to the front of the queue (a full round
-        // came first, so the source lies past the first 32 entries)
-        const int keep = total - taken;
-        if (taken > 0 && keep > 0) {
-            const uint32_t v = lane < keep ? queue[taken + lane] : 0u;
-            __syncwarp();
-            if (lane < keep) queue[lane] = v;
-            __syncwarp();
-        }
-        held = keep;
-        held_slot = slot;
-        hx0 = x0;
-        hy0 = y0;
-        hz0 = z0;
-    }
-    // the last tile's held entries, then its buffer
-    if (mine > 0) {
-        if (lane < held)
-            price_and_commit<DIM, NOFF, UNIFORM, false>(a, S.woff, S.contact, nullptr, S.win[held_slot], queue[lane],
-                                                        hx0, hy0, hz0, small_types);
-        __syncwarp();
-        lean_release<DIM>(a, tmap, S, mine - 1, mine, copies);
-    }
-    // finish the rotation: this thread's copied labels, then any past them
-    asm volatile("cp.async.wait_all;" ::: "memory");
-#pragma unroll
-    for (int k = 0; k < kRotate; ++k) {
-        const size_t l = rot_first + k * rot_stride;
-        if (l < (size_t)a.n_labels) {
-            int dv, ds;
-            unpack_delta(S.rot_prev[k * kLeanThreads + tid], dv, ds);
-            const int2 b = S.rot_base[k * kLeanThreads + tid];
-            a.vs_next_base[l] = make_int2(b.x + dv, b.y + ds);
-            a.vs_clear[l] = 0;
-        }
-    }
-    for (size_t l = rot_first + kRotate * rot_stride; l < (size_t)a.n_labels; l += rot_stride) {
-        int dv, ds;
-        unpack_delta(a.vs_prev[l], dv, ds);
-        const int2 b = a.vs_base[l];
-        a.vs_next_base[l] = make_int2(b.x + dv, b.y + ds);
-        a.vs_clear[l] = 0;
     }
 }
 
@@ -1288,44 +1035,6 @@ cudaError_t launch_cluster_sweep(const ResidentLaunch &r, cudaStream_t stream) {
 }
 
 template <int DIM, int NOFF, bool UNIFORM>
-static cudaError_t launch_lean(const SweepLaunch &a, const CUtensorMap &tmap, cudaStream_t stream) {
-    using T = Tile<DIM>;
-    static std::atomic<int> grid_cap_once{0};  // handles on other host threads may launch too
-    const size_t smem = sizeof(LeanSmem<DIM>) + 128;
-    if (!grid_cap_once.load(std::memory_order_acquire)) {
-        cudaError_t e = cudaFuncSetAttribute(lean_sweep_kernel<DIM, NOFF, UNIFORM>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e) return e;
-        int dev = 0, sms = 0, per_sm = 0;
-        if ((e = cudaGetDevice(&dev))) return e;
-        if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev))) return e;
-        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lean_sweep_kernel<DIM, NOFF, UNIFORM>,
-                                                               kLeanThreads, smem)))
-            return e;
-        grid_cap_once.store(sms * (per_sm > 0 ? per_sm : 1), std::memory_order_release);
-    }
-    const int tiles = ((a.g.w + T::TX - 1) / T::TX) * ((a.g.h + T::TY - 1) / T::TY) *
-                      (DIM == 3 ? (a.g.d + T::TZ - 1) / T::TZ : 1);
-    const int grid_cap = grid_cap_once.load(std::memory_order_acquire);
-    int grid = tiles < grid_cap ? tiles : grid_cap;
-    if (a.max_ctas > 0 && grid > a.max_ctas) grid = a.max_ctas;
-    // Programmatic launch: the grid may start its prologue while the previous
-    // kernel on the stream ends (the kernel waits before it reads pass data).
-    // GLAZIER_SWEEP_PDL=0 launches it plainly.
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kLeanThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = programmatic_launch();
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, lean_sweep_kernel<DIM, NOFF, UNIFORM>, a, tmap);
-}
-
-template <int DIM, int NOFF, bool UNIFORM>
 static cudaError_t launch(const SweepLaunch &a, cudaStream_t stream) {
     // the compile-time neighbourhood must be the one the host built
     for (int k = 0; k < NOFF; ++k)
@@ -1337,7 +1046,6 @@ static cudaError_t launch(const SweepLaunch &a, cudaStream_t stream) {
     else
         memset(&tmap, 0, sizeof tmap);
     if (a.direct) return launch_direct<DIM, NOFF, UNIFORM>(a, stream);
-    if (a.lean) return launch_lean<DIM, NOFF, UNIFORM>(a, tmap, stream);
     using T = Tile<DIM>;
     static std::atomic<int> grid_cap_once{0};  // handles on other host threads may launch too
     const size_t smem = sizeof(SweepSmem<DIM>) + 128;
@@ -1357,7 +1065,9 @@ static cudaError_t launch(const SweepLaunch &a, cudaStream_t stream) {
     const int grid_cap = grid_cap_once.load(std::memory_order_acquire);
     int grid = tiles < grid_cap ? tiles : grid_cap;
     if (a.max_ctas > 0 && grid > a.max_ctas) grid = a.max_ctas;
-    // programmatic launch as the lean kernel's
+    // Programmatic launch: the grid may start its prologue while the previous
+    // kernel on the stream ends (the kernel waits before it reads pass data).
+    // GLAZIER_SWEEP_PDL=0 launches it plainly.
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(kThreads);
@@ -1575,7 +1285,7 @@ __global__ void __launch_bounds__(kThreads, GLZ_SWEEP_MIN_BLOCKS)
 
 // ---------------------------------------------------------------- the lean ensemble
 //
-// The lean kernel's layout over an ensemble: warp-owned target shares, the
+// The layout above over an ensemble: warp-owned target shares, the
 // window ring refilled by the last warp out, queue entries carried into the
 // warp's next tile. Warps may be on different tiles, so each ring slot holds
 // its own copy of the tile's replica launch, with the pass's fields patched

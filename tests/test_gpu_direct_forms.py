@@ -9,7 +9,7 @@
   terms past contact, volume and surface.
 - The lean models' default choice either side of each of its sizes: the
   cluster up to (not with) 256^2 sites, in place up to one wave of blocks,
-  then gathered; planes of few rows, whose cluster has CTAs without rows or a
+  gathered up to one wave of those, then streamed by warps; planes of few rows, whose cluster has CTAs without rows or a
   CTA that is its own neighbour; and a plane whose cluster threads take four
   targets each.
 
@@ -101,7 +101,7 @@ def test_tables_in_shared_memory_and_past_it(device, kinds, width, every, monkey
 @pytest.mark.parametrize("w, h, d, kernel", [
     (30, 2, 1, "cluster"), (18, 4, 1, "cluster"), (66, 34, 1, "cluster"), (130, 50, 1, "cluster"),
     (254, 256, 1, "cluster"), (256, 256, 1, "direct"), (778, 778, 1, "direct"), (780, 780, 1, "gathered"),
-    (1254, 1252, 1, "gathered"), (1256, 1254, 1, "compact"), (2048, 2046, 1, "compact"), (2050, 2048, 1, "lean"),
+    (1100, 1102, 1, "gathered"), (1102, 1102, 1, "compact"), (2048, 2046, 1, "compact"), (2050, 2048, 1, "lean"),
     (80, 80, 80, "direct"), (88, 88, 88, "gathered"),
 ])
 @pytest.mark.parametrize("types", [1, 2])
@@ -218,4 +218,19 @@ def test_deaths_without_divisions_keep_no_moments(device):
         replay.step(chunk)
         _same(gpu, replay, 0)
     assert int((gpu.volumes()[1:] == 0).sum()) > 0
+    gpu.close()
+
+
+@pytest.mark.parametrize("w, h, d", [(32, 32, 1), (64, 66, 1), (126, 62, 1), (514, 70, 1), (18, 10, 6), (34, 30, 22)])
+@pytest.mark.parametrize("ctas", ["1", "2"])
+@pytest.mark.parametrize("types", [1, 2])
+def test_warps_that_stream_over_runs(device, w, h, d, ctas, types, monkeypatch):
+    """The lean models on one or two blocks' warps: runs of one whole step of
+    128 targets and less, of a step and a part, of many steps that carry
+    entries over, a last warp's short run and warps without a target."""
+    monkeypatch.setenv("GLAZIER_SWEEP_DIRECT", "0")
+    monkeypatch.setenv("GLAZIER_SWEEP_CTAS", ctas)
+    gpu, replay = _lean(device, w, h, d, types, 8 if d == 1 else 2)
+    assert gpu.sweep_kernel == "lean"
+    _same(gpu, replay, 0)
     gpu.close()
