@@ -149,12 +149,16 @@ constexpr int kBlockWide = 3;
 // one wave (at 128^3: 0.060 ms per MCS against 0.073 uncapped, 0.065 at 48);
 // small every-term passes keep 128 (uncapped they take up to 200, one block:
 // 48 against 70 us per MCS for the 512^2 tissue), large ones 64.
-constexpr int direct_blocks(int form, bool extras) {
-    return extras && (form == kPlain || form == kBlock) ? 2 : 4;
+// In place, a volume of several types also takes 128, so that its neighbours'
+// labels and types are in flight together (64 and 128 registers: 35.1 and
+// 28.9 us per MCS at 64^3 with 26 neighbours, 39.0 and 35.7 at 80^3; 31.1 and
+// 44.2 with 80).
+constexpr int direct_blocks(int form, bool extras, bool mixed_volume = false) {
+    return (extras && (form == kPlain || form == kBlock)) || (mixed_volume && form == kPlain) ? 2 : 4;
 }
 
 template <int DIM, int NOFF, bool UNIFORM, int FORM, int TERMS>
-__global__ void __launch_bounds__(kBlockThreads, direct_blocks(FORM, TERMS > 0))
+__global__ void __launch_bounds__(kBlockThreads, direct_blocks(FORM, TERMS > 0, DIM == 3 && !UNIFORM))
     direct_sweep_kernel(const __grid_constant__ SweepLaunch a) {
     constexpr bool EXTRAS = TERMS > 0;
     const int targets = (a.g.w / 2) * (a.g.h / 2) * (DIM == 3 ? a.g.d / 2 : 1);

@@ -69,38 +69,6 @@ __device__ __forceinline__ void direct_site(const SweepLaunch &a, int colour, in
     }
 }
 
-// The offsets of a neighbourhood along an axis, one more than each in two
-// bits, neighbour k's at bit 2 k.
-template <int DIM, int NOFF>
-__host__ __device__ constexpr uint64_t packed_offsets(int axis) {
-    uint64_t bits = 0;
-    for (int k = 0; k < NOFF; ++k) bits |= (uint64_t)(neighbour_offset<DIM, NOFF>(k, axis) + 1) << (2 * k);
-    return bits;
-}
-
-// The offset of neighbour `pick`: a shift of a constant an axis (the
-// 26-neighbourhood has a closed form), not a chain of selects or a table.
-template <int DIM, int NOFF>
-__device__ __forceinline__ void pick_offset(int pick, int &dx, int &dy, int &dz) {
-    if constexpr (DIM == 3 && NOFF == 26) {
-        dx = neighbour_offset<3, 26>(pick, 0);
-        dy = neighbour_offset<3, 26>(pick, 1);
-        dz = neighbour_offset<3, 26>(pick, 2);
-    } else {
-        constexpr uint64_t X = packed_offsets<DIM, NOFF>(0), Y = packed_offsets<DIM, NOFF>(1),
-                           Z = packed_offsets<DIM, NOFF>(2);
-        if constexpr (2 * NOFF <= 32) {
-            dx = (int)((uint32_t)X >> (2 * pick) & 3u) - 1;
-            dy = (int)((uint32_t)Y >> (2 * pick) & 3u) - 1;
-            dz = DIM == 3 ? (int)((uint32_t)Z >> (2 * pick) & 3u) - 1 : 0;
-        } else {
-            dx = (int)(X >> (2 * pick) & 3u) - 1;
-            dy = (int)(Y >> (2 * pick) & 3u) - 1;
-            dz = (int)(Z >> (2 * pick) & 3u) - 1;
-        }
-    }
-}
-
 // The label of the picked neighbour of (x, y, z).
 template <int DIM, int NOFF, class Access>
 __device__ __forceinline__ uint32_t picked_label(const SweepLaunch &a, const Access &acc, int x, int y, int z, int pick) {
