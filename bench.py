@@ -146,9 +146,9 @@ def measured_peak() -> tuple:
 
 # DRAM bytes (read + write) of one launch of the headline sweep kernel on the
 # 4096^2 workload, from an ncu capture of that kernel with cold caches
-# (profiles/lean_sweep_2d_4096.md), with the kernel it was measured on; a
+# (profiles/stream_sweep_2d_4096.md), with the kernel it was measured on; a
 # figure measured on another kernel is not reported.
-TRAFFIC = {"kernel": "lean", "bytes_per_launch": 80548862.0}
+TRAFFIC = {"kernel": "lean", "bytes_per_launch": 81738240.0}
 
 
 def ensemble_compare(mcs: int, device: int) -> dict:
