@@ -667,9 +667,8 @@ __global__ void __launch_bounds__(kThreads) backward_quads(const __grid_constant
     for (int k = threadIdx.x; k < a.n_grads; k += blockDim.x) global_row[k] = row[k];
 }
 
-// Planes of rows of whole multiples of four sites take several rounds a
-// launch: a block holds a tile of kTileX by kTileY sites of one species with
-// kHalo sites about it in shared memory and runs up to kHalo rounds there,
+// Planes take several rounds a launch (tile_plane says which): a block holds a
+// tile of kTileX by kTileY sites of one species with kHalo sites about it in shared memory and runs up to kHalo rounds there,
 // each valid one site less far out than the round before, so a round costs a
 // block barrier and not a launch, and neighbouring tiles repeat the rounds of
 // their common margin (1.4 times the sites at 64 x 32 with a halo of 4).
@@ -717,13 +716,19 @@ struct TileBackward {
 };
 
 // A thread's quads of a tile's region: region row and first column, the
-// lattice site they wrap to, and whether they are the tile's own.
+// lattice site they wrap to, and whether they are the tile's own. On rows of
+// whole quads (WHOLE) a quad is four sites in a line, read and written at
+// once; on others it may run past its row's end, from cell bend on at the
+// row's start, and the tile's own cells of the last are the first `count`.
+template <bool WHOLE>
 struct TileQuads {
+    int w;
+    int bend[kQuadsEach], count[kQuadsEach];
     int cell[kQuadsEach];  // offset in the region, -1 past its end
     int row[kQuadsEach], col[kQuadsEach];
     uint32_t site[kQuadsEach];
     bool mine[kQuadsEach];
-    __device__ __forceinline__ TileQuads(const Grid &g, int x0, int y0) {
+    __device__ __forceinline__ TileQuads(const Grid &g, int x0, int y0) : w(g.w) {
 #pragma unroll
         for (int n = 0; n < kQuadsEach; ++n) {
             const int q = (int)threadIdx.x + n * kTileThreads;
@@ -734,6 +739,34 @@ struct TileQuads {
             site[n] = (uint32_t)glz::wrap(y, g.h) * (uint32_t)g.w + (uint32_t)glz::wrap(x, g.w);
             mine[n] = row[n] >= kHalo && row[n] < kHalo + kTileY && col[n] >= 1 && col[n] < kRegionQuads - 1 &&
                       y < g.h && x < g.w;
+            bend[n] = g.w - glz::wrap(x, g.w);
+            count[n] = mine[n] ? g.w - x : 0;
+        }
+    }
+    // cell c of quad n is the tile's own
+    __device__ __forceinline__ bool own(int n, int c) const { return WHOLE ? mine[n] : c < count[n]; }
+    // quad n's cells of a lattice array, its first cell at site `at` of it
+    template <class T, class V>
+    __device__ __forceinline__ void load(const T *p, uint32_t at, int n, V v[4]) const {
+        if constexpr (WHOLE) {
+            ld4(p + at, v);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) v[c] = p[at + c - (c >= bend[n] ? (uint32_t)w : 0u)];
+        }
+    }
+    template <class T, class V>
+    __device__ __forceinline__ void load(const T *p, int n, V v[4]) const {
+        load(p, site[n], n, v);
+    }
+    // the tile's own cells of quad n to a lattice array
+    __device__ __forceinline__ void store(float *p, int n, const float v[4]) const {
+        if constexpr (WHOLE) {
+            if (mine[n]) st4(p + site[n], v);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                if (c < count[n]) p[site[n] + c] = v[c];
         }
     }
     // whether quad n has a site within `margin` of the tile
@@ -764,11 +797,12 @@ __device__ __forceinline__ void tile_rates(const float *sec, const float *upt, i
         rates[t] = t < n_types ? make_float2(sec[t * n_species + s], upt[t * n_species + s]) : make_float2(0.0f, 0.0f);
 }
 
+template <bool WHOLE>
 __global__ void __launch_bounds__(kTileThreads) tile_forward(const __grid_constant__ TileForward a) {
     __shared__ alignas(16) float region[2][kRegionX * kRegionY];
     __shared__ float2 rates[kTileTypes + 1];
     const int s = (int)blockIdx.z, k = a.k[s], rounds = a.steps * k;
-    const TileQuads Q(a.g, (int)blockIdx.x * kTileX, (int)blockIdx.y * kTileY);
+    const TileQuads<WHOLE> Q(a.g, (int)blockIdx.x * kTileX, (int)blockIdx.y * kTileY);
     grid_wait();
     tile_rates(a.sec, a.upt, s, a.n_species, a.n_types, rates);
     const float d = a.de[s], e = a.de[a.n_species + s];
@@ -776,7 +810,7 @@ __global__ void __launch_bounds__(kTileThreads) tile_forward(const __grid_consta
     for (int n = 0; n < kQuadsEach; ++n)
         if (Q.cell[n] >= 0) {
             float v[4];
-            ld4(a.in[s] + Q.site[n], v);
+            Q.load(a.in[s], n, v);
             st4(region[0] + Q.cell[n], v);
         }
     int at = 0;
@@ -784,7 +818,7 @@ __global__ void __launch_bounds__(kTileThreads) tile_forward(const __grid_consta
         int own[kQuadsEach][4];
 #pragma unroll
         for (int n = 0; n < kQuadsEach; ++n)
-            if (Q.cell[n] >= 0) ld4(a.owner + (size_t)t * a.g.sites + Q.site[n], own[n]);
+            if (Q.cell[n] >= 0) Q.load(a.owner + (size_t)t * a.g.sites, n, own[n]);
         for (int j = 0; j < k; ++j, ++r) {
             __syncthreads();  // the round before is in place (and the rates)
             const float *b = region[at];
@@ -797,7 +831,7 @@ __global__ void __launch_bounds__(kTileThreads) tile_forward(const __grid_consta
                 float h[4], v[4];
                 quad_step(b, Q.cell[n], d, e, h, v);
                 if (last) {
-                    if (keep && Q.mine[n]) st4(keep + Q.site[n], v);
+                    if (keep) Q.store(keep, n, v);
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
                         const bool cell = own[n][c] != kMedium;
@@ -809,7 +843,7 @@ __global__ void __launch_bounds__(kTileThreads) tile_forward(const __grid_consta
                     }
                 }
                 st4(next + Q.cell[n], v);
-                if (post && Q.mine[n]) st4(post + Q.site[n], v);
+                if (post) Q.store(post, n, v);
             }
             at ^= 1;
         }
@@ -826,6 +860,7 @@ __host__ __device__ constexpr size_t tile_backward_smem(int n_types) {
     return sizeof(double) * 2 * kTileThreads * (n_types + 1) + sizeof(float) * 2 * kRegionX * kRegionY;
 }
 
+template <bool WHOLE>
 __global__ void __launch_bounds__(kTileThreads, 2) tile_backward(const __grid_constant__ TileBackward a) {
     extern __shared__ __align__(16) unsigned char dynamic[];
     __shared__ float2 rates[kTileTypes + 1];
@@ -835,7 +870,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_backward(const __grid_co
     double *const by_type = reinterpret_cast<double *>(region + 2 * kRegionX * kRegionY) + tid;
     const int s = (int)blockIdx.z, k = a.k[s], rounds = a.steps * k;
     const int block = ((int)blockIdx.z * (int)gridDim.y + (int)blockIdx.y) * (int)gridDim.x + (int)blockIdx.x;
-    const TileQuads Q(a.g, (int)blockIdx.x * kTileX, (int)blockIdx.y * kTileY);
+    const TileQuads<WHOLE> Q(a.g, (int)blockIdx.x * kTileX, (int)blockIdx.y * kTileY);
     grid_wait();
     tile_rates(a.sec, a.upt, s, a.n_species, T, rates);
     const float d = a.de[s], e = a.de[a.n_species + s];
@@ -851,7 +886,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_backward(const __grid_co
     for (int n = 0; n < kQuadsEach; ++n)
         if (Q.cell[n] >= 0) {
             float v[4];
-            ld4(a.lam[s] + Q.site[n], v);
+            Q.load(a.lam[s], n, v);
             st4(region + Q.cell[n], v);
         }
     __syncthreads();
@@ -869,8 +904,8 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_backward(const __grid_co
 #pragma unroll
                 for (int n = 0; n < kQuadsEach; ++n)
                     if (Q.within(n, margin + 1)) {
-                        ld4(exch + Q.site[n], x[n]);
-                        ld4(a.owner + (size_t)t * a.g.sites + Q.site[n], own[n]);
+                        Q.load(exch, n, x[n]);
+                        Q.load(a.owner + (size_t)t * a.g.sites, n, own[n]);
                     }
 #pragma unroll
                 for (int n = 0; n < kQuadsEach; ++n) {
@@ -887,7 +922,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_backward(const __grid_co
                         const float lv = v2 < 0.0f ? 0.0f : l[c];
                         const float l1 = __fmul_rn(lv, __fsub_rn(1.0f, rate.y));
                         l[c] = cell ? l1 : l[c];
-                        if (Q.mine[n]) {
+                        if (Q.own(n, c)) {
                             double *const sum = by_type + 2 * o * kTileThreads;
                             sum[0] += (double)l1;
                             sum[kTileThreads] -= (double)__fmul_rn(lv, v1);
@@ -907,13 +942,14 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_backward(const __grid_co
                     const uint32_t W = (uint32_t)a.g.w, all = (uint32_t)a.g.sites, site = Q.site[n];
                     const uint32_t x = site - glz::udiv(a.g.div_w, site) * W;
                     float h[4], hu[4], hd[4], none[4] = {}, us[4];
-                    ld4(u + site, h);
-                    ld4(u + (site < W ? site + all - W : site - W), hu);
-                    ld4(u + (site + W >= all ? site + W - all : site + W), hd);
-                    quad_sums(false, h, u[x == 0 ? site + W - 1 : site - 1], u[x + 4 == W ? site + 4 - W : site + 4], hu,
+                    Q.load(u, site, n, h);
+                    Q.load(u, site < W ? site + all - W : site - W, n, hu);
+                    Q.load(u, site + W >= all ? site + W - all : site + W, n, hd);
+                    quad_sums(false, h, u[x == 0 ? site + W - 1 : site - 1], u[x + 4 >= W ? site + 4 - W : site + 4], hu,
                               hd, none, none, us);
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
+                        if (!Q.own(n, c)) continue;
                         gd += (double)__fmul_rn(l[c], __fsub_rn(us[c], __fmul_rn(4.0f, h[c])));
                         ge -= (double)__fmul_rn(l[c], h[c]);
                     }
@@ -928,7 +964,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) tile_backward(const __grid_co
         if (Q.mine[n]) {
             float v[4];
             ld4(region + at * kRegionX * kRegionY + Q.cell[n], v);
-            st4(a.lam_in[s] + Q.site[n], v);
+            Q.store(a.lam_in[s], n, v);
         }
     sums[0] = gd;
     sums[kTileThreads] = ge;
@@ -1025,11 +1061,17 @@ int blocks_for(const glz_adj *h) {
     return (int)((items + kThreads - 1) / kThreads);
 }
 
-// Planes that take the tile kernels: rows of whole quads, few enough owner
-// types, and few enough sites that the threads' running sums stay small
-// beside the fields (15 bytes a site of a species at four types).
+// Planes that take the tile kernels: few enough owner types, and few enough
+// sites that the threads' running sums stay small beside the fields (15 bytes
+// a site of a species at four types). Rows that are not whole quads take them
+// with more than one species or from 2^16 sites (forward and backward, a round
+// a launch and in tiles, us: 510 x 512 of two species, 50 steps, 274 + 1117
+// and 176 + 514; 98 x 96 of two, 30 steps, 115 + 319 and 90 + 243; of one
+// species 101 + 228 and 89 + 225 at 258 x 256, but 98 + 224 and 89 + 249 at
+// 194 x 200).
 bool tile_plane(const glz_adj *h) {
-    return h->g.dim == 2 && quads(h) && h->n_types <= kTileTypes && h->g.sites <= (1 << 20);
+    const bool rows = quads(h) || (h->g.w >= 8 && (h->n_species > 1 || h->g.sites >= (1 << 16)));
+    return h->g.dim == 2 && rows && h->n_types <= kTileTypes && h->g.sites <= (1 << 20);
 }
 // ... when every species' sub-steps fit a launch's rounds.
 bool tiled(const glz_adj *h) { return tile_plane(h) && h->kmax <= kHalo; }
@@ -1186,7 +1228,7 @@ int tile_keep(glz_adj *h, int sg, int local, int n, int len, float *last_out) {
                                               : (last_out ? last_out + (size_t)s * h->g.sites : nullptr);
             }
     }
-    CU(launch_blocks(tile_forward, tile_grid(h), kTileThreads, 0, h->stream, a));
+    CU(launch_blocks(quads(h) ? tile_forward<true> : tile_forward<false>, tile_grid(h), kTileThreads, 0, h->stream, a));
     return GLZ_OK;
 }
 
@@ -1234,7 +1276,7 @@ int tile_forward_to(glz_adj *h, int t_last) {
             a.k[s] = h->k[s];
             a.in[s] = cur + (size_t)s * sites;
         }
-        CU(launch_blocks(tile_forward, tile_grid(h), kTileThreads, 0, h->stream, a));
+        CU(launch_blocks(quads(h) ? tile_forward<true> : tile_forward<false>, tile_grid(h), kTileThreads, 0, h->stream, a));
         cur = dst;
     }
     return GLZ_OK;
@@ -1302,7 +1344,8 @@ int tile_backward_sequence(glz_adj *h) {
     a.fresh = 1;
     const dim3 grid = tile_grid(h);
     const size_t smem = tile_backward_smem(h->n_types);
-    CU(cudaFuncSetAttribute(tile_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const auto backward = quads(h) ? tile_backward<true> : tile_backward<false>;
+    CU(cudaFuncSetAttribute(backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int nseg = (h->steps + h->every - 1) / h->every;
     for (int sg = nseg - 1; sg >= 0; --sg) {
         const int t0 = sg * h->every, len = (t0 + h->every < h->steps ? t0 + h->every : h->steps) - t0;
@@ -1323,7 +1366,7 @@ int tile_backward_sequence(glz_adj *h) {
                         a.exch[s][r] = seg_state(h, sg, step, h->k[s], s);
                     }
             }
-            CU(launch_blocks(tile_backward, grid, kTileThreads, smem, h->stream, a));
+            CU(launch_blocks(backward, grid, kTileThreads, smem, h->stream, a));
             a.fresh = 0;
             cur = 1 - cur;
         }

@@ -1,7 +1,7 @@
 """The adjoint's tile kernels at the edges of tiles, launches and rounds.
 
 Lattices smaller than a tile, of odd heights and with a last tile of a few
-sites; up to four sub-steps a step (a launch takes four rounds) and five (the
+sites; rows that are not whole quads; up to four sub-steps a step (a launch takes four rounds) and five (the
 one-round kernels); steps and checkpoint intervals that do not divide a
 launch's steps; one to three species; 16 owner types (the most the tile
 kernels hold) and 17.
@@ -55,6 +55,17 @@ def _plain(params, fields0, owners, w, h, ns, nt):
     (72, 40, (1.2, 0.2), 4, 5),
     (72, 65, (0.1, 0.3, 0.7), 16, 6),
     (72, 65, (0.1, 0.3, 0.7), 17, 6),
+    # rows that are not whole quads: less than a region wide, a last tile of
+    # one to three sites, a quad of the margin across the row's end
+    (7, 6, (0.1,), 3, 9),
+    (7, 6, (0.1, 0.2), 3, 9),
+    (9, 7, (0.1, 0.6), 3, 9),
+    (62, 33, (0.1, 0.2), 4, 8),
+    (65, 32, (0.2, 0.05), 4, 11),
+    (66, 40, (1.0, 0.1), 4, 6),
+    (131, 70, (0.4, 0.1), 4, 7),
+    (198, 97, (0.1, 0.3, 0.7), 16, 6),
+    (258, 256, (0.1,), 3, 3),
 ])
 def test_the_tiles_match_a_plain_stencil(device, w, h, diffusion, nt, steps):
     import torch
