@@ -20,13 +20,12 @@
 //   - Pricing has no branch on the common path, so its reads and sums overlap.
 //   - The tally rotation is shared out over the grid and taken by each
 //     block's last threads.
-// Measured per MCS (the step graph, back to back), against the pass that read
-// its launch from shared memory and its tables where they lie, and launched
-// plainly: lean planes of four types 27.2 -> 16.2 us at 256^2 and 30.6 -> 18.9
-// at 512^2; the two-field tissue (length, chemotaxis; replayed) 55.5 -> 31.1 us at
-// 256^2, 62.1 -> 35.1 at 512^2 and 114.9 -> 62.7 at 1024^2. A pass of the
-// 256^2 plane is about 4 us, of which 0.8 is the graph's kernel-to-kernel
-// time and the rest the chain.
+// Measured per MCS, queued back to back, against the pass that read its launch
+// from shared memory and its tables where they lie, and launched plainly: lean
+// planes of two types 25.3 -> 14.7 us at 512^2; the two-field tissue (length,
+// chemotaxis) 55.5 -> 26.1 us at 256^2, 61.3 -> 27.3 at 512^2 and 223 -> 110
+// at 2048^2. A pass of a 256^2 lean plane is 2.5 us, of which 0.8 is the
+// kernel boundary and the rest the chain.
 
 #include <atomic>
 #include <cstdlib>

@@ -1,6 +1,6 @@
 // One copy attempt priced where it lies, shared by the kernels that read the
-// lattice in place: the direct sweep (direct.cu), and the resident, cluster
-// and direct ensemble sweeps (sweep.cu). A target's neighbours are other
+// lattice in place: the direct sweep (direct.cu), and the cluster and
+// direct ensemble sweeps (sweep.cu). A target's neighbours are other
 // colours, which no copy in the pass changes, so the labels it reads are the
 // pass's.
 #pragma once

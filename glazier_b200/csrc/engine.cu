@@ -971,8 +971,8 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
     // Models with other terms (length, chemotaxis, connectivity, motility,
     // drift, nematic, division and death) take the direct kernel at any size:
     // the tiled kernel's window staging costs more than it saves (per MCS of
-    // the two-field tissue, direct against tiled: 72 and 115 us at 1400^2, 130
-    // and 168 at 2048^2, 450 and 525 at 4096^2; of the infected slab's model
+    // the two-field tissue, direct against tiled: 63 and 115 us at 1400^2, 107
+    // and 168 at 2048^2, 353 and 525 at 4096^2; of the infected slab's model
     // 296 and 574 at 128^3, 461 and 750 at 160^3).
     h->direct = direct_mode == 1 || (direct_mode == -1 && (!h->lean || sites <= direct_most));
     // Past a number of targets a pass the direct kernel gathers each block's
@@ -980,8 +980,7 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
     // each warp streams over a run
     // (GLAZIER_SWEEP_COMPACT=0: neither, =1: the warp's, =2: the block's, at
     // any size). Per MCS of the two-field tissue, priced in place against
-    // gathered: 31.1 and 31.7 us at 256^2, 35.1 and 35.0 at 512^2, 51.6 and
-    // 36.6 at 640^2, 92.7 and 62.7 at 1024^2 (of the slab's model 147 and 162
+    // gathered: 27.3 and 30.7 us at 512^2, 75.1 and 41.2 at 1024^2 (of the slab's model 147 and 162
     // at 64 x 64 x 32, 179 and 191 at 96 x 96 x 64, 386 and 300 at 128^3), by
     // warps against by blocks 95.0 and 91.9 at 1800^2, 107 and 119 at 2048^2,
     // 353 and 435 at 4096^2. Of the lean plane: 11.9 and 13.9
