@@ -914,10 +914,10 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
     bool has_conn = false, has_division = false;
     for (int a = 0; a < nt * nt; ++a) contact[a] = (float)m->contact[a];
     for (int k = 0; k < nt; ++k) {
-        tv[k] = (float)at(m->target_volume, k);
         lv[k] = (float)at(m->lambda_volume, k);
-        ts[k] = (float)at(m->target_surface, k);
+        tv[k] = glz::weighted_target(at(m->target_volume, k), lv[k]);
         ls[k] = (float)at(m->lambda_surface, k);
+        ts[k] = glz::weighted_target(at(m->target_surface, k), ls[k]);
         tl[k] = at(m->target_length, k);
         ll[k] = at(m->lambda_length, k);
         divv[k] = at(m->division_volume, k);

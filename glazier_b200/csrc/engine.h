@@ -34,6 +34,11 @@ inline void set_dividers(Geometry &g) {
     g.div_hh = make_divider((uint32_t)(g.h / 2 > 0 ? g.h / 2 : 1));
 }
 
+// A type's target volume or surface as the kernels' tables hold it: zero where
+// the term's weight is zero, so that the term is a finite number times zero
+// whatever target the model states for it (infinite, NaN, or past f32).
+inline float weighted_target(double target, float weight) { return weight != 0.0f ? (float)target : 0.0f; }
+
 // Per-type tables in device memory, row-major [type][...], index 0 the medium.
 struct TypeTables {
     const float *contact;       // n_types * n_types

@@ -452,10 +452,11 @@ static int create_batched(int n, const glz_model *models, const uint32_t *const 
         float *tc = tables.data() + toff;
         for (int i = 0; i < nt * nt; ++i) tc[i] = (float)m.contact[i];
         for (int k = 0; k < nt; ++k) {
-            tc[nt * nt + k] = (float)at(m.target_volume, k);
-            tc[nt * nt + nt + k] = (float)at(m.lambda_volume, k);
-            tc[nt * nt + 2 * nt + k] = (float)at(m.target_surface, k);
-            tc[nt * nt + 3 * nt + k] = (float)at(m.lambda_surface, k);
+            const float lv = (float)at(m.lambda_volume, k), ls = (float)at(m.lambda_surface, k);
+            tc[nt * nt + k] = glz::weighted_target(at(m.target_volume, k), lv);
+            tc[nt * nt + nt + k] = lv;
+            tc[nt * nt + 2 * nt + k] = glz::weighted_target(at(m.target_surface, k), ls);
+            tc[nt * nt + 3 * nt + k] = ls;
         }
         float *dt = h->tables + toff;
         glz::SweepLaunch &a = descs[r].a;
@@ -479,10 +480,10 @@ static int create_batched(int n, const glz_model *models, const uint32_t *const 
         a.uniform_type = h->uniform ? t : -1;
         a.uniform_contact_exact = h->uniform;
         a.uniform_contact = (float)m.contact[t * nt + t];
-        a.u_target_volume = (float)at(m.target_volume, t);
-        a.u_lambda_volume = (float)at(m.lambda_volume, t);
-        a.u_target_surface = (float)at(m.target_surface, t);
-        a.u_lambda_surface = (float)at(m.lambda_surface, t);
+        a.u_target_volume = tc[nt * nt + t];
+        a.u_lambda_volume = tc[nt * nt + nt + t];
+        a.u_target_surface = tc[nt * nt + 2 * nt + t];
+        a.u_lambda_surface = tc[nt * nt + 3 * nt + t];
         a.use_tma = h->use_tma;
         a.error_flag = h->error_flag;
         descs[r].cell_off = rep.cell_off;

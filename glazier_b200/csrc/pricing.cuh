@@ -60,21 +60,29 @@ template <bool UNIFORM>
 __device__ __forceinline__ float size_terms(const SweepLaunch &a, const TypeTables &t, uint32_t old, uint32_t nw, int t_old, int t_new,
                                             int vol_old, int vol_new, int surf_old, int surf_new, int ds_old,
                                             int ds_new, float delta) {
-    // No branch: the medium, and a type whose weight is zero, add a zero,
-    // which leaves the sum's bits alone.
-    const float lv_old = old != 0 ? (UNIFORM ? a.u_lambda_volume : t.lambda_volume[t_old]) : 0.0f;
-    const float lv_new = nw != 0 ? (UNIFORM ? a.u_lambda_volume : t.lambda_volume[t_new]) : 0.0f;
-    const float ls_old = old != 0 ? (UNIFORM ? a.u_lambda_surface : t.lambda_surface[t_old]) : 0.0f;
-    const float ls_new = nw != 0 ? (UNIFORM ? a.u_lambda_surface : t.lambda_surface[t_new]) : 0.0f;
+    // No branch: the medium's side adds a zero chosen after its term is formed,
+    // and a type whose weight is zero has a zero target in the tables
+    // (weighted_target), so its term is a zero too. Chosen before the product
+    // instead, or with the target as the model states it, a target that is not
+    // finite, or whose double is not, would make 0 * inf of a term that the
+    // model does not have.
+    const float lv_old = UNIFORM ? a.u_lambda_volume : t.lambda_volume[t_old];
+    const float lv_new = UNIFORM ? a.u_lambda_volume : t.lambda_volume[t_new];
+    const float ls_old = UNIFORM ? a.u_lambda_surface : t.lambda_surface[t_old];
+    const float ls_new = UNIFORM ? a.u_lambda_surface : t.lambda_surface[t_new];
     const float ev_old = __fsub_rn((float)vol_old, UNIFORM ? a.u_target_volume : t.target_volume[t_old]);
     const float ev_new = __fsub_rn((float)vol_new, UNIFORM ? a.u_target_volume : t.target_volume[t_new]);
     const float es_old = __fsub_rn((float)surf_old, UNIFORM ? a.u_target_surface : t.target_surface[t_old]);
     const float es_new = __fsub_rn((float)surf_new, UNIFORM ? a.u_target_surface : t.target_surface[t_new]);
     const float d_old = (float)ds_old, d_new = (float)ds_new;
-    delta = __fadd_rn(delta, __fmul_rn(lv_old, __fsub_rn(1.0f, __fmul_rn(2.0f, ev_old))));
-    delta = __fadd_rn(delta, __fmul_rn(lv_new, __fadd_rn(__fmul_rn(2.0f, ev_new), 1.0f)));
-    delta = __fadd_rn(delta, __fmul_rn(ls_old, __fmul_rn(d_old, __fadd_rn(__fmul_rn(2.0f, es_old), d_old))));
-    delta = __fadd_rn(delta, __fmul_rn(ls_new, __fmul_rn(d_new, __fadd_rn(__fmul_rn(2.0f, es_new), d_new))));
+    const float v_old = __fmul_rn(lv_old, __fsub_rn(1.0f, __fmul_rn(2.0f, ev_old)));
+    const float v_new = __fmul_rn(lv_new, __fadd_rn(__fmul_rn(2.0f, ev_new), 1.0f));
+    const float s_old = __fmul_rn(ls_old, __fmul_rn(d_old, __fadd_rn(__fmul_rn(2.0f, es_old), d_old)));
+    const float s_new = __fmul_rn(ls_new, __fmul_rn(d_new, __fadd_rn(__fmul_rn(2.0f, es_new), d_new)));
+    delta = __fadd_rn(delta, old != 0 ? v_old : 0.0f);
+    delta = __fadd_rn(delta, nw != 0 ? v_new : 0.0f);
+    delta = __fadd_rn(delta, old != 0 ? s_old : 0.0f);
+    delta = __fadd_rn(delta, nw != 0 ? s_new : 0.0f);
     return delta;
 }
 
