@@ -1104,6 +1104,13 @@ float *seg_state(glz_adj *h, int sg, int local, int j, int s) {
     return h->seg + (((size_t)local * (h->kmax + 1) + j) * h->n_species + s) * (size_t)h->g.sites;
 }
 
+void drop_graphs(glz_adj *h) {
+    if (h->fwd_exec) cudaGraphExecDestroy(h->fwd_exec);
+    if (h->bwd_exec) cudaGraphExecDestroy(h->bwd_exec);
+    h->fwd_exec = h->bwd_exec = nullptr;
+    h->graph_k.clear();
+}
+
 int set_params(glz_adj *h, const double *params) {
     const int S = h->n_species, T = h->n_types;
     for (int s = 0; s < S; ++s)
@@ -1131,6 +1138,7 @@ int set_params(glz_adj *h, const double *params) {
     }
     CU(cudaMemcpyAsync(h->d_sec, h->staging, table_floats(h) * 4, cudaMemcpyHostToDevice, h->stream));
     if (h->seg_kmax != h->kmax) {
+        drop_graphs(h);  // they name the buffer freed here, and outlive it if the new one is refused
         cudaFree(h->seg);
         h->seg = nullptr;
         h->seg_kmax = -1;
@@ -1280,13 +1288,6 @@ int tile_forward_to(glz_adj *h, int t_last) {
         cur = dst;
     }
     return GLZ_OK;
-}
-
-void drop_graphs(glz_adj *h) {
-    if (h->fwd_exec) cudaGraphExecDestroy(h->fwd_exec);
-    if (h->bwd_exec) cudaGraphExecDestroy(h->bwd_exec);
-    h->fwd_exec = h->bwd_exec = nullptr;
-    h->graph_k.clear();
 }
 
 // Record what `body` queues on the handle's stream as a graph, instantiated
