@@ -285,6 +285,7 @@ __global__ void __launch_bounds__(kThreads) forward_quads(const __grid_constant_
 // `reduce_partials` sums the rows in block order at the end.
 constexpr int kBlocks = 148 * 8;
 constexpr int kWarps = kThreads / 32;
+constexpr int kMostTypes = 254;  // of a handle: an owner is a byte, and 255 the medium
 
 __device__ __forceinline__ double warp_sum(double v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -1330,6 +1331,21 @@ int forward_sequence(glz_adj *h) {
     return keep_segment(h, last, h->steps - t_last, h->final_out);
 }
 
+// Let `kernel` take up to `most` bytes of dynamic shared memory, the most any
+// handle asks of it: the setting is the kernel's, so a handle that set its own
+// need could leave it too low for one launching on another thread.
+template <class Kernel>
+int allow_smem(Kernel kernel, size_t most) {
+    CU(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    return GLZ_OK;
+}
+
+// The backward rounds' dynamic shared memory: each warp's (sec, upt) sums by
+// type, then the block's gradients.
+constexpr size_t round_backward_smem(int n_types, int n_species) {
+    return ((size_t)kWarps * 2 * n_types + 2 * n_species + (size_t)2 * n_types * n_species) * sizeof(double);
+}
+
 // backward_sequence by tile launches of several steps each.
 int tile_backward_sequence(glz_adj *h) {
     const int S = h->n_species;
@@ -1346,7 +1362,7 @@ int tile_backward_sequence(glz_adj *h) {
     const dim3 grid = tile_grid(h);
     const size_t smem = tile_backward_smem(h->n_types);
     const auto backward = quads(h) ? tile_backward<true> : tile_backward<false>;
-    CU(cudaFuncSetAttribute(backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int rc = allow_smem(backward, tile_backward_smem(kTileTypes))) return rc;
     const int nseg = (h->steps + h->every - 1) / h->every;
     for (int sg = nseg - 1; sg >= 0; --sg) {
         const int t0 = sg * h->every, len = (t0 + h->every < h->steps ? t0 + h->every : h->steps) - t0;
@@ -1397,13 +1413,13 @@ int backward_sequence(glz_adj *h) {
     a.upt = h->d_upt;
     a.de = h->d_de;
     a.partial = h->partial;
-    const size_t smem = ((size_t)kWarps * 2 * T + G) * sizeof(double);
+    const size_t smem = round_backward_smem(T, S);
     // owner types held in registers up to 4 or 8 types, else reduced per trip
     auto *backward = !quads(h) ? backward_round
                      : T <= 4  ? backward_quads<4>
                      : T <= 8  ? backward_quads<8>
                                : backward_quads<0>;
-    CU(cudaFuncSetAttribute(backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int rc = allow_smem(backward, round_backward_smem(kMostTypes, glz::kMaxSpecies))) return rc;
     const int nseg = (h->steps + h->every - 1) / h->every;
     for (int sg = nseg - 1; sg >= 0; --sg) {
         const int t0 = sg * h->every, len = (t0 + h->every < h->steps ? t0 + h->every : h->steps) - t0;
@@ -1444,7 +1460,7 @@ int glz_adj_create(int width, int height, int depth, int n_species, int n_types,
     if (!out) return fail(GLZ_INVALID, "null output handle");
     *out = nullptr;
     if (width <= 0 || height <= 0 || depth <= 0) return fail(GLZ_INVALID, "the lattice has a zero dimension");
-    if (n_species < 1 || n_species > glz::kMaxSpecies || n_types < 1 || n_types > 254 || steps < 1 ||
+    if (n_species < 1 || n_species > glz::kMaxSpecies || n_types < 1 || n_types > kMostTypes || steps < 1 ||
         checkpoint_every < 1)
         return fail(GLZ_INVALID, "species 1..8, types 1..254, steps and checkpoint interval >= 1");
     const long long sites = (long long)width * height * depth;

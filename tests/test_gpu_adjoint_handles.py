@@ -2,6 +2,8 @@
 
 from __future__ import annotations
 
+import threading
+
 import numpy as np
 import pytest
 
@@ -52,3 +54,54 @@ def test_a_refused_buffer_leaves_the_handle_usable(device):
     assert all(np.array_equal(a, b) for a, b in zip(_gradients(other, params, fields, weight), alone))
     adj.close()
     other.close()
+
+
+# (width, height, species, types): the tile kernels at one, four and 16 types,
+# the round kernels at 17, at 40, and on a row that is not whole quads
+SHAPES = [(64, 40, 2, 1), (64, 40, 2, 16), (72, 33, 1, 4), (64, 40, 2, 17), (64, 40, 2, 40), (66, 20, 1, 60)]
+
+
+def test_handles_of_different_types_side_by_side(device):
+    from glazier_b200.adjoint import FieldAdjoint
+
+    steps = 6
+    inputs = [_inputs(*shape, steps, seed) for seed, shape in enumerate(SHAPES)]
+
+    def make(i):
+        w, h, ns, nt = SHAPES[i]
+        return FieldAdjoint(w, h, 1, ns, nt, inputs[i][0], checkpoint_every=3)
+
+    want = []
+    for i in range(len(SHAPES)):
+        adj = make(i)
+        want.append(_gradients(adj, *inputs[i][1:]))
+        adj.close()
+
+    # alive together: graphs captured while the others' kernels were set up
+    handles = [make(i) for i in range(len(SHAPES))]
+    for _ in range(2):
+        for i, adj in enumerate(handles):
+            got = _gradients(adj, *inputs[i][1:])
+            assert all(np.array_equal(a, b) for a, b in zip(got, want[i])), f"handle {i}"
+    for adj in handles:
+        adj.close()
+
+    wrong = []
+
+    def drive(i):
+        try:
+            for _ in range(30):
+                adj = make(i)
+                got = _gradients(adj, *inputs[i][1:])
+                adj.close()
+                if not all(np.array_equal(a, b) for a, b in zip(got, want[i])):
+                    wrong.append(f"handle {i}")
+        except Exception as exc:  # reported on the main thread
+            wrong.append(f"handle {i}: {exc}")
+
+    threads = [threading.Thread(target=drive, args=(i,)) for i in range(len(SHAPES))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, wrong
