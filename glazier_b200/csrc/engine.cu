@@ -43,9 +43,22 @@ void prefault(void *p, size_t bytes) {
     if (bytes < kLeast) return;
     const size_t page = (size_t)sysconf(_SC_PAGESIZE);
     const size_t from = ((size_t)p + page - 1) / page * page, to = ((size_t)p + bytes) / page * page;
+    if (to <= from) return;
+    // A buffer whose last page is there has been used before, or is pinned:
+    // walking its pages would cost half as much as the copy into pinned memory
+    // (64 MB: 1.68 ms with the walk, 1.19 without) and a tenth of that into
+    // pageable memory (1 MB: 96 and 87 us). Managed memory stays where it is.
+    unsigned char there = 0;
+    if (mincore((void *)(to - page), page, &there) != 0 || (there & 1)) return;
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    if (at.type != cudaMemoryTypeUnregistered) return;
     // a hint: where the kernel or the mapping does not take it, the copy
     // faults the pages in as it did
-    if (to > from) madvise((void *)from, to - from, MADV_POPULATE_WRITE);
+    madvise((void *)from, to - from, MADV_POPULATE_WRITE);
 }
 }
 

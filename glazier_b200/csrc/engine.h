@@ -381,7 +381,7 @@ __device__ __forceinline__ int population_parity(const PopulationLaunch &a) {
 // call: a fresh buffer's pages otherwise fault one by one inside the driver's
 // copy, which takes five times as long as the copy itself (51 MB in 64
 // lattices: 22 ms, 15 with this, 4.3 into pages already mapped). Changes no
-// content; memory that is mapped costs a page walk.
+// content, and does nothing to a buffer that has its pages.
 void prefault(void *p, size_t bytes);
 
 // Record the message glz_last_error() returns on this thread.
