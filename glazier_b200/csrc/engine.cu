@@ -36,7 +36,10 @@ thread_local std::string g_error = "no error";
 #endif
 
 namespace glz {
-void set_last_error(const std::string &msg) { g_error = msg; }
+void set_last_error(const std::string &msg) {
+    g_error = msg;
+    cudaGetLastError();  // reported here, so not by the next launch's check too
+}
 
 void prefault(void *p, size_t bytes) {
     constexpr size_t kLeast = 64 * 1024;
@@ -65,7 +68,7 @@ void prefault(void *p, size_t bytes) {
 namespace {
 
 int fail(int code, const std::string &msg) {
-    g_error = msg;
+    glz::set_last_error(msg);
     return code;
 }
 

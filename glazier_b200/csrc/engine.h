@@ -384,7 +384,8 @@ __device__ __forceinline__ int population_parity(const PopulationLaunch &a) {
 // content, and does nothing to a buffer that has its pages.
 void prefault(void *p, size_t bytes);
 
-// Record the message glz_last_error() returns on this thread.
+// Record the message glz_last_error() returns on this thread, and clear CUDA's
+// own record of the thread's last error.
 void set_last_error(const std::string &msg);
 
 }  // namespace glz
