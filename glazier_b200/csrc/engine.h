@@ -298,7 +298,7 @@ constexpr float kDoseScale = 16777216.0f;
 // order) and the exact moment sums.
 struct RecountLaunch {
     Geometry g;
-    const uint32_t *labels;
+    uint32_t *labels;
     int n_labels;
     int2 *vs_base;
     long long *mom_base;
@@ -309,7 +309,10 @@ struct RecountLaunch {
     int *first;  // scratch per label: its first site in scan order
     int tracks;
     const float *nematic;  // with the nematic term: its sums follow the moments
-    int *error_flag;  // set to 2 when a label is not below n_labels
+    // Set to 2 when a label is not below n_labels; the recount of a lattice
+    // from outside (without `flags`) then makes the site medium, so that no
+    // sweep indexes an array with it.
+    int *error_flag;
     // Population models: the live count in device memory (n_labels is then
     // the capacity).
     const int *n_live;

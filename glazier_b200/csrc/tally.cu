@@ -44,7 +44,10 @@ __global__ void __launch_bounds__(256) first_sites_kernel(const __grid_constant_
     const uint32_t n_labels = (uint32_t)recount_labels(a);
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t l = i < (size_t)a.g.sites ? a.labels[i] : 0u;
-    if (l >= n_labels) l = 0u;  // recount_counts_kernel reports it
+    if (l >= n_labels) {
+        a.labels[i] = l = 0u;
+        atomicExch(a.error_flag, 2);
+    }
     first_site(a.first, l, (int)i);
 }
 

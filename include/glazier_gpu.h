@@ -97,7 +97,8 @@ int glz_gpu_step(glz_gpu *h, uint64_t steps);
  * types, fields and step count: a restart from a label field
  * (Simulation::from_labels, glazier-core/src/cpu.rs:151-175, as the
  * Blueprint's `initial.labels` uses it). Labels are checked on the device;
- * one not below the label count fails the next glz_gpu_step. */
+ * one not below the label count becomes medium and fails the next
+ * glz_gpu_step. */
 int glz_gpu_set_labels(glz_gpu *h, const uint32_t *labels, size_t sites);
 
 /* glz_gpu_set_labels from device memory of the handle's device (uint32 per
