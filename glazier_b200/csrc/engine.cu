@@ -1088,12 +1088,15 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
         h->n_bound = n_labels;
     }
 
+    // Everything a run starts from goes through the handle's own stream, which
+    // its kernels follow: the default stream, which they do not wait for, may
+    // be another user's and busy.
     if (ns > 0) {
         if ((rc = dev_alloc(&h->field_buf, (size_t)2 * ns * sites))) return bail(rc);
         std::vector<float> f((size_t)sites);
         for (int s = 0; s < ns; ++s) {
             for (long long i = 0; i < sites; ++i) f[i] = (float)(fields ? fields[(size_t)s * sites + i] : at(m->initial, s));
-            if (cudaMemcpy(h->field_ptr(s, 0), f.data(), sites * sizeof(float), cudaMemcpyHostToDevice))
+            if (cudaMemcpyAsync(h->field_ptr(s, 0), f.data(), sites * sizeof(float), cudaMemcpyHostToDevice, h->stream))
                 return bail(fail(GLZ_DRIVER, "field upload failed"));
         }
     }
@@ -1101,18 +1104,19 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
         std::vector<float> q(2 * (size_t)sites);
         for (size_t i = 0; i < q.size(); ++i) q[i] = (float)m->nematic[i];
         if ((rc = dev_alloc(&h->nematic, q.size()))) return bail(rc);
-        if (cudaMemcpy(h->nematic, q.data(), q.size() * sizeof(float), cudaMemcpyHostToDevice))
+        if (cudaMemcpyAsync(h->nematic, q.data(), q.size() * sizeof(float), cudaMemcpyHostToDevice, h->stream))
             return bail(fail(GLZ_DRIVER, "nematic field upload failed"));
     }
     if (h->has_motility) {
         std::vector<float> act((size_t)sites);
         for (long long i = 0; i < sites; ++i) act[i] = activity ? (float)activity[i] : 0.0f;
         if ((rc = dev_alloc(&h->activity, (size_t)sites))) return bail(rc);
-        if (cudaMemcpy(h->activity, act.data(), sites * sizeof(float), cudaMemcpyHostToDevice))
+        if (cudaMemcpyAsync(h->activity, act.data(), sites * sizeof(float), cudaMemcpyHostToDevice, h->stream))
             return bail(fail(GLZ_DRIVER, "activity upload failed"));
         if ((rc = dev_alloc(&h->pending, (size_t)(sites / g.ncol + 1)))) return bail(rc);
         if ((rc = dev_alloc(&h->pending_count, 2))) return bail(rc);
-        if (cudaMemset(h->pending_count, 0, 2 * sizeof(int))) return bail(fail(GLZ_DRIVER, "memset failed"));
+        if (cudaMemsetAsync(h->pending_count, 0, 2 * sizeof(int), h->stream))
+            return bail(fail(GLZ_DRIVER, "memset failed"));
     }
     if ((rc = dev_alloc(&h->error_flag, 1))) return bail(rc);
     if ((rc = dev_alloc(&h->clock, 1))) return bail(rc);
