@@ -190,7 +190,7 @@ int tiles_of(const glz_ens *h, const Replica &rep, int shape) {
 }
 
 // The runs' schedule, of replicas in their own order: what an ensemble starts
-// on and a candidate of the autotuner's, not one that callers name.
+// on, and a candidate of the autotuner's.
 constexpr int kRunsSchedule = 16;
 
 // Lay the replicas' tiles out in schedule order (`schedule` bit 0: largest
@@ -826,7 +826,7 @@ int glz_ens_autotune(glz_ens *h, uint64_t trial_steps, int *choice) {
 
 int glz_ens_set_schedule(glz_ens *h, int schedule, int max_ctas) {
     if (!h) return fail(GLZ_INVALID, "null handle");
-    if (schedule < 0 || schedule > 15 || max_ctas < 0) return fail(GLZ_INVALID, "no such schedule");
+    if (schedule < 0 || schedule > kRunsSchedule || max_ctas < 0) return fail(GLZ_INVALID, "no such schedule");
     return h->n > 0 ? set_schedule(h, schedule, max_ctas) : GLZ_OK;
 }
 
