@@ -276,9 +276,11 @@ int build_graph(glz_ens *h) {
     return GLZ_OK;
 }
 
-int run(glz_ens *h, uint64_t steps, bool graph, double *ms) {
-    if (graph)
-        if (int rc = build_graph(h)) return rc;
+// `steps` MCS of the batch, each a replay of its step graph. (The runs' kernels
+// read the clock before they wait for the kernel before them, which is only
+// right where a graph's start stands between the clock's advance and them.)
+int run(glz_ens *h, uint64_t steps, double *ms) {
+    if (int rc = build_graph(h)) return rc;
     cudaEvent_t a = nullptr, b = nullptr;
     if (ms) {
         CU(cudaEventCreate(&a));
@@ -286,10 +288,7 @@ int run(glz_ens *h, uint64_t steps, bool graph, double *ms) {
         CU(cudaEventRecord(a, h->stream));
     }
     for (uint64_t s = 0; s < steps; ++s) {
-        if (graph)
-            CU(cudaGraphLaunch(h->exec, h->stream));
-        else if (int rc = enqueue_step(h))
-            return rc;
+        CU(cudaGraphLaunch(h->exec, h->stream));
         h->step += 1;
         h->pass += h->ncol;
     }
@@ -692,7 +691,7 @@ static int step_mixed(glz_ens *h, uint64_t steps, double *ms) {
 // stream and each engine on its own stream from a host thread of its own,
 // all at once.
 static int step_all(glz_ens *h, uint64_t steps, double *ms) {
-    if (h->engines.empty()) return run(h, steps, true, ms);
+    if (h->engines.empty()) return run(h, steps, ms);
     bool replays = true;
     for (glz_gpu *g : h->engines) replays &= glz::engine_replays(g);
     if (replays) return step_mixed(h, steps, ms);
@@ -714,7 +713,7 @@ static int step_all(glz_ens *h, uint64_t steps, double *ms) {
         });
     int rc = GLZ_OK;
     if (h->n > 0)
-        rc = run(h, steps, true, nullptr);
+        rc = run(h, steps, nullptr);
     else
         h->step += (long long)steps;
     for (auto &t : threads) t.join();
@@ -806,8 +805,8 @@ int glz_ens_autotune(glz_ens *h, uint64_t trial_steps, int *choice) {
     for (auto [sch, g] : cands) {
         if ((rc = set_schedule(h, sch, g))) break;
         double ms = 0.0;
-        if ((rc = run(h, 1, true, nullptr))) break;  // warm the graph
-        if ((rc = run(h, trial_steps, true, &ms))) break;
+        if ((rc = run(h, 1, nullptr))) break;  // warm the graph
+        if ((rc = run(h, trial_steps, &ms))) break;
         if (ms < best) {
             best = ms;
             best_i = i;
