@@ -60,12 +60,13 @@ template <bool UNIFORM>
 __device__ __forceinline__ float size_terms(const SweepLaunch &a, const TypeTables &t, uint32_t old, uint32_t nw, int t_old, int t_new,
                                             int vol_old, int vol_new, int surf_old, int surf_new, int ds_old,
                                             int ds_new, float delta) {
-    // No branch: the medium's side adds a zero chosen after its term is formed,
-    // and a type whose weight is zero has a zero target in the tables
-    // (weighted_target), so its term is a zero too. Chosen before the product
-    // instead, or with the target as the model states it, a target that is not
-    // finite, or whose double is not, would make 0 * inf of a term that the
-    // model does not have.
+    // Every term is formed, so that their reads and products overlap, and the
+    // medium's side is left out at its add. A type whose weight is zero has a
+    // zero target in the tables (weighted_target), so its term is a zero,
+    // which leaves the sum's bits alone. A weight of zero for the medium, or
+    // targets as the model states them, would not do: where a target is not
+    // finite, or not in f32, 0 * inf is no zero. (Selecting between the term
+    // and a zero instead costs 1112 against 1102 us for 10 MCS at 4096^2.)
     const float lv_old = UNIFORM ? a.u_lambda_volume : t.lambda_volume[t_old];
     const float lv_new = UNIFORM ? a.u_lambda_volume : t.lambda_volume[t_new];
     const float ls_old = UNIFORM ? a.u_lambda_surface : t.lambda_surface[t_old];
@@ -79,10 +80,10 @@ __device__ __forceinline__ float size_terms(const SweepLaunch &a, const TypeTabl
     const float v_new = __fmul_rn(lv_new, __fadd_rn(__fmul_rn(2.0f, ev_new), 1.0f));
     const float s_old = __fmul_rn(ls_old, __fmul_rn(d_old, __fadd_rn(__fmul_rn(2.0f, es_old), d_old)));
     const float s_new = __fmul_rn(ls_new, __fmul_rn(d_new, __fadd_rn(__fmul_rn(2.0f, es_new), d_new)));
-    delta = __fadd_rn(delta, old != 0 ? v_old : 0.0f);
-    delta = __fadd_rn(delta, nw != 0 ? v_new : 0.0f);
-    delta = __fadd_rn(delta, old != 0 ? s_old : 0.0f);
-    delta = __fadd_rn(delta, nw != 0 ? s_new : 0.0f);
+    if (old != 0) delta = __fadd_rn(delta, v_old);
+    if (nw != 0) delta = __fadd_rn(delta, v_new);
+    if (old != 0) delta = __fadd_rn(delta, s_old);
+    if (nw != 0) delta = __fadd_rn(delta, s_new);
     return delta;
 }
 
