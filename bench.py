@@ -148,7 +148,7 @@ def measured_peak() -> tuple:
 # 4096^2 workload, from an ncu capture of that kernel with cold caches
 # (profiles/stream_sweep_2d_4096.md), with the kernel it was measured on; a
 # figure measured on another kernel is not reported.
-TRAFFIC = {"kernel": "lean", "bytes_per_launch": 81738240.0}
+TRAFFIC = {"kernel": "lean", "bytes_per_launch": 80020224.0}
 
 
 def ensemble_compare(mcs: int, device: int) -> dict:

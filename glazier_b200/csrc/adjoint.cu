@@ -1062,14 +1062,20 @@ int blocks_for(const glz_adj *h) {
     return (int)((items + kThreads - 1) / kThreads);
 }
 
-// Planes that take the tile kernels: few enough owner types, and few enough
-// sites that the threads' running sums stay small beside the fields (15 bytes
-// a site of a species at four types). Rows that are not whole quads take them
-// with more than one species or from 2^16 sites (forward and backward, a round
-// a launch and in tiles, us: 510 x 512 of two species, 50 steps, 274 + 1117
-// and 176 + 514; 98 x 96 of two, 30 steps, 115 + 319 and 90 + 243; of one
-// species 101 + 228 and 89 + 225 at 258 x 256, but 98 + 224 and 89 + 249 at
-// 194 x 200).
+// Planes that take the tile kernels, which pay up to about 1400^2 sites: past
+// it the running sums that every launch reads and writes (15 bytes a site of a
+// species at four types) no longer stay in L2 beside the fields. Forward and backward, a round a launch and
+// in tiles, us, 20 steps of two species: of four types 83 + 220 and 65 + 123
+// at 8 x 512, 88 + 224 and 66 + 127 at 16 x 512, 98 + 283 and 77 + 189 at
+// 512^2, 178 + 805 and 149 + 607 at 1024^2, 192 + 883 and 181 + 776 at 1100^2,
+// 275 + 1198 and 247 + 1169 at 1400^2, 506 + 2143 and 438 + 2303 at 2048^2
+// (one species 336 + 1143 and 252 + 1399); of 16 types 98 + 775 and 77 + 283
+// at 512^2, 178 + 2623 and 152 + 1059 at 1024^2, 503 + 8395 and 442 + 3990 at
+// 2048^2. The line is a size at which both few and many types gain.
+// Rows that are not whole quads take them with more than one species or from
+// 2^16 sites (510 x 512 of two species, 50 steps, 274 + 1117 and 176 + 514;
+// 98 x 96 of two, 30 steps, 115 + 319 and 90 + 243; of one species 101 + 228
+// and 89 + 225 at 258 x 256, but 98 + 224 and 89 + 249 at 194 x 200).
 bool tile_plane(const glz_adj *h) {
     const bool rows = quads(h) || (h->g.w >= 8 && (h->n_species > 1 || h->g.sites >= (1 << 16)));
     return h->g.dim == 2 && rows && h->n_types <= kTileTypes && h->g.sites <= (1 << 20);

@@ -122,7 +122,7 @@ constexpr int kBlock = 2;  // each block gathers the unlike of its targets into 
 // tiled kernel, windows by tensor copies through a ring in shared memory, took
 // 51.3, 103.7 and 131.3 us at these sizes (8192^2: 490 against 399; four
 // neighbours at 4096^2: 326 against 151; two types: 189 against 146). A pass
-// of 4096^2 is bound by issue, 61 % of cycles: 18.9 M warp instructions, and
+// of 4096^2 is bound by issue, 61 % of cycles: 18.8 M warp instructions, and
 // its reads are 1.5 lattices through L2 (2.3 TB/s).
 constexpr int kWarpK = 4;
 // A run's targets at most: longer ones leave the warps further apart in the

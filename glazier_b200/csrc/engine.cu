@@ -166,10 +166,10 @@ struct glz_gpu {
     uint64_t pass_no = 0, mcs = 0;
     bool use_tma = false;
     bool lean = false;    // the sweep prices contact, volume and surface only
-    bool direct = false;  // ... on a lattice small enough for the direct kernel
+    bool direct = false;  // the direct kernel, its form by size (lean planes from 2048^2, which always stream, have `lean` alone)
     int compact = 0;      // ... queueing a warp's unlike copies (1, large passes) or a block's (2)
-    bool cluster = false;   // ... a small plane with nothing between passes, in one cluster's shared memory
-    bool band = false;      // ... a large plane, streamed by row bands in one launch per call
+    bool cluster = false;   // a small lean plane with nothing between passes, in one cluster's shared memory
+    bool band = false;      // a lean plane, streamed by row bands in one launch per call
     unsigned *barrier = nullptr;  // the band sweep's grid barrier
     int max_ctas = 0;
     int uniform = -1;
@@ -971,7 +971,8 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
     }
     if (has_conn) g.ring_n = g.dim == 3 ? 26 : 8;  // the full Moore ring (connectivity.rs:23-29)
 
-    // GLAZIER_SWEEP_LEAN=0 keeps every model on the general sweep kernel.
+    // GLAZIER_SWEEP_LEAN=0 prices every model with every term's kernels: the
+    // direct ones, or with GLAZIER_SWEEP_DIRECT=0 too the tiled one.
     const char *lean_env = std::getenv("GLAZIER_SWEEP_LEAN");
     h->lean = !h->has_length && !h->tracks && !h->has_chemotaxis && !h->has_external && !h->has_motility && !has_conn &&
               !(lean_env && lean_env[0] == '0');
@@ -996,8 +997,13 @@ int glz_gpu_create(const glz_model *m, const uint32_t *labels, const uint8_t *ce
     // each warp streams over a run
     // (GLAZIER_SWEEP_COMPACT=0: neither, =1: the warp's, =2: the block's, at
     // any size). Per MCS of the two-field tissue, priced in place against
-    // gathered: 27.3 and 30.7 us at 512^2, 75.1 and 41.2 at 1024^2 (of the slab's model 147 and 162
-    // at 64 x 64 x 32, 179 and 191 at 96 x 96 x 64, 386 and 300 at 128^3), by
+    // gathered: 27.1 and 28.8 us at 512^2, 27.1 and 29.1 at 544^2, 32.9 and
+    // 29.9 at 552^2, 41.2 and 29.9 at 640^2, 76.8 and 43 at 1024^2; of the
+    // infection model 47.4 and 49.0 at 544^2, 52.8 and 50.0 at 560^2. The
+    // times cross where the in-place blocks no longer all fit (75,776 targets,
+    // 550^2); the line, 2^16 targets, lies a little before it, and gathering
+    // costs up to a tenth in between. Of the slab's model 147 and 162
+    // at 64 x 64 x 32, 179 and 191 at 96 x 96 x 64, 386 and 300 at 128^3; by
     // warps against by blocks 95.0 and 91.9 at 1800^2, 107 and 119 at 2048^2,
     // 353 and 435 at 4096^2. Of the lean plane: 11.9 and 13.9
     // at 512^2, 13.9 and 15.7 at 768^2 (a last target a thread of one wave of

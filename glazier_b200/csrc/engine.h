@@ -207,7 +207,7 @@ cudaError_t launch_apply_copies(const SweepLaunch &a, float *activity, cudaStrea
 cudaError_t launch_activity_decay(float *activity, int sites, cudaStream_t stream);
 
 // The batched ensemble: independent replicas of one neighbourhood, all their
-// tiles in one persistent launch per colour. Replica state lives in flat
+// runs of targets (or tiles) in one launch per colour. Replica state lives in flat
 // arrays; each replica's SweepLaunch holds its static fields (geometry,
 // tables, absolute label/type/colour-count pointers) and the kernel patches
 // the per-pass ones from the clock.

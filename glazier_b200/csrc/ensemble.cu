@@ -2,14 +2,14 @@
 //
 // Independent replicas of the plain sweep (contact, volume and surface terms;
 // lattices of any even sides, each with its own parameters and seed) share
-// flat device arrays and run as one persistent launch per colour over every
-// replica's tiles. One Monte Carlo step (the colour launches and a one-thread
+// flat device arrays and run as one launch per colour over every replica's
+// runs of targets (or tiles). One Monte Carlo step (the colour launches and a one-thread
 // clock advance) is captured once into a CUDA graph and replayed; the kernels
 // read the step and pass counters from the device clock, so the same graph
 // serves every step. A replica's results are bit-identical to a plain
 // glz_gpu_* run of the same start, whatever the schedule, so the autotuner
-// chooses the persistent grid and the order replicas' tiles are dealt in by
-// time alone.
+// chooses among runs, tile shapes, persistent grids and replica orders by time
+// alone.
 //
 // Replicas whose models state other terms (fields, length, connectivity,
 // division, death, motility, drift, nematic) are engines of their own. When

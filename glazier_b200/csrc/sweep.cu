@@ -1,11 +1,14 @@
-// The checkerboard Metropolis copy sweep: one launch per colour.
+// The checkerboard Metropolis copy sweep: the tiled kernel, the cluster sweep of
+// small planes, the ensemble's kernels, and the launches that choose between
+// these and the direct sweep (direct.cu).
 //
 // Replaces `cpm_sweep` of the reference device engine (glazier-cuda/src/
 // lib.rs:436-716). Same-colour targets are two apart on every axis, outside
 // any neighbourhood, so a pass's copies are independent and the labels a
 // target reads do not change during the pass.
 //
-// Layout of the work:
+// Layout of the work in the tiled kernel, which one lattice takes on request
+// only and whose pieces the ensemble's windowed kernels share:
 //   - Persistent CTAs walk the lattice tile by tile. A tile and its one-site
 //     halo are staged in shared memory; tiles clear of the periodic edge
 //     arrive by a TMA tensor copy issued one tile ahead into the other of two
@@ -1528,12 +1531,6 @@ __global__ void __launch_bounds__(kLeanThreads, GLZ_LEAN_MIN_BLOCKS)
 
 // ---------------------------------------------------------------- the direct ensemble
 //
-// A plane ensemble's pass with one block per tile of BX x BY targets of one
-// replica: the block finds its replica, copies the replica's launch into
-// shared memory with the pass's fields patched from the clock, and prices
-// every target of its tile where it lies (direct_target, as the direct
-// kernel does). The tile shape sets which sites a block's loads share; the
-// autotuner picks it by time, since the results do not depend on it.
 // Tile t of colour pass `colour` (pass number `pass`, step `step`): the
 // block finds the tile's replica, patches the replica's launch into `d` and
 // prices the tile's targets.

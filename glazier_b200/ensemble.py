@@ -1,8 +1,8 @@
 """A batch of independent Cellular Potts replicas run as one on the B200.
 
 The Python face of the ``glz_ens_*`` entry points: every replica whose model
-prices contact, volume and surface only goes through one persistent launch
-per colour, one Monte Carlo step replayed from a CUDA graph; a replica with
+prices contact, volume and surface only goes through one launch per
+colour, one Monte Carlo step replayed from a CUDA graph; a replica with
 fields, division, death or the other terms runs as its own engine beside the
 batch, at the same time. Each replica's results are bit-identical to a
 ``GpuSimulation`` run of the same start, so the schedule the autotuner picks
