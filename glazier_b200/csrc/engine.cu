@@ -757,6 +757,10 @@ int run_band(glz_gpu *h, uint64_t steps, double *ms) {
 
 int run_steps(glz_gpu *h, uint64_t steps, double *ms) {
     if (h->band) return run_band(h, steps, ms);
+    if (steps == 0) {  // nothing to run, nothing to wait for
+        if (ms) ms[0] = ms[1] = ms[2] = 0.0;
+        return GLZ_OK;
+    }
     // Steps are queued kernel by kernel: a pass takes the device longer than
     // its launch takes the host, and kernels launched programmatically on the
     // stream follow one another closer than a step graph's replays do (per

@@ -1,9 +1,9 @@
-"""An engine is set up on its own stream.
+"""What an engine waits for, and on which stream.
 
-With a second of another user's work queued on the default stream, an engine
-with every uploaded array (fields, nematic field, activity and its list of
-accepted copies) is made and stepped before that work ends, and the run is the
-replay's.
+An engine is set up on its own stream: with a second of another user's work
+queued on the default stream, an engine with every uploaded array (fields,
+nematic field, activity and its list of accepted copies) is made and stepped
+before that work ends, and the run is the replay's.
 """
 
 from __future__ import annotations
@@ -42,3 +42,19 @@ def test_the_default_stream_is_not_waited_for(device):
         assert np.array_equal(sim.field(k).astype(np.float32), replay.field(k))
     torch.cuda.synchronize()
     sim.close()
+
+
+def test_no_steps_wait_for_nothing(device):
+    """A call of no steps returns with its stream's earlier work still queued."""
+    import torch
+
+    with device.GpuSimulation.from_start(tiled(sheet_model(seed=3))) as sim:
+        before = sim.labels()
+        own = torch.cuda.ExternalStream(sim.stream)
+        with torch.cuda.stream(own):
+            torch.cuda._sleep(400_000_000)  # about a fifth of a second
+        sim.step(0)
+        assert sim.step_profiled(0) == (0.0, 0.0, 0.0)
+        assert not own.query(), "a call of no steps waited"
+        own.synchronize()
+        assert sim.mcs == 0 and np.array_equal(sim.labels(), before)
